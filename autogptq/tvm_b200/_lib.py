@@ -36,6 +36,7 @@ _SIGNATURES = {
     "b200gptq_gemm": (_c_int, [_c_void_p] * 8 + [_c_int] * 5 + [_c_void_p, _c_size_t, _c_void_p]),
     "b200gptq_sort_rows": (_c_int, [_c_void_p] * 3 + [_c_int] * 3 + [_c_void_p] * 3),
     "b200gptq_pack_fields": (_c_int, [_c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_void_p]),
+    "b200gptq_pack_linear": (_c_int, [_c_void_p, _c_int] + [_c_void_p] * 3 + [_c_int] * 4 + [_c_void_p] * 4),
     "b200gptq_tp_buffer_bytes": (_c_size_t, []),
     "b200gptq_gemv_tp": (_c_int, [_c_void_p] * 8 + [_c_int] * 5 + [_c_void_p, _c_size_t, _c_int, _c_int, _c_void_p,
                                   ctypes.c_longlong, _c_int, _c_int, _c_void_p]),
@@ -65,7 +66,8 @@ _SIGNATURES = {
 
 def _load() -> ctypes.CDLL:
     path = _build.LIB_PATH
-    if not os.path.isfile(path) or (_build.is_stale() and _build_possible()):
+    present = os.path.isfile(path) and os.path.isfile(_build.HOST_PATH)
+    if not present or (_build.is_stale() and _build_possible()):
         if not _build_possible():
             raise ImportError(
                 f"{path} is missing and nvcc is not available to build it; "
@@ -86,6 +88,9 @@ def _build_possible() -> bool:
 
 lib = _load()
 LIB_PATH = _build.LIB_PATH
+
+import torch  # noqa: E402,F401  (_host resolves its symbols from the libraries that torch loads)
+from . import _host  # noqa: E402  (the native call path; linked against the library loaded above)
 
 
 class B200GPTQError(RuntimeError):

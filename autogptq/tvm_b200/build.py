@@ -1,9 +1,10 @@
-"""Ahead-of-time build of ``libb200gptq.so`` (sm_100a only) with nvcc.
+"""Ahead-of-time build of ``libb200gptq.so`` (sm_100a only) with nvcc, and of ``_host`` with the host compiler.
 
 The library is plain CUDA C++ behind a C ABI: it links against the CUDA runtime
 and nothing else (no torch, no Python headers), and is placed next to this file
-so that it travels with the source tree.  ``python -m autogptq.tvm_b200.build``
-rebuilds it; :func:`build` is a no-op when the library is newer than every source.
+so that it travels with the source tree.  ``_host`` is a small CPython module (torch headers) that prepares a
+``QuantLinear.forward`` call in native code and calls the library.  ``python -m autogptq.tvm_b200.build``
+rebuilds both; :func:`build` is a no-op when they are newer than every source.
 """
 from __future__ import annotations
 
@@ -11,12 +12,15 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 INCLUDE = os.path.normpath(os.path.join(HERE, "..", "..", "include"))
 LIB_NAME = "libb200gptq.so"
 LIB_PATH = os.path.join(HERE, LIB_NAME)
+HOST_SRC = os.path.join(CSRC, "host", "host_call.cpp")
+HOST_PATH = os.path.join(HERE, "_host" + sysconfig.get_config_var("EXT_SUFFIX"))
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -33,16 +37,33 @@ def sources():
 
 
 def _deps():
-    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)]
+    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if os.path.isfile(os.path.join(CSRC, f))]
     deps += [os.path.join(INCLUDE, f) for f in os.listdir(INCLUDE)]
     return deps
 
 
+def _host_deps():
+    return [HOST_SRC] + [os.path.join(INCLUDE, f) for f in os.listdir(INCLUDE)]
+
+
+def _older(path, deps) -> bool:
+    return not os.path.isfile(path) or any(os.path.getmtime(d) > os.path.getmtime(path) for d in deps)
+
+
+def _host_command(out: str):
+    import torch
+    root = os.path.dirname(torch.__file__)
+    inc = os.path.join(root, "include")
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            "-I", inc, "-I", os.path.join(inc, "torch", "csrc", "api", "include"), "-I", sysconfig.get_paths()["include"],
+            "-I", os.path.join(cuda, "include"), HOST_SRC, "-o", out, "-L", HERE, f"-l:{LIB_NAME}", "-Wl,-rpath,$ORIGIN",
+            "-L", os.path.join(root, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python"]
+
+
 def is_stale() -> bool:
-    if not os.path.isfile(LIB_PATH):
-        return True
-    t = os.path.getmtime(LIB_PATH)
-    return any(os.path.getmtime(d) > t for d in _deps())
+    return _older(LIB_PATH, _deps()) or _older(HOST_PATH, _host_deps())
 
 
 def build(force: bool = False, verbose: bool = False, extra_flags=()) -> str:
@@ -94,6 +115,16 @@ def _build_locked(force: bool, verbose: bool, extra_flags) -> str:
     if r.returncode != 0:
         raise RuntimeError(f"link failed:\n{r.stdout}")
     os.replace(tmp, LIB_PATH)
+    if not force and not _older(HOST_PATH, _host_deps()):
+        return LIB_PATH      # (it binds the library at load time: a new library needs no new host module)
+    tmp = f"{HOST_PATH}.tmp.{os.getpid()}"
+    cmd = _host_command(tmp)
+    if verbose:
+        print(" ".join(cmd), file=sys.stderr)
+    r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"{cmd[0]} failed for {HOST_SRC}:\n{r.stdout}")
+    os.replace(tmp, HOST_PATH)
     return LIB_PATH
 
 

@@ -27,6 +27,8 @@ int sm_count() {
 int dequant_dispatch(const int32_t*, const int32_t*, const __half*, const int32_t*, int, int, int, int, int8_t*,
                      __half*, cudaStream_t);
 int pack_fields_dispatch(const int32_t*, int, int, int, int32_t*, cudaStream_t);
+int pack_linear_dispatch(const void*, int, const float*, const float*, const int32_t*, int, int, int, int, int32_t*,
+                         int32_t*, __half*, cudaStream_t);
 int sort_rows_dispatch(const int32_t*, const int32_t*, const int32_t*, int, int, int, int32_t*, int32_t*,
                        cudaStream_t);
 int gemv_generic_dispatch(const __half*, const int32_t*, const int32_t*, const __half*, const int32_t*,
@@ -104,6 +106,18 @@ int b200gptq_pack_fields(const int32_t* vals, int R, int C, int bits, int32_t* o
     if (bits != 2 && bits != 3 && bits != 4 && bits != 8) return B200GPTQ_ERR_BITS;
     if (R <= 0 || C <= 0 || R % 32 != 0) return B200GPTQ_ERR_SHAPE;
     return pack_fields_dispatch(vals, R, C, bits, out, static_cast<cudaStream_t>(stream));
+}
+
+int b200gptq_pack_linear(const void* weight, int dtype, const float* scales, const float* zeros, const int32_t* g_idx,
+                         int K, int N, int G, int bits, int32_t* qweight, int32_t* qzeros, void* scales_out,
+                         void* stream) {
+    if (!weight || !scales || !zeros || !g_idx || !qweight || !qzeros || !scales_out) return B200GPTQ_ERR_NULL_POINTER;
+    int gs = K;
+    if (int st = check_layer(K, N, bits, &gs)) return st;
+    if (G < 1 || dtype < B200GPTQ_F16 || dtype > B200GPTQ_F32) return B200GPTQ_ERR_SHAPE;
+    if (!aligned16(weight)) return B200GPTQ_ERR_ALIGNMENT;
+    return pack_linear_dispatch(weight, dtype, scales, zeros, g_idx, K, N, G, bits, qweight, qzeros,
+                                static_cast<__half*>(scales_out), static_cast<cudaStream_t>(stream));
 }
 
 int b200gptq_sort_rows(const int32_t* qweight, const int32_t* g_idx, const int32_t* perm, int K, int N, int bits,

@@ -1,0 +1,240 @@
+// Host side of one QuantLinear.forward call in native code.
+//
+// A decode GEMV runs for 3..10 us on the device; preparing its launch from Python (attribute look-ups, argument
+// conversion of a ctypes call, torch.empty) took 12..16 us per call and the GEMM's 27..31 us, so a loop of small calls
+// was bound by the host.  This module does the same checks and the same library call from C++: `Layer.run(x,
+// module.__dict__)` returns the output tensor, or None when anything about the call is not the prepared case (another
+// device, other buffers, a row count without a plan, a tensor subclass); the caller then takes the Python route,
+// which prepares what is missing.  Nothing here launches kernels of its own: the work goes through the C ABI.
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <unordered_map>
+
+#include "../../../../include/b200gptq.h"
+
+namespace {
+
+constexpr int kMaxGemvRows = 8;
+
+// Scratch buffers by (device, stream), registered by ops.get_workspace.  Read and written under the GIL.
+struct Scratch { void* ptr; size_t bytes; };
+struct KeyHash {
+    size_t operator()(const std::pair<int, void*>& k) const {
+        return std::hash<void*>()(k.second) * 31u + (size_t)k.first;
+    }
+};
+std::unordered_map<std::pair<int, void*>, Scratch, KeyHash>* g_scratch;
+PyObject* g_get_workspace;   // ops.get_workspace, for a stream without a large enough buffer
+
+PyObject *s_buffers, *s_qweight, *s_g_idx, *s_qzeros, *s_scales, *s_bias, *s_gemv_tuning;
+
+struct GemvEntry {
+    PyObject* owner;      // the ops.GemvPlan that owns the handle
+    const b200gptq_gemv_plan* plan;
+    size_t need;
+};
+
+struct Layer {
+    PyObject_HEAD
+    int K, N, bits, group_size, device;
+    // the buffers this object was prepared for: addresses of qweight / g_idx, identity of the others
+    const void *qweight_at, *g_idx_at;
+    PyObject *qzeros, *scales, *bias, *tuning;
+    GemvEntry gemv[kMaxGemvRows + 1];
+    // run-time layout for the GEMM (gemm_ok false: no tensor-core kernel for this layer)
+    bool gemm_ok;
+    const int32_t *qweight_run, *qzeros_run, *g_idx_run, *x_perm;
+    const void *scales_run, *bias_run;
+    PyObject* keep;       // keeps the tensors behind those addresses alive
+};
+
+inline bool address_is(PyObject* dict, PyObject* key, const void* at) {
+    PyObject* t = PyDict_GetItem(dict, key);
+    return t && THPVariable_Check(t) && THPVariable_Unpack(t).unsafeGetTensorImpl()->data() == at;
+}
+
+bool scratch_for(int device, cudaStream_t stream, size_t need, Scratch* out) {
+    auto it = g_scratch->find({device, (void*)stream});
+    if (it == g_scratch->end() || it->second.bytes < need) {
+        PyObject* r = PyObject_CallFunction(g_get_workspace, "in", device, (Py_ssize_t)need);
+        if (!r) return false;
+        Py_DECREF(r);
+        it = g_scratch->find({device, (void*)stream});
+        if (it == g_scratch->end() || it->second.bytes < need) {
+            PyErr_SetString(PyExc_RuntimeError, "no scratch buffer was registered for this stream");
+            return false;
+        }
+    }
+    *out = it->second;
+    return true;
+}
+
+// Layer.run(x, module_dict): the module's forward, or None where the prepared case does not apply.
+PyObject* layer_run(PyObject* self_, PyObject* const* args, Py_ssize_t nargs) {
+    Layer* self = reinterpret_cast<Layer*>(self_);
+    if (nargs != 2) { PyErr_SetString(PyExc_TypeError, "run(x, module_dict)"); return nullptr; }
+    PyObject *px = args[0], *dict = args[1];
+    if (!THPVariable_CheckExact(px) || !PyDict_Check(dict)) Py_RETURN_NONE;
+    const at::Tensor& x = THPVariable_Unpack(px);
+    const int64_t dims = x.dim();
+    if (!x.is_cuda() || x.scalar_type() != at::kHalf || dims < 1 || x.size(-1) != self->K || !x.is_contiguous() ||
+        x.get_device() != self->device)
+        Py_RETURN_NONE;
+    const int64_t M = x.numel() / self->K;
+    if (M < 1) Py_RETURN_NONE;
+    // the module's buffers are the ones this object was prepared for
+    PyObject* buffers = PyDict_GetItem(dict, s_buffers);
+    if (!buffers || !address_is(buffers, s_qweight, self->qweight_at) || !address_is(buffers, s_g_idx, self->g_idx_at))
+        Py_RETURN_NONE;
+    PyObject* bias = PyDict_GetItem(buffers, s_bias);
+    if (!bias) bias = PyDict_GetItem(dict, s_bias);
+    if ((bias ? bias : Py_None) != self->bias || PyDict_GetItem(buffers, s_qzeros) != self->qzeros ||
+        PyDict_GetItem(buffers, s_scales) != self->scales)
+        Py_RETURN_NONE;
+    const bool gemv = M <= kMaxGemvRows;
+    const GemvEntry* e = gemv ? &self->gemv[M] : nullptr;
+    if (gemv ? (!e->plan || PyDict_GetItem(dict, s_gemv_tuning) != self->tuning) : !self->gemm_ok) Py_RETURN_NONE;
+    if (c10::cuda::current_device() != self->device || M > INT32_MAX) Py_RETURN_NONE;
+
+    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)self->device).stream();
+    Scratch ws;
+    const size_t need = gemv ? e->need : b200gptq_workspace_bytes(B200GPTQ_OP_GEMM, (int)M, self->K, self->N, self->bits);
+    if (!scratch_for(self->device, stream, need, &ws)) return nullptr;
+    c10::SmallVector<int64_t, 4> shape(x.sizes().begin(), x.sizes().end());
+    shape.back() = self->N;
+    at::Tensor y;
+    try {
+        y = at::detail::empty_cuda(shape, at::kHalf, at::Device(at::kCUDA, (c10::DeviceIndex)self->device), std::nullopt);
+    } catch (const c10::Error&) {
+        Py_RETURN_NONE;   // (out of memory: the Python route raises it with its own type)
+    }
+    const void* xp = x.unsafeGetTensorImpl()->data();
+    void* yp = y.unsafeGetTensorImpl()->mutable_data();
+    int st;
+    if (gemv)
+        st = b200gptq_gemv_plan_run(e->plan, xp, yp, ws.ptr, ws.bytes, stream);
+    else
+        st = b200gptq_gemm(xp, self->qweight_run, self->qzeros_run, self->scales_run, self->g_idx_run, self->x_perm,
+                           self->bias_run, yp, (int)M, self->K, self->N, self->bits, self->group_size, ws.ptr, ws.bytes,
+                           stream);
+    if (st != B200GPTQ_OK) Py_RETURN_NONE;   // the Python route repeats the call and reports the status
+    return THPVariable_Wrap(std::move(y));
+}
+
+// Layer.set_gemv(rows, plan_owner, plan_handle, workspace_bytes)
+PyObject* layer_set_gemv(PyObject* self_, PyObject* args) {
+    Layer* self = reinterpret_cast<Layer*>(self_);
+    int rows;
+    PyObject* owner;
+    unsigned long long handle, need;
+    if (!PyArg_ParseTuple(args, "iOKK", &rows, &owner, &handle, &need)) return nullptr;
+    if (rows < 1 || rows > kMaxGemvRows) { PyErr_SetString(PyExc_ValueError, "rows"); return nullptr; }
+    GemvEntry& e = self->gemv[rows];
+    Py_INCREF(owner);
+    Py_XSETREF(e.owner, owner);
+    e.plan = reinterpret_cast<const b200gptq_gemv_plan*>((uintptr_t)handle);
+    e.need = (size_t)need;
+    Py_RETURN_NONE;
+}
+
+const void* tensor_address(PyObject* t) {
+    return t && THPVariable_Check(t) ? THPVariable_Unpack(t).unsafeGetTensorImpl()->data() : nullptr;
+}
+
+// Layer(K, N, bits, group_size, device, module_dict, gemm_ok, qweight_run, g_idx_run, x_perm)
+PyObject* layer_new(PyTypeObject* type, PyObject* args, PyObject*) {
+    int K, N, bits, group_size, device, gemm_ok;
+    PyObject *dict, *qw, *gi, *perm;
+    if (!PyArg_ParseTuple(args, "iiiiiOpOOO", &K, &N, &bits, &group_size, &device, &dict, &gemm_ok, &qw, &gi, &perm))
+        return nullptr;
+    PyObject* buffers = PyDict_Check(dict) ? PyDict_GetItem(dict, s_buffers) : nullptr;
+    if (!buffers) { PyErr_SetString(PyExc_TypeError, "module_dict"); return nullptr; }
+    PyObject *pq = PyDict_GetItem(buffers, s_qweight), *pg = PyDict_GetItem(buffers, s_g_idx),
+             *pz = PyDict_GetItem(buffers, s_qzeros), *ps = PyDict_GetItem(buffers, s_scales);
+    PyObject* bias = PyDict_GetItem(buffers, s_bias);
+    if (!bias) bias = PyDict_GetItem(dict, s_bias);
+    PyObject* tuning = PyDict_GetItem(dict, s_gemv_tuning);
+    if (!pq || !pg || !pz || !ps || !THPVariable_Check(pz) || !THPVariable_Check(ps) ||
+        (bias && bias != Py_None && !THPVariable_Check(bias))) {
+        PyErr_SetString(PyExc_TypeError, "the module lacks a buffer");
+        return nullptr;
+    }
+    PyObject* keep = PyTuple_Pack(7, qw, gi, perm, pz, ps, bias ? bias : Py_None, tuning ? tuning : Py_None);
+    if (!keep) return nullptr;
+    Layer* self = reinterpret_cast<Layer*>(type->tp_alloc(type, 0));
+    if (!self) { Py_DECREF(keep); return nullptr; }
+    self->K = K; self->N = N; self->bits = bits; self->group_size = group_size; self->device = device;
+    self->qweight_at = tensor_address(pq);
+    self->g_idx_at = tensor_address(pg);
+    self->qzeros = pz; self->scales = ps; self->bias = bias ? bias : Py_None; self->tuning = tuning;
+    self->gemm_ok = gemm_ok != 0;
+    self->qweight_run = static_cast<const int32_t*>(tensor_address(qw));
+    self->g_idx_run = static_cast<const int32_t*>(tensor_address(gi));
+    self->x_perm = static_cast<const int32_t*>(tensor_address(perm));
+    self->qzeros_run = static_cast<const int32_t*>(tensor_address(pz));
+    self->scales_run = tensor_address(ps);
+    self->bias_run = tensor_address(bias);
+    self->keep = keep;
+    return reinterpret_cast<PyObject*>(self);
+}
+
+void layer_dealloc(PyObject* self_) {
+    Layer* self = reinterpret_cast<Layer*>(self_);
+    for (auto& e : self->gemv) Py_XDECREF(e.owner);
+    Py_XDECREF(self->keep);
+    Py_TYPE(self_)->tp_free(self_);
+}
+
+PyMethodDef layer_methods[] = {
+    {"run", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(layer_run)), METH_FASTCALL, nullptr},
+    {"set_gemv", layer_set_gemv, METH_VARARGS, nullptr},
+    {nullptr, nullptr, 0, nullptr},
+};
+PyTypeObject LayerType = {PyVarObject_HEAD_INIT(nullptr, 0) "autogptq.tvm_b200._host.Layer", sizeof(Layer)};
+
+// set_scratch(device, stream, address, bytes)
+PyObject* set_scratch(PyObject*, PyObject* args) {
+    int device;
+    unsigned long long stream, address, bytes;
+    if (!PyArg_ParseTuple(args, "iKKK", &device, &stream, &address, &bytes)) return nullptr;
+    (*g_scratch)[{device, (void*)(uintptr_t)stream}] = Scratch{(void*)(uintptr_t)address, (size_t)bytes};
+    Py_RETURN_NONE;
+}
+PyObject* set_scratch_source(PyObject*, PyObject* fn) {
+    Py_INCREF(fn);
+    Py_XSETREF(g_get_workspace, fn);
+    Py_RETURN_NONE;
+}
+
+PyMethodDef module_methods[] = {
+    {"set_scratch", set_scratch, METH_VARARGS, nullptr},
+    {"set_scratch_source", set_scratch_source, METH_O, nullptr},
+    {nullptr, nullptr, 0, nullptr},
+};
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, module_methods};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__host(void) {
+    g_scratch = new std::unordered_map<std::pair<int, void*>, Scratch, KeyHash>();
+    s_buffers = PyUnicode_InternFromString("_buffers");
+    s_qweight = PyUnicode_InternFromString("qweight");
+    s_g_idx = PyUnicode_InternFromString("g_idx");
+    s_qzeros = PyUnicode_InternFromString("qzeros");
+    s_scales = PyUnicode_InternFromString("scales");
+    s_bias = PyUnicode_InternFromString("bias");
+    s_gemv_tuning = PyUnicode_InternFromString("gemv_tuning");
+    LayerType.tp_flags = Py_TPFLAGS_DEFAULT;
+    LayerType.tp_new = layer_new;
+    LayerType.tp_dealloc = layer_dealloc;
+    LayerType.tp_methods = layer_methods;
+    if (PyType_Ready(&LayerType) < 0) return nullptr;
+    PyObject* m = PyModule_Create(&module_def);
+    if (!m) return nullptr;
+    Py_INCREF(&LayerType);
+    if (PyModule_AddObject(m, "Layer", reinterpret_cast<PyObject*>(&LayerType)) < 0) return nullptr;
+    return m;
+}

@@ -50,7 +50,11 @@ def get_workspace(device: torch.device, nbytes: int) -> torch.Tensor:
         if ws is not None:
             new[16380:16384].copy_(ws[16380:16384])
         ws = _workspaces[key] = new
+        _lib._host.set_scratch(index, key[1], new.data_ptr(), size)
     return ws
+
+
+_lib._host.set_scratch_source(lambda index, nbytes: get_workspace(torch.device("cuda", index), nbytes))
 
 
 def check_status(device=None) -> None:
@@ -104,6 +108,38 @@ def pack_fields(vals, bits: int):
         st = _lib.lib.b200gptq_pack_fields(_ptr(vals), R, C, bits, _ptr(out), _stream(vals.device))
     _lib.check(st, "b200gptq_pack_fields")
     return out
+
+
+_PACK_DTYPES = {torch.float16: 0, torch.bfloat16: 1, torch.float32: 2}
+
+
+def can_pack_linear(weight, scales, zeros) -> bool:
+    """Whether :func:`pack_linear` takes these tensors: all on one CUDA device, the statistics in fp32 (with narrower
+    ones the reference's expression rounds its intermediates to their type)."""
+    return (weight.is_cuda and weight.dtype in _PACK_DTYPES and scales.dtype == zeros.dtype == torch.float32
+            and scales.device == weight.device == zeros.device)
+
+
+def pack_linear(weight, scales, zeros, g_idx, bits: int):
+    """``(qweight, qzeros, scales fp16 [G, N])`` of a linear ``weight [N, K]`` with ``scales`` / ``zeros`` fp32
+    ``[N, G]`` and ``g_idx`` int32 ``[K]``, in one launch (``b200gptq_pack_linear``)."""
+    N, K = weight.shape
+    G = scales.shape[1]
+    dev = weight.device
+    if tuple(scales.shape) != (N, G) or tuple(zeros.shape) != (N, G) or g_idx.numel() != K:
+        raise ValueError("scales and zeros must be [out, groups], g_idx [in]")
+    weight, scales, zeros = weight.contiguous(), scales.contiguous(), zeros.contiguous()
+    if weight.data_ptr() % 16:
+        weight = weight.clone()
+    g_idx = g_idx.to(device=dev, dtype=torch.int32).contiguous()
+    qweight = torch.empty((K // 32 * bits, N), dtype=torch.int32, device=dev)
+    qzeros = torch.empty((G, N // 32 * bits), dtype=torch.int32, device=dev)
+    scales16 = torch.empty((G, N), dtype=torch.float16, device=dev)
+    with torch.cuda.device(dev):
+        st = _lib.lib.b200gptq_pack_linear(_ptr(weight), _PACK_DTYPES[weight.dtype], _ptr(scales), _ptr(zeros), _ptr(g_idx),
+                                           K, N, G, bits, _ptr(qweight), _ptr(qzeros), _ptr(scales16), _stream(dev))
+    _lib.check(st, "b200gptq_pack_linear")
+    return qweight, qzeros, scales16
 
 
 def sort_rows(qweight, g_idx, bits: int):
@@ -220,8 +256,6 @@ class GemvPlan:
         _lib.check(st, "b200gptq_gemv_plan_create_ex")
         self._handle = handle
         self._need = _lib.workspace_bytes(_lib.OP_GEMV, M, self.K, self.N, bits)
-        self._index = self.device.index if self.device.index is not None else torch.cuda.current_device()
-        self._run = _lib.lib.b200gptq_gemv_plan_run
 
     def run(self, x, out=None):
         if not x.is_cuda or x.dtype != torch.float16 or not x.is_contiguous() or tuple(x.shape) != (self.M, self.xk):
@@ -230,26 +264,7 @@ class GemvPlan:
             out = torch.empty((self.M, self.N), dtype=torch.float16, device=x.device)
         ws = get_workspace(x.device, self._need)      # one buffer per (device, stream)
         st = _lib.lib.b200gptq_gemv_plan_run(self._handle, x.data_ptr(), out.data_ptr(), ws.data_ptr(), ws.numel(),
-                                             torch.cuda.current_stream(x.device).cuda_stream)
-        if st:
-            _lib.check(st, "b200gptq_gemv_plan_run")
-        return out
-
-    def launch(self, x, out_shape):
-        """:meth:`run` for a caller that has already checked ``x`` (contiguous fp16 on this plan's device, the plan's
-        row count): allocates ``out`` with ``out_shape`` and launches.  The host side of a decode GEMV is most of its
-        end-to-end time (25 us against 8 us on the device before this path existed), so nothing here builds a Stream
-        or a device-guard object unless the current device is another one."""
-        index = self._index
-        out = torch.empty(out_shape, dtype=torch.float16, device=self.device)
-        if torch._C._cuda_getDevice() != index:
-            with torch.cuda.device(index):
-                return self.run(x, out=out.view(self.M, self.N)).view(out_shape)
-        stream = torch._C._cuda_getCurrentRawStream(index)
-        ws = _workspaces.get((index, stream))
-        if ws is None or ws.numel() < self._need:
-            ws = get_workspace(self.device, self._need)
-        st = self._run(self._handle, x.data_ptr(), out.data_ptr(), ws.data_ptr(), ws.numel(), stream)
+                                             _stream(x.device))
         if st:
             _lib.check(st, "b200gptq_gemv_plan_run")
         return out

@@ -17,7 +17,7 @@ import numpy as np
 import torch
 import torch.nn as nn
 
-from . import ops
+from . import _lib, ops
 
 GEMV_MAX_M = 8
 
@@ -89,6 +89,7 @@ class QuantLinear(nn.Module):
         # (slices_per_sm, ctas_per_sm) of b200gptq_gemv_tuned, or None for the library defaults
         self.gemv_tuning = None
         self._plans = {}           # row count -> ops.GemvPlan (prepared launches of the decode GEMV)
+        self._native = None        # _host.Layer: the prepared call in native code, made by the first forward
 
     # ---- offline packing (CPU) ----------------------------------------------------------
     def pack(self, linear, scales, zeros, g_idx=None):
@@ -97,12 +98,18 @@ class QuantLinear(nn.Module):
         ``round((W + zero*scale) / fp16(scale))`` per row group and ``zeros - 1`` is stored.
         With the layer and the statistics on a CUDA device the whole procedure runs there (the
         reference packs with a Python loop over the rows on the CPU); the result is bit-identical."""
-        W = linear.weight.data.clone()
+        W = linear.weight.data
         if isinstance(linear, nn.Conv2d):
             W = W.flatten(1)
         elif type(linear).__name__ == "Conv1D":  # transformers.pytorch_utils.Conv1D keeps [in, out]
             W = W.t()
         self.g_idx = g_idx.clone() if g_idx is not None else self.g_idx
+        if ops.can_pack_linear(W, scales, zeros):
+            if linear.bias is not None:
+                self.bias = linear.bias.detach().clone().half()
+            self.qweight, self.qzeros, self.scales = ops.pack_linear(W, scales.detach(), zeros.detach(), self.g_idx, self.bits)
+            self._ready_for = None
+            return
         g = self.g_idx.long()
         scales = scales.t().contiguous()
         zeros = zeros.t().contiguous()
@@ -112,7 +119,7 @@ class QuantLinear(nn.Module):
             self.bias = linear.bias.detach().clone().half()
         intweight = torch.round((W.t() + scale_zeros[g]) / self.scales[g]).to(torch.int)
         if W.is_cuda:
-            # everything on the GPU: the same element-wise arithmetic, words built by b200gptq_pack_fields
+            # statistics narrower than fp32: the same expression element by element, words built by b200gptq_pack_fields
             self.qweight = ops.pack_fields(intweight.contiguous(), self.bits)
             zq = (zeros - 1).to(torch.int64).to(torch.int32)
             self.qzeros = ops.pack_fields(zq.t().contiguous(), self.bits).t().contiguous()
@@ -140,7 +147,10 @@ class QuantLinear(nn.Module):
         g = self.g_idx
         trivial = torch.equal(g, (torch.arange(K, device=dev, dtype=torch.int64) // self.groupsize).to(torch.int32))
         blocks = g.view(K // 32, 32)
-        block_uniform = bool((blocks == blocks[:, :1]).all().item())
+        lo, hi = torch.aminmax(g)
+        block_uniform, lo, hi = torch.stack([(blocks == blocks[:, :1]).all().to(g.dtype), lo, hi]).tolist()
+        if lo < 0 or hi >= self.scales.shape[0]:
+            raise ValueError(f"g_idx names group {lo if lo < 0 else hi}, the layer has {self.scales.shape[0]}")
         if trivial:
             self._qweight_run, self._g_idx_run, self._x_perm = self.qweight, None, None
         elif block_uniform:
@@ -161,6 +171,7 @@ class QuantLinear(nn.Module):
             b = g_run.view(K // 32, 32)
             self._gemm_ok = self.bits in (3, 4) and bool((b == b[:, :1]).all().item())
         self._plans = {}
+        self._native = None
         self._ready_for = (self.qweight.data_ptr(), self.g_idx.data_ptr())
 
     def _ready(self) -> bool:
@@ -178,18 +189,16 @@ class QuantLinear(nn.Module):
             y = quant_matmul(x2, self._qweight_run, self.qzeros, self.scales, self._g_idx_run, self._x_perm,
                              self.bias, self.bits, self.groupsize, self._gemm_ok)
             return y.reshape(x.shape[:-1] + (self.outfeatures,))
+        native = self._native
+        if native is not None:
+            # fp16, contiguous, on the layer's device, prepared before: checks, allocation and launch in one native call
+            y = native.run(x, self.__dict__)
+            if y is not None:
+                return y
         if not x.is_cuda:
             raise RuntimeError("QuantLinear.forward needs CUDA tensors: this backend has no CPU path")
         if not self._ready():
             self.post_init()
-        # decode: up to 8 rows, already fp16 and contiguous, a plan at hand -- one allocation and one library call
-        if x.dtype is torch.float16 and x.is_contiguous() and x.shape[-1] == self.infeatures:
-            M = x.numel() // self.infeatures
-            if 0 < M <= GEMV_MAX_M:
-                plan = self._plans.get((M, self.gemv_tuning))
-                if (plan is not None and plan._keep[5] is self._buffers.get("bias", self.__dict__.get("bias"))
-                        and x.get_device() == plan._index):
-                    return plan.launch(x, x.shape[:-1] + (self.outfeatures,))
         out_shape = x.shape[:-1] + (self.outfeatures,)
         x2 = x.half().reshape(-1, x.shape[-1])
         if not x2.is_contiguous():
@@ -204,9 +213,11 @@ class QuantLinear(nn.Module):
                 plan = self._plans[key] = ops.GemvPlan(self._qweight_run, self.qzeros, self.scales, self._g_idx_run,
                                                      self._x_perm, self.bias, M, self.bits, self.groupsize,
                                                      self.gemv_tuning)
+            self._prepare_native(M, plan)
             with torch.cuda.device(x2.device):
                 y = plan.run(x2)
         elif self._gemm_ok:
+            self._prepare_native()
             # measured on B200: from 9 rows on, one tensor-core pass (35-45 us for a 4096 x 12288 layer) beats two
             # or more GEMV passes
             y = ops.gemm(x2, *args, **kw)
@@ -227,6 +238,20 @@ class QuantLinear(nn.Module):
             for m0 in range(0, M, GEMV_MAX_M):
                 ops.gemv(x2[m0:m0 + GEMV_MAX_M], *args, out=y[m0:m0 + GEMV_MAX_M], **kw)
         return y.reshape(out_shape)
+
+    def _prepare_native(self, rows: int = 0, plan=None):
+        """Make the native call object for the current buffers (once), and hand it the plan of one more row count."""
+        if not self.qweight.is_cuda:
+            return
+        buffers = self._buffers
+        state = (self.gemv_tuning, self.bias, buffers["qzeros"], buffers["scales"])
+        if self._native is None or any(a is not b for a, b in zip(self._native_state, state)):
+            self._native_state = state
+            self._native = _lib._host.Layer(self.infeatures, self.outfeatures, self.bits, self.groupsize,
+                                            self.qweight.device.index, self.__dict__, self._gemm_ok, self._qweight_run,
+                                            self._g_idx_run, self._x_perm)
+        if plan is not None:
+            self._native.set_gemv(rows, plan, plan._handle.value, plan._need)
 
     # ---- the element-wise kernel in front of this layer folded into its read of x (decode batches only) ----
     def can_fold(self, rows: int, input_act: int) -> bool:

@@ -226,6 +226,23 @@ B200GPTQ_API int b200gptq_gemm_split(int M, int K, int N, int bits, int* splits,
  */
 B200GPTQ_API int b200gptq_pack_fields(const int32_t* vals, int R, int C, int bits, int32_t* out, void* stream);
 
+/* element types of b200gptq_pack_linear's weight */
+#define B200GPTQ_F16 0
+#define B200GPTQ_BF16 1
+#define B200GPTQ_F32 2
+
+/*
+ * QuantLinear.pack in one launch (auto_gptq/nn_modules/qlinear.py:77-175 of the reference).
+ *   weight  [N, K] of type `dtype`, the linear's weight
+ *   scales, zeros  fp32 [N, G];  g_idx int32 [K], group of row k (clamped to [0, G))
+ *   qweight int32 [K/32*bits, N]  round((w + zero * scale) / float(fp16(scale))), evaluated in fp32 with IEEE rounding
+ *   qzeros  int32 [G, N/32*bits]  zero - 1;   scales_out fp16 [G, N]
+ * Fields are not masked (see b200gptq_pack_fields).
+ */
+B200GPTQ_API int b200gptq_pack_linear(const void* weight, int dtype, const float* scales, const float* zeros,
+                                      const int32_t* g_idx, int K, int N, int G, int bits, int32_t* qweight,
+                                      int32_t* qzeros, void* scales_out, void* stream);
+
 /*
  * Re-order the rows of a packed layer so that rows of one group are adjacent
  * (stable sort of k by g_idx[k]).  Outputs:

@@ -79,3 +79,32 @@ def test_pack_fields_rejects_bad_arguments():
         ops.pack_fields(torch.zeros((32, 8), dtype=torch.int32, device=DEV), 5)
     with pytest.raises(RuntimeError):
         ops.pack_fields(torch.zeros((32, 8), dtype=torch.int32), 4)
+
+
+@pytest.mark.parametrize("bits,K,N,gs,dtype", [
+    (2, 32, 32, 32, torch.float16),           # smallest layer
+    (3, 1056, 64, 32, torch.float32),         # K is no multiple of the 256-row chunk
+    (4, 544, 96, -1, torch.bfloat16),
+    (8, 4128, 64, 8, torch.float16),          # 516 groups: the table does not fit, groups cut 32-row blocks
+])
+def test_one_launch_pack_equals_the_cpu_packer(bits, K, N, gs, dtype):
+    """b200gptq_pack_linear rounds a product with 1 / scale and falls back to the division near a half: random weights
+    (any fraction) and exact halves must give the words of the CPU route."""
+    gen = torch.Generator().manual_seed(bits + K)
+    size = gs if gs != -1 else K
+    G = -(-K // size)
+    scales = torch.rand(N, G, generator=gen) * 0.02 + 1e-3
+    zeros = torch.randint(1, 2 ** bits, (N, G), generator=gen).float()
+    g_idx = (torch.randperm(K, generator=gen) // size).to(torch.int32)
+    sel = g_idx.long()
+    W = (torch.rand(N, K, generator=gen) * (2 ** bits - 1) - zeros[:, sel]) * scales[:, sel]
+    s16 = scales[:, sel].half().float()
+    W[1] = ((torch.arange(K) % (2 ** bits - 1)).float() + 0.5) * s16[1] - (zeros * scales)[:, sel][1]
+    lin = nn.Linear(K, N, bias=False)
+    lin.weight.data = W.to(dtype)
+    a, b = QuantLinear(bits, gs, K, N, False), QuantLinear(bits, gs, K, N, False).to(DEV)
+    a.pack(lin, scales, zeros, g_idx)
+    b.pack(lin.to(DEV), scales.to(DEV), zeros.to(DEV), g_idx.to(DEV))
+    assert torch.equal(a.qweight, b.qweight.cpu())
+    assert torch.equal(a.qzeros, b.qzeros.cpu())
+    assert torch.equal(a.scales, b.scales.cpu())
