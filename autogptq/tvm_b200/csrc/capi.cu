@@ -36,20 +36,20 @@ int gemv_generic_dispatch(const __half*, const int32_t*, const int32_t*, const _
 size_t gemv_generic_workspace_bytes(int M, int K, int N);
 bool gemv_stream_supported(int M, int K, int N, int bits, int group_size);
 size_t gemv_stream_workspace_bytes(int M, int K, int N, int bits);
-int gemv_stream_dispatch(const __half*, const int32_t*, const int32_t*, const __half*, const int32_t*,
-                         const int32_t*, const __half*, __half*, int, int, int, int, int, void*, cudaStream_t);
-int gemv_stream_dispatch_knobs(const __half*, const int32_t*, const int32_t*, const __half*, const int32_t*,
-                               const __half*, __half*, int, int, int, int, int, void*, cudaStream_t, const int*);
 size_t gemm_workspace_bytes(int M, int K, int N, int bits);
 void gemm_split_query(int M, int K, int N, int* splits, int* ctas_per_sm);
 int gemm_dispatch(const __half*, const int32_t*, const int32_t*, const __half*, const int32_t*, const int32_t*,
                   const __half*, __half*, int, int, int, int, int, void*, size_t, cudaStream_t);
 
-struct GemvStreamPlan;
-GemvStreamPlan* gemv_stream_plan_create(const int32_t*, const __half*, bool, int, int, int, int, int, const int*, int*);
-int gemv_stream_plan_run(const GemvStreamPlan*, const __half*, const int32_t*, const int32_t*, const __half*, __half*,
-                         void*, cudaStream_t);
-void gemv_stream_plan_destroy(GemvStreamPlan*);
+struct GemvStripPlan;
+bool gemv_strip_supported(int M, int K, int N, int bits, int group_size);
+bool gemv_strip_gathers(int M, int K);
+GemvStripPlan* gemv_strip_plan_create(const int32_t*, const int32_t*, const __half*, bool, int, int, int, int, int, int, int, int*);
+int gemv_strip_run(const GemvStripPlan*, const __half*, const int32_t*, const __half*, __half*, void*, cudaStream_t);
+void gemv_strip_plan_destroy(GemvStripPlan*);
+int gemv_strip_dispatch(const __half*, const int32_t*, const int32_t*, const __half*, const int32_t*, const __half*, __half*,
+                        int, int, int, int, int, void*, int, int, cudaStream_t);
+int gather_x_dispatch(const __half*, const int32_t*, __half*, int, int, int, cudaStream_t);
 
 static inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
@@ -135,6 +135,8 @@ size_t b200gptq_workspace_bytes(int op, int M, int K, int N, int bits) {
     if (op == B200GPTQ_OP_GEMV) {
         size_t a = gemv_generic_workspace_bytes(M, K, N);
         size_t b = gemv_stream_workspace_bytes(M, K, N, bits);
+        const size_t c = kCounterBytes + (size_t)M * K * sizeof(__half);   // x gathered by a kernel of its own
+        if (c > b) b = c;
         return a > b ? a : b;
     }
     if (op == B200GPTQ_OP_GEMM) return gemm_workspace_bytes(M, K, N, bits);
@@ -190,6 +192,17 @@ static bool act_supported(int input_act, bool streams, const int32_t* x_perm) {
     return streams && !(input_act == B200GPTQ_ACT_SWIGLU && x_perm);
 }
 
+// A gather of more x than the kernel keeps in shared memory is done by a kernel of its own, into the scratch (ReLU, the
+// activation that is folded together with a gather, is element-wise and comes after it).
+static int gather_first(const __half** x, const int32_t** x_perm, int M, int K, void* workspace, cudaStream_t stream) {
+    if (!*x_perm || (gemv_strip_gathers(M, K) && aligned16(*x_perm))) return B200GPTQ_OK;
+    __half* xp = reinterpret_cast<__half*>(static_cast<char*>(workspace) + kCounterBytes);
+    const int st = gather_x_dispatch(*x, *x_perm, xp, M, K, 0, stream);
+    *x = xp;
+    *x_perm = nullptr;
+    return st;
+}
+
 int b200gptq_gemv_ex(const void* x, const int32_t* qweight, const int32_t* qzeros, const void* scales,
                      const int32_t* g_idx, const int32_t* x_perm, const void* bias, void* y, int M, int K, int N,
                      int bits, int group_size, void* workspace, size_t workspace_bytes, int slices_per_sm,
@@ -206,12 +219,12 @@ int b200gptq_gemv_ex(const void* x, const int32_t* qweight, const int32_t* qzero
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const bool streams = !g_idx && gemv_stream_supported(M, K, N, bits, group_size);
     if (!act_supported(input_act, streams, x_perm)) return B200GPTQ_ERR_SHAPE;
-    if (streams) {
-        const int knobs[6] = {slices_per_sm, ctas_per_sm, 0, 0, 0, input_act};
-        return gemv_stream_dispatch_knobs(static_cast<const __half*>(x), qweight, qzeros,
-                                          static_cast<const __half*>(scales), x_perm, static_cast<const __half*>(bias),
-                                          static_cast<__half*>(y), M, K, N, bits, group_size, workspace, st,
-                                          (slices_per_sm || ctas_per_sm || input_act) ? knobs : nullptr);
+    if (!g_idx && gemv_strip_supported(M, K, N, bits, group_size)) {
+        const __half* xh = static_cast<const __half*>(x);
+        if (int e = gather_first(&xh, &x_perm, M, K, workspace, st)) return e;
+        return gemv_strip_dispatch(xh, qweight, qzeros, static_cast<const __half*>(scales), x_perm,
+                                   static_cast<const __half*>(bias), static_cast<__half*>(y), M, K, N, bits, group_size,
+                                   workspace, ctas_per_sm, input_act, st);
     }
     return gemv_generic_dispatch(static_cast<const __half*>(x), qweight, qzeros, static_cast<const __half*>(scales),
                                  g_idx, x_perm, static_cast<const __half*>(bias), static_cast<__half*>(y), M, K, N,
@@ -224,7 +237,7 @@ struct b200gptq_gemv_plan {
     const __half *scales, *bias;
     int M, K, N, bits, group_size, slices_per_sm, ctas_per_sm;
     size_t workspace_need;
-    b200gptq::GemvStreamPlan* stream;   // NULL: the general kernel serves this problem
+    b200gptq::GemvStripPlan* strip;     // NULL: the general kernel serves this problem
 };
 
 int b200gptq_gemv_plan_create(b200gptq_gemv_plan** out, const int32_t* qweight, const int32_t* qzeros,
@@ -251,12 +264,11 @@ int b200gptq_gemv_plan_create_ex(b200gptq_gemv_plan** out, const int32_t* qweigh
           b200gptq_workspace_bytes(B200GPTQ_OP_GEMV, M, K, N, bits), nullptr};
     const bool streams = !g_idx && gemv_stream_supported(M, K, N, bits, group_size);
     if (!act_supported(input_act, streams, x_perm)) { delete p; return B200GPTQ_ERR_SHAPE; }
-    if (streams) {
-        const int knobs[6] = {slices_per_sm, ctas_per_sm, 0, 0, 0, input_act};
+    if (!g_idx && gemv_strip_supported(M, K, N, bits, group_size)) {
         int st = B200GPTQ_OK;
-        p->stream = gemv_stream_plan_create(qweight, p->scales, x_perm != nullptr, M, K, N, bits, group_size,
-                                            (slices_per_sm || ctas_per_sm || input_act) ? knobs : nullptr, &st);
-        if (!p->stream) { delete p; return st; }
+        const bool gather = x_perm != nullptr && gemv_strip_gathers(M, K) && aligned16(x_perm);
+        p->strip = gemv_strip_plan_create(qweight, qzeros, p->scales, gather, M, K, N, bits, group_size, ctas_per_sm, input_act, &st);
+        if (!p->strip) { delete p; return st; }
     }
     *out = p;
     return B200GPTQ_OK;
@@ -268,9 +280,12 @@ int b200gptq_gemv_plan_run(const b200gptq_gemv_plan* p, const void* x, void* y, 
     if (!aligned16(x) || !aligned16(y) || (workspace && !aligned16(workspace))) return B200GPTQ_ERR_ALIGNMENT;
     if (!workspace || workspace_bytes < p->workspace_need) return B200GPTQ_ERR_WORKSPACE;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (p->stream)
-        return gemv_stream_plan_run(p->stream, static_cast<const __half*>(x), p->qzeros, p->x_perm, p->bias,
-                                    static_cast<__half*>(y), workspace, st);
+    if (p->strip) {
+        const __half* xh = static_cast<const __half*>(x);
+        const int32_t* perm = p->x_perm;
+        if (int e = gather_first(&xh, &perm, p->M, p->K, workspace, st)) return e;
+        return gemv_strip_run(p->strip, xh, perm, p->bias, static_cast<__half*>(y), workspace, st);
+    }
     return gemv_generic_dispatch(static_cast<const __half*>(x), p->qweight, p->qzeros, p->scales, p->g_idx, p->x_perm,
                                  p->bias, static_cast<__half*>(y), p->M, p->K, p->N, p->bits, p->group_size, workspace,
                                  st);
@@ -278,7 +293,7 @@ int b200gptq_gemv_plan_run(const b200gptq_gemv_plan* p, const void* x, void* y, 
 
 void b200gptq_gemv_plan_destroy(b200gptq_gemv_plan* p) {
     if (!p) return;
-    if (p->stream) gemv_stream_plan_destroy(p->stream);
+    if (p->strip) gemv_strip_plan_destroy(p->strip);
     delete p;
 }
 

@@ -691,6 +691,17 @@ void gemm_split_query(int M, int K, int N, int* splits, int* ctas_per_sm) {
     *ctas_per_sm = g.per_sm;
 }
 
+// x copied in the order in which a product reads it: gathered through x_perm and / or in the 3-bit field order.
+int gather_x_dispatch(const __half* x, const int32_t* x_perm, __half* xp, int M, int K, int permute3, cudaStream_t stream) {
+    const size_t total = (size_t)M * K;
+    int blocks = (int)((total + 256 * 8 - 1) / (256 * 8));
+    if (blocks > 4 * sm_count()) blocks = 4 * sm_count();
+    if (blocks < 1) blocks = 1;
+    prep_x_kernel<<<blocks, 256, 0, stream>>>(x, x_perm, xp, M, K, permute3);
+    B200GPTQ_CUDA_TRY(cudaGetLastError());
+    return B200GPTQ_OK;
+}
+
 int gemm_dispatch(const __half* x, const int32_t* qweight, const int32_t* qzeros, const __half* scales,
                   const int32_t* g_idx, const int32_t* x_perm, const __half* bias, __half* y, int M, int K, int N,
                   int bits, int group_size, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
@@ -699,12 +710,7 @@ int gemm_dispatch(const __half* x, const int32_t* qweight, const int32_t* qzeros
     const __half* xt = x;
     if (bits == 3 || x_perm) {
         __half* xp = reinterpret_cast<__half*>(reinterpret_cast<char*>(workspace) + kCounterBytes);
-        const size_t total = (size_t)M * K;
-        int blocks = (int)((total + 256 * 8 - 1) / (256 * 8));
-        if (blocks > 4 * sm_count()) blocks = 4 * sm_count();
-        if (blocks < 1) blocks = 1;
-        prep_x_kernel<<<blocks, 256, 0, stream>>>(x, x_perm, xp, M, K, bits == 3 ? 1 : 0);
-        B200GPTQ_CUDA_TRY(cudaGetLastError());
+        if (int st = gather_x_dispatch(x, x_perm, xp, M, K, bits == 3 ? 1 : 0, stream)) return st;
         xt = xp;
     }
     float* partial = reinterpret_cast<float*>(reinterpret_cast<char*>(workspace) + kCounterBytes +

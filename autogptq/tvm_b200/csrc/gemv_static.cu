@@ -25,10 +25,6 @@ namespace b200gptq {
 
 int gemv_generic_dispatch(const __half*, const int32_t*, const int32_t*, const __half*, const int32_t*,
                           const int32_t*, const __half*, __half*, int, int, int, int, int, void*, cudaStream_t);
-bool gemv_stream_supported(int M, int K, int N, int bits, int group_size);
-int gemv_stream_dispatch(const __half*, const int32_t*, const int32_t*, const __half*, const int32_t*,
-                         const int32_t*, const __half*, __half*, int, int, int, int, int, void*, cudaStream_t);
-
 namespace {
 
 constexpr size_t kStaticScratchBytes = 4u << 20;  // 4 MiB per device
@@ -83,14 +79,8 @@ int b200gptq_gemv_static(const void* x, const int32_t* qweight, const int32_t* q
         return B200GPTQ_ERR_TOO_LARGE;
     void* scratch = nullptr;
     if (int st = static_scratch(&scratch)) return st;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (!g_idx && gemv_stream_supported(M, K, N, bits, group_size))
-        return gemv_stream_dispatch(static_cast<const __half*>(x), qweight, qzeros, static_cast<const __half*>(scales),
-                                    g_idx, x_perm, static_cast<const __half*>(bias), static_cast<__half*>(y), M, K, N,
-                                    bits, group_size, scratch, s);
-    return gemv_generic_dispatch(static_cast<const __half*>(x), qweight, qzeros, static_cast<const __half*>(scales),
-                                 g_idx, x_perm, static_cast<const __half*>(bias), static_cast<__half*>(y), M, K, N, bits,
-                                 group_size, scratch, s);
+    return b200gptq_gemv(x, qweight, qzeros, scales, g_idx, x_perm, bias, y, M, K, N, bits, group_size, scratch,
+                         kStaticScratchBytes, stream);
 }
 
 // The sticky status word of the built-in scratch on the current device (see b200gptq_workspace_status).

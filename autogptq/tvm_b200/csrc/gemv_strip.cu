@@ -1,0 +1,209 @@
+// Host side of the decode GEMV (gemv_strip.cuh): plan, tensor map, launch.
+#include <mutex>
+#include <new>
+
+#include "gemv_strip.cuh"
+
+namespace b200gptq {
+
+const void* gemv_strip_kernel_b2(int sub, int mode, int nt, int T, int warps);
+const void* gemv_strip_kernel_b3(int sub, int mode, int nt, int T, int warps);
+const void* gemv_strip_kernel_b4(int sub, int mode, int nt, int T, int warps);
+const void* gemv_strip_kernel_b8(int sub, int mode, int nt, int T, int warps);
+
+struct GemvStripPlan {
+    int M, K, N, smem, warps;
+    StripPlan plan;
+    CUtensorMap tmap_w, tmap_s, tmap_z;
+    const void* kernel;
+};
+
+namespace {
+
+constexpr int kSmemMax = 224 * 1024;      // dynamic shared memory of a CTA
+constexpr int kRawMax = 48 * 1024;        // largest x (all rows) that a CTA copies whole to gather from
+
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiledFn encode_tiled_fn() {
+    static const EncodeTiledFn fn = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            p = nullptr;
+        return reinterpret_cast<EncodeTiledFn>(p);
+    }();
+    return fn;
+}
+
+const void* strip_kernel(int bits, int sub, int mode, int nt, int T, int warps) {
+    switch (bits) {
+        case 2: return gemv_strip_kernel_b2(sub, mode, nt, T, warps);
+        case 3: return gemv_strip_kernel_b3(sub, mode, nt, T, warps);
+        case 4: return gemv_strip_kernel_b4(sub, mode, nt, T, warps);
+        case 8: return gemv_strip_kernel_b8(sub, mode, nt, T, warps);
+    }
+    return nullptr;
+}
+
+int set_attrs_once() {
+    static std::once_flag once[64];
+    static int result[64];
+    int dev = 0;
+    B200GPTQ_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return B200GPTQ_ERR_TOO_LARGE;
+    std::call_once(once[dev], [dev] {
+        cudaError_t e = cudaSuccess;
+        for (int b : {2, 3, 4, 8})
+            for (int sub : {1, 4})
+                for (int v = 0; v < 4; ++v)
+                    for (int i = 0; i < 8; ++i)
+                        if (const void* f = strip_kernel(b, sub, v == 3 ? kSeveral : v, v == 3 ? 2 : 1, 1 + i / 2, i & 1 ? 16 : 8))
+                            if (e == cudaSuccess)
+                                e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
+        result[dev] = (int)e;
+    });
+    if (result[dev] != 0) { set_last_cuda_error(result[dev]); return B200GPTQ_ERR_CUDA; }
+    return B200GPTQ_OK;
+}
+
+}  // namespace
+
+// Groups of whole 32-row blocks, up to 16 rows of x.
+bool gemv_strip_supported(int M, int K, int N, int bits, int group_size) {
+    (void)bits;
+    return M >= 1 && M <= 16 && N % kStripCols == 0 && K % 32 == 0 && (group_size % 32 == 0 || group_size >= K);
+}
+// A gather from a copy of x in shared memory; larger x is gathered by a kernel of its own first.
+bool gemv_strip_gathers(int M, int K) { return (size_t)M * K * 2 <= kRawMax; }
+
+int gemv_strip_prepare(GemvStripPlan* p, const int32_t* qweight, const int32_t* qzeros,
+                       const __half* scales, bool gather, int M, int K, int N, int bits, int group_size,
+                       int ctas_per_sm, int xact) {
+    if (int st = set_attrs_once()) return st;
+    p->M = M; p->K = K; p->N = N;
+    StripPlan& s = p->plan;
+    s.spg = group_size >= K ? K / 32 : group_size / 32;
+    s.groups = (K / 32 + s.spg - 1) / s.spg;
+    s.spg_inv = (unsigned int)((0x100000000ULL + s.spg - 1) / s.spg);     // (not used for 1)
+    s.gather = gather ? 1 : 0;
+    s.xact = xact;
+    // a unit lies in one group when groups are whole units (or there is only one)
+    const int sub = (s.spg % 4 == 0 || s.groups == 1) ? 1 : 4;
+    s.units = (K + kUnit - 1) / kUnit;
+    const int nt = M <= 8 ? 1 : 2;
+    // One and two rows: planes of x where they pay and fit; one row: x kept whole.
+    s.strips = N / kStripCols;
+    // One CTA per SM: each takes the same whole number of strips.
+    s.per_cta = (s.strips + sm_count() - 1) / sm_count();
+    const int plane_bytes = (s.units * M * ((bits == 3 ? 5 : 4) * 128 + 8) + 15) / 16 * 16;
+    const int mode = M <= 2 && bits != 8 && sub == 1 && s.per_cta > M && plane_bytes <= 96 * 1024 ? kInt
+                   : (M == 1 && K <= 65536 ? kOne : kSeveral);
+    const int tmax = mode == kInt ? 4 : (sub == 1 && nt == 1 ? 3 : 2);
+    s.rows_g = sub == 1 ? 1 : (s.spg == 1 ? 4 : (s.spg == 2 ? 2 : 3));
+    // Strips of a pass for W warps: a unit costs about half a strip's work on top of its strips, and the last pass is a whole
+    // one.  The rings take at least two slots and what is left of the shared memory.
+    struct Choice { int W, T, ring, fixed, kept; };
+    auto choose = [&](int W) {
+        Choice c = {W, 0, 0, 0, 0};
+        int best = 1 << 30;
+        // (a gather works from a copy of x that the sums overwrite: it needs every unit's x kept)
+        for (int kept = 1; kept >= (mode == kSeveral && !gather ? 0 : 1) && !c.T; --kept)
+            for (int t = 1; t <= tmax && t <= s.per_cta; ++t) {
+                const int slot = slot_bytes(bits, t) + const_bytes(bits, t, s.rows_g);
+                const int sums = W * M * t * kStripCols * 4, copy = gather || mode != kSeveral ? M * K * 2 : 0;
+                const int x = mode == kInt ? plane_bytes
+                            : (mode == kOne ? s.units * kUnit * 2 : (kept ? s.units : 2 * W) * M * kXPitch * 2);
+                const int f = x + (sums > copy ? sums : copy) + 1024, r = (kSmemMax - f) / (W * slot);
+                const int cost = ((s.per_cta + t - 1) / t) * (2 * t + 1);
+                if (f < kSmemMax && r >= 2 && cost <= best) { best = cost; c = {W, t, r, f, kept}; }
+            }
+        return c;
+    };
+    // Sixteen warps hide the latency of a unit better (4096 x 4096, 4 bits: 3.9 against 4.4 us, 11008 x 4096: 7.8 against
+    // 9.8), but their rings may only hold narrower passes that repeat strips (4096 x 12288: 8.1 against 6.2), and short K
+    // leaves some idle.  Sixteen rows of x take more than half of a thread's registers.
+    Choice c = choose(8);
+    if (nt == 1 && ctas_per_sm <= 1) {
+        const Choice w = choose(16);
+        auto work = [&](const Choice& v) { return (s.per_cta + v.T - 1) / v.T * v.T; };
+        if (w.T && (ctas_per_sm == 1 || !c.T || (s.units >= 16 && work(w) <= work(c)))) c = w;
+    }
+    if (!c.T) return B200GPTQ_ERR_TOO_LARGE;
+    const int W = c.W, T = c.T;
+    s.passes = (s.per_cta + T - 1) / T;
+    s.kept = c.kept;
+    const int longest = ((s.units + W - 1) / W) * s.passes;
+    s.ring = c.ring < longest ? c.ring : longest;
+    if (s.ring > kMaxRing) s.ring = kMaxRing;
+    p->warps = W;
+    p->smem = W * s.ring * (slot_bytes(bits, T) + const_bytes(bits, T, s.rows_g)) + c.fixed;
+    p->kernel = strip_kernel(bits, sub, mode, nt, T, W);
+    if (!p->kernel) return B200GPTQ_ERR_SHAPE;
+    const EncodeTiledFn encode = encode_tiled_fn();
+    if (!encode) { set_last_cuda_error((int)cudaErrorNotSupported); return B200GPTQ_ERR_CUDA; }
+    auto map = [&](CUtensorMap* m, CUtensorMapDataType type, int rank, const void* base, const cuuint64_t* dims,
+                   const cuuint64_t* strides, const cuuint32_t* box, CUtensorMapSwizzle swizzle) {
+        const cuuint32_t estr[3] = {1, 1, 1};
+        return encode(m, type, rank, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
+    // qweight [K/32*bits, N] as {32 columns, word-rows, N/32 strips}; scales [G, N]; qzeros as one run of words.  What lies
+    // past the end reads as zero.
+    const cuuint64_t wd[3] = {kStripCols, (cuuint64_t)(K / 32 * bits), (cuuint64_t)s.strips}, ws[2] = {(cuuint64_t)N * 4, kStripCols * 4};
+    const cuuint32_t wb[3] = {kStripCols, (cuuint32_t)(4 * bits), (cuuint32_t)T};
+    const cuuint64_t sd[2] = {(cuuint64_t)N, (cuuint64_t)s.groups}, ss[1] = {(cuuint64_t)N * 2};
+    const cuuint32_t sb[2] = {(cuuint32_t)(T * kStripCols), (cuuint32_t)s.rows_g};
+    const cuuint64_t zd[1] = {(cuuint64_t)s.groups * (N / 32 * bits)};
+    const cuuint32_t zb[1] = {(cuuint32_t)zero_words(bits, T)};
+    if (!map(&p->tmap_w, CU_TENSOR_MAP_DATA_TYPE_INT32, 3, qweight, wd, ws, wb, CU_TENSOR_MAP_SWIZZLE_128B) ||
+        !map(&p->tmap_s, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, scales, sd, ss, sb, CU_TENSOR_MAP_SWIZZLE_NONE) ||
+        !map(&p->tmap_z, CU_TENSOR_MAP_DATA_TYPE_INT32, 1, qzeros, zd, ws, zb, CU_TENSOR_MAP_SWIZZLE_NONE)) {
+        set_last_cuda_error((int)cudaErrorInvalidValue);
+        return B200GPTQ_ERR_CUDA;
+    }
+    return B200GPTQ_OK;
+}
+
+int gemv_strip_run(const GemvStripPlan* p, const __half* x, const int32_t* x_perm,
+                   const __half* bias, __half* y, void* workspace, cudaStream_t stream) {
+    unsigned int* status = reinterpret_cast<unsigned int*>(workspace);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(p->plan.strips < sm_count() ? p->plan.strips : sm_count());
+    cfg.blockDim = dim3(32 * p->warps);
+    cfg.dynamicSmemBytes = p->smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int M = p->M, K = p->K, N = p->N;
+    void* args[] = {const_cast<CUtensorMap*>(&p->tmap_w), const_cast<CUtensorMap*>(&p->tmap_s),
+                    const_cast<CUtensorMap*>(&p->tmap_z), &x, &x_perm, &bias, &y, &M, &K, &N,
+                    const_cast<StripPlan*>(&p->plan), &status};
+    B200GPTQ_CUDA_TRY(cudaLaunchKernelExC(&cfg, p->kernel, args));
+    return B200GPTQ_OK;
+}
+
+GemvStripPlan* gemv_strip_plan_create(const int32_t* qweight, const int32_t* qzeros, const __half* scales, bool gather, int M, int K, int N, int bits, int group_size,
+                                      int ctas_per_sm, int xact, int* status_out) {
+    GemvStripPlan* p = new (std::nothrow) GemvStripPlan;
+    if (!p) { *status_out = B200GPTQ_ERR_CUDA; return nullptr; }
+    *status_out = gemv_strip_prepare(p, qweight, qzeros, scales, gather, M, K, N, bits, group_size, ctas_per_sm, xact);
+    if (*status_out != B200GPTQ_OK) { delete p; return nullptr; }
+    return p;
+}
+void gemv_strip_plan_destroy(GemvStripPlan* p) { delete p; }
+
+int gemv_strip_dispatch(const __half* x, const int32_t* qweight, const int32_t* qzeros, const __half* scales,
+                        const int32_t* x_perm, const __half* bias, __half* y, int M, int K, int N, int bits, int group_size,
+                        void* workspace, int ctas_per_sm, int xact, cudaStream_t stream) {
+    GemvStripPlan p;
+    if (int st = gemv_strip_prepare(&p, qweight, qzeros, scales, x_perm != nullptr, M, K, N, bits, group_size, ctas_per_sm, xact)) return st;
+    return gemv_strip_run(&p, x, x_perm, bias, y, workspace, stream);
+}
+
+}  // namespace b200gptq

@@ -1,0 +1,8 @@
+// The 3-bit instantiations of the decode GEMV (a translation unit of their own, to compile side by side).
+#include "gemv_strip.cuh"
+
+namespace b200gptq {
+const void* gemv_strip_kernel_b3(int sub, int mode, int nt, int T, int warps) {
+    return strip_kernel_bits<3>(sub, mode, nt, T, warps);
+}
+}  // namespace b200gptq

@@ -1,0 +1,8 @@
+// The 8-bit instantiations of the decode GEMV (a translation unit of their own, to compile side by side).
+#include "gemv_strip.cuh"
+
+namespace b200gptq {
+const void* gemv_strip_kernel_b8(int sub, int mode, int nt, int T, int warps) {
+    return strip_kernel_bits<8>(sub, mode, nt, T, warps);
+}
+}  // namespace b200gptq

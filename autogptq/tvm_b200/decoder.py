@@ -168,10 +168,9 @@ class GPTQDecoder:
         self.layers = [DecoderLayer(cfg, i, self.rank, self.world, dev) for i in range(cfg.layers)]
         for L in self.layers:
             L.o.exchange = L.down.exchange = self.exchange
-            # in a decode step small kernels sit between the GEMVs: fewer, longer K slices and a footprint of a third
-            # of an SM measured fastest there (392 against 350 tokens/s on the Llama-7B architecture, one GPU)
-            for mod in (L.qkv, L.o, L.up, L.down):
-                mod.gemv_tuning = (2, 3)
+            if self.exchange is not None:
+                # the GEMVs with the exchange fused in: fewer, longer K slices and a footprint of a third of an SM
+                L.o.gemv_tuning = L.down.gemv_tuning = (2, 3)
         g = torch.Generator(device=dev).manual_seed(7)   # replicated tensors: the same seed on every rank
         self.embed = (0.02 * torch.randn(cfg.vocab, cfg.hidden, generator=g, device=dev)).half()
         self.pos_embed = None
@@ -401,7 +400,7 @@ class GPTQDecoder:
 
     #: work splits :meth:`tune` tries: (K slices per SM that the cluster size aims at, CTAs per SM that the footprint is
     #: sized for; 0 = the library's choice), ``None`` = the library's defaults for a GEMV on its own
-    TUNINGS = (None, (2, 0), (4, 0), (6, 0), (2, 3))
+    TUNINGS = (None, (2, 0), (4, 0), (6, 0), (2, 1), (2, 2), (2, 3))
 
     def tune(self, steps: int = 12, candidates=TUNINGS) -> dict:
         """Choose the GEMV work split of each kind of linear layer (qkv, o, up, down) by timing the captured decode

@@ -146,21 +146,22 @@ class QuantLinear(nn.Module):
         K = self.infeatures
         g = self.g_idx
         trivial = torch.equal(g, (torch.arange(K, device=dev, dtype=torch.int64) // self.groupsize).to(torch.int32))
-        blocks = g.view(K // 32, 32)
-        lo, hi = torch.aminmax(g)
-        block_uniform, lo, hi = torch.stack([(blocks == blocks[:, :1]).all().to(g.dtype), lo, hi]).tolist()
-        if lo < 0 or hi >= self.scales.shape[0]:
-            raise ValueError(f"g_idx names group {lo if lo < 0 else hi}, the layer has {self.scales.shape[0]}")
         if trivial:
             self._qweight_run, self._g_idx_run, self._x_perm = self.qweight, None, None
-        elif block_uniform:
-            self._qweight_run, self._g_idx_run, self._x_perm = self.qweight, g.contiguous(), None
         else:
-            qs, perm, gs = ops.sort_rows(self.qweight.contiguous(), g.contiguous(), self.bits)
-            sorted_trivial = torch.equal(
-                gs, (torch.arange(K, device=dev, dtype=torch.int64) // self.groupsize).to(torch.int32))
-            self._qweight_run, self._x_perm = qs, perm
-            self._g_idx_run = None if sorted_trivial else gs
+            blocks = g.view(K // 32, 32)
+            lo, hi = torch.aminmax(g)
+            block_uniform, lo, hi = torch.stack([(blocks == blocks[:, :1]).all().to(g.dtype), lo, hi]).tolist()
+            if lo < 0 or hi >= self.scales.shape[0]:
+                raise ValueError(f"g_idx names group {lo if lo < 0 else hi}, the layer has {self.scales.shape[0]}")
+            if block_uniform:
+                self._qweight_run, self._g_idx_run, self._x_perm = self.qweight, g.contiguous(), None
+            else:
+                qs, perm, gs = ops.sort_rows(self.qweight.contiguous(), g.contiguous(), self.bits)
+                sorted_trivial = torch.equal(
+                    gs, (torch.arange(K, device=dev, dtype=torch.int64) // self.groupsize).to(torch.int32))
+                self._qweight_run, self._x_perm = qs, perm
+                self._g_idx_run = None if sorted_trivial else gs
         # the tensor-core kernel takes one group per aligned 32-row block: true for every run-time g_idx built above
         # (block-uniform or sorted by group with whole blocks) except a NULL g_idx with a group size that is no
         # multiple of 32, and a sorted layout whose groups do not fill whole blocks

@@ -118,13 +118,10 @@ B200GPTQ_API int b200gptq_gemv(const void* x, const int32_t* qweight, const int3
  * default for that parameter; other kernels ignore them).  The reference tunes its kernels per shape and
  * per row bucket (tile tables of pycuda_warpper.py:77-127, NNI search results in .cache/handler_database.json);
  * here the kernel is one and what remains to tune is how it shares the GPU with its neighbours in the stream:
- *   slices_per_sm  the K range of a 256-column group is cut into as many slices (CTAs) as give the grid about
- *                  this many CTAs per SM (at most 8 slices).  Default 3 for one row of x, 2 otherwise.
- *   ctas_per_sm    shared-memory footprint: a CTA takes at most 1/ctas_per_sm of an SM, so that many CTAs -- of
- *                  this launch and of its neighbours -- can be resident together; a slice that does not fit is
- *                  streamed through a ring.  Default: 3 if the whole slice still fits, else 2.
- * Measured on B200: a chain of nothing but GEMVs (the benchmark's pool of layers) is fastest with the defaults;
- * a decode step, where small kernels sit between the GEMVs, is fastest with (2, 3).
+ *   slices_per_sm  used by the row-parallel GEMV (b200gptq_gemv_tp) only: the K range of a 256-column group is cut into
+ *                  as many slices (CTAs) as give the grid about this many CTAs per SM (at most 8 slices).
+ *   ctas_per_sm    1: sixteen warps per CTA, more: eight, 0: chosen by the sizes.  b200gptq_gemv_tp: shared-memory
+ *                  footprint, a CTA takes at most 1/ctas_per_sm of an SM.
  */
 B200GPTQ_API int b200gptq_gemv_tuned(const void* x, const int32_t* qweight, const int32_t* qzeros, const void* scales,
                         const int32_t* g_idx, const int32_t* x_perm, const void* bias, void* y,
@@ -179,7 +176,9 @@ B200GPTQ_API void b200gptq_gemv_plan_destroy(b200gptq_gemv_plan* plan);
  * B200GPTQ_PATH_GENERIC (a negative B200GPTQ_ERR_* code for an invalid problem).
  * Host-only; launches nothing.  has_g_idx != 0 means a non-NULL g_idx is passed.
  * The reference picks its kernel per (bits, N, K, M bucket) in
- * pycuda_warpper.py:138-189; this is the query for the same decision here.
+ * pycuda_warpper.py:138-189; this is the query for the same decision here.  PATH_STREAM stands for 3- and 4-bit layers
+ * whose groups are whole runs of 128 rows, the ones that also take an input activation; the streaming kernel itself serves
+ * every g_idx == NULL layer whose groups are whole 32-row blocks.
  */
 #define B200GPTQ_PATH_STREAM 1
 #define B200GPTQ_PATH_GENERIC 2

@@ -1,0 +1,55 @@
+"""The decode GEMV for groups of whole 32-row blocks at the edges of its work split: all bit widths, groups inside and
+across the 128-row units, a cut last unit, one strip of columns up to more strips than a pass, one row (byte planes, or fp16
+where the row is long), two rows (planes) and more rows (fp16), with and without a gather."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import gptq_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+if torch.cuda.is_available():
+    from autogptq.tvm_b200 import ops, synth
+    DEV = torch.device("cuda:0")
+
+CASES = [
+    # bits, K, N, gs, gather
+    (2, 32, 32, 32, False),            # a quarter of a unit, one strip
+    (2, 1184, 4800, 96, True),         # groups of three steps, cut last unit, more strips than CTAs
+    (2, 2048, 64, 128, False),
+    (3, 160, 96, 32, False),
+    (3, 1088, 5088, 64, True),
+    (3, 4224, 288, 128, True),
+    (3, 32768, 64, 128, False),        # planes of one row do not fit: fp16, the row kept whole
+    (3, 69632, 32, 128, False),        # nor does the row
+    (4, 992, 96, 32, True),
+    (4, 1056, 64, -1, False),          # one group, cut last unit
+    (4, 640, 19008, 128, False),       # 594 strips: five per CTA, overlapping passes
+    (4, 28672, 64, 1024, True),        # too long to gather from shared memory
+    (8, 96, 32, 32, False),
+    (8, 1152, 4832, 64, False),
+    (8, 2560, 160, -1, True),
+]
+
+
+@pytest.mark.parametrize("bits,K,N,gs,gather", CASES)
+@pytest.mark.parametrize("M", [1, 2, 3, 8])
+def test_gemv_vs_oracle(bits, K, N, gs, gather, M):
+    layer = synth.make_layer(bits, K, N, gs, False, bias=N % 96 == 0, seed=K + N + bits)
+    _, _, W = O.dequantize(layer.qweight.numpy(), layer.qzeros.numpy(), layer.scales.numpy(), layer.g_idx.numpy(), bits)
+    x = synth.make_x(M, K, seed=M)
+    perm = torch.randperm(K, generator=torch.Generator().manual_seed(K)).to(torch.int32) if gather else None
+    xg = x if perm is None else x[:, perm.long()]
+    bias = None if layer.bias is None else layer.bias.numpy()
+    d = layer.to(DEV)
+    run = lambda **kw: ops.gemv(x.to(DEV), d.qweight, d.qzeros, d.scales, None, bits, gs, bias=d.bias,
+                                x_perm=None if perm is None else perm.to(DEV), **kw)
+    ref = O.forward_fp64(xg.numpy(), W, bias)
+    # fp32 accumulation and one fp16 rounding: the weights are exact, the sums of powers of two that 2 and 3 bits subtract
+    # are up to 2^10 times the inputs in fp32
+    norm = np.linalg.norm(xg.numpy().astype(np.float64), axis=1, keepdims=True) * np.abs(W.astype(np.float64)).max()
+    for y in (run(), run(tuning=(2, 1))):       # eight warps and sixteen
+        err = np.abs(y.cpu().numpy().astype(np.float64) - ref)
+        assert np.all(err <= 2.0 ** -10 * np.abs(ref) + 2e-4 * norm), err.max()
+    ops.check_status(DEV)
