@@ -254,7 +254,8 @@ int b200gptq_gemv_plan_create_ex(b200gptq_gemv_plan** out, const int32_t* qweigh
     if (!out || !qweight || !qzeros || !scales) return B200GPTQ_ERR_NULL_POINTER;
     *out = nullptr;
     if (int st = check_layer(K, N, bits, &group_size)) return st;
-    if (M < 1 || M > 8) return B200GPTQ_ERR_SHAPE;
+    // (9 to 16 rows: only where the streaming kernel takes the layer)
+    if (M < 1 || M > (!g_idx && gemv_strip_supported(M, K, N, bits, group_size) ? 16 : 8)) return B200GPTQ_ERR_SHAPE;
     if (slices_per_sm < 0 || slices_per_sm > 8 || ctas_per_sm < 0 || ctas_per_sm > 4) return B200GPTQ_ERR_SHAPE;
     if (!aligned16(qweight) || !aligned16(scales) || !aligned16(qzeros)) return B200GPTQ_ERR_ALIGNMENT;
     b200gptq_gemv_plan* p = new (std::nothrow) b200gptq_gemv_plan;

@@ -17,7 +17,7 @@
 
 namespace {
 
-constexpr int kMaxGemvRows = 8;
+constexpr int kMaxGemvRows = 16;
 
 // Scratch buffers by (device, stream), registered by ops.get_workspace.  Read and written under the GIL.
 struct Scratch { void* ptr; size_t bytes; };
@@ -46,6 +46,7 @@ struct Layer {
     GemvEntry gemv[kMaxGemvRows + 1];
     // run-time layout for the GEMM (gemm_ok false: no tensor-core kernel for this layer)
     bool gemm_ok;
+    int gemv_rows;        // largest row count that goes through plans (8, or 16 where the streaming kernel takes the layer)
     const int32_t *qweight_run, *qzeros_run, *g_idx_run, *x_perm;
     const void *scales_run, *bias_run;
     PyObject* keep;       // keeps the tensors behind those addresses alive
@@ -94,7 +95,7 @@ PyObject* layer_run(PyObject* self_, PyObject* const* args, Py_ssize_t nargs) {
     if ((bias ? bias : Py_None) != self->bias || PyDict_GetItem(buffers, s_qzeros) != self->qzeros ||
         PyDict_GetItem(buffers, s_scales) != self->scales)
         Py_RETURN_NONE;
-    const bool gemv = M <= kMaxGemvRows;
+    const bool gemv = M <= self->gemv_rows;
     const GemvEntry* e = gemv ? &self->gemv[M] : nullptr;
     if (gemv ? (!e->plan || PyDict_GetItem(dict, s_gemv_tuning) != self->tuning) : !self->gemm_ok) Py_RETURN_NONE;
     if (c10::cuda::current_device() != self->device || M > INT32_MAX) Py_RETURN_NONE;
@@ -144,11 +145,11 @@ const void* tensor_address(PyObject* t) {
     return t && THPVariable_Check(t) ? THPVariable_Unpack(t).unsafeGetTensorImpl()->data() : nullptr;
 }
 
-// Layer(K, N, bits, group_size, device, module_dict, gemm_ok, qweight_run, g_idx_run, x_perm)
+// Layer(K, N, bits, group_size, device, module_dict, gemm_ok, gemv_rows, qweight_run, g_idx_run, x_perm)
 PyObject* layer_new(PyTypeObject* type, PyObject* args, PyObject*) {
-    int K, N, bits, group_size, device, gemm_ok;
+    int K, N, bits, group_size, device, gemm_ok, gemv_rows;
     PyObject *dict, *qw, *gi, *perm;
-    if (!PyArg_ParseTuple(args, "iiiiiOpOOO", &K, &N, &bits, &group_size, &device, &dict, &gemm_ok, &qw, &gi, &perm))
+    if (!PyArg_ParseTuple(args, "iiiiiOpiOOO", &K, &N, &bits, &group_size, &device, &dict, &gemm_ok, &gemv_rows, &qw, &gi, &perm))
         return nullptr;
     PyObject* buffers = PyDict_Check(dict) ? PyDict_GetItem(dict, s_buffers) : nullptr;
     if (!buffers) { PyErr_SetString(PyExc_TypeError, "module_dict"); return nullptr; }
@@ -171,6 +172,7 @@ PyObject* layer_new(PyTypeObject* type, PyObject* args, PyObject*) {
     self->g_idx_at = tensor_address(pg);
     self->qzeros = pz; self->scales = ps; self->bias = bias ? bias : Py_None; self->tuning = tuning;
     self->gemm_ok = gemm_ok != 0;
+    self->gemv_rows = gemv_rows < kMaxGemvRows ? gemv_rows : kMaxGemvRows;
     self->qweight_run = static_cast<const int32_t*>(tensor_address(qw));
     self->g_idx_run = static_cast<const int32_t*>(tensor_address(gi));
     self->x_perm = static_cast<const int32_t*>(tensor_address(perm));

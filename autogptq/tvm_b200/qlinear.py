@@ -20,6 +20,7 @@ import torch.nn as nn
 from . import _lib, ops
 
 GEMV_MAX_M = 8
+GEMV_WIDE_M = 16    # the streaming kernel takes up to 16 rows (a plan of 9..16 rows: b200gptq_gemv_plan_create)
 
 
 def _pack_fields(vals: torch.Tensor, bits: int) -> torch.Tensor:
@@ -80,6 +81,7 @@ class QuantLinear(nn.Module):
         self._qweight_run = None   # the weights the kernels read: qweight itself or its row-sorted copy
         self._g_idx_run = None     # None => rows use group k // groupsize
         self._x_perm = None        # None => no gather of x
+        self._gemv_rows = GEMV_MAX_M   # largest batch that goes through the GEMV
         self._gemm_ok = False      # the run-time layout meets the tensor-core kernel's one-group-per-32-rows rule
         # Row-parallel shard of a tensor-parallel model: forward_reduce() returns the sum over ranks.  `exchange` is an
         # exchange.PeerExchange (fused all-reduce for up to 8 rows), `tp_bias` the full bias that every rank adds after
@@ -171,6 +173,10 @@ class QuantLinear(nn.Module):
         else:
             b = g_run.view(K // 32, 32)
             self._gemm_ok = self.bits in (3, 4) and bool((b == b[:, :1]).all().item())
+        # 9 to 16 rows: one pass of the streaming GEMV beats the tensor-core kernel's 16-row tile, whose weight warps are
+        # the bottleneck (9216 x 9216, 3 bits: 20 against 40 us; 4096 x 4096, 4 bits: 8.3 against 16.6)
+        whole_blocks = self._g_idx_run is None and (self.groupsize % 32 == 0 or self.groupsize >= K)
+        self._gemv_rows = GEMV_WIDE_M if whole_blocks else GEMV_MAX_M
         self._plans = {}
         self._native = None
         self._ready_for = (self.qweight.data_ptr(), self.g_idx.data_ptr())
@@ -207,7 +213,7 @@ class QuantLinear(nn.Module):
         M = x2.shape[0]
         kw = dict(bias=self.bias, x_perm=self._x_perm)
         args = (self._qweight_run, self.qzeros, self.scales, self._g_idx_run, self.bits, self.groupsize)
-        if M <= GEMV_MAX_M:
+        if M <= self._gemv_rows:
             key = (M, self.gemv_tuning)
             plan = self._plans.get(key)
             if plan is None or plan._keep[5] is not self.bias:
@@ -219,8 +225,7 @@ class QuantLinear(nn.Module):
                 y = plan.run(x2)
         elif self._gemm_ok:
             self._prepare_native()
-            # measured on B200: from 9 rows on, one tensor-core pass (35-45 us for a 4096 x 12288 layer) beats two
-            # or more GEMV passes
+            # above that one tensor-core pass beats several GEMV passes
             y = ops.gemm(x2, *args, **kw)
         elif M > 64:
             # no tensor-core kernel for this layout and many rows: dequantise once with the library's kernel (the
@@ -249,8 +254,8 @@ class QuantLinear(nn.Module):
         if self._native is None or any(a is not b for a, b in zip(self._native_state, state)):
             self._native_state = state
             self._native = _lib._host.Layer(self.infeatures, self.outfeatures, self.bits, self.groupsize,
-                                            self.qweight.device.index, self.__dict__, self._gemm_ok, self._qweight_run,
-                                            self._g_idx_run, self._x_perm)
+                                            self.qweight.device.index, self.__dict__, self._gemm_ok, self._gemv_rows,
+                                            self._qweight_run, self._g_idx_run, self._x_perm)
         if plan is not None:
             self._native.set_gemv(rows, plan, plan._handle.value, plan._need)
 

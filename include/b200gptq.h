@@ -158,6 +158,7 @@ B200GPTQ_API int b200gptq_gemv_ex(const void* x, const int32_t* qweight, const i
  * and the library keeps no table).  The plan holds the layer's device pointers, not copies: the buffers must
  * outlive it and stay where they are.  A plan may be run from several threads and streams at once with
  * different workspaces.  plan_run has the semantics of b200gptq_gemv_tuned with the arguments given at creation.
+ * M may be up to 16 for a g_idx == NULL layer whose groups are whole 32-row blocks, otherwise up to 8.
  */
 typedef struct b200gptq_gemv_plan b200gptq_gemv_plan;
 B200GPTQ_API int b200gptq_gemv_plan_create(b200gptq_gemv_plan** out, const int32_t* qweight, const int32_t* qzeros,

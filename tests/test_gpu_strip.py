@@ -46,10 +46,30 @@ def test_gemv_vs_oracle(bits, K, N, gs, gather, M):
     run = lambda **kw: ops.gemv(x.to(DEV), d.qweight, d.qzeros, d.scales, None, bits, gs, bias=d.bias,
                                 x_perm=None if perm is None else perm.to(DEV), **kw)
     ref = O.forward_fp64(xg.numpy(), W, bias)
-    # fp32 accumulation and one fp16 rounding: the weights are exact, the sums of powers of two that 2 and 3 bits subtract
-    # are up to 2^10 times the inputs in fp32
+    # One fp16 rounding of the result, and the weights: the oracle rounds scale * (q - zero) to fp16, the kernel does not.  That
+    # is up to 2^-11 |w| each with independent signs, a standard deviation of 2^-11 / sqrt(3) * norm(x) * rms(w); the largest
+    # of 1e5 outputs is at 4.5 of them, and rms(w) is below a third of max |w| here: 2^-11 * norm(x) * max |w|.  The fp32
+    # sums (2 and 3 bits subtract sums of powers of two up to 2^10 times the inputs) stay far below that.
     norm = np.linalg.norm(xg.numpy().astype(np.float64), axis=1, keepdims=True) * np.abs(W.astype(np.float64)).max()
     for y in (run(), run(tuning=(2, 1))):       # eight warps and sixteen
         err = np.abs(y.cpu().numpy().astype(np.float64) - ref)
-        assert np.all(err <= 2.0 ** -10 * np.abs(ref) + 2e-4 * norm), err.max()
+        assert np.all(err <= 2.0 ** -10 * np.abs(ref) + 2.0 ** -11 * norm), err.max()
+    ops.check_status(DEV)
+
+
+@pytest.mark.parametrize("bits,K,N,gs,gather", [(2, 544, 96, 32, True), (3, 1152, 4832, 128, False), (3, 1184, 64, 64, True),
+                                                (4, 4096, 4800, 128, True), (4, 992, 32, 32, False), (8, 288, 9632, -1, False)])
+@pytest.mark.parametrize("M", [9, 16])
+def test_plan_of_nine_to_sixteen_rows_vs_oracle(bits, K, N, gs, gather, M):
+    layer = synth.make_layer(bits, K, N, gs, False, bias=True, seed=K + N + bits)
+    _, _, W = O.dequantize(layer.qweight.numpy(), layer.qzeros.numpy(), layer.scales.numpy(), layer.g_idx.numpy(), bits)
+    x = synth.make_x(M, K, seed=M)
+    perm = torch.randperm(K, generator=torch.Generator().manual_seed(K)).to(torch.int32) if gather else None
+    xg = x if perm is None else x[:, perm.long()]
+    d = layer.to(DEV)
+    plan = ops.GemvPlan(d.qweight, d.qzeros, d.scales, None, None if perm is None else perm.to(DEV), d.bias, M, bits, gs)
+    ref = O.forward_fp64(xg.numpy(), W, layer.bias.numpy())
+    norm = np.linalg.norm(xg.numpy().astype(np.float64), axis=1, keepdims=True) * np.abs(W.astype(np.float64)).max()
+    err = np.abs(plan.run(x.to(DEV)).cpu().numpy().astype(np.float64) - ref)
+    assert np.all(err <= 2.0 ** -10 * np.abs(ref) + 2.0 ** -11 * norm), err.max()
     ops.check_status(DEV)
