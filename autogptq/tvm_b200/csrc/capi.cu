@@ -37,7 +37,7 @@ size_t gemv_generic_workspace_bytes(int M, int K, int N);
 bool gemv_stream_supported(int M, int K, int N, int bits, int group_size);
 size_t gemv_stream_workspace_bytes(int M, int K, int N, int bits);
 size_t gemm_workspace_bytes(int M, int K, int N, int bits);
-void gemm_split_query(int M, int K, int N, int* splits, int* ctas_per_sm);
+void gemm_split_query(int M, int K, int N, int bits, int* splits, int* ctas_per_sm);
 int gemm_dispatch(const __half*, const int32_t*, const int32_t*, const __half*, const int32_t*, const int32_t*,
                   const __half*, __half*, int, int, int, int, int, void*, size_t, cudaStream_t);
 
@@ -163,9 +163,8 @@ int b200gptq_gemm_split(int M, int K, int N, int bits, int* splits, int* ctas_pe
     if (!splits || !ctas_per_sm) return B200GPTQ_ERR_NULL_POINTER;
     int group_size = -1;
     if (int st = check_layer(K, N, bits, &group_size)) return st;
-    if (bits != 3 && bits != 4) return B200GPTQ_ERR_BITS;
     if (M < 1) return B200GPTQ_ERR_SHAPE;
-    gemm_split_query(M, K, N, splits, ctas_per_sm);
+    gemm_split_query(M, K, N, bits, splits, ctas_per_sm);
     return B200GPTQ_OK;
 }
 
@@ -303,7 +302,6 @@ int b200gptq_gemm(const void* x, const int32_t* qweight, const int32_t* qzeros, 
                   int bits, int group_size, void* workspace, size_t workspace_bytes, void* stream) {
     if (!x || !qweight || !qzeros || !scales || !y) return B200GPTQ_ERR_NULL_POINTER;
     if (int st = check_layer(K, N, bits, &group_size)) return st;
-    if (bits != 3 && bits != 4) return B200GPTQ_ERR_BITS;
     if (M < 1) return B200GPTQ_ERR_SHAPE;
     // the kernel takes one group per aligned 32-row block: without a g_idx that holds only for such group sizes
     if (!g_idx && group_size % 32 != 0) return B200GPTQ_ERR_GROUPS;

@@ -1,0 +1,699 @@
+// Prefill dequant-GEMM for more than 64 rows of x (2- and 8-bit layers: any number): pairs of CTAs on one tcgen05 tile.
+//
+//   y[M, N] = x[M, K] @ W[K, N] (+ bias),   W[k, n] = scales[g, n] * (q[k, n] - zero[g, n]),  rounded once to fp16
+//
+// Like gemm.cu the product is computed transposed, y^T = W^T x^T, with the dequantised weights as the A operand in tensor
+// memory.  There one CTA took 128 columns x 256 rows and read all 256 rows of x itself: 1.6 GB of x through L2 for 2048 rows
+// of 4096 x 12288, 36 KB per 64-row k-tile against the 550 clk its products take, which is what bounded it (182 us; with
+// a quarter of the products 152, without the dequantisation 166).  Here two CTAs of a cluster share a 256-column tile
+// (tcgen05 cta_group::2): each holds and dequantises its own 128 columns and HALF of the rows of x.
+//
+//   warp 0      TMA: packed weights, scales and zero-points of 128 rows of K, into a ring of their own that runs ahead of
+//               the products as far as shared memory allows (they come from DRAM, x from L2)
+//   warp 1      TMA: this CTA's rows of x, into the stages; completion is counted in the first CTA of the pair
+//   warp 2      first CTA: issues tcgen05.mma for both (M = 256 columns, N = TN rows of x, K = 16); allocates tensor memory
+//   warps 4..11 epilogue: accumulators -> y
+//   warps 12..27  four groups of four that take 64-row k-tiles in turn: a thread owns one column, dequantises it to the exact
+//               fp16 values of the reference (auto_gptq/nn_modules/qlinear.py:242: one rounding) in the natural order of k and
+//               stores them into the stage's A buffer in tensor memory.  (A warp per 32-row block spent as many instructions
+//               on hand-overs as on weights: 790 clk per k-tile whatever the number of rows.)
+//
+// The pairs are persistent: the rings run on from one tile to the next, so only the drain of the accumulators stands
+// between two tiles (nothing, where two sets of accumulators fit: up to 128 rows).  A stage is released in both CTAs by one
+// multicast tcgen05.commit.  Every wait is bounded: on expiry the kernel raises a sticky status word, unwinds, frees its
+// tensor memory and returns.
+//
+// Replaces the TVM-generated wmma kernels src/kernels/gemm_kernel.cu:25-142 of the reference.
+#include <cuda.h>
+
+#include <mutex>
+
+#include "common.cuh"
+
+namespace b200gptq {
+
+namespace {
+
+constexpr int BN = 128;                  // columns per CTA
+constexpr int BK = 64;                   // rows of K per stage
+constexpr int kGroups = 4, kGroupWarps = 4;
+constexpr int kFirstEpiWarp = 4, kEpiWarps = 8, kFirstWeightWarp = kFirstEpiWarp + kEpiWarps;
+constexpr int kThreads = 32 * (kFirstWeightWarp + kGroups * kGroupWarps);
+constexpr int kMaxStages = 14, kMaxW = 16;
+constexpr int kTmemCols = 512;           // accumulators in columns [0, TN), 32 columns of A per stage behind them
+constexpr int kSmemMax = 222 * 1024;
+constexpr int kStatusWord = kMaxCounters - 1;
+constexpr int kMaxSplits = 4;
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ bool elect_one() {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok));
+    return ok != 0;
+}
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// On a barrier of the other CTA.  What it announces lies in tensor memory, ordered by the tcgen05 fences around it; no
+// ordinary memory is handed over, so the default scope serves (with .cluster scope on arrive and wait: 244 us instead of
+// 187 for 2048 rows of 4096 x 12288, a memory barrier and an L1 invalidation per hand-over).
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+__device__ __forceinline__ void mbar_expect(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(bar), "r"(parity), "r"(4000u) : "memory");
+    return ok != 0;
+}
+// Bounded wait: gives up after ~2e9 clocks or as soon as another warp of the CTA has.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+    if (mbar_try(bar, parity)) return true;
+    const long long t0 = clock64();
+    while (true) {
+        for (int i = 0; i < 8; ++i)
+            if (mbar_try(bar, parity)) return true;
+        if (*abort_flag) return false;
+        if (clock64() - t0 > 2000000000LL) { *abort_flag = 1; return false; }
+    }
+}
+__device__ __forceinline__ uint32_t in_cta(uint32_t local, uint32_t rank) {   // the same shared-memory offset in CTA `rank`
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tma_1d(uint32_t dst, const CUtensorMap* map, int x, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.1d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2}], [%3];"
+                 ::"r"(dst), "l"(map), "r"(x), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void tma_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
+}
+// into this CTA's shared memory, counted on a barrier of the pair's first CTA
+__device__ __forceinline__ void tma_2d_pair(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t cluster_bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+        ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(cluster_bar) : "memory");
+}
+__device__ __forceinline__ void mma_commit_pair(uint32_t bar) {   // arrives at this offset in both CTAs
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                 ::"r"(bar), "h"((unsigned short)3) : "memory");
+}
+__device__ __forceinline__ void mma_pair(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+}
+// (the registers pass through the wait, so that nothing reads them before it)
+__device__ __forceinline__ void tmem_wait_ld(uint32_t (&r)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+                 :: "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+        ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
+          "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
+}
+// K-major, 128-byte-swizzled operand tile: rows of 128 bytes, 8-row groups 1024 bytes apart.
+__device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr) {
+    uint64_t d = 0;
+    d |= (uint64_t)((saddr >> 4) & 0x3FFF);   // start address, 16-byte units
+    d |= (uint64_t)1 << 16;                    // leading byte offset (unused for swizzled K-major)
+    d |= (uint64_t)(1024 >> 4) << 32;          // stride byte offset: next 8-row group
+    d |= (uint64_t)1 << 46;                    // descriptor version of sm_100
+    d |= (uint64_t)2 << 61;                    // SWIZZLE_128B
+    return d;
+}
+
+__device__ __forceinline__ uint32_t lop3_and_or(uint32_t a, uint32_t mask, uint32_t magic) {
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(a), "r"(mask), "r"(magic));
+    return r;
+}
+__device__ __forceinline__ __half2 as_h2(uint32_t u) { return *reinterpret_cast<__half2*>(&u); }
+// fp16 exponent pattern that turns a field at bit p of a 16-bit half into 2^(10-p) + field
+__host__ __device__ constexpr uint32_t magic_at(int p) { return (uint32_t)(25 - p) << 10; }
+__host__ __device__ constexpr uint32_t magic2(int lo, int hi) { return magic_at(lo) | (magic_at(hi) << 16); }
+// 2^(10-lo) + z, 2^(10-hi) + z
+template <int LO, int HI>
+__device__ __forceinline__ __half2 offsets(__half2 z2) { return __hadd2(as_h2(magic2(LO, HI)), z2); }
+// (field + offset) pair -> scale * (field - zero): the subtraction is exact in fp16 and the product is rounded once
+__device__ __forceinline__ uint32_t finish(uint32_t biased, __half2 offset_plus_zero, __half2 scale2) {
+    const __half2 r = __hmul2(__hsub2(as_h2(biased), offset_plus_zero), scale2);
+    return *reinterpret_cast<const uint32_t*>(&r);
+}
+
+// One 32-row block of one column -> 16 pairs in the natural order of k.
+template <int BITS> struct Block;
+
+// Byte b of a word replicated into all four lanes: low nibble in the low half, high nibble in the high half.
+template <> struct Block<4> {
+    __device__ static __forceinline__ void run(const uint32_t (&w)[4], __half2 s2, __half2 z2, uint32_t (&out)[16]) {
+        const __half2 o = offsets<0, 4>(z2);
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+            out[i] = finish(lop3_and_or(__byte_perm(w[i >> 2], 0u, 0x1111u * (i & 3)), 0x00f0000fu, magic2(0, 4)), o, s2);
+    }
+};
+template <> struct Block<8> {
+    __device__ static __forceinline__ void run(const uint32_t (&w)[8], __half2 s2, __half2 z2, uint32_t (&out)[16]) {
+        const __half2 o = offsets<0, 0>(z2);
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+            out[i] = finish(__byte_perm(w[i >> 1], 0x64646464u, (i & 1) ? 0x4342 : 0x4140), o, s2);
+    }
+};
+template <> struct Block<2> {
+    __device__ static __forceinline__ void run(const uint32_t (&w)[2], __half2 s2, __half2 z2, uint32_t (&out)[16]) {
+        const __half2 o0 = offsets<0, 2>(z2), o1 = offsets<4, 6>(z2);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const uint32_t rep = __byte_perm(w[i >> 2], 0u, 0x1111u * (i & 3));     // four fields
+            out[2 * i] = finish(lop3_and_or(rep, 0x000c0003u, magic2(0, 2)), o0, s2);
+            out[2 * i + 1] = finish(lop3_and_or(rep, 0x00c00030u, magic2(4, 6)), o1, s2);
+        }
+    }
+};
+// Pair i sits at bits 6 i .. 6 i + 5 of the 96-bit run.  The two bytes around it are copied into both halves; where the
+// pair starts at bit 6 of a byte (every fourth) the run is shifted by 4 bits first.
+template <> struct Block<3> {
+    __device__ static __forceinline__ void run(const uint32_t (&w)[3], __half2 s2, __half2 z2, uint32_t (&out)[16]) {
+        const __half2 o0 = offsets<0, 3>(z2), o2 = offsets<2, 5>(z2), o4 = offsets<4, 7>(z2);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const int shift = (6 * i) % 8 == 6 ? 4 : 0, bit = 6 * i - shift, p = bit % 8;   // p = 0, 2 or 4
+            const int wi = bit / 32, by = (bit % 32) / 8;
+            const uint32_t lo = w[wi], hi = wi < 2 ? w[wi + 1] : 0u;
+            const uint32_t a = shift ? (bit % 32 + shift + 6 <= 32 ? lo >> 4 : __funnelshift_r(lo, hi, 4)) : lo;
+            // bytes by, by + 1 of (a, next word); pairs without a shift that cross into the next word start at byte 3
+            const uint32_t rep = __byte_perm(a, shift ? 0u : hi, by * 0x0101u + 0x1010u * (by + 1));
+            const uint32_t v = lop3_and_or(rep, (7u << p) | (7u << (p + 19)), p == 0 ? magic2(0, 3) : (p == 2 ? magic2(2, 5) : magic2(4, 7)));
+            out[i] = finish(v, p == 0 ? o0 : (p == 2 ? o2 : o4), s2);
+        }
+    }
+};
+
+__host__ __device__ constexpr int zero_words(int bits) { return bits % 4 == 0 ? 4 * bits : (4 * bits + 3 + 3) & ~3; }
+__host__ __device__ constexpr int w_unit_bytes(int bits) { return 4 * bits * BN * 4; }      // packed weights of 128 rows
+// a slot of the weight ring: packed rows | scales [group][column] | zero-point words of each group
+__host__ __device__ constexpr int w_slot_bytes(int bits, int rows_g) { return w_unit_bytes(bits) + rows_g * (BN * 2 + 128); }
+
+// Field of column `col` (0 .. 127) plus one, from words in shared memory.
+template <int BITS>
+__device__ __forceinline__ uint32_t zero_of(const uint8_t* row, int col) {
+    const int bit = BITS * col;
+    uint32_t v = row[bit >> 3];
+    if (BITS == 8) return v + 1u;
+    if (BITS == 3) v |= (uint32_t)row[(bit >> 3) + 1] << 8;
+    return ((v >> (bit & 7)) & ((1u << BITS) - 1u)) + 1u;
+}
+
+struct PairArgs {
+    int M, K, N, spg, groups_in_slot, TN, S, SW, acc_sets, splits;
+    int pairs, row_tiles, tiles;         // 256-column tiles, TN-row tiles, all tiles (with the runs of K)
+    unsigned int spg_inv;                // ceil(2^32 / spg), spg = 32-row blocks per group
+};
+
+template <int BITS>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
+                 const __grid_constant__ CUtensorMap tmap_s, const __grid_constant__ CUtensorMap tmap_z,
+                 const int32_t* __restrict__ g_idx, const int32_t* __restrict__ qzeros, const __half* __restrict__ scales,
+                 const __half* __restrict__ bias, __half* __restrict__ y, const PairArgs p, unsigned int* __restrict__ status,
+                 float* __restrict__ partial) {
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t raw = smem_u32(smem_raw), base = (raw + 1023u) & ~1023u;
+    uint8_t* base_ptr = smem_raw + (base - raw);
+    __shared__ __align__(8) uint64_t bars[2 * kMaxW + 2 * kMaxStages + 4];
+    __shared__ uint32_t tmem_base_holder;
+    __shared__ volatile int abort_flag;
+    __shared__ unsigned int arrived;
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = blockIdx.x & 1;             // cluster rank; 0 issues the products
+    const int K = p.K, N = p.N, TN = p.TN, S = p.S, SW = p.SW, TH = TN / 2;
+    const int RB = K / 32, KT_all = (K + BK - 1) / BK, U_all = (K + 127) / 128;
+    const int cluster = blockIdx.x >> 1, clusters = gridDim.x >> 1;
+    const uint32_t x_bytes = (uint32_t)TH * BK * 2;
+    const int w_slot = w_slot_bytes(BITS, p.groups_in_slot);
+    const uint32_t w_off = S * x_bytes;
+
+    const uint32_t bar_base = smem_u32(bars);
+    auto w_full = [&](int s) { return bar_base + 8u * s; };
+    auto w_empty = [&](int s) { return bar_base + 8u * (kMaxW + s); };
+    auto full = [&](int s) { return bar_base + 8u * (2 * kMaxW + s); };             // x of both CTAs and A of both CTAs
+    auto empty = [&](int s) { return bar_base + 8u * (2 * kMaxW + kMaxStages + s); };
+    auto acc_full = [&](int a) { return bar_base + 8u * (2 * kMaxW + 2 * kMaxStages + a); };
+    auto acc_empty = [&](int a) { return bar_base + 8u * (2 * kMaxW + 2 * kMaxStages + 2 + a); };
+
+    if (threadIdx.x == 0) {
+        abort_flag = 0;
+        for (int s = 0; s < SW; ++s) { mbar_init(w_full(s), 1); mbar_init(w_empty(s), 2 * kGroupWarps); }   // two k-tiles
+        for (int s = 0; s < S; ++s) {
+            mbar_init(full(s), 1 + 2 * kGroupWarps);     // the first CTA's expect_tx arrive, a group of weight warps in each
+            mbar_init(empty(s), 1);                      // tcgen05.commit
+        }
+        for (int a = 0; a < 2; ++a) { mbar_init(acc_full(a), 1); mbar_init(acc_empty(a), 2 * kEpiWarps); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 2) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
+                     ::"r"(smem_u32(&tmem_base_holder)), "r"((uint32_t)kTmemCols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    cluster_sync();                                      // barriers of both CTAs exist, tensor memory is allocated
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem_base = tmem_base_holder, tmem_a = tmem_base + (uint32_t)(p.acc_sets * TN);
+    asm volatile("griddepcontrol.launch_dependents;");
+    // what a preceding kernel may still be writing: x; what it may still be reading: y and the scratch
+    if (warp != 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+
+    // A tile: 256 columns x TN rows x a run of 128-row units.
+    struct Tile { int n0, m0, z, u0, u1, kt0, KT; };
+    auto tile_at = [&](int t) {
+        Tile v;
+        const int pr = t % p.pairs, r = t / p.pairs, row = r % p.row_tiles;
+        v.z = r / p.row_tiles;
+        v.n0 = (2 * pr + rank) * BN;
+        v.m0 = row * TN;
+        v.u0 = (int)(((long long)v.z * U_all) / p.splits);
+        v.u1 = (int)(((long long)(v.z + 1) * U_all) / p.splits);
+        v.kt0 = 2 * v.u0;
+        v.KT = min(2 * v.u1, KT_all) - v.kt0;
+        return v;
+    };
+    // group of a 32-row block without a division (140 clk each, in the one warp that feeds every k-tile)
+    auto group_at = [&](int rb) { return p.spg == 1 ? rb : (int)__umulhi((unsigned int)rb, p.spg_inv); };
+    const int zwords = N / 32 * BITS;
+
+    if (warp == 0) {
+        // ===== packed weights, scales, zero-points.  (With a g_idx the number of groups is not known here, so boxes could not
+        //       be clipped to the arrays: the weight warps read scales and zero-points themselves.) =====
+        const int rows_g = g_idx ? 0 : p.groups_in_slot;
+        const uint32_t tx = w_unit_bytes(BITS) + rows_g * (BN * 2 + zero_words(BITS) * 4);
+        int s = 0, round = 0;
+        bool ok = true;
+        for (int t = cluster; t < p.tiles && ok; t += clusters) {
+            const Tile v = tile_at(t);
+            const int zn = v.n0 / 32 * BITS;
+            for (int u = v.u0; u < v.u1; ++u) {
+                const int g0 = group_at(4 * u);
+                if (round > 0) ok = mbar_wait(w_empty(s), (round - 1) & 1, &abort_flag);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                if (elect_one()) {
+                    const uint32_t dst = base + w_off + s * w_slot, bar = w_full(s);
+                    mbar_expect(bar, tx);
+                    tma_2d(dst, &tmap_w, v.n0, u * 4 * BITS, bar);
+                    if (rows_g) tma_2d(dst + w_unit_bytes(BITS), &tmap_s, v.n0, g0, bar);
+                    for (int r = 0; r < rows_g; ++r)
+                        tma_1d(dst + w_unit_bytes(BITS) + rows_g * BN * 2 + r * 128, &tmap_z, ((g0 + r) * zwords + zn) & ~3, bar);
+                }
+                __syncwarp();
+                if (++s == SW) { s = 0; ++round; }
+            }
+        }
+    } else if (warp == 1) {
+        // ===== this CTA's rows of x =====
+        const uint32_t first_full = in_cta(full(0), 0);
+        int s = 0, round = 0;
+        bool ok = true;
+        for (int t = cluster; t < p.tiles && ok; t += clusters) {
+            const Tile v = tile_at(t);
+            for (int kt = 0; kt < v.KT; ++kt) {
+                if (round > 0) ok = mbar_wait(empty(s), (round - 1) & 1, &abort_flag);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                if (elect_one()) {
+                    if (rank == 0) mbar_expect(full(s), 2 * x_bytes);
+                    tma_2d_pair(base + s * x_bytes, &tmap_x, (v.kt0 + kt) * BK, v.m0 + rank * TH, first_full + 8u * s);
+                }
+                __syncwarp();
+                if (++s == S) { s = 0; ++round; }
+            }
+        }
+    } else if (warp == 2) {
+        // ===== products, for both CTAs =====
+        if (rank == 0 && elect_one()) {
+            const uint32_t idesc = (1u << 4) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(2 * BN >> 4) << 24);
+            bool ok = true;
+            int s = 0, round = 0, set = 0, used = 0;     // used: times the sets have gone round
+            for (int t = cluster; t < p.tiles && ok; t += clusters) {
+                const Tile v = tile_at(t);
+                if (used > 0) ok = mbar_wait(acc_empty(set), (used - 1) & 1, &abort_flag);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t acc = tmem_base + (uint32_t)(set * TN);
+                for (int kt = 0; kt < v.KT; ++kt) {
+                    ok = mbar_wait(full(s), round & 1, &abort_flag);
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint64_t bdesc = make_smem_desc(base + s * x_bytes);
+                    const uint32_t a_addr = tmem_a + 32u * s;
+#pragma unroll
+                    for (int k16 = 0; k16 < BK / 16; ++k16)
+                        mma_pair(acc, a_addr + 8u * k16, bdesc + 2u * k16, idesc, (kt > 0 || k16 > 0) ? 1u : 0u);
+                    mma_commit_pair(empty(s));
+                    if (++s == S) { s = 0; ++round; }
+                }
+                if (ok) mma_commit_pair(acc_full(set));
+                if (++set == p.acc_sets) { set = 0; ++used; }
+            }
+        }
+    } else if (warp >= kFirstWeightWarp) {
+        // ===== dequantisation =====
+        const int ww = warp - kFirstWeightWarp, quarter = warp & 3;   // tensor-memory lanes 32 * quarter .. + 31
+        const int wgroup = ww / kGroupWarps, col = 32 * quarter + lane;
+        const uint32_t lane_a = tmem_a + ((uint32_t)(32 * quarter) << 16);
+        const uint32_t first_full = in_cta(full(0), 0);
+        const bool early_words = BITS % 4 != 0 && (zwords & 3);       // zero-point boxes may start early
+        bool ok = true;
+        int s = wgroup % S, round = wgroup / S, ws = 0, wround = 0, at_unit = 0;   // slot ws holds the at_unit-th unit so far
+        int kt = wgroup, unit_base = 0;
+        for (int t = cluster; t < p.tiles && ok; t += clusters) {
+            const Tile v = tile_at(t);
+            for (; kt < v.KT; kt += kGroups) {
+                const int unit = unit_base + (kt >> 1);
+                ws += unit - at_unit;
+                at_unit = unit;
+                while (ws >= SW) { ws -= SW; ++wround; }
+                const int rb = 2 * (v.kt0 + kt);
+                __half sc[2];
+                uint32_t z[2];
+                if (g_idx) {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int grp = __ldg(g_idx + 32 * min(rb + h, RB - 1));
+                        sc[h] = __float2half(0.f);
+                        z[h] = 1;
+                        if (v.n0 + col < N) {
+                            sc[h] = __ldg(scales + (size_t)grp * N + v.n0 + col);
+                            z[h] = (uint32_t)zero_point<BITS>(qzeros + (size_t)grp * zwords, v.n0 + col);
+                        }
+                    }
+                }
+                ok = mbar_wait(w_full(ws), wround & 1, &abort_flag);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                const uint8_t* src = base_ptr + w_off + ws * w_slot;
+                const uint32_t* pw = reinterpret_cast<const uint32_t*>(src) + (kt & 1) * 2 * BITS * BN + col;
+                uint32_t w[2][BITS];
+#pragma unroll
+                for (int r = 0; r < 2 * BITS; ++r) w[r / BITS][r % BITS] = pw[r * BN];
+                if (!g_idx) {
+                    const int g0 = group_at(rb & ~3);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        // (one group in the slot: both blocks read the same constants)
+                        const int r = p.groups_in_slot == 1 ? 0 : min(group_at(rb + h) - g0, p.groups_in_slot - 1);
+                        const int early = early_words ? ((g0 + r) * zwords + v.n0 / 32 * BITS) & 3 : 0;
+                        sc[h] = reinterpret_cast<const __half*>(src + w_unit_bytes(BITS) + r * BN * 2)[col];
+                        z[h] = zero_of<BITS>(src + w_unit_bytes(BITS) + p.groups_in_slot * BN * 2 + r * 128 + 4 * early, col);
+                    }
+                }
+                __syncwarp();
+                // each slot is left by two k-tiles; the last k-tile of a tile may be alone in its slot
+                if (lane == 0 || (lane == 1 && kt + 1 == v.KT && !(kt & 1))) mbar_arrive(w_empty(ws));
+                if (round > 0) {
+                    ok = mbar_wait(empty(s), (round - 1) & 1, &abort_flag);   // the products that read this buffer have retired
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                }
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t out[16];
+                    Block<BITS>::run(w[h], __half2half2(sc[h]), __half2half2(__ushort2half_rn((unsigned short)z[h])), out);
+                    tmem_st16(lane_a + 32u * s + 16 * h, out);
+                }
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(first_full + 8u * s);
+                s += kGroups;
+                while (s >= S) { s -= S; ++round; }
+            }
+            kt -= v.KT;                                   // this group's first k-tile of the next tile
+            unit_base += v.u1 - v.u0;
+        }
+    } else if (warp >= kFirstEpiWarp) {
+        // ===== accumulators (lane = column, tensor-memory column = row of x) -> y =====
+        const int quarter = warp & 3, half = (warp - kFirstEpiWarp) >> 2, col = 32 * quarter + lane;
+        const uint32_t lane_acc = tmem_base + ((uint32_t)(32 * quarter) << 16);
+        const uint32_t first_empty = in_cta(acc_empty(0), 0);
+        const int M = p.M, rows_pad = p.row_tiles * TN;
+        bool ok = true;
+        int set = 0, used = 0;
+        for (int t = cluster; t < p.tiles; t += clusters) {
+            const Tile v = tile_at(t);
+            const int n = v.n0 + col;
+            const bool col_ok = v.n0 + 32 * quarter < N;     // (N is a multiple of 32: whole warps)
+            const float b = (bias && col_ok) ? __half2float(bias[n]) : 0.f;
+            // two lanes exchange values so that each stores a pair of columns of every other row
+            auto store_rows = [&](int m, float (&x)[16]) {
+                const int left = col_ok ? M - m - (lane & 1) : 0;
+                __half* dst = y + (size_t)(m + (lane & 1)) * N + (n & ~1);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float give = (lane & 1) ? x[2 * i] : x[2 * i + 1];
+                    const float got = __shfl_xor_sync(0xffffffffu, give, 1);
+                    const __half2 h = (lane & 1) ? __floats2half2_rn(got, x[2 * i + 1]) : __floats2half2_rn(x[2 * i], got);
+                    if (2 * i < left) *reinterpret_cast<__half2*>(dst) = h;
+                    dst += 2 * (size_t)N;
+                }
+            };
+            if (ok) ok = mbar_wait(acc_full(set), used & 1, &abort_flag);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            float* mine = partial + (size_t)v.z * rows_pad * N;
+            const int chunks = min(TN, M - v.m0 + 15) / 16;          // 16 rows each; the next one is loaded meanwhile
+            const uint32_t acc = lane_acc + (uint32_t)(set * TN);
+            uint32_t r[16], next[16] = {};
+            if (half < chunks) { tmem_ld16(acc + 16u * half, r); tmem_wait_ld(r); }
+#pragma unroll 1
+            for (int c = half; c < chunks; c += 2) {
+                if (c + 2 < chunks) tmem_ld16(acc + 16u * (c + 2), next);
+                const int m = v.m0 + 16 * c;
+                if (p.splits == 1) {
+                    float x[16];
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) x[i] = __uint_as_float(r[i]) + b;
+                    store_rows(m, x);
+                } else if (col_ok) {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i)
+                        if (m + i < M) mine[(size_t)(m + i) * N + n] = __uint_as_float(r[i]);
+                }
+                tmem_wait_ld(next);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) r[i] = next[i];
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(first_empty + 8u * set);
+            if (++set == p.acc_sets) { set = 0; ++used; }
+        }
+        if (p.splits > 1) __threadfence();               // the fp32 sums, before this CTA is counted in below
+    }
+
+    if (p.splits > 1) {
+        // ===== split K (one tile per pair): the last CTA of a tile to arrive adds the runs in order, with all its warps: a warp
+        //       takes rows, a lane four columns.  (One column per lane and only the epilogue warps: 13 us for 77 rows.)
+        //       Reached whatever happened before, so that the tile's counter returns to zero. =====
+        __syncthreads();
+        const Tile v = tile_at(cluster);
+        unsigned int* counter = status + (cluster % (p.pairs * p.row_tiles)) * 2 + rank;
+        if (threadIdx.x == 0) arrived = atomicAdd(counter, 1u);
+        __syncthreads();
+        if (arrived == (unsigned int)p.splits - 1u) {
+            __threadfence();
+            const int n = v.n0 + 4 * lane;
+            const int rows = n < N ? min(TN, p.M - v.m0) : 0;
+            float bf[4] = {0.f, 0.f, 0.f, 0.f};
+            if (bias && n < N)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) bf[c] = __half2float(bias[n + c]);
+            const size_t run = (size_t)p.row_tiles * TN * N;
+#pragma unroll 2
+            for (int i = warp; i < rows; i += kThreads / 32) {
+                const float* src = partial + (size_t)(v.m0 + i) * N + n;
+                float4 part[kMaxSplits];
+#pragma unroll
+                for (int z = 0; z < kMaxSplits; ++z)
+                    part[z] = z < p.splits ? __ldcg(reinterpret_cast<const float4*>(src + z * run)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                float4 x = part[0];
+#pragma unroll
+                for (int z = 1; z < kMaxSplits; ++z) { x.x += part[z].x; x.y += part[z].y; x.z += part[z].z; x.w += part[z].w; }
+                __half2 h[2] = {__floats2half2_rn(x.x + bf[0], x.y + bf[1]), __floats2half2_rn(x.z + bf[2], x.w + bf[3])};
+                *reinterpret_cast<uint2*>(y + (size_t)(v.m0 + i) * N + n) = *reinterpret_cast<const uint2*>(h);
+            }
+            if (threadIdx.x == 0) *counter = 0u;
+        }
+    }
+
+    // ===== teardown: every role arrives here, also after a timed-out wait; neither CTA leaves before the other has =====
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    __syncwarp();
+    cluster_sync();
+    if (threadIdx.x == 0 && abort_flag) atomicExch(status + kStatusWord, 1u);
+    if (warp == 2)
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)kTmemCols) : "memory");
+}
+
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiledFn encode_tiled_fn() {
+    static const EncodeTiledFn fn = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            p = nullptr;
+        return reinterpret_cast<EncodeTiledFn>(p);
+    }();
+    return fn;
+}
+
+// Rows of x per tile: the shortest sum over waves of (k-tiles x clocks per k-tile + drain of the accumulators, where there is
+// one set).  A k-tile costs its four products (TN / 2 clk each, measured) but no less than the weight warps take.
+int pick_rows(int M, int N, int K, int splits) {
+    const long long pairs = (N + 2 * BN - 1) / (2 * BN), slots = sm_count() / 2;
+    const long long kt = ((K + BK - 1) / BK + splits - 1) / splits;
+    long long best = -1;
+    int tn = 256;
+    for (int t = 256; t >= 32; t -= 32) {
+        if (splits > 1 && t < M && t < 256) break;       // (a tile per pair)
+        const long long rows = (M + t - 1) / t;
+        const long long per_kt = 2 * t + 8 > 370 ? 2 * t + 8 : 370;
+        const long long cost = ((pairs * rows * splits + slots - 1) / slots) * (kt * per_kt + (t > 128 ? 8 * t : 300)) + 12 * t;
+        if (best < 0 || cost < best) { best = cost; tn = t; }
+    }
+    return tn;
+}
+
+template <int BITS>
+int launch(const __half* x, const int32_t* qweight, const int32_t* qzeros, const __half* scales, const int32_t* g_idx,
+           const __half* bias, __half* y, int M, int K, int N, int group_size, int splits, unsigned int* status,
+           float* partial, cudaStream_t stream) {
+    const EncodeTiledFn encode = encode_tiled_fn();
+    if (!encode) { set_last_cuda_error((int)cudaErrorNotSupported); return B200GPTQ_ERR_CUDA; }
+    const int groups = (K + group_size - 1) / group_size;
+    PairArgs a = {};
+    a.M = M; a.K = K; a.N = N; a.splits = splits;
+    a.spg = group_size >= K ? (K + 31) / 32 : (group_size >= 32 ? group_size / 32 : 1);
+    a.spg_inv = (unsigned int)((0x100000000ULL + a.spg - 1) / a.spg);                 // (not used for 1)
+    a.groups_in_slot = a.spg % 4 == 0 || groups == 1 ? 1 : (a.spg == 1 ? 4 : (a.spg == 2 ? 2 : 3));
+    const int TN = a.TN = pick_rows(M, N, K, splits);
+    a.acc_sets = TN <= 128 ? 2 : 1;
+    const int x_stage = TN / 2 * BK * 2, w_slot = w_slot_bytes(BITS, a.groups_in_slot);
+    a.S = (kTmemCols - a.acc_sets * TN) / 32;
+    if (a.S > kMaxStages) a.S = kMaxStages;
+    a.SW = (kSmemMax - 1024 - a.S * x_stage) / w_slot;
+    if (a.SW > kMaxW) a.SW = kMaxW;
+    if (a.SW < 3) return B200GPTQ_ERR_TOO_LARGE;
+    const int smem = a.S * x_stage + a.SW * w_slot + 1024;
+    a.pairs = (N + 2 * BN - 1) / (2 * BN);
+    a.row_tiles = (M + TN - 1) / TN;
+    const long long tiles = (long long)a.pairs * a.row_tiles * splits;
+    if (tiles > 0x7fffffff || (splits > 1 && 2LL * a.pairs * a.row_tiles >= kMaxCounters - 1)) return B200GPTQ_ERR_TOO_LARGE;
+    a.tiles = (int)tiles;
+    auto map = [&](CUtensorMap* m, CUtensorMapDataType type, int rank, const void* ptr, const cuuint64_t* dims,
+                   const cuuint64_t* strides, const cuuint32_t* box, CUtensorMapSwizzle swizzle) {
+        const cuuint32_t estr[2] = {1, 1};
+        return encode(m, type, rank, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
+    CUtensorMap tx, tw, ts, tz;
+    const cuuint64_t xd[2] = {(cuuint64_t)K, (cuuint64_t)M}, xs[1] = {(cuuint64_t)K * 2};
+    const cuuint32_t xb[2] = {BK, (cuuint32_t)(TN / 2)};
+    const cuuint64_t wd[2] = {(cuuint64_t)N, (cuuint64_t)(K / 32 * BITS)}, ws[1] = {(cuuint64_t)N * 4};
+    const cuuint32_t wb[2] = {BN, 4 * BITS};
+    const cuuint64_t sd[2] = {(cuuint64_t)N, (cuuint64_t)groups}, ss[1] = {(cuuint64_t)N * 2};
+    const cuuint32_t sb[2] = {BN, (cuuint32_t)a.groups_in_slot};
+    const cuuint64_t zd[1] = {(cuuint64_t)groups * (N / 32 * BITS)};
+    const cuuint32_t zb[1] = {(cuuint32_t)zero_words(BITS)};
+    if (!map(&tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, x, xd, xs, xb, CU_TENSOR_MAP_SWIZZLE_128B) ||
+        !map(&tw, CU_TENSOR_MAP_DATA_TYPE_INT32, 2, qweight, wd, ws, wb, CU_TENSOR_MAP_SWIZZLE_NONE) ||
+        !map(&ts, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, scales, sd, ss, sb, CU_TENSOR_MAP_SWIZZLE_NONE) ||
+        !map(&tz, CU_TENSOR_MAP_DATA_TYPE_INT32, 1, qzeros, zd, ws, zb, CU_TENSOR_MAP_SWIZZLE_NONE)) {
+        set_last_cuda_error((int)cudaErrorInvalidValue);
+        return B200GPTQ_ERR_CUDA;
+    }
+    static std::once_flag once[64];
+    static int result[64];
+    int dev = 0;
+    B200GPTQ_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return B200GPTQ_ERR_TOO_LARGE;
+    std::call_once(once[dev], [dev] {
+        result[dev] = (int)cudaFuncSetAttribute(gemm_pair_kernel<BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
+    });
+    if (result[dev] != 0) { set_last_cuda_error(result[dev]); return B200GPTQ_ERR_CUDA; }
+    cudaLaunchConfig_t cfg = {};
+    const int pairs_of_sms = sm_count() / 2;
+    cfg.gridDim = dim3(2 * (a.tiles < pairs_of_sms ? a.tiles : pairs_of_sms));
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    B200GPTQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_pair_kernel<BITS>, tx, tw, ts, tz, g_idx, qzeros, scales, bias, y, a, status,
+                                         partial));
+    return B200GPTQ_OK;
+}
+
+}  // namespace
+
+// fp32 partial sums of a launch whose k-tiles are cut into `splits` runs
+size_t gemm_pair_partial_bytes(int M, int K, int N, int splits) {
+    if (splits == 1) return 0;
+    const int tn = pick_rows(M, N, K, splits);
+    return (size_t)splits * ((M + tn - 1) / tn * tn) * N * sizeof(float);
+}
+
+int gemm_pair_dispatch(const __half* x, const int32_t* qweight, const int32_t* qzeros, const __half* scales, const int32_t* g_idx,
+                       const __half* bias, __half* y, int M, int K, int N, int bits, int group_size, int splits,
+                       unsigned int* status, float* partial, cudaStream_t stream) {
+    switch (bits) {
+        case 2: return launch<2>(x, qweight, qzeros, scales, g_idx, bias, y, M, K, N, group_size, splits, status, partial, stream);
+        case 3: return launch<3>(x, qweight, qzeros, scales, g_idx, bias, y, M, K, N, group_size, splits, status, partial, stream);
+        case 4: return launch<4>(x, qweight, qzeros, scales, g_idx, bias, y, M, K, N, group_size, splits, status, partial, stream);
+        case 8: return launch<8>(x, qweight, qzeros, scales, g_idx, bias, y, M, K, N, group_size, splits, status, partial, stream);
+    }
+    return B200GPTQ_ERR_BITS;
+}
+
+}  // namespace b200gptq

@@ -1,5 +1,4 @@
 // Host side of the decode GEMV (gemv_strip.cuh): plan, tensor map, launch.
-#include <mutex>
 #include <new>
 
 #include "gemv_strip.cuh"
@@ -48,27 +47,6 @@ const void* strip_kernel(int bits, int sub, int mode, int nt, int T, int warps) 
     return nullptr;
 }
 
-int set_attrs_once() {
-    static std::once_flag once[64];
-    static int result[64];
-    int dev = 0;
-    B200GPTQ_CUDA_TRY(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64) return B200GPTQ_ERR_TOO_LARGE;
-    std::call_once(once[dev], [dev] {
-        cudaError_t e = cudaSuccess;
-        for (int b : {2, 3, 4, 8})
-            for (int sub : {1, 4})
-                for (int v = 0; v < 4; ++v)
-                    for (int i = 0; i < 8; ++i)
-                        if (const void* f = strip_kernel(b, sub, v == 3 ? kSeveral : v, v == 3 ? 2 : 1, 1 + i / 2, i & 1 ? 16 : 8))
-                            if (e == cudaSuccess)
-                                e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
-        result[dev] = (int)e;
-    });
-    if (result[dev] != 0) { set_last_cuda_error(result[dev]); return B200GPTQ_ERR_CUDA; }
-    return B200GPTQ_OK;
-}
-
 }  // namespace
 
 // Groups of whole 32-row blocks, up to 16 rows of x.
@@ -82,7 +60,6 @@ bool gemv_strip_gathers(int M, int K) { return (size_t)M * K * 2 <= kRawMax; }
 int gemv_strip_prepare(GemvStripPlan* p, const int32_t* qweight, const int32_t* qzeros,
                        const __half* scales, bool gather, int M, int K, int N, int bits, int group_size,
                        int ctas_per_sm, int xact) {
-    if (int st = set_attrs_once()) return st;
     p->M = M; p->K = K; p->N = N;
     StripPlan& s = p->plan;
     s.spg = group_size >= K ? K / 32 : group_size / 32;
@@ -142,6 +119,8 @@ int gemv_strip_prepare(GemvStripPlan* p, const int32_t* qweight, const int32_t* 
     p->smem = W * s.ring * (slot_bytes(bits, T) + const_bytes(bits, T, s.rows_g)) + c.fixed;
     p->kernel = strip_kernel(bits, sub, mode, nt, T, W);
     if (!p->kernel) return B200GPTQ_ERR_SHAPE;
+    // (only the one that is used: raising the limit loads a kernel, and there are a hundred)
+    B200GPTQ_CUDA_TRY(cudaFuncSetAttribute(p->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
     const EncodeTiledFn encode = encode_tiled_fn();
     if (!encode) { set_last_cuda_error((int)cudaErrorNotSupported); return B200GPTQ_ERR_CUDA; }
     auto map = [&](CUtensorMap* m, CUtensorMapDataType type, int rank, const void* base, const cuuint64_t* dims,

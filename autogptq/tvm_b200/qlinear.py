@@ -169,10 +169,10 @@ class QuantLinear(nn.Module):
         # multiple of 32, and a sorted layout whose groups do not fill whole blocks
         g_run = self._g_idx_run
         if g_run is None:
-            self._gemm_ok = self.bits in (3, 4) and self.groupsize % 32 == 0
+            self._gemm_ok = self.groupsize % 32 == 0
         else:
             b = g_run.view(K // 32, 32)
-            self._gemm_ok = self.bits in (3, 4) and bool((b == b[:, :1]).all().item())
+            self._gemm_ok = bool((b == b[:, :1]).all().item())
         # 9 to 16 rows: one pass of the streaming GEMV beats the tensor-core kernel's 16-row tile, whose weight warps are
         # the bottleneck (9216 x 9216, 3 bits: 20 against 40 us; 4096 x 4096, 4 bits: 8.3 against 16.6)
         whole_blocks = self._g_idx_run is None and (self.groupsize % 32 == 0 or self.groupsize >= K)
@@ -238,8 +238,7 @@ class QuantLinear(nn.Module):
             if self.bias is not None:
                 y = y + self.bias
         else:
-            # 2- and 8-bit layers, and layers whose groups cut through 32-row blocks, have no tensor-core kernel:
-            # GEMV passes of up to 8 rows
+            # layers whose groups cut through 32-row blocks have no tensor-core kernel: GEMV passes of up to 8 rows
             y = torch.empty((M, self.outfeatures), dtype=torch.float16, device=x2.device)
             for m0 in range(0, M, GEMV_MAX_M):
                 ops.gemv(x2[m0:m0 + GEMV_MAX_M], *args, out=y[m0:m0 + GEMV_MAX_M], **kw)

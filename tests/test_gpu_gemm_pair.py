@@ -1,0 +1,48 @@
+"""The tensor-core kernel for pairs of SMs (more than 64 rows; 2 and 8 bits at any number) at the edges of its split: column
+tiles with one CTA or part of one beyond the layer, cut k-tiles and units, one to four groups per unit, more tiles than pairs
+(persistent), one and two sets of accumulators, and K split over pairs."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+if torch.cuda.is_available():
+    from autogptq.tvm_b200 import ops, synth
+    DEV = torch.device("cuda:0")
+
+CASES = [
+    # bits, K, N, gs, M, gather
+    (4, 32, 32, 32, 65, False),           # half a k-tile, one quarter of one CTA
+    (4, 4128, 9632, 64, 700, False),      # odd number of k-tiles, several tiles per pair
+    (3, 1184, 288, 96, 257, True),        # three-block groups, zero-point rows that start inside a 16-byte word
+    (3, 2048, 19200, 128, 300, False),
+    (2, 1056, 96, 32, 20, True),
+    (2, 640, 4832, -1, 130, False),
+    (8, 2080, 4128, 128, 9, False),
+    (8, 96, 640, 32, 513, False),
+    (4, 11008, 4096, 64, 77, False),      # four runs of K
+    (8, 11008, 1056, 32, 128, True),
+]
+
+
+@pytest.mark.parametrize("bits,K,N,gs,M,gather", CASES)
+def test_gemm_against_dequantised_product(bits, K, N, gs, M, gather):
+    """The (bit-exact, separately tested) dequantised weights times x in fp32; twice, and with the groups as a g_idx, to the bit."""
+    d = synth.make_layer(bits, K, N, gs, False, bias=True, seed=K + N, device=DEV)
+    x = synth.make_x(M, K, seed=M, device=DEV)
+    perm = torch.randperm(K, device=DEV).to(torch.int32) if gather else None
+    run = lambda g: ops.gemm(x, d.qweight, d.qzeros, d.scales, g, bits, gs, bias=d.bias, x_perm=perm)
+    y = run(None)
+    _, W = ops.dequantize(d.qweight, d.qzeros, d.scales, d.g_idx, bits, gs, want_q=False)
+    xg = (x if perm is None else x[:, perm.long()]).double()
+    ref = xg @ W.double() + d.bias.double()
+    # fp32 accumulation of K exact products (rounded or truncated: 2^-23 each) and one fp16 rounding
+    bound = 2.0 ** -11 * ref.abs() + K * 2.0 ** -23 * (xg.abs() @ W.double().abs()) + 2.0 ** -24
+    assert bool(((y.double() - ref).abs() <= bound).all())
+    assert torch.equal(y, run(None)) and torch.equal(y, run(d.g_idx))
+    ops.check_status(DEV)
+
+
+def test_split_of_the_cases_above():
+    assert ops.gemm_split(77, 11008, 4096, 4)[0] == 4
+    assert ops.gemm_split(128, 11008, 1056, 8)[0] == 4
