@@ -17,22 +17,14 @@ __device__ __forceinline__ float warp_sum(float v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
-__device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
 
-// x[b,:] += add[b,:] (optional); h[b,:] = norm(x[b,:]) * w (+ beta).  rms != 0: RMSNorm, else LayerNorm.
-// One CTA of 256 threads per row; H is a multiple of 8.
-// Programmatic dependent launch: every kernel of the decode step is launched with the attribute that lets it
-// become resident while its predecessor in the stream is still running.  It reads and writes nothing of the
-// step's data before the predecessor has completed (griddepcontrol.wait), and only then lets its own successor
-// in (so at most two kernels of the chain are resident at a time).  Without the launch attribute both
-// instructions do nothing.
+// Programmatic dependent launch: every kernel of the decode step lets its successor become resident at once and reads and
+// writes nothing of the step's data before its predecessor has completed (griddepcontrol.wait; completion includes the
+// predecessor's own wait, so the chain is ordered).  Letting the successor in only after the own wait put its launch latency
+// on the path of every kernel of a step.  Without the launch attribute both instructions do nothing.
 __device__ __forceinline__ void pdl_enter() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 bool pdl_enabled() {
@@ -70,54 +62,69 @@ cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
-__global__ void __launch_bounds__(256)
+// x[b,:] += add[b,:] (optional); h[b,:] = norm(x[b,:]) * w (+ beta).  rms != 0: RMSNorm, else LayerNorm.
+// One CTA per row, eight values per thread and pass (P passes) kept in registers; H is a multiple of 8.  A row is 8..24 KB, so
+// this is one chain of latencies: w and beta are constants and loaded before the wait.
+template <int P>
+__global__ void __launch_bounds__(1024)
 add_norm_kernel(__half* __restrict__ x, const __half* __restrict__ add, const __half* __restrict__ w,
                 const __half* __restrict__ beta, __half* __restrict__ h, int H, float eps, int rms) {
-    extern __shared__ float row[];  // H floats
-    __shared__ float red[2][8];
+    __shared__ float red[2][32];
+    const int b = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
+    uint4 wv[P], bv[P], v[P];
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+        const int i = 8 * (tid + p * nt);
+        wv[p] = bv[p] = v[p] = make_uint4(0, 0, 0, 0);
+        if (i < H) {
+            wv[p] = *reinterpret_cast<const uint4*>(w + i);
+            if (beta) bv[p] = *reinterpret_cast<const uint4*>(beta + i);
+        }
+    }
     pdl_enter();
-    const int b = blockIdx.x, tid = threadIdx.x;
     __half* xr = x + (size_t)b * H;
     float s = 0.f, s2 = 0.f;
-    for (int i = tid * 8; i < H; i += 256 * 8) {
-        uint4 v = *reinterpret_cast<const uint4*>(xr + i);
-        __half2* p = reinterpret_cast<__half2*>(&v);
-        if (add) {
-            const uint4 a = *reinterpret_cast<const uint4*>(add + (size_t)b * H + i);
-            const __half2* q = reinterpret_cast<const __half2*>(&a);
 #pragma unroll
-            for (int k = 0; k < 4; ++k) p[k] = __hadd2(p[k], q[k]);
-            *reinterpret_cast<uint4*>(xr + i) = v;
-        }
+    for (int p = 0; p < P; ++p) {
+        const int i = 8 * (tid + p * nt);
+        if (i < H) {
+            v[p] = *reinterpret_cast<const uint4*>(xr + i);
+            __half2* q = reinterpret_cast<__half2*>(&v[p]);
+            if (add) {
+                const uint4 a = *reinterpret_cast<const uint4*>(add + (size_t)b * H + i);
+                const __half2* qa = reinterpret_cast<const __half2*>(&a);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const float2 f = __half22float2(p[k]);
-            row[i + 2 * k] = f.x; row[i + 2 * k + 1] = f.y;
-            s += f.x + f.y; s2 += f.x * f.x + f.y * f.y;
+                for (int k = 0; k < 4; ++k) q[k] = __hadd2(q[k], qa[k]);
+                *reinterpret_cast<uint4*>(xr + i) = v[p];
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float2 f = __half22float2(q[k]);
+                s += f.x + f.y; s2 += f.x * f.x + f.y * f.y;
+            }
         }
     }
     s = warp_sum(s); s2 = warp_sum(s2);
     if ((tid & 31) == 0) { red[0][tid >> 5] = s; red[1][tid >> 5] = s2; }
     __syncthreads();
-    float ts = 0.f, ts2 = 0.f;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) { ts += red[0][k]; ts2 += red[1][k]; }
+    const bool has = (tid & 31) < (nt + 31) / 32;
+    const float ts = warp_sum(has ? red[0][tid & 31] : 0.f), ts2 = warp_sum(has ? red[1][tid & 31] : 0.f);
     const float mean = rms ? 0.f : ts / H;
     const float var = rms ? ts2 / H : fmaxf(ts2 / H - mean * mean, 0.f);
     const float inv = rsqrtf(var + eps);
-    for (int i = tid * 8; i < H; i += 256 * 8) {
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+        const int i = 8 * (tid + p * nt);
+        if (i >= H) continue;
         uint4 o;
         __half2* po = reinterpret_cast<__half2*>(&o);
-        const uint4 wv = *reinterpret_cast<const uint4*>(w + i);
-        const __half2* pw = reinterpret_cast<const __half2*>(&wv);
-        uint4 bv = make_uint4(0, 0, 0, 0);
-        if (beta) bv = *reinterpret_cast<const uint4*>(beta + i);
-        const __half2* pb = reinterpret_cast<const __half2*>(&bv);
+        const __half2 *q = reinterpret_cast<const __half2*>(&v[p]), *pw = reinterpret_cast<const __half2*>(&wv[p]),
+                      *pb = reinterpret_cast<const __half2*>(&bv[p]);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const float2 fw = __half22float2(pw[k]), fb = __half22float2(pb[k]);
+            const float2 f = __half22float2(q[k]), fw = __half22float2(pw[k]), fb = __half22float2(pb[k]);
             // RMSNorm rounds the normalised value to fp16 before the weight, as the usual fp16 modules do
-            float a0 = (row[i + 2 * k] - mean) * inv, a1 = (row[i + 2 * k + 1] - mean) * inv;
+            float a0 = (f.x - mean) * inv, a1 = (f.y - mean) * inv;
             if (rms) { a0 = __half2float(__float2half_rn(a0)); a1 = __half2float(__float2half_rn(a1)); }
             po[k] = __floats2half2_rn(a0 * fw.x + fb.x, a1 * fw.y + fb.y);
         }
@@ -158,57 +165,64 @@ __global__ void rope_cache_kernel(const __half* __restrict__ qkv, const __half* 
     *reinterpret_cast<__half2*>(v_cache + c_off) = v2;
 }
 
-__device__ __forceinline__ float ld_cluster_f32(const float* local_ptr, uint32_t rank) {
+__device__ __forceinline__ void st_cluster_f32(const float* local_ptr, uint32_t rank, float v) {
     uint32_t remote;
-    float v;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
                  : "=r"(remote) : "r"((uint32_t)__cvta_generic_to_shared(local_ptr)), "r"(rank));
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
-    return v;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(v) : "memory");
 }
 
-// Single-query attention over the cache positions 0..pos[0] (inclusive).  A cluster of kAttnSplit CTAs
-// of 16 warps serves one (head, b); the 32-position chunks are dealt round-robin to all warps of the
-// cluster, so a prompt of ~2000 tokens is still one chunk per warp.  Scores: each lane owns ONE position
-// and reads that key row with 128-bit loads (all 32 rows in flight together); softmax statistics once per
-// 32 positions; values: each lane owns HD/32 dims, the 32 probabilities are broadcast by shuffle and the
-// 32 value rows are read coalesced.  Online softmax per warp; warps are combined through shared memory
-// and the CTAs of the cluster through distributed shared memory by the cluster's first CTA.
+// Single-query attention over the cache positions 0..pos[0] (inclusive).  A cluster of SPLIT CTAs of eight warps serves one
+// (head, b).  HD / 8 lanes share a position (16 bytes of its key and value each); a warp takes kAttnRows = 8 (16 for 64
+// dims) adjacent positions at a time, the blocks dealt round-robin to all warps of the cluster whatever the length is, so
+// that the keys AND values of a warp's first block are requested together with the position and the query: one round trip to
+// memory, not four (a lane per position for the scores, then the values eight at a time: 14.7 us of a Llama-7B layer's 57 at
+// 550 positions).  Rows past the position are loaded too (inside the cache) and given weight zero.  Each group of lanes keeps
+// its own online softmax; groups are combined by shuffles, warps through shared memory, and the CTAs push their results into
+// the first one's shared memory.
 //
 // STEP = true is the whole attention part of a decode step in one launch: `q` is then qkv[b, 3, heads, hd] of the
 // new token; every CTA rotates q and the new k itself (the same fp16 arithmetic as rope_cache_kernel), uses the new
 // k and v from shared memory for position pos[0], and the cluster's first CTA writes them into the caches for the
 // steps to come -- rope_cache_kernel + attn_decode_kernel without the launch in between.
-//
-// SPLIT CTAs (a cluster) of WARPS warps share one (sequence, head): the launcher picks the pair so that the whole grid
-// is resident at once (128 registers per thread: 16 warps per SM) -- 4 x 16 for a single sequence, down to one CTA
-// of 4 warps per (sequence, head) for a batch.
-template <int HD, bool STEP, int SPLIT, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
+constexpr int kAttnWarps = 8;
+template <int HD, bool STEP, int SPLIT>
+__global__ void __launch_bounds__(kAttnWarps * 32, 2)
 attn_decode_kernel(const __half* __restrict__ q, const __half* __restrict__ k_cache,
                    const __half* __restrict__ v_cache, const long long* __restrict__ pos, __half* __restrict__ out,
                    int heads, int max_seq, float scale, const __half* __restrict__ cos_t,
                    const __half* __restrict__ sin_t, int rope, __half* k_write, __half* v_write) {
-    // k_write / v_write (STEP): the same caches, for the one row this kernel writes; that row is never read through
-    // k_cache / v_cache here (position pos[0] is served from shared memory), so the read-only path stays valid.
-    constexpr int PER = HD / 32;
-    static_assert(WARPS * 32 >= HD / 2 && WARPS * 32 >= HD, "the prologue takes one thread per element");
+    // k_write / v_write (STEP): the same caches, for the one row this kernel writes; what is read of that row through
+    // k_cache / v_cache is not used (position pos[0] is served from shared memory).
+    constexpr int LP = HD / 8, GROUPS = 32 / LP, U = 4, ROWS = U * GROUPS;    // lanes per position; positions per block
+    static_assert(kAttnWarps * 32 >= HD, "one thread per element in the prologue and the combination");
     __shared__ __align__(16) __half q_sm[HD];
     __shared__ __align__(16) __half knew_sm[STEP ? HD : 8], vnew_sm[STEP ? HD : 8];
-    __shared__ float sm_m[WARPS], sm_l[WARPS], sm_acc[WARPS][HD];
-    __shared__ float cta_m, cta_l, cta_acc[HD];   // this CTA's partial result, read by the cluster's first CTA
-    pdl_enter();
+    __shared__ float sm_m[kAttnWarps], sm_l[kAttnWarps];
+    __shared__ __align__(16) float sm_acc[kAttnWarps][HD];
+    __shared__ float part_m[SPLIT], part_l[SPLIT], part_acc[SPLIT][HD];       // first CTA: results of the cluster's CTAs
     const int split = blockIdx.x % SPLIT, head = blockIdx.x / SPLIT, b = blockIdx.y;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = lane / LP, dim = (lane % LP) * 8;
+    if constexpr (SPLIT > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    pdl_enter();
+    const size_t base = ((size_t)b * heads + head) * (size_t)max_seq * HD;
+    const int stride = kAttnWarps * SPLIT * ROWS;
+    uint4 kv[U], vv[U];
+    auto request = [&](int t0) {
+#pragma unroll
+        for (int i = 0; i < U; ++i) {
+            const int t = min(t0 + i * GROUPS + grp, max_seq - 1);
+            kv[i] = *reinterpret_cast<const uint4*>(k_cache + base + (size_t)t * HD + dim);
+            vv[i] = *reinterpret_cast<const uint4*>(v_cache + base + (size_t)t * HD + dim);
+        }
+    };
+    int t0 = (warp * SPLIT + split) * ROWS;
+    if (t0 < max_seq) request(t0);
     const long long p64 = pos[0];
     if (STEP && (p64 < 0 || p64 >= max_seq)) return;   // a position outside the caches: refused by the whole cluster
     const int P = STEP ? (int)p64 : -1;                // the position whose key and value are in shared memory
     // positions served from the caches: 0..pos[0] (never past their end); STEP: 0..pos[0]-1, the new one comes last
     const int L = STEP ? P : (p64 < 0 ? 0 : (p64 >= max_seq ? max_seq : (int)p64 + 1));
-    const size_t base = ((size_t)b * heads + head) * (size_t)max_seq * HD;
     if constexpr (STEP) {
         if (threadIdx.x < HD / 2) {
             const int i = threadIdx.x;   // pair index
@@ -238,132 +252,139 @@ attn_decode_kernel(const __half* __restrict__ q, const __half* __restrict__ k_ca
         if (threadIdx.x < HD) q_sm[threadIdx.x] = q[((size_t)b * heads + head) * HD + threadIdx.x];
     }
     __syncthreads();
-    float acc[PER];
+    float qf[8], acc[8];
+    {
+        const uint4 raw = *reinterpret_cast<const uint4*>(q_sm + dim);
+        const __half2* h = reinterpret_cast<const __half2*>(&raw);
 #pragma unroll
-    for (int d = 0; d < PER; ++d) acc[d] = 0.f;
-    float m = -INFINITY, l = 0.f;
-    for (int t0 = (warp * SPLIT + split) * 32; t0 < L; t0 += WARPS * SPLIT * 32) {
-        const int t = t0 + lane;
-        // ---- score of this lane's position ----
-        float dot = -INFINITY;
-        if (t < L) {
-            const uint4* kp = reinterpret_cast<const uint4*>(k_cache + base + (size_t)t * HD);
-            uint4 kv[HD / 8];
-#pragma unroll
-            for (int i = 0; i < HD / 8; ++i) kv[i] = kp[i];
-            float s = 0.f;
-#pragma unroll
-            for (int i = 0; i < HD / 8; ++i) {
-                const __half2* k2 = reinterpret_cast<const __half2*>(&kv[i]);
-                const __half2* q2 = reinterpret_cast<const __half2*>(q_sm + 8 * i);
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float2 kf = __half22float2(k2[e]), qf = __half22float2(q2[e]);
-                    s = fmaf(kf.x, qf.x, s);
-                    s = fmaf(kf.y, qf.y, s);
-                }
-            }
-            dot = s * scale;
+        for (int e = 0; e < 4; ++e) {
+            const float2 f = __half22float2(h[e]);
+            qf[2 * e] = f.x; qf[2 * e + 1] = f.y;
         }
-        const float m_new = fmaxf(m, warp_max(dot));
-        const float pexp = (t < L) ? __expf(dot - m_new) : 0.f;
+    }
+    auto dot8 = [&](const uint4& raw) {     // over the lane's 8 dims, summed over the position's lanes
+        const __half2* h = reinterpret_cast<const __half2*>(&raw);
+        float s = 0.f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float2 f = __half22float2(h[e]);
+            s = fmaf(f.x, qf[2 * e], s);
+            s = fmaf(f.y, qf[2 * e + 1], s);
+        }
+#pragma unroll
+        for (int o = 1; o < LP; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        return s * scale;
+    };
+    auto add8 = [&](const uint4& raw, float p) {
+        const __half2* h = reinterpret_cast<const __half2*>(&raw);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float2 f = __half22float2(h[e]);
+            acc[2 * e] = fmaf(p, f.x, acc[2 * e]);
+            acc[2 * e + 1] = fmaf(p, f.y, acc[2 * e + 1]);
+        }
+    };
+    constexpr float kNone = -1e30f;         // below every score; finite, so that differences are
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc[e] = 0.f;
+    float m = kNone, l = 0.f;
+    while (t0 < L) {
+        uint4 kc[U], vc[U];
+#pragma unroll
+        for (int i = 0; i < U; ++i) { kc[i] = kv[i]; vc[i] = vv[i]; }
+        const int t = t0 + grp;
+        t0 += stride;
+        if (t0 < L) request(t0);            // the next block is on its way while this one is worked on
+        float sc[U], m_new = m;
+#pragma unroll
+        for (int i = 0; i < U; ++i) {
+            sc[i] = dot8(kc[i]);
+            if (t + i * GROUPS < L) m_new = fmaxf(m_new, sc[i]);
+        }
         const float corr = __expf(m - m_new);
-        l = l * corr + warp_sum(pexp);
-        m = m_new;
+        l *= corr;
 #pragma unroll
-        for (int d = 0; d < PER; ++d) acc[d] *= corr;
-        // ---- values: lanes own dims, positions are walked together ----
-        const int n = min(32, L - t0);
-        const __half* vp = v_cache + base + (size_t)t0 * HD + lane * PER;
-#pragma unroll 8
-        for (int i = 0; i < n; ++i) {
-            const float p = __shfl_sync(0xffffffffu, pexp, i);
-            if constexpr (PER == 4) {
-                const uint2 raw = *reinterpret_cast<const uint2*>(vp + (size_t)i * HD);
-                const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&raw.x));
-                const float2 c = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
-                acc[0] = fmaf(p, a.x, acc[0]); acc[1] = fmaf(p, a.y, acc[1]);
-                acc[2] = fmaf(p, c.x, acc[2]); acc[3] = fmaf(p, c.y, acc[3]);
-            } else {
-                const float2 a = __half22float2(*reinterpret_cast<const __half2*>(vp + (size_t)i * HD));
-                acc[0] = fmaf(p, a.x, acc[0]); acc[1] = fmaf(p, a.y, acc[1]);
+        for (int e = 0; e < 8; ++e) acc[e] *= corr;
+#pragma unroll
+        for (int i = 0; i < U; ++i)
+            if (t + i * GROUPS < L) {
+                const float p = __expf(sc[i] - m_new);
+                l += p;
+                add8(vc[i], p);
             }
-        }
+        m = m_new;
     }
     if (STEP && split == 0 && warp == 0) {
-        // the new position: key and value are in shared memory; one more step of the online softmax for this warp
-        float part = 0.f;
+        // the new position: key and value are in shared memory; one more step of the online softmax for the first group
+        const float s = dot8(*reinterpret_cast<const uint4*>(knew_sm + dim));
+        if (grp == 0) {
+            const float m_new = fmaxf(m, s), p = __expf(s - m_new), corr = __expf(m - m_new);
+            l = l * corr + p;
+            m = m_new;
 #pragma unroll
-        for (int d = 0; d < PER; ++d)
-            part = fmaf(__half2float(knew_sm[lane * PER + d]), __half2float(q_sm[lane * PER + d]), part);
-        const float dot = warp_sum(part) * scale;
-        const float m_new = fmaxf(m, dot);
-        const float pexp = __expf(dot - m_new), corr = __expf(m - m_new);
-        l = l * corr + pexp;
-        m = m_new;
-#pragma unroll
-        for (int d = 0; d < PER; ++d) acc[d] = fmaf(pexp, __half2float(vnew_sm[lane * PER + d]), acc[d] * corr);
-    }
-    if (lane == 0) { sm_m[warp] = m; sm_l[warp] = l; }
-#pragma unroll
-    for (int d = 0; d < PER; ++d) sm_acc[warp][lane * PER + d] = acc[d];
-    __syncthreads();
-    if (warp == 0) {   // combine the 16 warps of this CTA
-        float gm = -INFINITY;
-#pragma unroll
-        for (int w = 0; w < WARPS; ++w) gm = fmaxf(gm, sm_m[w]);
-        float gl = 0.f, wgt[WARPS];
-#pragma unroll
-        for (int w = 0; w < WARPS; ++w) {
-            wgt[w] = (sm_m[w] == -INFINITY) ? 0.f : __expf(sm_m[w] - gm);
-            gl += sm_l[w] * wgt[w];
+            for (int e = 0; e < 8; ++e) acc[e] *= corr;
+            add8(*reinterpret_cast<const uint4*>(vnew_sm + dim), p);
         }
-        if (lane == 0) { cta_m = gm; cta_l = gl; }
+    }
+    // ---- the warp's groups ----
+    float gm = m;
 #pragma unroll
-        for (int d = 0; d < PER; ++d) {
-            float v = 0.f;
+    for (int o = LP; o < 32; o <<= 1) gm = fmaxf(gm, __shfl_xor_sync(0xffffffffu, gm, o));
+    const float wgt = __expf(m - gm);
+    l *= wgt;
 #pragma unroll
-            for (int w = 0; w < WARPS; ++w) v += sm_acc[w][lane * PER + d] * wgt[w];
-            cta_acc[lane * PER + d] = v;
+    for (int e = 0; e < 8; ++e) acc[e] *= wgt;
+#pragma unroll
+    for (int o = LP; o < 32; o <<= 1) {
+        l += __shfl_xor_sync(0xffffffffu, l, o);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], o);
+    }
+    if (lane == 0) { sm_m[warp] = gm; sm_l[warp] = l; }
+    if (grp == 0) {
+        *reinterpret_cast<float4*>(&sm_acc[warp][dim]) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+        *reinterpret_cast<float4*>(&sm_acc[warp][dim + 4]) = make_float4(acc[4], acc[5], acc[6], acc[7]);
+    }
+    __syncthreads();
+    // ---- the CTA's warps: one dim per thread ----
+    const int d = threadIdx.x;
+    float cm = kNone, cl = 0.f, ca = 0.f;
+#pragma unroll
+    for (int w = 0; w < kAttnWarps; ++w) cm = fmaxf(cm, sm_m[w]);
+    if (d < HD) {
+#pragma unroll
+        for (int w = 0; w < kAttnWarps; ++w) {
+            const float e = __expf(sm_m[w] - cm);
+            cl += sm_l[w] * e;
+            ca += sm_acc[w][d] * e;
         }
     }
     if constexpr (SPLIT == 1) {
-        __syncwarp();
-        if (warp == 0) {
-#pragma unroll
-            for (int d = 0; d < PER; ++d)
-                out[((size_t)b * heads + head) * HD + lane * PER + d] = __float2half_rn(cta_acc[lane * PER + d] / cta_l);
-        }
+        if (d < HD) out[((size_t)b * heads + head) * HD + d] = __float2half_rn(ca / cl);
         return;
-    }
-    cluster_sync_all();   // every CTA's (cta_m, cta_l, cta_acc) is visible to the cluster
-    if (split == 0 && warp == 0) {
-        float pm[SPLIT], pl[SPLIT], pa[SPLIT][PER];
-#pragma unroll
-        for (int r = 0; r < SPLIT; ++r) {   // all remote reads in flight together
-            pm[r] = ld_cluster_f32(&cta_m, r);
-            pl[r] = ld_cluster_f32(&cta_l, r);
-#pragma unroll
-            for (int d = 0; d < PER; ++d) pa[r][d] = ld_cluster_f32(&cta_acc[lane * PER + d], r);
+    } else {
+        // ---- the cluster's CTAs: pushed into the first one, which the barrier's first phase has shown to be running ----
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (d < HD) {
+            st_cluster_f32(&part_acc[split][d], 0u, ca);
+            if (d == 0) { st_cluster_f32(&part_m[split], 0u, cm); st_cluster_f32(&part_l[split], 0u, cl); }
         }
-        float gm = -INFINITY;
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        if (split != 0) return;
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (d < HD) {
+            float tm = kNone, tl = 0.f, ta = 0.f;
 #pragma unroll
-        for (int r = 0; r < SPLIT; ++r) gm = fmaxf(gm, pm[r]);
-        float gl = 0.f, wgt[SPLIT];
+            for (int r = 0; r < SPLIT; ++r) tm = fmaxf(tm, part_m[r]);
 #pragma unroll
-        for (int r = 0; r < SPLIT; ++r) {
-            wgt[r] = (pm[r] == -INFINITY) ? 0.f : __expf(pm[r] - gm);
-            gl += pl[r] * wgt[r];
-        }
-#pragma unroll
-        for (int d = 0; d < PER; ++d) {
-            float v = 0.f;
-#pragma unroll
-            for (int r = 0; r < SPLIT; ++r) v += pa[r][d] * wgt[r];
-            out[((size_t)b * heads + head) * HD + lane * PER + d] = __float2half_rn(v / gl);
+            for (int r = 0; r < SPLIT; ++r) {
+                const float e = __expf(part_m[r] - tm);
+                tl += part_l[r] * e;
+                ta += part_acc[r][d] * e;
+            }
+            out[((size_t)b * heads + head) * HD + d] = __float2half_rn(ta / tl);
         }
     }
-    cluster_sync_all();   // keep every CTA's shared memory alive until it has been read
 }
 
 // act[b, i] = silu(u[b, i]) * u[b, I + i]  (gated != 0)   or   relu(u[b, i])  (gated == 0)
@@ -528,22 +549,22 @@ pick_final_kernel(const __half* __restrict__ slots, int world, long long* __rest
 using namespace b200gptq;
 
 namespace {
-// One launch of the attention kernel.  A (sequence, head) gets as many warps as keep the whole grid resident at once:
-// the kernel takes 128 registers per thread, so an SM holds 16 warps.
+// One launch of the attention kernel.  A (sequence, head) gets up to eight CTAs, as many as keep the whole grid resident
+// (two per SM) and as have a block of positions for each of their warps.
 template <int HD, bool STEP>
 cudaError_t launch_attention(const __half* q, const __half* k_cache, const __half* v_cache, const long long* pos,
                              __half* out, int batch, int heads, int max_seq, float scale, const __half* cos_t,
                              const __half* sin_t, int rope, __half* k_write, __half* v_write, void* stream) {
-    const long long pairs = (long long)batch * heads;
-    const long long warps_each = (16LL * sm_count()) / pairs;
-#define B200GPTQ_ATTN(SPLIT, WARPS)                                                                                    \
-    launch_pdl(attn_decode_kernel<HD, STEP, SPLIT, WARPS>, dim3(heads * SPLIT, batch), dim3(WARPS * 32), 0, stream,    \
+    const long long pairs = (long long)batch * heads, slots = 2LL * sm_count();
+    const int per_cta = kAttnWarps * 4 * 32 / (HD / 8);
+    auto fits = [&](int split) { return pairs * split <= slots && max_seq > (split / 2) * per_cta; };
+#define B200GPTQ_ATTN(SPLIT)                                                                                           \
+    launch_pdl(attn_decode_kernel<HD, STEP, SPLIT>, dim3(heads * SPLIT, batch), dim3(kAttnWarps * 32), 0, stream,      \
                SPLIT, q, k_cache, v_cache, pos, out, heads, max_seq, scale, cos_t, sin_t, rope, k_write, v_write)
-    if (warps_each >= 64) return B200GPTQ_ATTN(4, 16);
-    if (warps_each >= 32) return B200GPTQ_ATTN(4, 8);
-    if (warps_each >= 16) return B200GPTQ_ATTN(4, 4);
-    if (warps_each >= 8) return B200GPTQ_ATTN(1, 8);
-    return B200GPTQ_ATTN(1, 4);
+    if (fits(8)) return B200GPTQ_ATTN(8);
+    if (fits(4)) return B200GPTQ_ATTN(4);
+    if (fits(2)) return B200GPTQ_ATTN(2);
+    return B200GPTQ_ATTN(1);
 #undef B200GPTQ_ATTN
 }
 }  // namespace
@@ -554,10 +575,13 @@ B200GPTQ_API int b200gptq_add_norm(void* x, const void* add, const void* w, cons
                                    int H, float eps, int rms, void* stream) {
     if (!x || !w || !h) return B200GPTQ_ERR_NULL_POINTER;
     if (rows <= 0 || H <= 0 || H % 8 != 0 || H > 12288) return B200GPTQ_ERR_SHAPE;
-    B200GPTQ_CUDA_TRY(launch_pdl(add_norm_kernel, dim3(rows), dim3(256), H * sizeof(float), stream, 1,
-                                 static_cast<__half*>(x), static_cast<const __half*>(add),
-                                 static_cast<const __half*>(w), static_cast<const __half*>(beta),
-                                 static_cast<__half*>(h), H, eps, rms));
+    const int threads = H >= 8192 ? 1024 : (H / 8 + 31) / 32 * 32;
+    auto launch = [&](auto* kernel) {
+        return launch_pdl(kernel, dim3(rows), dim3(threads), 0, stream, 1, static_cast<__half*>(x),
+                          static_cast<const __half*>(add), static_cast<const __half*>(w), static_cast<const __half*>(beta),
+                          static_cast<__half*>(h), H, eps, rms);
+    };
+    B200GPTQ_CUDA_TRY(H <= 8192 ? launch(add_norm_kernel<1>) : launch(add_norm_kernel<2>));
     return B200GPTQ_OK;
 }
 
