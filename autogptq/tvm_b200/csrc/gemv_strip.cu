@@ -82,10 +82,9 @@ int gemv_strip_prepare(GemvStripPlan* p, const int32_t* qweight, const int32_t* 
     s.rows_g = sub == 1 ? 1 : (s.spg == 1 ? 4 : (s.spg == 2 ? 2 : 3));
     // Strips of a pass for W warps: a unit costs about half a strip's work on top of its strips, and the last pass is a whole
     // one.  The rings take at least two slots and what is left of the shared memory.
-    struct Choice { int W, T, ring, fixed, kept; };
+    struct Choice { int W, T, ring, fixed, kept, cost; };
     auto choose = [&](int W) {
-        Choice c = {W, 0, 0, 0, 0};
-        int best = 1 << 30;
+        Choice c = {W, 0, 0, 0, 0, 1 << 30};
         // (a gather works from a copy of x that the sums overwrite: it needs every unit's x kept)
         for (int kept = 1; kept >= (mode == kSeveral && !gather ? 0 : 1) && !c.T; --kept)
             for (int t = 1; t <= tmax && t <= s.per_cta; ++t) {
@@ -95,18 +94,19 @@ int gemv_strip_prepare(GemvStripPlan* p, const int32_t* qweight, const int32_t* 
                             : (mode == kOne ? s.units * kUnit * 2 : (kept ? s.units : 2 * W) * M * kXPitch * 2);
                 const int f = x + (sums > copy ? sums : copy) + 1024, r = (kSmemMax - f) / (W * slot);
                 const int cost = ((s.per_cta + t - 1) / t) * (2 * t + 1);
-                if (f < kSmemMax && r >= 2 && cost <= best) { best = cost; c = {W, t, r, f, kept}; }
+                if (f < kSmemMax && r >= 2 && cost <= c.cost) c = {W, t, r, f, kept, cost};
             }
         return c;
     };
     // Sixteen warps hide the latency of a unit better (4096 x 4096, 4 bits: 3.9 against 4.4 us, 11008 x 4096: 7.8 against
-    // 9.8), but their rings may only hold narrower passes that repeat strips (4096 x 12288: 8.1 against 6.2), and short K
-    // leaves some idle.  Sixteen rows of x take more than half of a thread's registers.
+    // 9.8), but their rings may only hold narrow passes (4096 x 12288: 8.1 against 6.2, and 12 % of a Llama-7B step), short K
+    // leaves some idle and a long row of x leaves their rings little room (36864 x 9216, 3 bits: 47 against 43).  Sixteen rows
+    // of x take more than half of a thread's registers.
     Choice c = choose(8);
     if (nt == 1 && ctas_per_sm <= 1) {
         const Choice w = choose(16);
-        auto work = [&](const Choice& v) { return (s.per_cta + v.T - 1) / v.T * v.T; };
-        if (w.T && (ctas_per_sm == 1 || !c.T || (s.units >= 16 && work(w) <= work(c)))) c = w;
+        const bool pays = s.units >= 16 && 10 * w.cost <= 11 * c.cost && (mode != kOne || K <= 16384);
+        if (w.T && (ctas_per_sm == 1 || !c.T || pays)) c = w;
     }
     if (!c.T) return B200GPTQ_ERR_TOO_LARGE;
     const int W = c.W, T = c.T;

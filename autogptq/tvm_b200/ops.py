@@ -366,6 +366,17 @@ def rope_cache(qkv, cos, sin, pos, q_out, k_cache, v_cache, heads: int, hd: int,
     return q_out
 
 
+def rope_prompt(qkv, cos, sin, q_out, k_cache, v_cache, seq: int, heads: int, hd: int, rope: bool):
+    """:func:`rope_cache` for a whole prompt: ``qkv`` ``[B * seq, 3*heads*hd]`` of tokens 0 .. seq-1 -> rotated ``q_out``
+    ``[B, seq, heads, hd]`` and the caches (``b200gptq_rope_prompt``)."""
+    B, max_seq = k_cache.shape[0], k_cache.shape[2]
+    with torch.cuda.device(qkv.device):
+        st = _lib.lib.b200gptq_rope_prompt(_ptr(qkv), _ptr(cos), _ptr(sin), _ptr(q_out), _ptr(k_cache), _ptr(v_cache), B, seq,
+                                           heads, hd, max_seq, 1 if rope else 0, _stream(qkv.device))
+    _lib.check(st, "b200gptq_rope_prompt")
+    return q_out
+
+
 def attn_decode(q, k_cache, v_cache, pos, out, heads: int, hd: int):
     B, max_seq = k_cache.shape[0], k_cache.shape[2]
     with torch.cuda.device(q.device):

@@ -359,6 +359,8 @@ B200GPTQ_API int b200gptq_tp_probe(const void* device_ptr, unsigned int* host_ou
  *   b200gptq_add_norm     x[rows,H] += add (nullable); h = RMSNorm(x)*w (rms != 0) or LayerNorm(x)*w + beta
  *   b200gptq_rope_cache   one new token per sequence: qkv[b,3,heads,hd] -> rotated q_out[b,heads,hd]; rotated k
  *                         and v written at position pos[0] of the caches [b,heads,max_seq,hd]; rope == 0: no rotation
+ *   b200gptq_rope_prompt  the same for a whole prompt of `seq` tokens at positions 0 .. seq-1: qkv[b,seq,3,heads,hd] ->
+ *                         q_out[b,seq,heads,hd] and the caches; hd a multiple of 8
  *   b200gptq_attn_decode  out[b,heads*hd] = softmax(q k^T * scale) v over cache positions 0..pos[0]; hd in {64,128}
  *   b200gptq_attn_step    b200gptq_rope_cache followed by b200gptq_attn_decode as ONE launch (same caches bit for bit,
  *                         same output up to the order of the softmax accumulation): rotates
@@ -372,6 +374,9 @@ B200GPTQ_API int b200gptq_add_norm(void* x, const void* add, const void* w, cons
 B200GPTQ_API int b200gptq_rope_cache(const void* qkv, const void* cos_t, const void* sin_t, const void* pos,
                                      void* q_out, void* k_cache, void* v_cache, int batch, int heads, int hd,
                                      int max_seq, int rope, void* stream);
+B200GPTQ_API int b200gptq_rope_prompt(const void* qkv, const void* cos_t, const void* sin_t, void* q_out, void* k_cache,
+                                      void* v_cache, int batch, int seq, int heads, int hd, int max_seq, int rope,
+                                      void* stream);
 B200GPTQ_API int b200gptq_attn_decode(const void* q, const void* k_cache, const void* v_cache, const void* pos,
                                       void* out, int batch, int heads, int hd, int max_seq, float scale,
                                       void* stream);
