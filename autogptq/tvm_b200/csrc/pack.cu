@@ -66,16 +66,27 @@ int launch_pack(const int32_t* vals, int R, int C, int32_t* out, cudaStream_t st
 //
 // As a chain of framework kernels this was eleven launches with five fp32 [K, N] intermediates: 1.0 ms for
 // 4096 x 11008; the bound is one read of the weight and one write of the words, 17 us there.  A CTA takes 32 output
-// columns (rows of `weight`) and a part of K: 256 k of every row are loaded with coalesced 16-byte reads into shared
-// memory, a thread then owns one column and one 32-row block (128-bit reads, rows 16 bytes apart in banks) and writes
-// its words, 128 bytes per warp and word-row.  (zero * scale, 1 / scale) of the 32 columns x all groups sit in shared
-// memory, column fastest, so that a look-up by any g_idx is one conflict-free 8-byte read.
+// columns (rows of `weight`) and a part of K: 256 k of every row come into shared memory with coalesced 16-byte
+// asynchronous copies, the next 256 while these are packed (57 us for 4096 x 11008 when a chunk's copy and its packing
+// took turns).  A thread then owns one column and one 32-row block (128-bit reads, rows 16 bytes apart in banks) and
+// writes its words, 128 bytes per warp and word-row.  (zero * scale, 1 / scale) of the 32 columns x all groups sit in
+// shared memory, column fastest, so that a look-up by any g_idx is one conflict-free 8-byte read; the rows are one entry
+// longer than the columns, so that the table is written without conflicts from coalesced reads of [N, G] too.  scales and
+// qzeros are left to CTAs of their own.  4096 x 11008, 4 bits, groups of 128 in act-order: 35 us; in order, where a row
+// block is one group and needs no look-ups, 31 us.
 //
-// An IEEE division per element would be most of the arithmetic.  t = a * (1 / s) is within |t| * 2^-22 of the rounded
-// quotient (two roundings of 2^-24 and the quotient's own), so rounding t gives the same integer unless t lies that
-// close to a half; a 32-row block with such an element (or with a NaN, an infinity, |t| >= 2^20) is redone with the
-// division.  Quantised weights are integer multiples of the scale up to rounding, so that is rare.
-constexpr int kPackCols = 32, kPackChunk = 256, kPackThreads = 256;
+// What remains is the start of a CTA (its table) and the instructions of an element, 20 of them once (25 us at full issue):
+// - No IEEE division.  With r = 1 / s rounded, a * r is within a relative 2^-24 of a / s and the rounded quotient within
+//   another, so for 0 <= q < 2^bits rounding a * r gives the integer that rounding the quotient gives unless a * r lies within
+//   2^bits * 2^-22 of a half.  u = a * r + 1.5 * 2^23 in one fma is that integer in the low bits of a float; d, also one fma,
+//   the rest.
+// - A field is added to its word as (bits of u) << position, what 1.5 * 2^23 leaves there is a constant of the word.  That
+//   takes 0 <= q < 2^bits: the upper bits of all u's or'ed and and'ed are then those of 1.5 * 2^23.  (So a NaN or an
+//   infinity is seen too.)
+// A 32-row block with an element close to a half or out of range is redone with the division and the unmasked insert.
+// Quantised weights are multiples of the scale within the range up to rounding, so that is rare.
+constexpr int kPackCols = 32, kPackChunk = 256, kPackThreads = 256, kPackPitch = kPackCols + 1;
+constexpr int kPackCtas = 5;                  // per SM: what the registers and two tiles of fp16 allow
 constexpr int kPackTableMax = 128 * 1024;     // bytes of the table; more groups are read from global memory
 
 template <typename T> struct PackIn;
@@ -95,90 +106,180 @@ __device__ __forceinline__ void pack_insert(uint32_t (&w)[BITS], int j, uint32_t
     }
 }
 
+constexpr float kRound = 12582912.f;           // 1.5 * 2^23: adding it rounds to an integer, ties to even
+constexpr uint32_t kRoundBits = 0x4B400000u;   // (its bits)
+// What kRound's bits add up to in word i of a block (fields that lie in two words are added without them).
+template <int BITS>
+__device__ constexpr uint32_t pack_bias(int i) {
+    uint32_t c = 0u;
+    for (int j = 0; j < kRowsPerBlock; ++j) {
+        const int bit = BITS * j, sh = bit & 31;
+        if ((bit >> 5) == i && sh + BITS <= 32) c += kRoundBits << sh;
+    }
+    return c;
+}
+
+// A 32-row block with the division.  A call of its own: inlined, its loads in flight took the registers of the usual path.
 template <int BITS, typename T>
-__global__ void __launch_bounds__(kPackThreads)
+__device__ __noinline__ void pack_divided(const T* row, const int* gr, const float* scales, const float* zeros, int32_t* out,
+                                          int N) {
+    uint32_t w[BITS];
+#pragma unroll
+    for (int i = 0; i < BITS; ++i) w[i] = 0u;
+#pragma unroll
+    for (int j = 0; j < kRowsPerBlock; ++j) {
+        const float sf = scales[gr[j]], s = __half2float(__float2half_rn(sf));
+        const float a = __fadd_rn(PackIn<T>::get(row[j]), __fmul_rn(zeros[gr[j]], sf));
+        pack_insert<BITS>(w, j, (uint32_t)(int)rintf(__fdiv_rn(a, s)));
+    }
+#pragma unroll
+    for (int i = 0; i < BITS; ++i) out[(size_t)i * N] = (int32_t)w[i];
+}
+
+template <int BITS, typename T>
+__global__ void __launch_bounds__(kPackThreads, kPackCtas)
 pack_linear_kernel(const T* __restrict__ weight, const float* __restrict__ scales, const float* __restrict__ zeros,
                    const int32_t* __restrict__ g_idx, int K, int N, int G, int chunks_per_cta, int use_table,
                    int32_t* __restrict__ qweight, int32_t* __restrict__ qzeros, __half* __restrict__ scales_out) {
     constexpr int VEC = 16 / (int)sizeof(T);                       // elements of one 16-byte read
     constexpr int PITCH = kPackChunk + VEC;                        // elements of a tile row: 16 bytes of padding
+    constexpr int TILE = kPackCols * PITCH;
     extern __shared__ __align__(16) unsigned char pack_smem[];
-    T* tile = reinterpret_cast<T*>(pack_smem);                     // [32][PITCH]
-    int* gs = reinterpret_cast<int*>(pack_smem + sizeof(T) * kPackCols * PITCH);   // groups of the chunk's rows
-    float2* table = reinterpret_cast<float2*>(gs + kPackChunk);    // [G][32] (zero * scale, 1 / scale)
+    T* tiles = reinterpret_cast<T*>(pack_smem);                    // two of [32][PITCH]
+    int* groups = reinterpret_cast<int*>(pack_smem + 2 * sizeof(T) * TILE);        // two of: groups of the chunk's rows
+    float2* table = reinterpret_cast<float2*>(groups + 2 * kPackChunk);            // [G][33] (zero * scale, 1 / scale)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int n0 = blockIdx.x * kPackCols, n = n0 + lane;
-    auto entry = [&](int g, float& s) {
-        const float sf = scales[(size_t)n * G + g];
-        s = __half2float(__float2half_rn(sf));
-        return make_float2(__fmul_rn(zeros[(size_t)n * G + g], sf), __frcp_rn(s));
-    };
-    if (use_table)
-        for (int g = warp; g < G; g += kPackThreads / 32) { float s; table[g * kPackCols + lane] = entry(g, s); }
-    if (blockIdx.y == 0) {
-        for (int g = warp; g < G; g += kPackThreads / 32)
-            scales_out[(size_t)g * N + n] = __float2half_rn(scales[(size_t)n * G + g]);
-        for (int g = threadIdx.x; g < G; g += kPackThreads) {
-            uint32_t w[BITS];
-#pragma unroll
-            for (int i = 0; i < BITS; ++i) w[i] = 0u;
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-                pack_insert<BITS>(w, j, (uint32_t)(long long)(zeros[(size_t)(n0 + j) * G + g] - 1.f));
-#pragma unroll
-            for (int i = 0; i < BITS; ++i) qzeros[(size_t)g * (N / 32 * BITS) + blockIdx.x * BITS + i] = (int32_t)w[i];
-        }
-    }
-    const int c_end = min((K + kPackChunk - 1) / kPackChunk, (int)(blockIdx.y + 1) * chunks_per_cta);
-    for (int c = blockIdx.y * chunks_per_cta; c < c_end; ++c) {
+    const int c_begin = blockIdx.y * chunks_per_cta, c_end = min((K + kPackChunk - 1) / kPackChunk, c_begin + chunks_per_cta);
+    auto fetch = [&](int c, int buf) {
         const int k0 = c * kPackChunk;
-        __syncthreads();                                           // the previous chunk has been read (and: the table is there)
 #pragma unroll
         for (int i = threadIdx.x; i < kPackCols * kPackChunk / VEC; i += kPackThreads) {
             const int r = i / (kPackChunk / VEC), e = (i % (kPackChunk / VEC)) * VEC;
             if (k0 + e < K)
-                *reinterpret_cast<uint4*>(tile + r * PITCH + e) =
-                    __ldcs(reinterpret_cast<const uint4*>(weight + (size_t)(n0 + r) * K + k0 + e));
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
+                             ::"r"((uint32_t)__cvta_generic_to_shared(tiles + buf * TILE + r * PITCH + e)), "l"(weight + (size_t)(n0 + r) * K + k0 + e)
+                             : "memory");
         }
-        if (k0 + (int)threadIdx.x < K)      // an index outside the groups is refused by the host when the layer is used
-            gs[threadIdx.x] = min(max(__ldg(g_idx + k0 + threadIdx.x), 0), G - 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // (an index outside the groups is refused by the host when the layer is used)
+    auto group_of = [&](int c) {
+        const int k = c * kPackChunk + threadIdx.x;
+        return k < K ? min(max(__ldg(g_idx + k), 0), G - 1) : 0;
+    };
+    if (blockIdx.y == gridDim.y - 1) {
+        // scales and zero-points of the strip, 128 groups at a time: read along the groups, written along the columns
+        constexpr int GT = 128;
+        float* st = reinterpret_cast<float*>(pack_smem);
+        float* zt = st + GT * kPackPitch;
+        for (int g0 = 0; g0 < G; g0 += GT) {
+            const int count = min(GT, G - g0);
+            for (int g = lane; g < count; g += 32)
+#pragma unroll
+                for (int r = 0; r < kPackCols; r += kPackThreads / 32) {
+                    const size_t at = (size_t)(n0 + r + warp) * G + g0 + g;
+                    st[g * kPackPitch + r + warp] = scales[at];
+                    zt[g * kPackPitch + r + warp] = zeros[at];
+                }
+            __syncthreads();
+            for (int g = warp; g < count; g += kPackThreads / 32)
+                scales_out[(size_t)(g0 + g) * N + n] = __float2half_rn(st[g * kPackPitch + lane]);
+            for (int g = threadIdx.x; g < count; g += kPackThreads) {
+                uint32_t w[BITS];
+#pragma unroll
+                for (int i = 0; i < BITS; ++i) w[i] = 0u;
+#pragma unroll
+                for (int j = 0; j < 32; ++j)
+                    pack_insert<BITS>(w, j, (uint32_t)(long long)(zt[g * kPackPitch + j] - 1.f));
+#pragma unroll
+                for (int i = 0; i < BITS; ++i)
+                    qzeros[(size_t)(g0 + g) * (N / 32 * BITS) + blockIdx.x * BITS + i] = (int32_t)w[i];
+            }
+            __syncthreads();
+        }
+        return;
+    }
+    fetch(c_begin, 0);
+    int g_next = group_of(c_begin);
+    auto entry = [&](size_t at) {                                  // at: [N, G]
+        const float sf = scales[at];
+        return make_float2(__fmul_rn(zeros[at], sf), __frcp_rn(__half2float(__float2half_rn(sf))));
+    };
+    if (use_table)
+        for (int g = lane; g < G; g += 32)
+#pragma unroll
+            for (int r = 0; r < kPackCols; r += kPackThreads / 32)
+                table[g * kPackPitch + r + warp] = entry((size_t)(n0 + r + warp) * G + g);
+    for (int c = c_begin; c < c_end; ++c) {
+        const int buf = (c - c_begin) & 1;
+        groups[buf * kPackChunk + threadIdx.x] = g_next;
+        if (c + 1 < c_end) {                                       // (the barrier that ended the last turn freed its buffers)
+            fetch(c + 1, buf ^ 1);
+            g_next = group_of(c + 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
         __syncthreads();
-        const int rb = k0 / kRowsPerBlock + warp;
-        if (rb * kRowsPerBlock >= K) continue;
-        const T* row = tile + lane * PITCH + warp * kRowsPerBlock;
-        const int* gr = gs + warp * kRowsPerBlock;
-        uint32_t w[BITS];
+        const int rb = c * (kPackChunk / kRowsPerBlock) + warp;
+        if (rb * kRowsPerBlock < K) {
+            const T* row = tiles + buf * TILE + lane * PITCH + warp * kRowsPerBlock;
+            const int* gr = groups + buf * kPackChunk + warp * kRowsPerBlock;
+            uint32_t w[BITS];
+            float far = 0.f;                                       // largest distance from an integer
+            uint32_t any = 0u, all = ~0u;
+            auto block = [&](auto look_up) {
 #pragma unroll
-        for (int i = 0; i < BITS; ++i) w[i] = 0u;
-        bool close = false;                                        // some quotient is too close to a half, or not finite
+                for (int i = 0; i < BITS; ++i) w[i] = 0u - pack_bias<BITS>(i);
 #pragma unroll
-        for (int j0 = 0; j0 < kRowsPerBlock; j0 += VEC) {
-            const uint4 raw = *reinterpret_cast<const uint4*>(row + j0);
-            const T* v = reinterpret_cast<const T*>(&raw);
+                for (int j0 = 0; j0 < kRowsPerBlock; j0 += VEC) {
+                    const uint4 raw = *reinterpret_cast<const uint4*>(row + j0);
+                    const T* v = reinterpret_cast<const T*>(&raw);
 #pragma unroll
-            for (int i = 0; i < VEC; ++i) {
-                const int g = gr[j0 + i];
-                float s;
-                const float2 e = use_table ? table[g * kPackCols + lane] : entry(g, s);
-                const float t = __fadd_rn(PackIn<T>::get(v[i]), e.x) * e.y;
-                const float u = __fadd_rn(t, 12582912.f);          // 1.5 * 2^23: rounds t to an integer, ties to even
-                const float d = fabsf(t - __fadd_rn(u, -12582912.f));
-                close |= !(d < fmaf(fabsf(t), -4.76837158203125e-7f, 0.5f));   // |t| * 2^-21
-                pack_insert<BITS>(w, j0 + i, (uint32_t)(__float_as_int(u) - 0x4B400000));
+                    for (int i = 0; i < VEC; i += 2) {
+                        uint32_t ub[2];
+                        float d[2];
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const float2 e = look_up(j0 + i + h);
+                            const float a = __fadd_rn(PackIn<T>::get(v[i + h]), e.x), u = fmaf(a, e.y, kRound);
+                            d[h] = fmaf(a, e.y, -__fadd_rn(u, -kRound));
+                            ub[h] = __float_as_uint(u);
+                            const int bit = BITS * (j0 + i + h), wi = bit >> 5, sh = bit & 31;
+                            if (sh + BITS <= 32) {
+                                w[wi] += ub[h] << sh;
+                            } else {
+                                w[wi] += (ub[h] - kRoundBits) << sh;
+                                w[wi + 1] += (ub[h] - kRoundBits) >> (32 - sh);
+                            }
+                        }
+                        far = fmaxf(far, fmaxf(fabsf(d[0]), fabsf(d[1])));
+                        any |= ub[0] | ub[1];
+                        all &= ub[0] & ub[1];
+                    }
+                }
+            };
+            const int g_lane = gr[lane], g_first = __shfl_sync(0xffffffffu, g_lane, 0);
+            if (__all_sync(0xffffffffu, g_lane == g_first)) {      // rows in order, groups of whole blocks
+                const float2 e = use_table ? table[g_first * kPackPitch + lane] : entry((size_t)n * G + g_first);
+                block([&](int) { return e; });
+            } else if (use_table) {
+                block([&](int j) { return table[gr[j] * kPackPitch + lane]; });
+            } else {
+                block([&](int j) { return entry((size_t)n * G + gr[j]); });
+            }
+            const bool redo = far > 0.5f - (1 << BITS) * 4.76837158203125e-7f || (any >> BITS) != (kRoundBits >> BITS) ||
+                              (all >> BITS) != (kRoundBits >> BITS);                     // (2^bits * 2^-21)
+            int32_t* out = qweight + (size_t)rb * BITS * N + n;
+            if (redo) {
+                pack_divided<BITS, T>(row, gr, scales + (size_t)n * G, zeros + (size_t)n * G, out, N);
+            } else {
+#pragma unroll
+                for (int i = 0; i < BITS; ++i) out[(size_t)i * N] = (int32_t)w[i];
             }
         }
-        if (close) {
-#pragma unroll
-            for (int i = 0; i < BITS; ++i) w[i] = 0u;
-#pragma unroll
-            for (int j = 0; j < kRowsPerBlock; ++j) {
-                float s;
-                const float2 e = entry(gr[j], s);
-                pack_insert<BITS>(w, j, (uint32_t)(int)rintf(__fdiv_rn(__fadd_rn(PackIn<T>::get(row[j]), e.x), s)));
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < BITS; ++i) qweight[(size_t)(rb * BITS + i) * N + n] = (int32_t)w[i];
+        __syncthreads();
     }
 }
 
@@ -186,9 +287,9 @@ template <int BITS, typename T>
 int launch_pack_linear(const void* weight, const float* scales, const float* zeros, const int32_t* g_idx, int K, int N,
                        int G, int32_t* qweight, int32_t* qzeros, __half* scales_out, cudaStream_t stream) {
     const int chunks = (K + kPackChunk - 1) / kPackChunk, strips = N / kPackCols;
-    const long long table = (long long)G * kPackCols * sizeof(float2);
+    const long long table = (long long)G * kPackPitch * sizeof(float2);
     const int use_table = table <= kPackTableMax;
-    const size_t smem = sizeof(T) * kPackCols * (kPackChunk + 16 / sizeof(T)) + kPackChunk * sizeof(int) + (use_table ? table : 0);
+    const size_t smem = 2 * (sizeof(T) * kPackCols * (kPackChunk + 16 / sizeof(T)) + kPackChunk * sizeof(int)) + (use_table ? table : 0);
     static std::once_flag once[64];
     static int result[64];
     int dev = 0;
@@ -199,11 +300,17 @@ int launch_pack_linear(const void* weight, const float* scales, const float* zer
                                                 200 * 1024);
     });
     if (result[dev] != 0) { set_last_cuda_error(result[dev]); return B200GPTQ_ERR_CUDA; }
-    // K is cut until the grid fills the device about four times over: every cut builds the table of its columns again
-    int parts = (8 * sm_count() + strips - 1) / strips;
-    if (parts > chunks) parts = chunks;
-    const int per = (chunks + parts - 1) / parts;
-    dim3 grid(strips, (chunks + per - 1) / per);
+    // K is cut so that the waves of the grid are full and short: a CTA costs its chunks, the start of its pipeline and its
+    // table (an entry about as much as four elements).
+    const int resident = sm_count() * (smem * kPackCtas <= 220 * 1024 ? kPackCtas : (int)(220 * 1024 / smem));
+    int per = chunks;
+    long long best = -1;
+    for (int p = 1; p <= chunks; ++p) {
+        const int c = (chunks + p - 1) / p, ctas = strips * ((chunks + c - 1) / c);
+        const long long cost = (long long)((ctas + resident - 1) / resident) * (64 * (c + 1) + G);
+        if (best < 0 || cost < best) { best = cost; per = c; }
+    }
+    dim3 grid(strips, (chunks + per - 1) / per + 1);
     pack_linear_kernel<BITS, T><<<grid, kPackThreads, smem, stream>>>(static_cast<const T*>(weight), scales, zeros, g_idx, K, N,
                                                                       G, per, use_table, qweight, qzeros, scales_out);
     B200GPTQ_CUDA_TRY(cudaGetLastError());

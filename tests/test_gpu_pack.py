@@ -108,3 +108,25 @@ def test_one_launch_pack_equals_the_cpu_packer(bits, K, N, gs, dtype):
     assert torch.equal(a.qweight, b.qweight.cpu())
     assert torch.equal(a.qzeros, b.qzeros.cpu())
     assert torch.equal(a.scales, b.scales.cpu())
+
+
+@pytest.mark.parametrize("bits", [2, 3, 4, 8])
+@pytest.mark.parametrize("K,N,gs", [(288, 32, 32), (4480, 64, 32)])     # (140 groups: more than one tile of the zero-points)
+def test_one_launch_pack_in_order_and_out_of_range(bits, K, N, gs):
+    """Rows in group order take no table; fields outside 0..2^bits-1 spill into their neighbours as the CPU route has them."""
+    gen = torch.Generator().manual_seed(bits + K)
+    G = K // gs
+    scales = 2.0 ** torch.randint(-8, -3, (N, G), generator=gen).float()
+    zeros = torch.randint(1, 2 ** bits, (N, G), generator=gen).float()
+    sel = torch.arange(K) // gs
+    q = torch.randint(0, 2 ** bits, (N, K), generator=gen).float()
+    for i, wrong in enumerate([-1., 2. ** bits, 300., -4194304., -9437184., 2.**24]):
+        q[3 + i, 17 * i + 9] = wrong
+    lin = nn.Linear(K, N, bias=False)
+    lin.weight.data = (q - zeros[:, sel]) * scales[:, sel]
+    a, b = QuantLinear(bits, gs, K, N, False), QuantLinear(bits, gs, K, N, False).to(DEV)
+    a.pack(lin, scales, zeros)
+    b.pack(lin.to(DEV), scales.to(DEV), zeros.to(DEV))
+    assert torch.equal(a.qweight, b.qweight.cpu())
+    assert torch.equal(a.qzeros, b.qzeros.cpu())
+    assert torch.equal(a.scales, b.scales.cpu())
