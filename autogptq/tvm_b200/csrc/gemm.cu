@@ -225,9 +225,10 @@ template <> struct Dequant<3> {
 };
 
 // ---- x pre-pass: gather through x_perm and/or permute each 32-block into the 3-bit field order ----
-// One row of x and 2048 of its values per CTA, eight per thread: a row of x stays in L1 while its values are picked.  (One
+// One row of x and 1024 of its values per CTA, eight per thread: a row of x stays in L1 while its values are picked.  Four
+// warps of 32 registers fit beside the decode GEMV, so that they are there when it ends.  (One
 // 2-byte value per thread and pass with a division: 7.8 us for 16 x 9216, 24 us for 1495 x 1856.)
-constexpr int kPrepValues = 2048;
+constexpr int kPrepValues = 1024;
 constexpr unsigned long long order8(int first) {
     constexpr unsigned char o[32] = {0, 3, 1, 7, 2, 8, 4, 9, 5, 10, 6, 11, 12, 17, 13, 18,
                                      14, 19, 15, 20, 16, 21, 22, 27, 23, 28, 24, 29, 25, 30, 26, 31};
@@ -239,7 +240,6 @@ __global__ void __launch_bounds__(kPrepValues / 8)
 prep_x_kernel(const __half* __restrict__ x, const int32_t* __restrict__ x_perm, __half* __restrict__ xp, int K, int permute3) {
     const int k0 = blockIdx.x * kPrepValues + 8 * threadIdx.x;
     asm volatile("griddepcontrol.launch_dependents;");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
     if (k0 >= K) return;
     constexpr unsigned long long O0 = order8(0), O1 = order8(8), O2 = order8(16), O3 = order8(24);
     const int part = (k0 >> 3) & 3;
@@ -250,6 +250,7 @@ prep_x_kernel(const __half* __restrict__ x, const int32_t* __restrict__ x_perm, 
         src[i] = permute3 ? (k0 & ~31) + (int)((o >> (8 * i)) & 0xffu) : k0 + i;
         if (x_perm) src[i] = __ldg(x_perm + src[i]);
     }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const unsigned short* row = reinterpret_cast<const unsigned short*>(x) + (size_t)blockIdx.y * K;
     unsigned short v[8];
 #pragma unroll

@@ -82,19 +82,22 @@ int gemv_strip_prepare(GemvStripPlan* p, const int32_t* qweight, const int32_t* 
     s.rows_g = sub == 1 ? 1 : (s.spg == 1 ? 4 : (s.spg == 2 ? 2 : 3));
     // Strips of a pass for W warps: a unit costs about half a strip's work on top of its strips, and the last pass is a whole
     // one.  The rings take at least two slots and what is left of the shared memory.
-    struct Choice { int W, T, ring, fixed, kept, cost; };
+    struct Choice { int W, T, ring, fixed, bufs, cost; };
     auto choose = [&](int W) {
         Choice c = {W, 0, 0, 0, 0, 1 << 30};
         // (a gather works from a copy of x that the sums overwrite: it needs every unit's x kept)
-        for (int kept = 1; kept >= (mode == kSeveral && !gather ? 0 : 1) && !c.T; --kept)
+        // x that is not kept: as many units ahead as leave the weights three slots, one ahead being the least
+        for (int bufs = 5; bufs >= (mode == kSeveral && !gather ? 2 : 5) && c.bufs != 5; --bufs)
             for (int t = 1; t <= tmax && t <= s.per_cta; ++t) {
                 const int slot = slot_bytes(bits, t) + const_bytes(bits, t, s.rows_g);
                 const int sums = W * M * t * kStripCols * 4, copy = gather || mode != kSeveral ? M * K * 2 : 0;
                 const int x = mode == kInt ? plane_bytes
-                            : (mode == kOne ? s.units * kUnit * 2 : (kept ? s.units : 2 * W) * M * kXPitch * 2);
+                            : (mode == kOne ? s.units * kUnit * 2 : (bufs == 5 ? s.units : bufs * W) * M * kXPitch * 2);
                 const int f = x + (sums > copy ? sums : copy) + 1024, r = (kSmemMax - f) / (W * slot);
                 const int cost = ((s.per_cta + t - 1) / t) * (2 * t + 1);
-                if (f < kSmemMax && r >= 2 && cost <= c.cost) c = {W, t, r, f, kept, cost};
+                const int least = bufs == 3 || bufs == 4 ? 3 : 2;
+                if (bufs != 5 && bufs > 2 && s.units / W < bufs - 1) continue;
+                if (f < kSmemMax && r >= least && (cost < c.cost || (cost == c.cost && bufs == c.bufs))) c = {W, t, r, f, bufs, cost};
             }
         return c;
     };
@@ -111,7 +114,8 @@ int gemv_strip_prepare(GemvStripPlan* p, const int32_t* qweight, const int32_t* 
     if (!c.T) return B200GPTQ_ERR_TOO_LARGE;
     const int W = c.W, T = c.T;
     s.passes = (s.per_cta + T - 1) / T;
-    s.kept = c.kept;
+    s.kept = c.bufs == 5;
+    s.x_bufs = s.kept ? 2 : c.bufs;
     const int longest = ((s.units + W - 1) / W) * s.passes;
     s.ring = c.ring < longest ? c.ring : longest;
     if (s.ring > kMaxRing) s.ring = kMaxRing;

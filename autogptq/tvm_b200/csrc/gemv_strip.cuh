@@ -15,8 +15,9 @@
 //    filled before griddepcontrol.wait; with eight warps the footprint is half an SM, so under programmatic dependent
 //    launch the next launch's weights arrive while this one computes.
 //  * One row of x: a warp puts its whole slice of x into shared memory in the order of the B registers, once.  Several
-//    rows: copied one unit ahead with cp.async and permuted as they are read.  Which k a lane multiplies is free as long
-//    as x is read in the same order.
+//    rows: copied with cp.async and permuted as they are read; all of x at once where it fits, else one to three units ahead
+//    (one unit ahead is an L2 latency per unit: 16 rows, 9216 x 9216, 3 bits 29 us, two ahead 21).  Which k a lane multiplies
+//    is free as long as x is read in the same order.
 //  * One or two rows, 2 to 4 bits, whole units per group: products on the integer tensor path.  A byte of weights is q << p, one
 //    AND per four fields and no shift; x is fixed point per unit (|X| < 2^22: exact for every
 //    element within 2^-12 of the unit's largest), shifted by what its weight byte lacks and split into four signed byte
@@ -360,7 +361,8 @@ struct StripPlan {
     int groups;
     unsigned int spg_inv;   // ceil(2^32 / spg)
     int rows_g;       // groups whose constants a slot holds
-    int kept;         // several rows: every unit's x has a place of its own (otherwise two in turn)
+    int kept;         // several rows: every unit's x has a place of its own
+    int x_bufs;       // otherwise: places of a warp, 2..4, used in turn
     int gather;       // x is picked through x_perm from a copy of it in shared memory
     int xact;         // activation applied to x as it is read: 0 none, 1 SwiGLU, 2 ReLU
 };
@@ -389,8 +391,12 @@ __device__ __forceinline__ uint32_t act_swiglu2(uint32_t gv, uint32_t uv) {
 
 // SUB: groups of a unit that are scaled apart (1: a group is a whole number of units).  NT: rows of x / 8.
 // MODE: kSeveral, kOne, kInt.  T: strips of a pass.  W: warps of a CTA.
+// Registers: two CTAs of eight warps fit on an SM; sixteen warps, or sixteen rows of x, leave 4096 or 8192 of an SM's for the
+// kernel that comes next.  With all of them taken, the gather of x between two products of 8 rows, 9216 x 9216, 3 bits, only
+// started when a CTA ended, and the next product's weights after that: 22 us against 16.6 (and 14.3 against 14.1 where
+// nothing is gathered).
 template <int BITS, int SUB, int NT, int MODE, int T, int W>
-__global__ void __launch_bounds__(32 * W, W == 8 && NT == 1 ? 2 : 1)
+__global__ void __maxnreg__(W == 16 ? 120 : NT == 1 ? 128 : 224)
 gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_s,
                   const __grid_constant__ CUtensorMap tmap_z, const __half* __restrict__ x,
                   const int32_t* __restrict__ x_perm, const __half* __restrict__ bias, __half* __restrict__ y, int M_rows, int K, int N, const StripPlan plan,
@@ -423,10 +429,10 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     uint8_t* p_const = aligned + (size_t)W * R * SLOT + (size_t)warp * R * cbytes;
     uint8_t* base_x = aligned + (size_t)W * R * (SLOT + cbytes);
     // one row: [unit][quad lane][16 registers]; planes: [unit][step]..., then (factor, sum) [unit][row]; several rows:
-    // [unit][row][natural halves], or two units in turn per warp
+    // [unit][row][natural halves], or a few units in turn per warp
     const int unit_x = ONE ? kUnit * 2 : (INT ? int_unit_bytes<BITS>(M) : M * kXPitch * 2);
-    const int x_units = ROWS && !plan.kept ? 2 * W : plan.units;
-    uint8_t* p_x = base_x + (size_t)(ROWS && !plan.kept ? 2 * warp : u_begin) * unit_x;
+    const int x_units = ROWS && !plan.kept ? plan.x_bufs * W : plan.units;
+    uint8_t* p_x = base_x + (size_t)(ROWS && !plan.kept ? plan.x_bufs * warp : u_begin) * unit_x;
     float2* p_f = reinterpret_cast<float2*>(base_x + (size_t)plan.units * unit_x) + (size_t)u_begin * M;
     uint8_t* base_r = base_x + (size_t)x_units * unit_x + (INT ? (plan.units * M * 8 + 15) / 16 * 16 : 0);
     float* red = reinterpret_cast<float*>(base_r);                                 // [warp][m][column of the pass]
@@ -683,8 +689,9 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     static_assert(L::kRows % 4 == 0, "strips start on lines 0 or 4 of the swizzle pattern");
 
     int slot = 0, parity = 0, buf = 0;
+    if (ROWS && async_x && !plan.kept && nu > 0)          // x that is not kept: x_bufs - 1 units (no more than nu) ahead
+        for (int i = 0; i < plan.x_bufs - 1; ++i) fetch_x(i, i);
     for (int p = 0, win = 0; p < plan.passes; ++p, win = min(win + T, last_window)) {
-        if (ROWS && async_x && !plan.kept && nu > 0) fetch_x(0, buf);
 #pragma unroll 1
         for (int u = 0; u < nu; ++u) {
             const uint8_t* src = p_ring + slot * SLOT;
@@ -749,17 +756,22 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                 }
             } else {
                 __half* xs = reinterpret_cast<__half*>(p_x + (size_t)(plan.kept ? u : buf) * unit_x);
-                buf ^= 1;
                 if (!plan.kept) {
                     if (async_x) {
-                        asm volatile("cp.async.wait_group 0;" ::: "memory");
+                        if (plan.x_bufs == 4) asm volatile("cp.async.wait_group 2;" ::: "memory");
+                        else if (plan.x_bufs == 3) asm volatile("cp.async.wait_group 1;" ::: "memory");
+                        else asm volatile("cp.async.wait_group 0;" ::: "memory");
                         __syncwarp();
-                        if (u + 1 < nu) fetch_x(u + 1, buf);
+                        // into the place of the unit before this one; also for the next pass
+                        const int ahead = u + plan.x_bufs - 1, to = buf == 0 ? plan.x_bufs - 1 : buf - 1;
+                        if (ahead < nu || p + 1 < plan.passes) fetch_x(ahead < nu ? ahead : ahead - nu, to);
+                        else asm volatile("cp.async.commit_group;" ::: "memory");    // keeps the count of groups
                     } else {
                         for (int m = 0; m < M; ++m)
                             *reinterpret_cast<uint2*>(xs + m * kXPitch + 4 * lane) = load4(m, (u_begin + u) * kUnit + 4 * lane);
                         __syncwarp();
                     }
+                    if (++buf == plan.x_bufs) buf = 0;
                 }
 #pragma unroll
                 for (int nt = 0; nt < NT; ++nt) {

@@ -58,7 +58,9 @@ def test_gemv_vs_oracle(bits, K, N, gs, gather, M):
 
 
 @pytest.mark.parametrize("bits,K,N,gs,gather", [(2, 544, 96, 32, True), (3, 1152, 4832, 128, False), (3, 1184, 64, 64, True),
-                                                (4, 4096, 4800, 128, True), (4, 992, 32, 32, False), (8, 288, 9632, -1, False)])
+                                                (4, 4096, 4800, 128, True), (4, 992, 32, 32, False), (8, 288, 9632, -1, False),
+                                                # x does not fit: places in turn, three and four of them, several passes
+                                                (3, 6144, 9632, 128, False), (4, 12288, 4832, 128, False)])
 @pytest.mark.parametrize("M", [9, 16])
 def test_plan_of_nine_to_sixteen_rows_vs_oracle(bits, K, N, gs, gather, M):
     layer = synth.make_layer(bits, K, N, gs, False, bias=True, seed=K + N + bits)
