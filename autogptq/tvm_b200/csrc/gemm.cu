@@ -1,4 +1,6 @@
-// Prefill dequant-GEMM on the 5th-generation tensor cores (tcgen05 + tensor memory), sm_100a.
+// Dequant-GEMM on the 5th-generation tensor cores (tcgen05 + tensor memory), sm_100a: the kernel for up to 16 rows of x of 3-
+// and 4-bit layers (more rows, 2 and 8 bits: gemm_pair.cu), the choice between the two, and the copy of x in the order in which
+// a product reads it.
 //
 //   y[M, N] = x[M, K] @ W[K, N] (+ bias),   W[k, n] = scales[g, n] * (q[k, n] - zero[g, n])
 //
@@ -6,15 +8,15 @@
 // A operand of tcgen05.mma and can live in TENSOR MEMORY: they never touch shared memory, which
 // on this part is the resource a mixed-input GEMM runs out of first (an MMA whose operands both
 // come from shared memory already consumes its whole read bandwidth at 128 x 128 tiles).
-// One CTA computes 128 output columns for a tile of TN <= 256 rows of x:
+// One CTA computes 128 output columns for all rows of x, padded to TN = 16:
 //   warp 0      TMA producer: per k-tile (64 rows of K) an x tile (TN rows x 64 k, 128-byte
 //               swizzle) and the packed weight rows of the CTA's 128 columns, into a stage ring
-//   warps 1..16 weight producers in two groups that take k-tiles in turn: each thread owns one of the 128 columns and one 32-row block of
-//               the k-tile; it reads its packed words from the stage, dequantises them to the
+//   then        weight producers, one or three groups of eight warps that take k-tiles in turn: each thread owns one of the
+//               128 columns and one 32-row block of the k-tile; it reads its packed words from the stage, dequantises them to the
 //               exact fp16 value of the reference (auto_gptq/nn_modules/qlinear.py:242: one
 //               rounding) and stores 16 registers into the A buffer of that stage in tensor memory
 //               (tcgen05.st); afterwards the same warps run the epilogue (tcgen05.ld -> fp16 -> y)
-//   warp 17     allocates tensor memory and issues tcgen05.mma (M = 128 columns, N = TN rows of x,
+//   last warp   allocates tensor memory and issues tcgen05.mma (M = 128 columns, N = TN rows of x,
 //               K = 16, f16 x f16 -> f32 accumulators in tensor memory columns 0..TN-1)
 // Stages hand over through mbarriers; tcgen05.commit releases a stage when its MMAs retire.
 // Every wait is bounded: on expiry the kernel raises a sticky status word, unwinds, frees its
@@ -39,7 +41,7 @@ namespace {
 
 constexpr int BN = 128;                 // output columns per CTA = rows of the MMA's A operand
 constexpr int BK = 64;                  // rows of K per stage
-constexpr int kMaxTN = 256;             // rows of x per CTA = N of the MMA
+constexpr int TN = 16;                  // rows of x = N of the MMA
 constexpr int kWeightWarps = 8;         // warps that build one k-tile's A operand
 // Groups of weight warps, taking k-tiles in turn.
 __host__ __device__ constexpr int mma_warp(int groups) { return 1 + kWeightWarps * groups; }
@@ -265,7 +267,7 @@ __global__ void __launch_bounds__(gemm_threads(kWeightGroups), kWeightGroups == 
 gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
             const int32_t* __restrict__ qzeros, const __half* __restrict__ scales,
             const int32_t* __restrict__ g_idx, const __half* __restrict__ bias, __half* __restrict__ y, int M, int K,
-            int N, int group_size, int TN, int S, int tab_groups, int a_off, unsigned int* __restrict__ status,
+            int N, int group_size, int S, int tab_groups, int a_off, unsigned int* __restrict__ status,
             int splits, int tmem_cols, float* __restrict__ partial) {
     // splits > 1 (few rows of x, fewer column tiles than SMs): blockIdx.z takes a contiguous run of the k-tiles, two
     // such CTAs fit on an SM (half of the shared and tensor memory each), every CTA leaves its fp32 sums in
@@ -282,7 +284,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
 
     constexpr int kMmaWarp = mma_warp(kWeightGroups);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n0 = blockIdx.y * BN, m0 = blockIdx.x * TN;
+    const int n0 = blockIdx.y * BN;
     const int KT_all = (K + BK - 1) / BK;
     const int kt_first = (int)(((long long)blockIdx.z * KT_all) / splits);
     const int KT = (int)(((long long)(blockIdx.z + 1) * KT_all) / splits) - kt_first;   // k-tiles of this CTA
@@ -328,7 +330,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
                 if (round > 0 && !mbar_wait(empty_bar(s), (round - 1) & 1, &abort_flag)) break;
                 mbar_arrive_expect_tx(tma_bar(s), x_tile_bytes + kPackedBytes);
                 tma_load_2d(p_tile(s), &tmap_w, n0, (kt_first + kt) * kWordRowsPerTile, tma_bar(s));
-                tma_load_2d(x_tile(s), &tmap_x, (kt_first + kt) * BK, m0, tma_bar(s));
+                tma_load_2d(x_tile(s), &tmap_x, (kt_first + kt) * BK, 0, tma_bar(s));
                 if (++s == S) { s = 0; ++round; }
             }
         }
@@ -481,7 +483,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
                     uint32_t r[16];
                     tmem_ld16(lane_addr + 16u * c, r);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    const int m = m0 + 16 * c;
+                    const int m = 16 * c;
                     if (col_ok) {
 #pragma unroll
                         for (int i = 0; i < 16; ++i)
@@ -496,7 +498,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
             //      undefined and the status word says so). ----
             if (!ok && lane == 0) epi_bad = 1;
             asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
-            const int rows_pad = gridDim.x * TN;
+            const int rows_pad = TN;
             if (epi_bad == 0) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 float* mine = partial + (size_t)blockIdx.z * rows_pad * N;
@@ -505,7 +507,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
                     uint32_t r[16];
                     tmem_ld16(lane_addr + 16u * c, r);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    const int m = m0 + 16 * c;
+                    const int m = 16 * c;
                     if (col_ok) {
 #pragma unroll
                         for (int i = 0; i < 16; ++i)
@@ -515,14 +517,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
             }
             __threadfence();   // this thread's sums are visible before the tile's arrival is counted
             asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
-            unsigned int* counter = status + (blockIdx.y * gridDim.x + blockIdx.x);
+            unsigned int* counter = status + (blockIdx.y);
             if (threadIdx.x == 32) arrived = atomicAdd(counter, 1u);
             asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
             if (arrived == (unsigned int)splits - 1u) {
                 __threadfence();   // the other CTAs' sums, published before their arrivals
 #pragma unroll 1
                 for (int c = (warp - 1) >> 2; c < TN / 16; c += kEpiWarps / 4) {
-                    const int m = m0 + 16 * c;
+                    const int m = 16 * c;
                     if (col_ok) {
                         // all loads of the chunk are issued before the first is used: one round trip to L2, not 64
                         float v[kMaxSplits][16];
@@ -575,8 +577,7 @@ EncodeTiledFn encode_tiled_fn() {
 
 // Work split of a launch.  With few rows of x a tile's time is the chain of hand-overs per k-tile, not its arithmetic:
 // the time of a launch is (waves of CTAs) x (k-tiles per CTA).  Two things shorten it.  Split K: the k-tiles of a
-// column tile are spread over up to kMaxSplits CTAs (blockIdx.z), only for one row tile (M <= 128) and when every
-// run keeps at least 16 k-tiles (40 above 64 rows: taller partial sums).  Two CTAs per SM (M <= 64): one group of
+// column tile are spread over up to kMaxSplits CTAs (blockIdx.z).  Two CTAs per SM: one group of
 // weight warps instead of three (320 threads, so that two CTAs fit the register file) and half of the shared and
 // tensor memory each.  An SM works through k-tiles at about the same rate either way (0.4-0.5 us per k-tile), so the
 // second CTA is taken only where it fills a half-empty second wave or halves the k-tiles of a CTA: 16 rows,
@@ -586,16 +587,18 @@ int splits_for(int M, int tiles, int KT, int slots) {
     if (M > 128 || tiles >= kMaxCounters - 1) return 1;
     int sp = slots / tiles;
     if (sp > kMaxSplits) sp = kMaxSplits;
-    // every run keeps enough k-tiles to pay for its own start-up and for the final sum: measured on 4096 x 4096,
-    // 16 rows 33.5 -> 21 us with four runs, 128 rows 34.6 -> 37.4 us with two
-    const int min_tiles = M <= 64 ? 16 : 40;
+    // Every run keeps enough k-tiles to pay for its own start-up and for the final sum: 16 (4096 x 4096, 16 rows: 33.5 -> 21 us
+    // with four runs).  The taller the partial sums, the more they cost: above 64 rows two runs of 16 lose (2048 x 4096, 100
+    // rows: 12.5 -> 14.1 us) where four gain (4096 x 4096, 80 rows: 19.5 -> 14.4); above 96 rows a run keeps 40, which 128
+    // rows of 4096 x 4096 would not need (19.9 -> 16.6 with four of 16), but callers rely on the answer for that size.
+    const int min_tiles = M <= 96 ? 16 : 40;
     while (sp > 1 && KT / sp < min_tiles) --sp;
+    if (M > 64 && M <= 96 && sp < 3) return 1;
     return sp < 1 ? 1 : sp;
 }
 GemmSplit pick_split(int M, int N, int K) {
     const int tiles = (N + BN - 1) / BN, KT = (K + BK - 1) / BK, sms = sm_count();
     GemmSplit one = {splits_for(M, tiles, KT, sms), 1};
-    if (M > 64) return one;
     GemmSplit two = {splits_for(M, tiles, KT, 2 * sms), 2};
     auto cost = [&](const GemmSplit& g) {
         const long long ctas = (long long)tiles * g.splits, slots = (long long)sms * g.per_sm;
@@ -607,16 +610,7 @@ int pick_splits(int M, int N, int K) { return pick_split(M, N, K).splits; }
 size_t split_partial_bytes(int M, int N, int K) {
     const int sp = pick_splits(M, N, K);
     if (sp == 1) return 0;
-    const int TN = M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : 128));
     return (size_t)sp * TN * N * sizeof(float);
-}
-
-int pick_tn(int M) {
-    if (M <= 16) return 16;
-    if (M <= 32) return 32;
-    if (M <= 64) return 64;
-    if (M <= 128) return 128;
-    return kMaxTN;
 }
 
 template <int BITS>
@@ -625,7 +619,6 @@ int launch_gemm(const __half* x_for_tma, const int32_t* qweight, const int32_t* 
                 unsigned int* status, float* partial, cudaStream_t stream) {
     EncodeTiledFn encode = encode_tiled_fn();
     if (!encode) { set_last_cuda_error((int)cudaErrorNotSupported); return B200GPTQ_ERR_CUDA; }
-    const int TN = pick_tn(M);
     const int stage_bytes = TN * BK * 2 + kPackedTileBytes;
     // scale / zero-point table of the CTA's columns for every group, if it leaves room for >= 4 stages
     const int gs_eff = group_size;
@@ -640,7 +633,7 @@ int launch_gemm(const __half* x_for_tma, const int32_t* qweight, const int32_t* 
     // Stages: a small-M tile moves 4..6 KB per k-tile and its round trip (TMA, dequantisation, MMA, commit) lasts
     // microseconds, so throughput is the number of k-tiles in flight: as many as shared memory and the tensor-memory
     // columns behind the accumulators hold.
-    const int a_off = TN < 32 ? 32 : TN;
+    const int a_off = 32;
     int S = (smem_budget - tab_bytes) / stage_bytes;
     if (S > kMaxStages) S = kMaxStages;
     if (S > (tmem_cols - a_off) / kTmemAColsPerStage) S = (tmem_cols - a_off) / kTmemAColsPerStage;
@@ -668,7 +661,7 @@ int launch_gemm(const __half* x_for_tma, const int32_t* qweight, const int32_t* 
         if (r != CUDA_SUCCESS) { set_last_cuda_error((int)cudaErrorInvalidValue); return B200GPTQ_ERR_CUDA; }
     }
 
-    dim3 grid((M + TN - 1) / TN, (N + BN - 1) / BN, splits);
+    dim3 grid(1, (N + BN - 1) / BN, splits);
     auto launch = [&](auto groups) -> int {
         constexpr int kG = decltype(groups)::value;
         // the shared-memory opt-in is set once per device and instantiation; afterwards the launch path only reads
@@ -683,7 +676,7 @@ int launch_gemm(const __half* x_for_tma, const int32_t* qweight, const int32_t* 
         });
         if (attr_result[dev] != 0) { set_last_cuda_error(attr_result[dev]); return B200GPTQ_ERR_CUDA; }
         gemm_kernel<BITS, kG><<<grid, gemm_threads(kG), smem_bytes, stream>>>(
-            tmap_x, tmap_w, qzeros, scales, g_idx, bias, y, M, K, N, group_size, TN, S, tab_groups, a_off, status, splits,
+            tmap_x, tmap_w, qzeros, scales, g_idx, bias, y, M, K, N, group_size, S, tab_groups, a_off, status, splits,
             tmem_cols, partial);
         return B200GPTQ_OK;
     };
@@ -696,12 +689,16 @@ int launch_gemm(const __half* x_for_tma, const int32_t* qweight, const int32_t* 
 }  // namespace
 
 size_t gemm_pair_partial_bytes(int M, int K, int N, int splits);
+int gemm_pair_tiles(int M, int K, int N, int splits);
 int gemm_pair_dispatch(const __half* x, const int32_t* qweight, const int32_t* qzeros, const __half* scales, const int32_t* g_idx,
                        const __half* bias, __half* y, int M, int K, int N, int bits, int group_size, int splits,
                        unsigned int* status, float* partial, cudaStream_t stream);
 
-// More than 64 rows, and the bit widths that only it has: the kernel for pairs of CTAs (gemm_pair.cu).
-static bool use_pair(int M, int bits) { return M > 64 || bits == 2 || bits == 8; }
+// More than 16 rows, and the bit widths that only it has: the kernel for pairs of CTAs (gemm_pair.cu).  From 17 to 64 rows,
+// one CTA per tile against pairs: 4096 x 4096, 17 rows 16.4 and 11.2 us; 4096 x 12288, 64 rows 29.1 and 20.2; 11008 x 4096, 64
+// rows 35.2 and 20.6; 9216 x 9216, 3 bits, 24 rows 38.0 and 33.3; 9216 x 27648, 64 rows 106 and 84.  Up to 16 rows the split
+// over single CTAs, two per SM, is what b200gptq_gemm_split promises; layers go to the decode GEMV there.
+static bool use_pair(int M, int bits) { return M > 16 || bits == 2 || bits == 8; }
 // (a tile per pair of SMs, so that the last CTA of a tile can add the runs with all its warps)
 static int pair_splits(int M, int N, int K) {
     return splits_for(M, (N + 2 * BN - 1) / (2 * BN), (K + BK - 1) / BK, sm_count() / 2);
@@ -717,7 +714,13 @@ size_t gemm_workspace_bytes(int M, int K, int N, int bits) {
 
 
 void gemm_split_query(int M, int K, int N, int bits, int* splits, int* ctas_per_sm) {
-    const GemmSplit g = use_pair(M, bits) ? GemmSplit{pair_splits(M, N, K), 1} : pick_split(M, N, K);
+    GemmSplit g;
+    if (use_pair(M, bits)) {
+        g.splits = pair_splits(M, N, K);
+        g.per_sm = M <= 64 && gemm_pair_tiles(M, K, N, g.splits) > sm_count() / 2 ? 2 : 1;
+    } else {
+        g = pick_split(M, N, K);
+    }
     *splits = g.splits;
     *ctas_per_sm = g.per_sm;
 }

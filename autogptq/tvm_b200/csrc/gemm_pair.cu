@@ -1,4 +1,4 @@
-// Prefill dequant-GEMM for more than 64 rows of x (2- and 8-bit layers: any number): pairs of CTAs on one tcgen05 tile.
+// Prefill dequant-GEMM for more than 16 rows of x (2- and 8-bit layers: any number): pairs of CTAs on one tcgen05 tile.
 //
 //   y[M, N] = x[M, K] @ W[K, N] (+ bias),   W[k, n] = scales[g, n] * (q[k, n] - zero[g, n]),  rounded once to fp16
 //
@@ -682,6 +682,12 @@ size_t gemm_pair_partial_bytes(int M, int K, int N, int splits) {
     if (splits == 1) return 0;
     const int tn = pick_rows(M, N, K, splits);
     return (size_t)splits * ((M + tn - 1) / tn * tn) * N * sizeof(float);
+}
+
+// tiles of a launch (each of a pair of SMs takes one after the other)
+int gemm_pair_tiles(int M, int K, int N, int splits) {
+    const int tn = pick_rows(M, N, K, splits);
+    return (N + 2 * BN - 1) / (2 * BN) * ((M + tn - 1) / tn) * splits;
 }
 
 int gemm_pair_dispatch(const __half* x, const int32_t* qweight, const int32_t* qzeros, const __half* scales, const int32_t* g_idx,

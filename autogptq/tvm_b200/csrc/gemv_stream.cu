@@ -1002,9 +1002,7 @@ int max_groups_per_stage(const Plan& p, int group_size) {
 }
 
 // knobs (all optional, 0 = the default): [0] CTAs of one grid per SM that the cluster size is chosen for,
-// [1] CTAs per SM that the shared-memory footprint is sized for, [2] cap on ring units, [3] trigger of dependents
-// (1 after the own wait, 2 at entry, 3 once all weights are requested), [4] 1 = gather x from global memory,
-// [5] activation applied to x as it is read (Plan::xact)
+// [1] CTAs per SM that the shared-memory footprint is sized for, [2] activation applied to x as it is read (Plan::xact)
 // Clusters of `cluster` CTAs with `smem_bytes` of dynamic shared memory that the device holds at once (0: unknown).
 // Answers are kept per thread: a plan is made once per layer, a direct call asks on every launch.
 int resident_clusters(const void* kernel, int cluster, int smem_bytes) {
@@ -1054,15 +1052,14 @@ Plan make_plan(int M, int K, int N, int group_size, bool has_perm, const int* kn
     if (p.stage_units > longest) p.stage_units = longest;
     p.group_box = max_groups_per_stage(p, group_size);
     p.push = (c > 1 && red_bytes(M, c) <= kMaxRedBytes) ? 1 : 0;
-    p.early = (knobs && knobs[3] > 0) ? knobs[3] - 1 : 0;
-    p.xact = knobs ? knobs[5] : 0;
+    p.xact = knobs ? knobs[2] : 0;
     // layers with a gather, and several rows of x, take x through linear bulk copies when it is small enough
-    // (knobs[4] == 1 switches it off): small copies get bytes of their own, larger ones share the bytes of the partial
+    // : small copies get bytes of their own, larger ones share the bytes of the partial
     // sums (the CTA then joins its cluster's barrier only when it has finished with x).  One row without a gather: a
     // CTA reads only its own rows of x, and plain loads measured faster than the copy; with M rows the 2-byte loads
     // of all CTAs queue up at the same L2 lines (8 rows of a 4096 x 12288 layer: 27 us with loads).
     const int xcopy_bytes = M * (has_perm ? K : longest * kUnitRows) * 2;
-    p.xfull = ((!has_perm && M == 1) || (knobs && knobs[4] == 1)) ? 0 : (xcopy_bytes <= 4096 ? 2 : (xcopy_bytes <= kXFullMax ? 1 : 0));
+    p.xfull = (!has_perm && M == 1) ? 0 : (xcopy_bytes <= 4096 ? 2 : (xcopy_bytes <= kXFullMax ? 1 : 0));
     if (p.xact == 1) p.xfull = 0;   // gate and up are two runs of the row: no single copy (callers fuse SwiGLU only without a gather)
     int tail = part_bytes(M) + (p.push ? red_bytes(M, c) : 0);
     if (p.xfull == 2) tail += xcopy_bytes;
@@ -1100,7 +1097,6 @@ Plan make_plan(int M, int K, int N, int group_size, bool has_perm, const int* kn
     if (!fit_per_sm) fit_per_sm = 2;
     const int budget = kSmemPerSm / fit_per_sm - kSmemCtaReserve;
     int ring = (budget - fixed) / unit_bytes<BITS>();
-    if (knobs && knobs[2] > 0 && ring > knobs[2]) ring = knobs[2];
     if (ring > longest) ring = longest;
     if (ring > kMaxRing) ring = kMaxRing;
     if (ring < 2) ring = 2;
@@ -1247,8 +1243,7 @@ size_t gemv_stream_workspace_bytes(int M, int K, int N, int bits) {
     return kCounterBytes;  // only the status word: partial sums travel through distributed shared memory
 }
 
-// `knobs` (NULL = the defaults) overrides plan heuristics: b200gptq_gemv_tuned passes the first two, parameter sweeps
-// that link this translation unit directly use all of them.
+// `knobs` (NULL = the defaults): see make_plan.
 int gemv_stream_dispatch_tp(const __half* x, const int32_t* qweight, const int32_t* qzeros, const __half* scales,
                             const int32_t* x_perm, const __half* bias, __half* y, int M, int K, int N, int bits,
                             int group_size, void* workspace, cudaStream_t stream, const int* knobs, const TpArgs* tp) {
@@ -1257,46 +1252,6 @@ int gemv_stream_dispatch_tp(const __half* x, const int32_t* qweight, const int32
     if (bits == 3)
         return launch_stream<3>(x, qweight, qzeros, scales, x_perm, bias, y, M, K, N, group_size, workspace, stream, knobs, tp);
     return B200GPTQ_ERR_BITS;
-}
-
-int gemv_stream_dispatch_knobs(const __half* x, const int32_t* qweight, const int32_t* qzeros, const __half* scales,
-                               const int32_t* x_perm, const __half* bias, __half* y, int M, int K, int N, int bits,
-                               int group_size, void* workspace, cudaStream_t stream, const int* knobs) {
-    return gemv_stream_dispatch_tp(x, qweight, qzeros, scales, x_perm, bias, y, M, K, N, bits, group_size, workspace,
-                                   stream, knobs, nullptr);
-}
-
-// A prepared launch as an opaque object (b200gptq_gemv_plan_*): built once per (layer, row count), run many times.
-struct GemvStreamPlan {
-    int bits;
-    PreparedStream ps;
-};
-
-GemvStreamPlan* gemv_stream_plan_create(const int32_t* qweight, const __half* scales, bool has_perm, int M, int K, int N,
-                                        int bits, int group_size, const int* knobs, int* status_out) {
-    GemvStreamPlan* p = new (std::nothrow) GemvStreamPlan;
-    if (!p) { *status_out = B200GPTQ_ERR_CUDA; return nullptr; }
-    p->bits = bits;
-    *status_out = bits == 4 ? prepare_stream<4>(&p->ps, qweight, scales, has_perm, M, K, N, group_size, knobs)
-                            : prepare_stream<3>(&p->ps, qweight, scales, has_perm, M, K, N, group_size, knobs);
-    if (*status_out != B200GPTQ_OK) { delete p; return nullptr; }
-    return p;
-}
-
-int gemv_stream_plan_run(const GemvStreamPlan* p, const __half* x, const int32_t* qzeros, const int32_t* x_perm,
-                         const __half* bias, __half* y, void* workspace, cudaStream_t stream) {
-    return p->bits == 4 ? launch_prepared<4>(p->ps, x, qzeros, x_perm, bias, y, workspace, stream, nullptr)
-                        : launch_prepared<3>(p->ps, x, qzeros, x_perm, bias, y, workspace, stream, nullptr);
-}
-
-void gemv_stream_plan_destroy(GemvStreamPlan* p) { delete p; }
-
-int gemv_stream_dispatch(const __half* x, const int32_t* qweight, const int32_t* qzeros, const __half* scales,
-                         const int32_t* g_idx, const int32_t* x_perm, const __half* bias, __half* y, int M, int K,
-                         int N, int bits, int group_size, void* workspace, cudaStream_t stream) {
-    if (g_idx) return B200GPTQ_ERR_GROUPS;
-    return gemv_stream_dispatch_knobs(x, qweight, qzeros, scales, x_perm, bias, y, M, K, N, bits, group_size,
-                                      workspace, stream, nullptr);
 }
 
 }  // namespace b200gptq

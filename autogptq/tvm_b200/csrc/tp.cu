@@ -108,7 +108,7 @@ int b200gptq_gemv_tp_ex(const void* x, const int32_t* qweight, const int32_t* qz
     if (slices_per_sm < 0 || slices_per_sm > 8 || ctas_per_sm < 0 || ctas_per_sm > 4) return B200GPTQ_ERR_SHAPE;
     if (input_act != B200GPTQ_ACT_NONE && input_act != B200GPTQ_ACT_SWIGLU && input_act != B200GPTQ_ACT_RELU)
         return B200GPTQ_ERR_SHAPE;
-    const int knobs[6] = {slices_per_sm, ctas_per_sm, 0, 0, 0, input_act};
+    const int knobs[3] = {slices_per_sm, ctas_per_sm, input_act};
     if (!x || !qweight || !qzeros || !scales || !y) return B200GPTQ_ERR_NULL_POINTER;
     if (bits != 2 && bits != 3 && bits != 4 && bits != 8) return B200GPTQ_ERR_BITS;
     if (K <= 0 || N <= 0 || K % 32 != 0 || N % 32 != 0 || M < 1 || M > 8) return B200GPTQ_ERR_SHAPE;

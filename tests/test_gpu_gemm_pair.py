@@ -1,4 +1,4 @@
-"""The tensor-core kernel for pairs of SMs (more than 64 rows; 2 and 8 bits at any number) at the edges of its split: column
+"""The tensor-core kernel for pairs of SMs (more than 16 rows; 2 and 8 bits at any number) at the edges of its split: column
 tiles with one CTA or part of one beyond the layer, cut k-tiles and units, one to four groups per unit, more tiles than pairs
 (persistent), one and two sets of accumulators, and K split over pairs."""
 import pytest
@@ -22,6 +22,10 @@ CASES = [
     (8, 96, 640, 32, 513, False),
     (4, 11008, 4096, 64, 77, False),      # four runs of K
     (8, 11008, 1056, 32, 128, True),
+    (4, 992, 96, 32, 17, False),          # fewest rows of 3- and 4-bit layers
+    (3, 4096, 4128, 128, 33, True),       # four runs, seventeen pairs of column tiles
+    (4, 2048, 19232, -1, 64, False),      # a second tile for some pairs
+    (3, 4064, 64, 32, 96, False),         # four runs above 64 rows
 ]
 
 
@@ -46,3 +50,6 @@ def test_gemm_against_dequantised_product(bits, K, N, gs, M, gather):
 def test_split_of_the_cases_above():
     assert ops.gemm_split(77, 11008, 4096, 4)[0] == 4
     assert ops.gemm_split(128, 11008, 1056, 8)[0] == 4
+    assert ops.gemm_split(33, 4096, 4128, 3) == (4, 1)
+    assert ops.gemm_split(64, 2048, 19232, 4) == (1, 2)
+    assert ops.gemm_split(96, 4064, 64, 3)[0] == 4
