@@ -1,4 +1,5 @@
-// Decode GEMV, streaming form (M <= 8, bits in {3,4}, groups = k / group_size).
+// Decode GEMV of the tensor-parallel path, streaming form (M <= 8, bits in {3,4}, groups = k / group_size): clusters that can
+// hand their sums to the exchange between GPUs.  (On one GPU: gemv_strip.cuh.)
 //
 //   y[m, n] = sum_k x[m, xk(k)] * scales[g, n] * (q[k, n] - zero[g, n]),   g = k / group_size
 //
@@ -416,8 +417,6 @@ struct Plan {
     int push;         // 1: the K slices are combined by pushing partial sums into the first CTA's shared memory
     int xfull;        // x is bulk-copied to shared memory before it is re-ordered (the whole of x for layers with x_perm,
                       // the CTA's rows otherwise): 2 into bytes of its own, 1 into the bytes of the partial sums, 0 not
-    int early;        // when dependents may be launched: 0 once this CTA has passed its own wait, 1 as soon as it runs,
-                      // 2 once all its weights are requested
     int xact;         // activation applied to x as it is read: 0 none, 1 SwiGLU (x holds [gate | up], 2 K values per
                       // row), 2 ReLU -- the element-wise kernel between two linears of a decode step folded into the second
 };
@@ -561,7 +560,6 @@ gemv_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     // matched by the wait in front of the first store into another CTA; a CTA that gathers x through `part` / `red`
     // arrives only when it has finished with those bytes
     if (push && !xfull_aliased) cluster_arrive();
-    if (plan.early == 1) asm volatile("griddepcontrol.launch_dependents;");
 
     const int g = lane >> 2, j = lane & 3;
     const int lane_col = warp * 32 + 4 * g;  // first of the lane's 4 columns inside the column group
@@ -610,7 +608,7 @@ gemv_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     };
 
     int slot = 0, round = 0;
-    bool first = true, triggered = false;
+    bool first = true;
     for (int kb_a = kb_begin, st = 0; kb_a < kb_end; kb_a += S, ++st) {
         const int kb_b = min(kb_a + S, kb_end);
         const int nu = kb_b - kb_a;
@@ -649,7 +647,7 @@ gemv_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         // scales, zero-points and gather indices requested.
         auto await_x = [&]() {
             asm volatile("griddepcontrol.wait;" ::: "memory");
-            if (plan.early == 0) asm volatile("griddepcontrol.launch_dependents;");
+            asm volatile("griddepcontrol.launch_dependents;");
             if (use_xfull) {
                 // A gather straight from global memory would send every CTA's 2-byte requests to the same few
                 // L2 lines at the same moment; one linear bulk copy of x per CTA and a gather from shared memory
@@ -798,12 +796,6 @@ gemv_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         bool scales_ready = false;
 #pragma unroll 1
         for (int kb = kb_a; kb < kb_b; ++kb) {
-            if (plan.early == 2 && !triggered && kb + R >= kb_end) {
-                // every unit of this CTA has been requested: CTAs of the next launch may come in and queue their
-                // weights behind it without delaying it
-                asm volatile("griddepcontrol.launch_dependents;");
-                triggered = true;
-            }
             mbar_wait(full_bar(slot), round & 1, &gave_up);
             uint4 cur[T::kVecs];
             const uint8_t* src = ring + slot * UB;

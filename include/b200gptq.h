@@ -100,7 +100,7 @@ B200GPTQ_API int b200gptq_workspace_status(const void* workspace, void* stream, 
  *           were re-ordered by b200gptq_sort_rows() is evaluated.
  *
  * Any g_idx is accepted, but g_idx == NULL is the fast-path contract: only then
- * (and with bits in {3,4}, K and group_size multiples of 128) does the call run
+ * (and with groups of whole 32-row blocks) does the call run
  * the streaming tensor-map kernel; every non-NULL g_idx, even one equal to
  * k / group_size, runs the general kernel, which looks groups up per row block.
  * Callers that hold a checkpoint's g_idx should compare it with k / group_size
@@ -187,7 +187,7 @@ B200GPTQ_API int b200gptq_gemv_path(int M, int K, int N, int bits, int group_siz
 
 /*
  * Prefill GEMM, any M >= 1 (meant for M >= 16):  y = x @ W (+ bias) on the
- * tcgen05 tensor cores with fp32 accumulators in tensor memory.  bits in {3,4}.
+ * tcgen05 tensor cores with fp32 accumulators in tensor memory.  bits in {2,3,4,8}.
  * Replaces the TVM `m16 .. m256` kernel launches of pycuda_warpper.py:150-189
  * (kernels: src/kernels/gemm_kernel.cu:25-142); no M padding is needed.
  *
