@@ -86,8 +86,10 @@ int gemv_strip_prepare(GemvStripPlan* p, const int32_t* qweight, const int32_t* 
     auto choose = [&](int W) {
         Choice c = {W, 0, 0, 0, 0, 1 << 30};
         // (a gather works from a copy of x that the sums overwrite: it needs every unit's x kept)
-        // x that is not kept: as many units ahead as leave the weights three slots, one ahead being the least
-        for (int bufs = 5; bufs >= (mode == kSeveral && !gather ? 2 : 5) && c.bufs != 5; --bufs)
+        // x that is not kept: as many units ahead as leave the weights three slots, one ahead being the least.  Nine rows and
+        // more are fetched again in every pass rather than kept where that saves a pass (9216 x 9216, 2 bits, 9 rows: 24 ->
+        // 18.5 us).
+        for (int bufs = 5; bufs >= (mode == kSeveral && !gather ? 2 : 5) && (nt == 2 || c.bufs != 5); --bufs)
             for (int t = 1; t <= tmax && t <= s.per_cta; ++t) {
                 const int slot = slot_bytes(bits, t) + const_bytes(bits, t, s.rows_g);
                 const int sums = W * M * t * kStripCols * 4, copy = gather || mode != kSeveral ? M * K * 2 : 0;
