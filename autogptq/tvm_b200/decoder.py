@@ -436,7 +436,7 @@ class GPTQDecoder:
         depends on the kernels around the GEMV (4-5 % of a Llama-7B step, 2-3 % of an OPT-66B step on one B200).
         Position and tokens are restored; cache rows past the current position are used as scratch.  With several
         ranks every rank calls this at the same point and all take the split that is fastest for the slowest rank.
-        Returns {kind: tuning}; a batch of more than 8 rows does not run GEMVs and is left alone."""
+        Returns {kind: tuning}; a batch of more than 8 rows is left alone."""
         kinds = ("qkv", "o", "up", "down")
         chosen = {k: getattr(self.layers[0], k).gemv_tuning for k in kinds}
         if self.batch > 8 or self._pos_host + steps + 3 > self.cfg.max_seq:

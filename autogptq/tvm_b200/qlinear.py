@@ -4,8 +4,8 @@ Mirrors the constructor / ``pack`` / ``forward`` surface of the reference's TVM
 module (``auto_gptq/nn_modules/qlinear_tvm.py:10-158``) but keeps the standard
 AutoGPTQ buffers of ``auto_gptq/nn_modules/qlinear.py:40-59`` (``qweight``,
 ``qzeros``, ``scales``, ``g_idx``, ``bias``), so ordinary GPTQ checkpoints load
-unchanged.  ``forward`` runs on the GPU only: M <= 8 rows go to the decode GEMV,
-more rows to the tcgen05 dequant-GEMM.  There is no M padding, no per-shape
+unchanged.  ``forward`` runs on the GPU only: up to 16 rows (8 where groups cut
+32-row blocks) go to the decode GEMV, more rows to the tcgen05 dequant-GEMM.  There is no M padding, no per-shape
 kernel cache and no tuner (the reference's ``tvm_untils/cache.py`` and
 ``pycuda_warpper.py`` have no counterpart here).
 """
