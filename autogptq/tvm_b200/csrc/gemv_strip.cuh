@@ -480,24 +480,32 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
 
     const bool gather = plan.gather != 0;
     // What does not need x is done before the wait.  Byte planes: a lane's rows of a 128-row unit, and where they lie in x for its
-    // first unit (3 bits, 4096 x 11008 with a gather 9.4 -> 8.2 us, without 8.5 -> 7.9).  3 bits in fp16: where the rows of its
-    // first 32-row block lie.
-    int row[8], pre[8], first[8];
+    // first two units (3 bits, 4096 x 11008 with a gather 9.4 -> 8.2 us, without 8.5 -> 7.9).  3 bits in fp16: where its four rows
+    // of the first units lie.
+    int row[8], pre[8], first[2][8];
     if constexpr (INT) {
         I::item((lane >> 2) & 3, lane & 3, row, pre);
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
             const int k = (u_begin + (lane >> 4)) * kUnit + row[e];
-            first[e] = !gather || k >= K ? min(k, K - 1) : __ldg(x_perm + k);
-            asm volatile("" : "+r"(row[e]), "+r"(pre[e]), "+r"(first[e]));
+            first[0][e] = !gather || k >= K ? min(k, K - 1) : __ldg(x_perm + k);
+            asm volatile("" : "+r"(row[e]), "+r"(pre[e]), "+r"(first[0][e]));
+        }
+        if (gather && nu > 2) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                first[1][e] = __ldg(x_perm + min((u_begin + 2 + (lane >> 4)) * kUnit + row[e], K - 1));
+                asm volatile("" : "+r"(first[1][e]));
+            }
         }
     }
     constexpr bool BLOCKS = ONE && BITS == 3 && SUB == 1;
-    uint4 first4[8];
+    constexpr int EARLY = 4;
+    uint4 first4[EARLY];
     if (BLOCKS && gather) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            first4[e] = __ldg(reinterpret_cast<const uint4*>(x_perm + min(u_begin * kUnit + 32 * lane + 4 * e, K - 4)));
+        for (int e = 0; e < EARLY; ++e) {
+            first4[e] = __ldg(reinterpret_cast<const uint4*>(x_perm + min((u_begin + e) * kUnit + 4 * lane, K - 4)));
             asm volatile("" : "+r"(first4[e].x), "+r"(first4[e].y), "+r"(first4[e].z), "+r"(first4[e].w));
         }
     }
@@ -586,12 +594,22 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     if constexpr (ONE) {
         // the warp's slice of x in the order of the B registers: piece (unit, quad lane, step) is four registers
         if constexpr (BITS == 3 && SUB == 1) {
-            for (int i = lane; i < nu * 4; i += 32) {   // a 32-row block at a time: its pairs cross the 8-row pieces
+            // a 32-row block at a time: its pairs cross the 8-row pieces.  A gather picks its rows with all lanes first, into the
+            // bytes that the block is written back to.
+            if (gather) {
+                auto put = [&](int u, uint2 v) { *reinterpret_cast<uint2*>(p_x + u * kUnit * 2 + 8 * lane) = v; };
+#pragma unroll
+                for (int u = 0; u < EARLY; ++u)
+                    if (u < nu) put(u, pick4(0, (u_begin + u) * kUnit + 4 * lane, first4[u]));
+                for (int u = EARLY; u < nu; ++u) put(u, load4(0, (u_begin + u) * kUnit + 4 * lane));
+                __syncwarp();
+            }
+            for (int i = lane; i < nu * 4; i += 32) {
                 uint32_t xr[16], b[16];
 #pragma unroll
                 for (int e = 0; e < 8; ++e) {
-                    const int k = u_begin * kUnit + 32 * i + 4 * e;
-                    const uint2 v = gather && i == lane ? pick4(0, k, first4[e]) : load4(0, k);
+                    const uint2 v = gather ? *reinterpret_cast<const uint2*>(p_x + i * 64 + 8 * e)
+                                           : load4(0, u_begin * kUnit + 32 * i + 4 * e);
                     xr[2 * e] = v.x; xr[2 * e + 1] = v.y;
                 }
                 L::b_block(xr, b);
@@ -625,10 +643,10 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                 const bool active = q < nu * 16;
                 const int k0 = (u_begin + u) * kUnit;
                 unsigned short h[8];
-                if (staged && q0 == 0 && (BITS != 4 || gather)) {
+                if (staged && (q0 == 0 || (gather && q0 == 32)) && (BITS != 4 || gather)) {
 #pragma unroll
                     for (int e = 0; e < 8; ++e) {
-                        h[e] = active && k0 + row[e] < K ? raw[(size_t)m * K + first[e]] : (unsigned short)0;
+                        h[e] = active && k0 + row[e] < K ? raw[(size_t)m * K + (q0 == 0 ? first[0][e] : first[1][e])] : (unsigned short)0;
                         if (plan.xact) h[e] = (unsigned short)act_relu2(h[e]);
                     }
                 } else if constexpr (BITS == 4) {      // a run of eight rows
