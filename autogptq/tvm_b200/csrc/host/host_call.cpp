@@ -40,7 +40,7 @@ struct GemvEntry {
 struct Layer {
     PyObject_HEAD
     int K, N, bits, group_size, device;
-    // the buffers this object was prepared for: addresses of qweight / g_idx, identity of the others
+    // the buffers this object was prepared for: addresses of qweight / g_idx, identity and addresses of the others
     const void *qweight_at, *g_idx_at;
     PyObject *qzeros, *scales, *bias, *tuning;
     GemvEntry gemv[kMaxGemvRows + 1];
@@ -52,6 +52,9 @@ struct Layer {
     PyObject* keep;       // keeps the tensors behind those addresses alive
 };
 
+inline const void* tensor_address(PyObject* t) {
+    return t && THPVariable_Check(t) ? THPVariable_Unpack(t).unsafeGetTensorImpl()->data() : nullptr;
+}
 inline bool address_is(PyObject* dict, PyObject* key, const void* at) {
     PyObject* t = PyDict_GetItem(dict, key);
     return t && THPVariable_Check(t) && THPVariable_Unpack(t).unsafeGetTensorImpl()->data() == at;
@@ -94,6 +97,10 @@ PyObject* layer_run(PyObject* self_, PyObject* const* args, Py_ssize_t nargs) {
     if (!bias) bias = PyDict_GetItem(dict, s_bias);
     if ((bias ? bias : Py_None) != self->bias || PyDict_GetItem(buffers, s_qzeros) != self->qzeros ||
         PyDict_GetItem(buffers, s_scales) != self->scales)
+        Py_RETURN_NONE;
+    // (`tensor.data = other` keeps the tensor and moves its numbers)
+    if (tensor_address(self->qzeros) != self->qzeros_run || tensor_address(self->scales) != self->scales_run ||
+        tensor_address(self->bias) != self->bias_run)
         Py_RETURN_NONE;
     const bool gemv = M <= self->gemv_rows;
     const GemvEntry* e = gemv ? &self->gemv[M] : nullptr;
@@ -141,10 +148,6 @@ PyObject* layer_set_gemv(PyObject* self_, PyObject* args) {
     Py_RETURN_NONE;
 }
 
-const void* tensor_address(PyObject* t) {
-    return t && THPVariable_Check(t) ? THPVariable_Unpack(t).unsafeGetTensorImpl()->data() : nullptr;
-}
-
 // Layer(K, N, bits, group_size, device, module_dict, gemm_ok, gemv_rows, qweight_run, g_idx_run, x_perm)
 PyObject* layer_new(PyTypeObject* type, PyObject* args, PyObject*) {
     int K, N, bits, group_size, device, gemm_ok, gemv_rows;
@@ -163,7 +166,8 @@ PyObject* layer_new(PyTypeObject* type, PyObject* args, PyObject*) {
         PyErr_SetString(PyExc_TypeError, "the module lacks a buffer");
         return nullptr;
     }
-    PyObject* keep = PyTuple_Pack(7, qw, gi, perm, pz, ps, bias ? bias : Py_None, tuning ? tuning : Py_None);
+    // (the stored qweight and g_idx too: as long as they live nothing else can come to lie at their addresses)
+    PyObject* keep = PyTuple_Pack(9, pq, pg, qw, gi, perm, pz, ps, bias ? bias : Py_None, tuning ? tuning : Py_None);
     if (!keep) return nullptr;
     Layer* self = reinterpret_cast<Layer*>(type->tp_alloc(type, 0));
     if (!self) { Py_DECREF(keep); return nullptr; }

@@ -55,6 +55,11 @@ def _pack_fields(vals: torch.Tensor, bits: int) -> torch.Tensor:
     return words.to(torch.int32)
 
 
+def _same(a, b) -> bool:
+    """Of two results of ``QuantLinear._constants``: the same tensors at the same addresses."""
+    return all(s is t for s, t in zip(a[:3], b[:3])) and a[3:] == b[3:]
+
+
 class QuantLinear(nn.Module):
     def __init__(self, bits, groupsize, infeatures, outfeatures, bias):
         super().__init__()
@@ -90,7 +95,7 @@ class QuantLinear(nn.Module):
         self.tp_bias = None
         # (slices_per_sm, ctas_per_sm) of b200gptq_gemv_tuned, or None for the library defaults
         self.gemv_tuning = None
-        self._plans = {}           # row count -> ops.GemvPlan (prepared launches of the decode GEMV)
+        self._plans = {}           # (rows, tuning, activation) -> (ops.GemvPlan, the _constants it was made from)
         self._native = None        # _host.Layer: the prepared call in native code, made by the first forward
 
     # ---- offline packing (CPU) ----------------------------------------------------------
@@ -214,12 +219,7 @@ class QuantLinear(nn.Module):
         kw = dict(bias=self.bias, x_perm=self._x_perm)
         args = (self._qweight_run, self.qzeros, self.scales, self._g_idx_run, self.bits, self.groupsize)
         if M <= self._gemv_rows:
-            key = (M, self.gemv_tuning)
-            plan = self._plans.get(key)
-            if plan is None or plan._keep[5] is not self.bias:
-                plan = self._plans[key] = ops.GemvPlan(self._qweight_run, self.qzeros, self.scales, self._g_idx_run,
-                                                     self._x_perm, self.bias, M, self.bits, self.groupsize,
-                                                     self.gemv_tuning)
+            plan = self._plan(M)
             self._prepare_native(M, plan)
             with torch.cuda.device(x2.device):
                 y = plan.run(x2)
@@ -244,14 +244,29 @@ class QuantLinear(nn.Module):
                 ops.gemv(x2[m0:m0 + GEMV_MAX_M], *args, out=y[m0:m0 + GEMV_MAX_M], **kw)
         return y.reshape(out_shape)
 
+    def _constants(self):
+        """What a prepared launch holds beside the rows themselves: these tensors, and where their numbers lie (``.data``
+        may have been replaced)."""
+        t = (self.qzeros, self.scales, self.bias)
+        return t + tuple(None if v is None else v.data_ptr() for v in t)
+
+    def _plan(self, rows: int, input_act: int = 0):
+        """The prepared GEMV of this row count, made anew when a tensor that it points to has been replaced."""
+        key, now = (rows, self.gemv_tuning, input_act), self._constants()
+        made = self._plans.get(key)
+        if made is None or not _same(made[1], now):
+            plan = ops.GemvPlan(self._qweight_run, self.qzeros, self.scales, self._g_idx_run, self._x_perm, self.bias, rows,
+                                self.bits, self.groupsize, self.gemv_tuning, input_act)
+            made = self._plans[key] = (plan, now)
+        return made[0]
+
     def _prepare_native(self, rows: int = 0, plan=None):
         """Make the native call object for the current buffers (once), and hand it the plan of one more row count."""
         if not self.qweight.is_cuda:
             return
-        buffers = self._buffers
-        state = (self.gemv_tuning, self.bias, buffers["qzeros"], buffers["scales"])
-        if self._native is None or any(a is not b for a, b in zip(self._native_state, state)):
-            self._native_state = state
+        now = self._constants()
+        if self._native is None or not _same(self._native_state, now) or self._native_tuning is not self.gemv_tuning:
+            self._native_state, self._native_tuning = now, self.gemv_tuning
             self._native = _lib._host.Layer(self.infeatures, self.outfeatures, self.bits, self.groupsize,
                                             self.qweight.device.index, self.__dict__, self._gemm_ok, self._gemv_rows,
                                             self._qweight_run, self._g_idx_run, self._x_perm)
@@ -276,12 +291,7 @@ class QuantLinear(nn.Module):
         if not u2.is_contiguous():
             u2 = u2.contiguous()
         M = u2.shape[0]
-        key = (M, self.gemv_tuning, input_act)
-        plan = self._plans.get(key)
-        if plan is None or plan._keep[5] is not self.bias:
-            plan = self._plans[key] = ops.GemvPlan(self._qweight_run, self.qzeros, self.scales, self._g_idx_run,
-                                                 self._x_perm, self.bias, M, self.bits, self.groupsize,
-                                                 self.gemv_tuning, input_act)
+        plan = self._plan(M, input_act)
         with torch.cuda.device(u2.device):
             y = plan.run(u2)
         return y.reshape(u.shape[:-1] + (self.outfeatures,))
