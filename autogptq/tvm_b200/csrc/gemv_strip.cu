@@ -78,15 +78,15 @@ int gemv_strip_prepare(GemvStripPlan* p, const int32_t* qweight, const int32_t* 
     // One CTA per SM: each takes the same whole number of strips.
     s.per_cta = (s.strips + sm_count() - 1) / sm_count();
     const int plane_bytes = (s.units * M * ((bits == 3 ? 5 : 4) * 128 + 8) + 15) / 16 * 16;
-    const int mode = M <= 2 && bits != 8 && sub == 1 && s.per_cta > (bits == 3 ? 2 * M : M) && plane_bytes <= 96 * 1024 ? kInt
-                   : (M == 1 && K <= 65536 ? kOne : kSeveral);
-    const int tmax = mode == kInt ? 4 : (sub == 1 && nt == 1 ? 3 : 2);
+    int mode = M <= 2 && bits != 8 && sub == 1 && s.per_cta > (bits == 3 ? 2 * M : M) && plane_bytes <= 96 * 1024 ? kInt
+             : (M == 1 && K <= 65536 ? kOne : kSeveral);
     s.rows_g = sub == 1 ? 1 : (s.spg == 1 ? 4 : (s.spg == 2 ? 2 : 3));
     // Strips of a pass for W warps: a unit costs about half a strip's work on top of its strips, and the last pass is a whole
     // one.  The rings take at least two slots and what is left of the shared memory.
     struct Choice { int W, T, ring, fixed, bufs, cost; };
     auto choose = [&](int W) {
         Choice c = {W, 0, 0, 0, 0, 1 << 30};
+        const int tmax = mode == kInt ? 4 : (sub == 1 && nt == 1 ? 3 : 2);
         // (a gather works from a copy of x that the sums overwrite: it needs every unit's x kept)
         // x that is not kept: as many units ahead as leave the weights three slots, one ahead being the least.  Nine rows and
         // more are fetched again in every pass rather than kept where that saves a pass (9216 x 9216, 2 bits, 9 rows: 24 ->
@@ -110,6 +110,15 @@ int gemv_strip_prepare(GemvStripPlan* p, const int32_t* qweight, const int32_t* 
     // leaves some idle and a long row of x leaves their rings little room (36864 x 9216, 3 bits: 47 against 43).  Sixteen rows
     // of x take more than half of a thread's registers.
     Choice c = choose(8);
+    if (mode == kOne && !gather) {
+        // A long row in operand order and its copy, 4 bytes per value, leave the rings little room or none (8 bits from 39 000
+        // values on, 3 and 4 bits from 46 000).  The form for several rows keeps x once, or a few units of it, and is taken where
+        // that allows wider passes (4 bits, 40960 x 8192: 59 against 48 us; 8 bits, 32768 x 8192: 66 against 45).
+        mode = kSeveral;
+        const Choice several = choose(8);
+        if (!c.T || several.cost < c.cost) c = several;
+        else mode = kOne;
+    }
     if (nt == 1 && ctas_per_sm <= 1) {
         const Choice w = choose(16);
         const bool pays = s.units >= 16 && 10 * w.cost <= 11 * c.cost && (mode != kOne || K <= 16384);

@@ -23,6 +23,9 @@ CASES = [
     (3, 4224, 288, 128, True),
     (3, 32768, 64, 128, False),        # planes of one row do not fit: fp16, the row kept whole
     (3, 69632, 32, 128, False),        # nor does the row
+    (4, 49152, 64, 128, False),        # nor the row and its copy, one row included
+    (2, 65536, 96, 64, False),
+    (8, 40960, 32, 32, False),
     (4, 992, 96, 32, True),
     (4, 1056, 64, -1, False),          # one group, cut last unit
     (4, 640, 19008, 128, False),       # 594 strips: five per CTA, overlapping passes
@@ -74,4 +77,16 @@ def test_plan_of_nine_to_sixteen_rows_vs_oracle(bits, K, N, gs, gather, M):
     norm = np.linalg.norm(xg.numpy().astype(np.float64), axis=1, keepdims=True) * np.abs(W.astype(np.float64)).max()
     err = np.abs(plan.run(x.to(DEV)).cpu().numpy().astype(np.float64) - ref)
     assert np.all(err <= 2.0 ** -10 * np.abs(ref) + 2.0 ** -11 * norm), err.max()
+    ops.check_status(DEV)
+
+
+@pytest.mark.parametrize("bits,K", [(4, 1024), (3, 4096), (4, 57344)])     # planes or fp16, the row kept, and too long for that
+@pytest.mark.parametrize("gated", [False, True])
+@pytest.mark.parametrize("M", [1, 3])
+def test_folded_activation_equals_the_kernel_in_front(bits, K, gated, M):
+    layer = synth.make_layer(bits, K, 4832, 128, False, seed=K, device=DEV)
+    u = synth.make_x(M, 2 * K if gated else K, seed=M, device=DEV)
+    a = ops.act(u, torch.empty((M, K), dtype=torch.float16, device=DEV), K, gated)
+    args = (layer.qweight, layer.qzeros, layer.scales, None, bits, 128)
+    assert torch.equal(ops.gemv(u, *args, input_act=1 if gated else 2), ops.gemv(a, *args))
     ops.check_status(DEV)
