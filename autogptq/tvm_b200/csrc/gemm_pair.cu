@@ -29,19 +29,20 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "ring_rules.h"
 
 namespace b200gptq {
 
 namespace {
 
-constexpr int BN = 128;                  // columns per CTA
-constexpr int BK = 64;                   // rows of K per stage
-constexpr int kGroups = 4, kGroupWarps = 4;
+constexpr int BN = kPairColumns;         // columns per CTA
+constexpr int BK = kPairKTile;           // rows of K per stage
+constexpr int kGroups = kPairGroups, kGroupWarps = 4;
 constexpr int kFirstEpiWarp = 4, kEpiWarps = 8, kFirstWeightWarp = kFirstEpiWarp + kEpiWarps;
 constexpr int kThreads = 32 * (kFirstWeightWarp + kGroups * kGroupWarps);
-constexpr int kMaxStages = 14, kMaxW = 16;
-constexpr int kTmemCols = 512;           // accumulators in columns [0, TN), 32 columns of A per stage behind them
-constexpr int kSmemMax = 222 * 1024;
+constexpr int kMaxStages = kPairMaxStages, kMaxW = kPairMaxSlots;
+constexpr int kTmemCols = kPairTmemCols; // accumulators in columns [0, TN), 32 columns of A per stage behind them
+constexpr int kSmemMax = kPairSmem;
 constexpr int kStatusWord = kMaxCounters - 1;
 constexpr int kMaxSplits = 4;
 
@@ -219,11 +220,6 @@ template <> struct Block<3> {
     }
 };
 
-__host__ __device__ constexpr int zero_words(int bits) { return bits % 4 == 0 ? 4 * bits : (4 * bits + 3 + 3) & ~3; }
-__host__ __device__ constexpr int w_unit_bytes(int bits) { return 4 * bits * BN * 4; }      // packed weights of 128 rows
-// a slot of the weight ring: packed rows | scales [group][column] | zero-point words of each group
-__host__ __device__ constexpr int w_slot_bytes(int bits, int rows_g) { return w_unit_bytes(bits) + rows_g * (BN * 2 + 128); }
-
 // Field of column `col` (0 .. 127) plus one, from words in shared memory.
 template <int BITS>
 __device__ __forceinline__ uint32_t zero_of(const uint8_t* row, int col) {
@@ -236,6 +232,7 @@ __device__ __forceinline__ uint32_t zero_of(const uint8_t* row, int col) {
 
 struct PairArgs {
     int M, K, N, spg, groups_in_slot, TN, S, SW, acc_sets, splits;
+    int ahead;                           // fills of the weight ring in flight at most (ring_rules.h)
     int pairs, row_tiles, tiles;         // 256-column tiles, TN-row tiles, all tiles (with the runs of K)
     unsigned int spg_inv;                // ceil(2^32 / spg), spg = 32-row blocks per group
 };
@@ -261,7 +258,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     const int RB = K / 32, KT_all = (K + BK - 1) / BK, U_all = (K + 127) / 128;
     const int cluster = blockIdx.x >> 1, clusters = gridDim.x >> 1;
     const uint32_t x_bytes = (uint32_t)TH * BK * 2;
-    const int w_slot = w_slot_bytes(BITS, p.groups_in_slot);
+    const int w_slot = pair_slot_bytes(BITS, p.groups_in_slot);
     const uint32_t w_off = S * x_bytes;
 
     const uint32_t bar_base = smem_u32(bars);
@@ -318,24 +315,30 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
         // ===== packed weights, scales, zero-points.  (With a g_idx the number of groups is not known here, so boxes could not
         //       be clipped to the arrays: the weight warps read scales and zero-points themselves.) =====
         const int rows_g = g_idx ? 0 : p.groups_in_slot;
-        const uint32_t tx = w_unit_bytes(BITS) + rows_g * (BN * 2 + zero_words(BITS) * 4);
-        int s = 0, round = 0;
+        const uint32_t tx = pair_unit_bytes(BITS) + rows_g * (BN * 2 + pair_zero_words(BITS) * 4);
+        int s = 0, round = 0, left = p.ahead, ls = 0, lround = 0;     // the fill that has to have completed: slot ls
         bool ok = true;
         for (int t = cluster; t < p.tiles && ok; t += clusters) {
             const Tile v = tile_at(t);
             const int zn = v.n0 / 32 * BITS;
             for (int u = v.u0; u < v.u1; ++u) {
                 const int g0 = group_at(4 * u);
-                if (round > 0) ok = mbar_wait(w_empty(s), (round - 1) & 1, &abort_flag);
+                if (left > 0) {
+                    --left;
+                } else {                                              // (long done when a slot becomes free, as a rule)
+                    ok = mbar_wait(w_full(ls), lround & 1, &abort_flag);
+                    if (++ls == SW) { ls = 0; ++lround; }
+                }
+                if (round > 0) ok = ok && mbar_wait(w_empty(s), (round - 1) & 1, &abort_flag);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 if (elect_one()) {
                     const uint32_t dst = base + w_off + s * w_slot, bar = w_full(s);
                     mbar_expect(bar, tx);
                     tma_2d(dst, &tmap_w, v.n0, u * 4 * BITS, bar);
-                    if (rows_g) tma_2d(dst + w_unit_bytes(BITS), &tmap_s, v.n0, g0, bar);
+                    if (rows_g) tma_2d(dst + pair_unit_bytes(BITS), &tmap_s, v.n0, g0, bar);
                     for (int r = 0; r < rows_g; ++r)
-                        tma_1d(dst + w_unit_bytes(BITS) + rows_g * BN * 2 + r * 128, &tmap_z, ((g0 + r) * zwords + zn) & ~3, bar);
+                        tma_1d(dst + pair_unit_bytes(BITS) + rows_g * BN * 2 + r * 128, &tmap_z, ((g0 + r) * zwords + zn) & ~3, bar);
                 }
                 __syncwarp();
                 if (++s == SW) { s = 0; ++round; }
@@ -435,8 +438,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
                         // (one group in the slot: both blocks read the same constants)
                         const int r = p.groups_in_slot == 1 ? 0 : min(group_at(rb + h) - g0, p.groups_in_slot - 1);
                         const int early = early_words ? ((g0 + r) * zwords + v.n0 / 32 * BITS) & 3 : 0;
-                        sc[h] = reinterpret_cast<const __half*>(src + w_unit_bytes(BITS) + r * BN * 2)[col];
-                        z[h] = zero_of<BITS>(src + w_unit_bytes(BITS) + p.groups_in_slot * BN * 2 + r * 128 + 4 * early, col);
+                        sc[h] = reinterpret_cast<const __half*>(src + pair_unit_bytes(BITS) + r * BN * 2)[col];
+                        z[h] = zero_of<BITS>(src + pair_unit_bytes(BITS) + p.groups_in_slot * BN * 2 + r * 128 + 4 * early, col);
                     }
                 }
                 __syncwarp();
@@ -615,13 +618,11 @@ int launch(const __half* x, const int32_t* qweight, const int32_t* qzeros, const
     a.spg_inv = (unsigned int)((0x100000000ULL + a.spg - 1) / a.spg);                 // (not used for 1)
     a.groups_in_slot = a.spg % 4 == 0 || groups == 1 ? 1 : (a.spg == 1 ? 4 : (a.spg == 2 ? 2 : 3));
     const int TN = a.TN = pick_rows(M, N, K, splits);
-    a.acc_sets = TN <= 128 ? 2 : 1;
-    const int x_stage = TN / 2 * BK * 2, w_slot = w_slot_bytes(BITS, a.groups_in_slot);
-    a.S = (kTmemCols - a.acc_sets * TN) / 32;
-    if (a.S > kMaxStages) a.S = kMaxStages;
-    a.SW = (kSmemMax - 1024 - a.S * x_stage) / w_slot;
-    if (a.SW > kMaxW) a.SW = kMaxW;
-    if (a.SW < 3) return B200GPTQ_ERR_TOO_LARGE;
+    // (with K split every pair has one tile, so that no group meets the end of one)
+    const PairRings rings = pair_rings(BITS, a.groups_in_slot, TN, splits > 1 ? 2 : (K + BK - 1) / BK);
+    a.acc_sets = rings.acc_sets; a.S = rings.stages; a.SW = rings.slots; a.ahead = rings.ahead;
+    const int x_stage = TN / 2 * BK * 2, w_slot = pair_slot_bytes(BITS, a.groups_in_slot);
+    if (a.ahead < 1) return B200GPTQ_ERR_TOO_LARGE;
     const int smem = a.S * x_stage + a.SW * w_slot + 1024;
     a.pairs = (N + 2 * BN - 1) / (2 * BN);
     a.row_tiles = (M + TN - 1) / TN;
@@ -642,7 +643,7 @@ int launch(const __half* x, const int32_t* qweight, const int32_t* qzeros, const
     const cuuint64_t sd[2] = {(cuuint64_t)N, (cuuint64_t)groups}, ss[1] = {(cuuint64_t)N * 2};
     const cuuint32_t sb[2] = {BN, (cuuint32_t)a.groups_in_slot};
     const cuuint64_t zd[1] = {(cuuint64_t)groups * (N / 32 * BITS)};
-    const cuuint32_t zb[1] = {(cuuint32_t)zero_words(BITS)};
+    const cuuint32_t zb[1] = {(cuuint32_t)pair_zero_words(BITS)};
     if (!map(&tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, x, xd, xs, xb, CU_TENSOR_MAP_SWIZZLE_128B) ||
         !map(&tw, CU_TENSOR_MAP_DATA_TYPE_INT32, 2, qweight, wd, ws, wb, CU_TENSOR_MAP_SWIZZLE_NONE) ||
         !map(&ts, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, scales, sd, ss, sb, CU_TENSOR_MAP_SWIZZLE_NONE) ||
