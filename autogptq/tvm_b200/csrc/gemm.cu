@@ -34,6 +34,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "ring_rules.h"
 
 namespace b200gptq {
 
@@ -637,6 +638,7 @@ int launch_gemm(const __half* x_for_tma, const int32_t* qweight, const int32_t* 
     int S = (smem_budget - tab_bytes) / stage_bytes;
     if (S > kMaxStages) S = kMaxStages;
     if (S > (tmem_cols - a_off) / kTmemAColsPerStage) S = (tmem_cols - a_off) / kTmemAColsPerStage;
+    if (split.per_sm == 1) S = ring_in_whole_turns(S, kGroups);
     if (S < 2) return B200GPTQ_ERR_TOO_LARGE;
     const int smem_bytes = S * stage_bytes + tab_bytes + 1024;  // + slack to align the ring to 1024 bytes
 
