@@ -65,7 +65,9 @@ cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
 // x[b,:] += add[b,:] (optional); h[b,:] = norm(x[b,:]) * w (+ beta).  rms != 0: RMSNorm, else LayerNorm.
 // One CTA per row, eight values per thread and pass (P passes) kept in registers; H is a multiple of 8.  A row is 8..24 KB, so
 // this is one chain of latencies: w and beta are constants and loaded before the wait.
-template <int P>
+// CENTRED: LayerNorm whose variance is summed around the mean, in a second reduction.  Of E[x^2] - mean^2 a mean a few hundred
+// times the spread leaves nothing in fp32.
+template <int P, bool CENTRED>
 __global__ void __launch_bounds__(1024)
 add_norm_kernel(__half* __restrict__ x, const __half* __restrict__ add, const __half* __restrict__ w,
                 const __half* __restrict__ beta, __half* __restrict__ h, int H, float eps, int rms) {
@@ -110,7 +112,25 @@ add_norm_kernel(__half* __restrict__ x, const __half* __restrict__ add, const __
     const bool has = (tid & 31) < (nt + 31) / 32;
     const float ts = warp_sum(has ? red[0][tid & 31] : 0.f), ts2 = warp_sum(has ? red[1][tid & 31] : 0.f);
     const float mean = rms ? 0.f : ts / H;
-    const float var = rms ? ts2 / H : fmaxf(ts2 / H - mean * mean, 0.f);
+    float var = rms ? ts2 / H : fmaxf(ts2 / H - mean * mean, 0.f);
+    if constexpr (CENTRED) {
+        s2 = 0.f;
+#pragma unroll
+        for (int p = 0; p < P; ++p)
+            if (8 * (tid + p * nt) < H) {
+                const __half2* q = reinterpret_cast<const __half2*>(&v[p]);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float2 f = __half22float2(q[k]);
+                    s2 += (f.x - mean) * (f.x - mean) + (f.y - mean) * (f.y - mean);
+                }
+            }
+        s2 = warp_sum(s2);
+        __syncthreads();                    // (red has been read)
+        if ((tid & 31) == 0) red[1][tid >> 5] = s2;
+        __syncthreads();
+        var = warp_sum(has ? red[1][tid & 31] : 0.f) / H;
+    }
     const float inv = rsqrtf(var + eps);
 #pragma unroll
     for (int p = 0; p < P; ++p) {
@@ -639,7 +659,12 @@ B200GPTQ_API int b200gptq_add_norm(void* x, const void* add, const void* w, cons
                           static_cast<const __half*>(add), static_cast<const __half*>(w), static_cast<const __half*>(beta),
                           static_cast<__half*>(h), H, eps, rms);
     };
-    B200GPTQ_CUDA_TRY(H <= 8192 ? launch(add_norm_kernel<1>) : launch(add_norm_kernel<2>));
+    // A prompt: its rows fill the SMs and hide most of the second reduction (512 x 4096: 3.7 against 4.1 us).  In a decode step
+    // of up to 16 rows a norm is on the path of every kernel after it; summed around the mean, or around any value near it, it took
+    // 0.15 to 0.36 us more, 1.5 to 4 % of a small OPT step.
+    const bool centred = !rms && rows > 16;
+    B200GPTQ_CUDA_TRY(H <= 8192 ? (centred ? launch(add_norm_kernel<1, true>) : launch(add_norm_kernel<1, false>))
+                                : (centred ? launch(add_norm_kernel<2, true>) : launch(add_norm_kernel<2, false>)));
     return B200GPTQ_OK;
 }
 

@@ -358,6 +358,7 @@ B200GPTQ_API int b200gptq_tp_probe(const void* device_ptr, unsigned int* host_ou
  * that a batch-1 decode step is a handful of launches instead of dozens of element-wise kernels.
  *
  *   b200gptq_add_norm     x[rows,H] += add (nullable); h = RMSNorm(x)*w (rms != 0) or LayerNorm(x)*w + beta
+ *                         (more than 16 rows: the variance is summed around the mean; up to 16, E[x^2] - mean^2 in fp32)
  *   b200gptq_rope_cache   one new token per sequence: qkv[b,3,heads,hd] -> rotated q_out[b,heads,hd]; rotated k
  *                         and v written at position pos[0] of the caches [b,heads,max_seq,hd]; rope == 0: no rotation
  *   b200gptq_rope_prompt  the same for a whole prompt of `seq` tokens at positions 0 .. seq-1: qkv[b,seq,3,heads,hd] ->
