@@ -52,8 +52,14 @@ struct Layer {
     PyObject* keep;       // keeps the tensors behind those addresses alive
 };
 
+// Tensors that stand for something else: wrappers without memory of their own (vmap, grad and their kin), views whose values
+// are not what lies in memory.
+const c10::DispatchKeySet kNotPlain({c10::DispatchKey::Python, c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::BatchedNestedTensor,
+                                     c10::DispatchKey::FuncTorchGradWrapper, c10::DispatchKey::Functionalize, c10::DispatchKey::Conjugate,
+                                     c10::DispatchKey::Negative, c10::DispatchKey::ZeroTensor});
+
 inline const void* tensor_address(PyObject* t) {
-    return t && THPVariable_Check(t) ? THPVariable_Unpack(t).unsafeGetTensorImpl()->data() : nullptr;
+    return t && t != Py_None && THPVariable_Check(t) ? THPVariable_Unpack(t).unsafeGetTensorImpl()->data() : nullptr;
 }
 inline bool address_is(PyObject* dict, PyObject* key, const void* at) {
     PyObject* t = PyDict_GetItem(dict, key);
@@ -76,13 +82,11 @@ bool scratch_for(int device, cudaStream_t stream, size_t need, Scratch* out) {
     return true;
 }
 
-// Layer.run(x, module_dict): the module's forward, or None where the prepared case does not apply.
-PyObject* layer_run(PyObject* self_, PyObject* const* args, Py_ssize_t nargs) {
-    Layer* self = reinterpret_cast<Layer*>(self_);
-    if (nargs != 2) { PyErr_SetString(PyExc_TypeError, "run(x, module_dict)"); return nullptr; }
-    PyObject *px = args[0], *dict = args[1];
+// The module's forward, or None where the prepared case does not apply.
+PyObject* run_prepared(Layer* self, PyObject* px, PyObject* dict) {
     if (!THPVariable_CheckExact(px) || !PyDict_Check(dict)) Py_RETURN_NONE;
     const at::Tensor& x = THPVariable_Unpack(px);
+    if (x.key_set().has_any(kNotPlain)) Py_RETURN_NONE;
     const int64_t dims = x.dim();
     if (!x.is_cuda() || x.scalar_type() != at::kHalf || dims < 1 || x.size(-1) != self->K || !x.is_contiguous() ||
         x.get_device() != self->device)
@@ -99,8 +103,9 @@ PyObject* layer_run(PyObject* self_, PyObject* const* args, Py_ssize_t nargs) {
         PyDict_GetItem(buffers, s_scales) != self->scales)
         Py_RETURN_NONE;
     // (`tensor.data = other` keeps the tensor and moves its numbers)
-    if (tensor_address(self->qzeros) != self->qzeros_run || tensor_address(self->scales) != self->scales_run ||
-        tensor_address(self->bias) != self->bias_run)
+    auto at = [](PyObject* t) { return THPVariable_Unpack(t).unsafeGetTensorImpl()->data(); };
+    if (at(self->qzeros) != self->qzeros_run || at(self->scales) != self->scales_run ||
+        (self->bias_run && at(self->bias) != self->bias_run))
         Py_RETURN_NONE;
     const bool gemv = M <= self->gemv_rows;
     const GemvEntry* e = gemv ? &self->gemv[M] : nullptr;
@@ -113,12 +118,7 @@ PyObject* layer_run(PyObject* self_, PyObject* const* args, Py_ssize_t nargs) {
     if (!scratch_for(self->device, stream, need, &ws)) return nullptr;
     c10::SmallVector<int64_t, 4> shape(x.sizes().begin(), x.sizes().end());
     shape.back() = self->N;
-    at::Tensor y;
-    try {
-        y = at::detail::empty_cuda(shape, at::kHalf, at::Device(at::kCUDA, (c10::DeviceIndex)self->device), std::nullopt);
-    } catch (const c10::Error&) {
-        Py_RETURN_NONE;   // (out of memory: the Python route raises it with its own type)
-    }
+    at::Tensor y = at::detail::empty_cuda(shape, at::kHalf, at::Device(at::kCUDA, (c10::DeviceIndex)self->device), std::nullopt);
     const void* xp = x.unsafeGetTensorImpl()->data();
     void* yp = y.unsafeGetTensorImpl()->mutable_data();
     int st;
@@ -130,6 +130,17 @@ PyObject* layer_run(PyObject* self_, PyObject* const* args, Py_ssize_t nargs) {
                            stream);
     if (st != B200GPTQ_OK) Py_RETURN_NONE;   // the Python route repeats the call and reports the status
     return THPVariable_Wrap(std::move(y));
+}
+
+// Layer.run(x, module_dict).  No C++ exception leaves here: out of memory, or a tensor that has no address, is met again by
+// the Python route, which raises it with its own type.
+PyObject* layer_run(PyObject* self_, PyObject* const* args, Py_ssize_t nargs) {
+    if (nargs != 2) { PyErr_SetString(PyExc_TypeError, "run(x, module_dict)"); return nullptr; }
+    try {
+        return run_prepared(reinterpret_cast<Layer*>(self_), args[0], args[1]);
+    } catch (const std::exception&) {
+        Py_RETURN_NONE;
+    }
 }
 
 // Layer.set_gemv(rows, plan_owner, plan_handle, workspace_bytes)
@@ -149,7 +160,7 @@ PyObject* layer_set_gemv(PyObject* self_, PyObject* args) {
 }
 
 // Layer(K, N, bits, group_size, device, module_dict, gemm_ok, gemv_rows, qweight_run, g_idx_run, x_perm)
-PyObject* layer_new(PyTypeObject* type, PyObject* args, PyObject*) {
+PyObject* make_layer(PyTypeObject* type, PyObject* args) {
     int K, N, bits, group_size, device, gemm_ok, gemv_rows;
     PyObject *dict, *qw, *gi, *perm;
     if (!PyArg_ParseTuple(args, "iiiiiOpiOOO", &K, &N, &bits, &group_size, &device, &dict, &gemm_ok, &gemv_rows, &qw, &gi, &perm))
@@ -185,6 +196,15 @@ PyObject* layer_new(PyTypeObject* type, PyObject* args, PyObject*) {
     self->bias_run = tensor_address(bias);
     self->keep = keep;
     return reinterpret_cast<PyObject*>(self);
+}
+
+PyObject* layer_new(PyTypeObject* type, PyObject* args, PyObject*) {
+    try {
+        return make_layer(type, args);
+    } catch (const std::exception& e) {      // a tensor without an address
+        PyErr_SetString(PyExc_RuntimeError, e.what());
+        return nullptr;
+    }
 }
 
 void layer_dealloc(PyObject* self_) {

@@ -63,3 +63,28 @@ def test_replaced_tensors_with_a_folded_activation(name):
     mod.forward_act(x, _lib.ACT_RELU)
     setattr(mod, name, getattr(b, name))
     assert torch.equal(mod.forward_act(x, _lib.ACT_RELU), _fresh(mod).forward_act(x, _lib.ACT_RELU))
+
+
+def _outcome(f):
+    try:
+        return f()
+    except Exception as e:      # noqa: BLE001  (its type is what is compared)
+        return type(e)
+
+
+@pytest.mark.parametrize("M", [1, 32])
+def test_wrapped_tensors_take_the_python_route(M):
+    """Tensors without memory of their own (vmap, grad, jvp) raise in Python, as they do before the native call object exists."""
+    mod, x = _module(synth.make_layer(BITS, K, N, GS, False, bias=True, seed=1, device=DEV)), synth.make_x(M, K, seed=3, device=DEV)
+    want = mod(x)
+    transforms = [lambda: torch.func.vmap(mod)(torch.stack([x, x])),
+                  lambda: torch.func.grad(lambda t: mod(t).float().sum())(x),
+                  lambda: torch.func.jvp(mod, (x,), (x,))[0]]
+    for f in transforms:
+        mod(x)
+        assert mod._native is not None
+        got = _outcome(f)
+        mod._native = None
+        plain = _outcome(f)
+        assert got is plain if isinstance(plain, type) else torch.equal(got, plain)
+    assert torch.equal(mod(x), want)
