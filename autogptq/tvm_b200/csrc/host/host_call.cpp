@@ -19,8 +19,9 @@ namespace {
 
 constexpr int kMaxGemvRows = 16;
 
-// Scratch buffers by (device, stream), registered by ops.get_workspace.  Read and written under the GIL.
-struct Scratch { void* ptr; size_t bytes; };
+// Scratch buffers by (device, stream), registered by ops.get_workspace.  Read and written under the GIL; `owner` is the
+// tensor, held while it is registered and by a call that works without the GIL.
+struct Scratch { PyObject* owner; void* ptr; size_t bytes; };
 struct KeyHash {
     size_t operator()(const std::pair<int, void*>& k) const {
         return std::hash<void*>()(k.second) * 31u + (size_t)k.first;
@@ -50,6 +51,20 @@ struct Layer {
     const int32_t *qweight_run, *qzeros_run, *g_idx_run, *x_perm;
     const void *scales_run, *bias_run;
     PyObject* keep;       // keeps the tensors behind those addresses alive
+};
+
+// A reference held for the time of a call.
+struct Held {
+    PyObject* o;
+    explicit Held(PyObject* p) : o(p) { Py_XINCREF(o); }
+    ~Held() { Py_XDECREF(o); }
+    Held(const Held&) = delete;
+    Held& operator=(const Held&) = delete;
+};
+// The GIL given up for the time of a scope.
+struct WithoutGil {
+    PyThreadState* state = PyEval_SaveThread();
+    ~WithoutGil() { PyEval_RestoreThread(state); }
 };
 
 // Tensors that stand for something else: wrappers without memory of their own (vmap, grad and their kin), views whose values
@@ -116,18 +131,26 @@ PyObject* run_prepared(Layer* self, PyObject* px, PyObject* dict) {
     Scratch ws;
     const size_t need = gemv ? e->need : b200gptq_workspace_bytes(B200GPTQ_OP_GEMM, (int)M, self->K, self->N, self->bits);
     if (!scratch_for(self->device, stream, need, &ws)) return nullptr;
+    // What another thread may replace while this one has given up the GIL.  (`self`, its tensors and x are held by the caller.)
+    const b200gptq_gemv_plan* plan = gemv ? e->plan : nullptr;
+    const Held scratch(ws.owner), owner(gemv ? e->owner : nullptr);
     c10::SmallVector<int64_t, 4> shape(x.sizes().begin(), x.sizes().end());
     shape.back() = self->N;
-    at::Tensor y = at::detail::empty_cuda(shape, at::kHalf, at::Device(at::kCUDA, (c10::DeviceIndex)self->device), std::nullopt);
-    const void* xp = x.unsafeGetTensorImpl()->data();
-    void* yp = y.unsafeGetTensorImpl()->mutable_data();
+    at::Tensor y;
     int st;
-    if (gemv)
-        st = b200gptq_gemv_plan_run(e->plan, xp, yp, ws.ptr, ws.bytes, stream);
-    else
-        st = b200gptq_gemm(xp, self->qweight_run, self->qzeros_run, self->scales_run, self->g_idx_run, self->x_perm,
-                           self->bias_run, yp, (int)M, self->K, self->N, self->bits, self->group_size, ws.ptr, ws.bytes,
-                           stream);
+    {
+        // A launch waits while the device's queue is full, an allocation may wait for the device: other threads go on.
+        const WithoutGil released;
+        y = at::detail::empty_cuda(shape, at::kHalf, at::Device(at::kCUDA, (c10::DeviceIndex)self->device), std::nullopt);
+        const void* xp = x.unsafeGetTensorImpl()->data();
+        void* yp = y.unsafeGetTensorImpl()->mutable_data();
+        if (gemv)
+            st = b200gptq_gemv_plan_run(plan, xp, yp, ws.ptr, ws.bytes, stream);
+        else
+            st = b200gptq_gemm(xp, self->qweight_run, self->qzeros_run, self->scales_run, self->g_idx_run, self->x_perm,
+                               self->bias_run, yp, (int)M, self->K, self->N, self->bits, self->group_size, ws.ptr, ws.bytes,
+                               stream);
+    }
     if (st != B200GPTQ_OK) Py_RETURN_NONE;   // the Python route repeats the call and reports the status
     return THPVariable_Wrap(std::move(y));
 }
@@ -221,12 +244,23 @@ PyMethodDef layer_methods[] = {
 };
 PyTypeObject LayerType = {PyVarObject_HEAD_INIT(nullptr, 0) "autogptq.tvm_b200._host.Layer", sizeof(Layer)};
 
-// set_scratch(device, stream, address, bytes)
+// set_scratch(device, stream, tensor, bytes)
 PyObject* set_scratch(PyObject*, PyObject* args) {
     int device;
-    unsigned long long stream, address, bytes;
-    if (!PyArg_ParseTuple(args, "iKKK", &device, &stream, &address, &bytes)) return nullptr;
-    (*g_scratch)[{device, (void*)(uintptr_t)stream}] = Scratch{(void*)(uintptr_t)address, (size_t)bytes};
+    unsigned long long stream, bytes;
+    PyObject* tensor;
+    if (!PyArg_ParseTuple(args, "iKOK", &device, &stream, &tensor, &bytes)) return nullptr;
+    const void* address = nullptr;
+    try {
+        address = tensor_address(tensor);
+    } catch (const std::exception&) {
+    }
+    if (!address) { PyErr_SetString(PyExc_TypeError, "set_scratch: a tensor"); return nullptr; }
+    Scratch& s = (*g_scratch)[{device, (void*)(uintptr_t)stream}];
+    PyObject* before = s.owner;
+    Py_INCREF(tensor);
+    s = Scratch{tensor, const_cast<void*>(address), (size_t)bytes};
+    Py_XDECREF(before);
     Py_RETURN_NONE;
 }
 PyObject* set_scratch_source(PyObject*, PyObject* fn) {

@@ -50,7 +50,7 @@ def get_workspace(device: torch.device, nbytes: int) -> torch.Tensor:
         if ws is not None:
             new[16380:16384].copy_(ws[16380:16384])
         ws = _workspaces[key] = new
-        _lib._host.set_scratch(index, key[1], new.data_ptr(), size)
+        _lib._host.set_scratch(index, key[1], new, size)
     return ws
 
 

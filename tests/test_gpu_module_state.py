@@ -88,3 +88,54 @@ def test_wrapped_tensors_take_the_python_route(M):
         plain = _outcome(f)
         assert got is plain if isinstance(plain, type) else torch.equal(got, plain)
     assert torch.equal(mod(x), want)
+
+
+def test_other_threads_go_on_while_a_launch_waits():
+    """The device's queue is full behind a kernel of most of a second; the launches that wait for it hold no GIL."""
+    import threading
+    import time
+    mod, x = _module(synth.make_layer(BITS, K, N, GS, False, bias=True, seed=1, device=DEV)), synth.make_x(1, K, seed=3, device=DEV)
+    want = mod(x)
+    mod(x)
+    torch.cuda.synchronize()
+    outs = []
+
+    def work():
+        torch.cuda._sleep(1_500_000_000)
+        outs.extend([mod(x) for _ in range(4000)][-1:])
+
+    t = threading.Thread(target=work)
+    t.start()
+    longest, last = 0.0, time.perf_counter()
+    while t.is_alive():
+        time.sleep(0.005)
+        now = time.perf_counter()
+        longest, last = max(longest, now - last), now
+    t.join()
+    torch.cuda.synchronize()
+    assert torch.equal(outs[0], want)
+    assert longest < 0.25, f"this thread stood still for {longest:.2f} s"
+
+
+def test_threads_and_streams_share_a_module():
+    """Four threads, each on a stream of its own, in the rows' three routes, while the scratch of each stream grows."""
+    import threading
+    mod = _module(synth.make_layer(BITS, K, N, GS, True, bias=True, seed=1, device=DEV))
+    xs = [synth.make_x(M, K, seed=M, device=DEV) for M in (1, 16, 32, 1500)]
+    want = [mod(x) for x in xs]
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(50):
+                for x, w in list(zip(xs, want))[i:] + list(zip(xs, want))[:i]:
+                    y = mod(x)
+                    if not torch.equal(y, w):
+                        wrong.append((i, x.shape[0]))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert not wrong
+    ops.check_status(DEV)
