@@ -219,12 +219,13 @@ class QuantLinear(nn.Module):
         kw = dict(bias=self.bias, x_perm=self._x_perm)
         args = (self._qweight_run, self.qzeros, self.scales, self._g_idx_run, self.bits, self.groupsize)
         if M <= self._gemv_rows:
-            plan = self._plan(M)
-            self._prepare_native(M, plan)
+            now = self._constants()
+            plan = self._plan(M, now)
+            self._prepare_native(now, M, plan)
             with torch.cuda.device(x2.device):
                 y = plan.run(x2)
         elif self._gemm_ok:
-            self._prepare_native()
+            self._prepare_native(self._constants())
             # above that one tensor-core pass beats several GEMV passes
             y = ops.gemm(x2, *args, **kw)
         elif M > 64:
@@ -247,28 +248,30 @@ class QuantLinear(nn.Module):
     def _constants(self):
         """What a prepared launch holds beside the rows themselves: these tensors, and where their numbers lie (``.data``
         may have been replaced)."""
-        t = (self.qzeros, self.scales, self.bias)
-        return t + tuple(None if v is None else v.data_ptr() for v in t)
+        b = self._buffers
+        qzeros, scales, bias = b["qzeros"], b["scales"], b.get("bias", self.__dict__.get("bias"))
+        return qzeros, scales, bias, qzeros.data_ptr(), scales.data_ptr(), None if bias is None else bias.data_ptr()
 
-    def _plan(self, rows: int, input_act: int = 0):
-        """The prepared GEMV of this row count, made anew when a tensor that it points to has been replaced."""
-        key, now = (rows, self.gemv_tuning, input_act), self._constants()
+    def _plan(self, rows: int, now, input_act: int = 0):
+        """The prepared GEMV of this row count, made anew when a tensor that it points to is not the one in ``now``
+        (``_constants``) any more."""
+        key = (rows, self.gemv_tuning, input_act)
         made = self._plans.get(key)
         if made is None or not _same(made[1], now):
-            plan = ops.GemvPlan(self._qweight_run, self.qzeros, self.scales, self._g_idx_run, self._x_perm, self.bias, rows,
-                                self.bits, self.groupsize, self.gemv_tuning, input_act)
+            plan = ops.GemvPlan(self._qweight_run, now[0], now[1], self._g_idx_run, self._x_perm, now[2], rows, self.bits,
+                                self.groupsize, self.gemv_tuning, input_act)
             made = self._plans[key] = (plan, now)
         return made[0]
 
-    def _prepare_native(self, rows: int = 0, plan=None):
+    def _prepare_native(self, now, rows: int = 0, plan=None):
         """Make the native call object for the current buffers (once), and hand it the plan of one more row count."""
-        if not self.qweight.is_cuda:
+        device = self._buffers["qweight"].device
+        if device.type != "cuda":
             return
-        now = self._constants()
         if self._native is None or not _same(self._native_state, now) or self._native_tuning is not self.gemv_tuning:
             self._native_state, self._native_tuning = now, self.gemv_tuning
             self._native = _lib._host.Layer(self.infeatures, self.outfeatures, self.bits, self.groupsize,
-                                            self.qweight.device.index, self.__dict__, self._gemm_ok, self._gemv_rows,
+                                            device.index, self.__dict__, self._gemm_ok, self._gemv_rows,
                                             self._qweight_run, self._g_idx_run, self._x_perm)
         if plan is not None:
             self._native.set_gemv(rows, plan, plan._handle.value, plan._need)
@@ -291,7 +294,7 @@ class QuantLinear(nn.Module):
         if not u2.is_contiguous():
             u2 = u2.contiguous()
         M = u2.shape[0]
-        plan = self._plan(M, input_act)
+        plan = self._plan(M, self._constants(), input_act)
         with torch.cuda.device(u2.device):
             y = plan.run(u2)
         return y.reshape(u.shape[:-1] + (self.outfeatures,))
