@@ -190,6 +190,13 @@ class QuantLinear(nn.Module):
         b = self._buffers    # (a tensor on another device has another address, so the addresses say it all)
         return self._ready_for == (b["qweight"].data_ptr(), b["g_idx"].data_ptr())
 
+    def __getstate__(self):
+        """For ``copy.deepcopy`` and ``torch.save``: prepared launches hold addresses of this process and are made anew."""
+        state = dict(self.__dict__, _plans={}, _native=None, _ready_for=None)
+        for name in ("_native_state", "_native_tuning"):
+            state.pop(name, None)
+        return state
+
     # ---- forward --------------------------------------------------------------------------
     def forward(self, x):
         if torch.compiler.is_compiling():

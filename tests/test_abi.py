@@ -53,3 +53,24 @@ def test_quantlinear_refuses_cpu_tensors_and_bad_bits():
     assert layer.g_idx.tolist()[:3] == [0, 0, 0] and int(layer.g_idx[-1]) == 1
     with pytest.raises(RuntimeError):
         layer(torch.zeros(1, 256))
+
+
+def test_a_prepared_module_can_be_copied_and_saved():
+    """The native call object and the plans stay behind (they hold addresses); everything else travels."""
+    import copy
+    import io
+    import torch
+    from autogptq.tvm_b200 import QuantLinear, _lib
+    m = QuantLinear(4, 128, 256, 64, True)
+    m.bias.normal_()
+    m._native = _lib._host.Layer(256, 64, 4, 128, 0, m.__dict__, True, 16, m.qweight, None, None)
+    m._native_state, m._native_tuning = m._constants(), None
+    m._plans = {(1, None, 0): (ctypes.c_void_p(1), m._constants())}
+    m._ready_for = (m.qweight.data_ptr(), m.g_idx.data_ptr())
+    f = io.BytesIO()
+    torch.save(m, f)
+    f.seek(0)
+    for c in (copy.deepcopy(m), torch.load(f, weights_only=False)):
+        assert c._native is None and c._plans == {} and not c._ready()
+        assert torch.equal(c.bias, m.bias) and torch.equal(c.g_idx, m.g_idx) and c.groupsize == 128
+    assert m._native is not None and m._ready()

@@ -139,3 +139,18 @@ def test_threads_and_streams_share_a_module():
     [t.join() for t in threads]
     assert not wrong
     ops.check_status(DEV)
+
+
+@pytest.mark.parametrize("act", [False, True])
+def test_copies_of_a_used_module(act):
+    import copy
+    import io
+    mod = _module(synth.make_layer(BITS, K, N, GS, act, bias=True, seed=1, device=DEV))
+    xs = [synth.make_x(M, K, seed=M, device=DEV) for M in ROWS]
+    want = [mod(x) for x in xs]
+    f = io.BytesIO()
+    torch.save(mod, f)
+    f.seek(0)
+    for c in (copy.deepcopy(mod), torch.load(f, weights_only=False)):
+        for _ in range(2):
+            assert all(torch.equal(c(x), w) for x, w in zip(xs, want))
