@@ -685,12 +685,6 @@ size_t gemm_pair_partial_bytes(int M, int K, int N, int splits) {
     return (size_t)splits * ((M + tn - 1) / tn * tn) * N * sizeof(float);
 }
 
-// tiles of a launch (each of a pair of SMs takes one after the other)
-int gemm_pair_tiles(int M, int K, int N, int splits) {
-    const int tn = pick_rows(M, N, K, splits);
-    return (N + 2 * BN - 1) / (2 * BN) * ((M + tn - 1) / tn) * splits;
-}
-
 int gemm_pair_dispatch(const __half* x, const int32_t* qweight, const int32_t* qzeros, const __half* scales, const int32_t* g_idx,
                        const __half* bias, __half* y, int M, int K, int N, int bits, int group_size, int splits,
                        unsigned int* status, float* partial, cudaStream_t stream) {

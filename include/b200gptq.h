@@ -209,9 +209,9 @@ B200GPTQ_API int b200gptq_gemm(const void* x, const int32_t* qweight, const int3
 
 /*
  * How b200gptq_gemm divides this problem on the current device: *splits = runs that one tile's K is cut into
- * (1 = none; their fp32 partial sums are added in a fixed order); *ctas_per_sm = 2 where an SM works on two tiles of up to
- * 64 rows, up to 16 rows of 3- and 4-bit layers side by side (two thread blocks, half of the shared and tensor memory
- * each), otherwise one after the other; else 1.  Host-only; launches nothing.  The reference picks
+ * (1 = none; their fp32 partial sums are added in a fixed order); *ctas_per_sm = thread blocks per SM: 2 (half of the
+ * shared and tensor memory each) only for up to 16 rows of 3- and 4-bit layers, else 1.  Host-only; launches nothing.  The
+ * reference picks
  * a tile per (bits, N, K, M bucket) from its tuned table (pycuda_warpper.py:77-127); this is the query for the
  * corresponding decision here, so that a test can tell which form it exercised.
  */

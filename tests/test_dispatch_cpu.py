@@ -87,14 +87,19 @@ def test_registered_operator_has_a_shape_rule():
 
 def test_gemm_work_split_rule():
     """b200gptq_gemm_split is host-only (without a device it plans for 148 SMs): K is split only for up to 128 rows
-    and while every run keeps 16 k-tiles (40 above 64 rows); the second CTA per SM comes only for up to 64 rows and
-    only where it shortens waves x k-tiles."""
+    and while every run keeps 16 k-tiles (40 above 96 rows; from 65 rows on into no fewer than three); more than 16 rows, and 2 and
+    8 bits, run on pairs of SMs, one CTA each; the second CTA per SM comes only below that and only where it shortens waves x
+    k-tiles."""
     from autogptq.tvm_b200 import ops
     assert ops.gemm_split(16, 4096, 4096, 4) == (4, 1)        # 32 column tiles on 148 SMs: four runs of 16 k-tiles
-    assert ops.gemm_split(128, 4096, 4096, 4) == (1, 1)       # 32 k-tiles per run would be too few above 64 rows
+    assert ops.gemm_split(128, 4096, 4096, 4) == (1, 1)       # 16 k-tiles per run would be too few above 96 rows
+    assert ops.gemm_split(96, 4096, 4096, 4) == (4, 1)        # 16 pairs of column tiles on 74 pairs of SMs: four runs
+    assert ops.gemm_split(96, 2048, 4096, 4) == (1, 1)        # two runs would be too few above 64 rows
     assert ops.gemm_split(128, 11008, 4096, 4) == (4, 1)      # 172 k-tiles: four runs of 43
     assert ops.gemm_split(16, 4096, 12288, 4) == (3, 2)       # 96 tiles: three runs, two CTAs per SM
-    assert ops.gemm_split(64, 9216, 27648, 3) == (1, 2)       # 216 tiles: one wave of two per SM instead of two waves
+    assert ops.gemm_split(64, 9216, 27648, 3) == (1, 1)       # 108 pairs of column tiles: never two CTAs of a pair kernel per SM
+    assert ops.gemm_split(16, 9216, 27648, 3) == (1, 2)       # 216 tiles: one wave of two per SM instead of two waves
+    assert ops.gemm_split(16, 4096, 12288, 8)[1] == 1         # 8 bits: pairs at any number of rows
     assert ops.gemm_split(16, 9216, 9216, 3)[0] > 1
     assert ops.gemm_split(256, 4096, 4096, 4) == (1, 1)       # more than one row tile: never split
     assert ops.gemm_split(2048, 4096, 12288, 4) == (1, 1)

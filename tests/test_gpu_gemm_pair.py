@@ -51,5 +51,5 @@ def test_split_of_the_cases_above():
     assert ops.gemm_split(77, 11008, 4096, 4)[0] == 4
     assert ops.gemm_split(128, 11008, 1056, 8)[0] == 4
     assert ops.gemm_split(33, 4096, 4128, 3) == (4, 1)
-    assert ops.gemm_split(64, 2048, 19232, 4) == (1, 2)
+    assert ops.gemm_split(64, 2048, 19232, 4) == (1, 1)
     assert ops.gemm_split(96, 4064, 64, 3)[0] == 4
