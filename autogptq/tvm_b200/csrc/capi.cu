@@ -155,8 +155,8 @@ int b200gptq_workspace_status(const void* workspace, void* stream, unsigned int*
 int b200gptq_gemv_path(int M, int K, int N, int bits, int group_size, int has_g_idx) {
     if (int st = check_layer(K, N, bits, &group_size)) return st;
     if (M < 1 || M > 8) return B200GPTQ_ERR_SHAPE;
-    return (!has_g_idx && gemv_stream_supported(M, K, N, bits, group_size)) ? B200GPTQ_PATH_STREAM
-                                                                           : B200GPTQ_PATH_GENERIC;
+    return (!has_g_idx && gemv_strip_supported(M, K, N, bits, group_size)) ? B200GPTQ_PATH_STREAM
+                                                                          : B200GPTQ_PATH_GENERIC;
 }
 
 int b200gptq_gemm_split(int M, int K, int N, int bits, int* splits, int* ctas_per_sm) {

@@ -214,11 +214,13 @@ def gemv(x, qweight, qzeros, scales, g_idx, bits: int, group_size: int, bias=Non
 
 
 def can_fold_act(M: int, K: int, N: int, bits: int, group_size: int, has_g_idx: bool, has_perm: bool, input_act: int) -> bool:
-    """Whether ``b200gptq_gemv_ex`` folds ``input_act`` into this GEMV (only the streaming kernel does, and SwiGLU not
-    together with a gather); otherwise the caller runs :func:`act` first."""
+    """Whether ``b200gptq_gemv_ex`` folds ``input_act`` into this GEMV (only the streaming kernel does, for 3 and 4 bits and
+    groups of whole runs of 128 rows, and SwiGLU not together with a gather); otherwise the caller runs :func:`act` first."""
     if not input_act:
         return True
     if _lib.gemv_path(M, K, N, bits, group_size, has_g_idx) != _lib.PATH_STREAM:
+        return False
+    if bits not in (3, 4) or K % 128 != 0 or (group_size != -1 and group_size % 128 != 0):
         return False
     return not (input_act == _lib.ACT_SWIGLU and has_perm)
 

@@ -177,9 +177,7 @@ B200GPTQ_API void b200gptq_gemv_plan_destroy(b200gptq_gemv_plan* plan);
  * B200GPTQ_PATH_GENERIC (a negative B200GPTQ_ERR_* code for an invalid problem).
  * Host-only; launches nothing.  has_g_idx != 0 means a non-NULL g_idx is passed.
  * The reference picks its kernel per (bits, N, K, M bucket) in
- * pycuda_warpper.py:138-189; this is the query for the same decision here.  PATH_STREAM stands for 3- and 4-bit layers
- * whose groups are whole runs of 128 rows, the ones that also take an input activation; the streaming kernel itself serves
- * every g_idx == NULL layer whose groups are whole 32-row blocks.
+ * pycuda_warpper.py:138-189; this is the query for the same decision here.
  */
 #define B200GPTQ_PATH_STREAM 1
 #define B200GPTQ_PATH_GENERIC 2

@@ -51,3 +51,28 @@ def test_every_folded_activation_has_a_plan(bits, act):
     for M in (1, 2, 8):
         for K in list(range(128, 20000, 1280)) + list(range(20480, 140000, 2560)):
             assert _create(M, K, 8192, bits, 128, False, 0, act) != TOO_LARGE, (M, K)
+
+
+def test_the_query_for_folding_and_the_library_agree():
+    """ops.can_fold_act says what b200gptq_gemv_plan_create_ex refuses (with the shape's status) and what it does not."""
+    from autogptq.tvm_b200 import ops
+    refused = 0
+    for M in (1, 3, 8):
+        for K in (128, 96, 256, 4096, 4128):
+            for bits in (2, 3, 4, 8):
+                for group in (32, 64, 128, 256, -1):
+                    for perm in (False, True):
+                        for act in (_lib.ACT_SWIGLU, _lib.ACT_RELU):
+                            folds = ops.can_fold_act(M, K, 96, bits, group, False, perm, act)
+                            assert (_create(M, K, 96, bits, group, perm, 0, act) != -3) == folds, (M, K, bits, group, perm, act)
+                            refused += not folds
+    assert refused
+
+
+def test_the_path_query_names_the_kernel():
+    for bits in (2, 3, 4, 8):
+        for K, group, streams in ((256, 32, True), (256, 64, True), (256, 128, True), (256, -1, True), (96, -1, True), (256, 16, False),
+                                  (288, 48, False)):
+            want = _lib.PATH_STREAM if streams else _lib.PATH_GENERIC
+            assert _lib.gemv_path(1, K, 96, bits, group, False) == want
+            assert _lib.gemv_path(8, K, 96, bits, group, True) == _lib.PATH_GENERIC

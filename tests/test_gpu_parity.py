@@ -136,7 +136,7 @@ def test_gemv_vs_oracle(bits, K, N, gs, act, bias, M, explicit_g_idx):
     d = layer.to(DEV)
     g = d.g_idx if explicit_g_idx else None
     path = _lib.gemv_path(M, K, N, bits, gs, g is not None)
-    streams = (not explicit_g_idx) and bits in (3, 4) and K % 128 == 0 and (gs == -1 or gs % 128 == 0)
+    streams = (not explicit_g_idx) and (gs == -1 or gs % 32 == 0)
     assert path == (_lib.PATH_STREAM if streams else _lib.PATH_GENERIC)
     y = ops.gemv(x.to(DEV), d.qweight, d.qzeros, d.scales, g, bits, gs, bias=d.bias)
     _check_output(y, x.numpy(), W, None if layer.bias is None else layer.bias.numpy())
