@@ -627,6 +627,8 @@ pick_final_kernel(const __half* __restrict__ slots, int world, long long* __rest
 using namespace b200gptq;
 
 namespace {
+bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+
 // One launch of the attention kernel.  A (sequence, head) gets up to eight CTAs, as many as keep the whole grid resident
 // (two per SM) and as have a block of positions for each of their warps.
 template <int HD, bool STEP>
@@ -687,9 +689,8 @@ B200GPTQ_API int b200gptq_rope_prompt(const void* qkv, const void* cos_t, const 
     if (!qkv || !q_out || !k_cache || !v_cache || (rope && (!cos_t || !sin_t))) return B200GPTQ_ERR_NULL_POINTER;
     if (batch <= 0 || batch > 65535 || seq <= 0 || seq > 65535 || seq > max_seq || heads <= 0 || hd <= 0 || hd % 8 != 0)
         return B200GPTQ_ERR_SHAPE;
-    if ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(q_out) | reinterpret_cast<uintptr_t>(k_cache) |
-         reinterpret_cast<uintptr_t>(v_cache) | reinterpret_cast<uintptr_t>(cos_t) | reinterpret_cast<uintptr_t>(sin_t)) & 15u)
-        return B200GPTQ_ERR_ALIGNMENT;
+    for (const void* p : {qkv, cos_t, sin_t, (const void*)q_out, (const void*)k_cache, (const void*)v_cache})
+        if (!aligned16(p)) return B200GPTQ_ERR_ALIGNMENT;
     B200GPTQ_CUDA_TRY(launch_pdl(rope_prompt_kernel, dim3((heads * hd / 8 + 255) / 256, seq, batch), dim3(256), 0, stream, 1,
                                  static_cast<const __half*>(qkv), static_cast<const __half*>(cos_t),
                                  static_cast<const __half*>(sin_t), static_cast<__half*>(q_out), static_cast<__half*>(k_cache),
@@ -702,6 +703,7 @@ B200GPTQ_API int b200gptq_attn_decode(const void* q, const void* k_cache, const 
                                       void* stream) {
     if (!q || !k_cache || !v_cache || !pos || !out) return B200GPTQ_ERR_NULL_POINTER;
     if (batch <= 0 || heads <= 0 || (hd != 64 && hd != 128)) return B200GPTQ_ERR_SHAPE;
+    if (!aligned16(k_cache) || !aligned16(v_cache)) return B200GPTQ_ERR_ALIGNMENT;      // (read 16 bytes at a time)
     const __half* qh = static_cast<const __half*>(q);
     const __half* kh = static_cast<const __half*>(k_cache);
     const __half* vh = static_cast<const __half*>(v_cache);
@@ -723,6 +725,7 @@ B200GPTQ_API int b200gptq_attn_step(const void* qkv, const void* cos_t, const vo
                                     int max_seq, int rope, float scale, void* stream) {
     if (!qkv || !k_cache || !v_cache || !pos || !out || (rope && (!cos_t || !sin_t))) return B200GPTQ_ERR_NULL_POINTER;
     if (batch <= 0 || heads <= 0 || (hd != 64 && hd != 128)) return B200GPTQ_ERR_SHAPE;
+    if (!aligned16(k_cache) || !aligned16(v_cache)) return B200GPTQ_ERR_ALIGNMENT;      // (read 16 bytes at a time)
     const __half* qh = static_cast<const __half*>(qkv);
     const __half* kh = static_cast<const __half*>(k_cache);
     const __half* vh = static_cast<const __half*>(v_cache);
@@ -746,7 +749,7 @@ B200GPTQ_API int b200gptq_attn_step(const void* qkv, const void* cos_t, const vo
 B200GPTQ_API int b200gptq_act(const void* u, void* act, int rows, int I, int gated, void* stream) {
     if (!u || !act) return B200GPTQ_ERR_NULL_POINTER;
     if (rows <= 0 || I <= 0 || I % 2 != 0) return B200GPTQ_ERR_SHAPE;
-    if (I % 8 == 0 && rows <= 65535 && ((reinterpret_cast<uintptr_t>(u) | reinterpret_cast<uintptr_t>(act)) & 15u) == 0) {
+    if (I % 8 == 0 && rows <= 65535 && aligned16(u) && aligned16(act)) {
         B200GPTQ_CUDA_TRY(launch_pdl(act8_kernel, dim3((I / 8 + 255) / 256, rows), dim3(256), 0, stream, 1,
                                      static_cast<const __half*>(u), static_cast<__half*>(act), I, gated));
         return B200GPTQ_OK;

@@ -361,7 +361,8 @@ B200GPTQ_API int b200gptq_tp_probe(const void* device_ptr, unsigned int* host_ou
  *                         and v written at position pos[0] of the caches [b,heads,max_seq,hd]; rope == 0: no rotation
  *   b200gptq_rope_prompt  the same for a whole prompt of `seq` tokens at positions 0 .. seq-1: qkv[b,seq,3,heads,hd] ->
  *                         q_out[b,seq,heads,hd] and the caches; hd a multiple of 8
- *   b200gptq_attn_decode  out[b,heads*hd] = softmax(q k^T * scale) v over cache positions 0..pos[0]; hd in {64,128}
+ *   b200gptq_attn_decode  out[b,heads*hd] = softmax(q k^T * scale) v over cache positions 0..pos[0]; hd in {64,128}; caches
+ *                         16-byte aligned (also for attn_step)
  *   b200gptq_attn_step    b200gptq_rope_cache followed by b200gptq_attn_decode as ONE launch (same caches bit for bit,
  *                         same output up to the order of the softmax accumulation): rotates
  *                         q and the new k inside the attention kernel, attends to the new position from shared

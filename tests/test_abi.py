@@ -74,3 +74,13 @@ def test_a_prepared_module_can_be_copied_and_saved():
         assert c._native is None and c._plans == {} and not c._ready()
         assert torch.equal(c.bias, m.bias) and torch.equal(c.g_idx, m.g_idx) and c.groupsize == 128
     assert m._native is not None and m._ready()
+
+
+def test_attention_refuses_caches_that_are_not_aligned():
+    """Keys and values are read 16 bytes at a time; the check comes before anything is launched (the addresses are made up)."""
+    from autogptq.tvm_b200 import _lib
+    a, off = 0x100000, 0x100008
+    for k, v in ((off, a), (a, off)):
+        for hd in (64, 128):
+            assert _lib.lib.b200gptq_attn_decode(a, k, v, a, a, 1, 8, hd, 256, 1.0, None) == -4
+            assert _lib.lib.b200gptq_attn_step(a, a, a, a, k, v, a, 1, 8, hd, 256, 1, 1.0, None) == -4
