@@ -425,8 +425,9 @@ class GPTQDecoder:
         self.pos.copy_(saved_pos)
         self.tokens.copy_(saved_tok)
 
-    #: work splits :meth:`tune` tries: (K slices per SM that the cluster size aims at, CTAs per SM that the footprint is
-    #: sized for; 0 = the library's choice), ``None`` = the library's defaults for a GEMV on its own
+    #: work splits :meth:`tune` tries, ``None`` = the library's defaults.  With the exchange fused in: (K slices per SM that the
+    #: cluster size aims at, CTAs per SM that the footprint is sized for; 0 = the library's choice).  Otherwise only the second
+    #: number counts (1: sixteen warps per CTA, more: eight), and what comes to the same is measured once.
     TUNINGS = (None, (2, 0), (4, 0), (6, 0), (2, 1), (2, 2), (2, 3))
 
     def tune(self, steps: int = 12, candidates=TUNINGS) -> dict:
@@ -467,11 +468,14 @@ class GPTQDecoder:
         for kind in kinds:
             if not isinstance(getattr(self.layers[0], kind), QuantLinear):
                 continue
-            times = []
+            times, split = {}, getattr(self.layers[0], kind).exchange is not None
             for cand in candidates:
+                same = cand if split else min(cand[1], 2) if cand else 0
+                if same in times:
+                    continue
                 apply(kind, cand)
-                times.append(step_ms())
-            chosen[kind] = candidates[times.index(min(times))]
+                times[same] = (step_ms(), cand)
+            chosen[kind] = min(times.values(), key=lambda t: t[0])[1]
             apply(kind, chosen[kind])
         self.capture()
         return chosen

@@ -32,9 +32,9 @@ def test_graph_decode_equals_eager_decode(arch, bits, desc_act):
 
 @pytest.mark.parametrize("arch,bits,desc_act", [("llama", 4, False), ("opt", 3, True)])
 def test_tuning_in_place_keeps_the_state_and_the_result(arch, bits, desc_act):
-    """GPTQDecoder.tune(): every kind of linear gets one of the candidate work splits, position and tokens are as
-    before, and the logits of the next step stay within the output contract of the untuned decoder's (a different
-    split of K changes the order of the fp32 sums only)."""
+    """GPTQDecoder.tune(): every kind of linear gets one of the candidate work splits that differ on one GPU, position and
+    tokens are as before, and the logits of the next step stay within the output contract of the untuned decoder's (a
+    different split of K changes the order of the fp32 sums only)."""
     cfg = _small(arch, bits, desc_act)
     prompt = torch.randint(0, cfg.vocab, (1, 12), generator=torch.Generator().manual_seed(1)).to(DEV)
     ref = decoder.GPTQDecoder(cfg, batch=1, device=DEV)
@@ -44,7 +44,8 @@ def test_tuning_in_place_keeps_the_state_and_the_result(arch, bits, desc_act):
     m.prefill(prompt)
     pos, tok = int(m.pos), m.tokens.clone()
     chosen = m.tune(steps=4)
-    assert set(chosen) == {"qkv", "o", "up", "down"} and all(c in m.TUNINGS for c in chosen.values())
+    assert set(chosen) == {"qkv", "o", "up", "down"}
+    assert all(c in (None, (2, 1), (2, 2)) for c in chosen.values()), "the first of the candidates that come to the same"
     assert int(m.pos) == pos and torch.equal(m.tokens, tok) and m._pos_host == pos
     for L in m.layers:
         assert L.qkv.gemv_tuning == chosen["qkv"] and L.down.gemv_tuning == chosen["down"]
@@ -180,11 +181,13 @@ def test_greedy_pick_matches_argmax(rows, ld, valid):
 
 
 @pytest.mark.parametrize("hd", [64, 128])
-@pytest.mark.parametrize("B,heads,pos", [(1, 8, 200), (2, 30, 200), (4, 30, 97), (8, 30, 255), (16, 24, 130), (3, 5, 0)])
-def test_single_query_attention_matches_fp32_softmax(hd, B, heads, pos):
-    """b200gptq_attn_decode against softmax(q k^T / sqrt(hd)) v in fp32, for every way the launcher divides the work:
-    from a cluster of four 16-warp CTAs per (sequence, head) for one sequence down to one 4-warp CTA for a batch."""
-    max_seq = 256
+@pytest.mark.parametrize("B,heads,pos,max_seq", [(1, 8, 200, 256), (2, 30, 200, 256), (4, 30, 97, 256), (8, 30, 255, 256), (16, 24, 130, 256),
+                                                 (3, 5, 0, 256), (1, 32, 1000, 1024), (1, 32, 1023, 1024), (1, 36, 0, 1024), (1, 40, 700, 1024),
+                                                 (2, 30, 515, 1024), (4, 30, 511, 1024), (1, 32, 5, 768), (1, 8, 300, 301)])
+def test_single_query_attention_matches_fp32_softmax(hd, B, heads, pos, max_seq):
+    """b200gptq_attn_decode against softmax(q k^T / sqrt(hd)) v in fp32, for every way the launcher divides the work: a cluster
+    of eight, four or two CTAs per (sequence, head), as many as are resident together and as the cache has blocks for, down to
+    one CTA; positions before, at and behind the blocks' edges."""
     g = torch.Generator().manual_seed(hd + pos + B)
     q = torch.randn(B, heads * hd, generator=g).half().to(DEV)
     kc = torch.randn(B, heads, max_seq, hd, generator=g).half().to(DEV)
@@ -197,13 +200,15 @@ def test_single_query_attention_matches_fp32_softmax(hd, B, heads, pos):
     assert torch.allclose(got.float(), want, rtol=2e-3, atol=2e-3)
 
 
-@pytest.mark.parametrize("hd,rope,B,heads,pos", [(128, True, 1, 4, 37), (64, False, 3, 6, 0), (128, True, 2, 3, 255), (64, True, 1, 2, 100),
-                                                 (128, True, 16, 24, 130), (64, True, 8, 30, 70), (128, False, 4, 30, 33), (128, True, 2, 30, 200)])
-def test_attention_step_equals_its_two_kernels(hd, rope, B, heads, pos):
+@pytest.mark.parametrize("hd,rope,B,heads,pos,max_seq", [
+    (128, True, 1, 4, 37, 256), (64, False, 3, 6, 0, 256), (128, True, 2, 3, 255, 256), (64, True, 1, 2, 100, 256),
+    (128, True, 16, 24, 130, 256), (64, True, 8, 30, 70, 256), (128, False, 4, 30, 33, 256), (128, True, 2, 30, 200, 256),
+    (128, True, 1, 32, 900, 1024), (64, True, 1, 32, 1023, 1024), (128, False, 1, 36, 0, 1024), (64, False, 2, 30, 600, 1024),
+    (128, True, 4, 16, 513, 1024), (128, True, 1, 32, 300, 768)])
+def test_attention_step_equals_its_two_kernels(hd, rope, B, heads, pos, max_seq):
     """b200gptq_attn_step (rotary + cache write + attention in one launch) against b200gptq_rope_cache followed by
     b200gptq_attn_decode: the same caches bit for bit, the same attention output up to the order in which the new
     position enters the online softmax."""
-    max_seq = 256
     g = torch.Generator().manual_seed(hd + pos)
     qkv = torch.randn(B, 3 * heads * hd, generator=g).half().to(DEV)
     kc = torch.randn(B, heads, max_seq, hd, generator=g).half().to(DEV)
