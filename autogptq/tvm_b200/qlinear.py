@@ -55,6 +55,20 @@ def _pack_fields(vals: torch.Tensor, bits: int) -> torch.Tensor:
     return words.to(torch.int32)
 
 
+def row_rules(K: int, groupsize: int, has_g_idx: bool, uniform: bool):
+    """``(gemm_ok, gemv_rows)`` of a run-time layout: whether the tensor-core kernel takes it (one group per aligned 32-row
+    block; ``uniform`` says so of a ``g_idx``), and the largest batch that goes through the GEMV in one pass.
+
+    9 to 16 rows: one pass of the streaming GEMV, where it takes the layer, beats the tensor-core kernel's 16-row tile, whose
+    weight warps are the bottleneck (9216 x 9216, 3 bits: 20 against 40 us; 4096 x 4096, 4 bits: 8.3 against 16.6).  It is also
+    where results change by a rounding: the GEMM multiplies the reference's fp16 ``scale * (q - zero)``, the GEMV the exact field
+    and the scale in fp32 (2.1e-4 against 2.8e-4 from the exact product)."""
+    whole_blocks = groupsize % 32 == 0
+    gemm_ok = uniform if has_g_idx else whole_blocks
+    streams = not has_g_idx and (whole_blocks or groupsize >= K)
+    return gemm_ok, GEMV_WIDE_M if streams else GEMV_MAX_M
+
+
 def _same(a, b) -> bool:
     """Of two results of ``QuantLinear._constants``: the same tensors at the same addresses."""
     return all(s is t for s, t in zip(a[:3], b[:3])) and a[3:] == b[3:]
@@ -169,19 +183,13 @@ class QuantLinear(nn.Module):
                     gs, (torch.arange(K, device=dev, dtype=torch.int64) // self.groupsize).to(torch.int32))
                 self._qweight_run, self._x_perm = qs, perm
                 self._g_idx_run = None if sorted_trivial else gs
-        # the tensor-core kernel takes one group per aligned 32-row block: true for every run-time g_idx built above
-        # (block-uniform or sorted by group with whole blocks) except a NULL g_idx with a group size that is no
-        # multiple of 32, and a sorted layout whose groups do not fill whole blocks
-        g_run = self._g_idx_run
-        if g_run is None:
-            self._gemm_ok = self.groupsize % 32 == 0
-        else:
+        # true for every run-time g_idx built above (block-uniform, or sorted by group with whole blocks) except a sorted
+        # layout whose groups do not fill whole blocks
+        g_run, uniform = self._g_idx_run, True
+        if g_run is not None:
             b = g_run.view(K // 32, 32)
-            self._gemm_ok = bool((b == b[:, :1]).all().item())
-        # 9 to 16 rows: one pass of the streaming GEMV beats the tensor-core kernel's 16-row tile, whose weight warps are
-        # the bottleneck (9216 x 9216, 3 bits: 20 against 40 us; 4096 x 4096, 4 bits: 8.3 against 16.6)
-        whole_blocks = self._g_idx_run is None and (self.groupsize % 32 == 0 or self.groupsize >= K)
-        self._gemv_rows = GEMV_WIDE_M if whole_blocks else GEMV_MAX_M
+            uniform = bool((b == b[:, :1]).all().item())
+        self._gemm_ok, self._gemv_rows = row_rules(K, self.groupsize, g_run is not None, uniform)
         self._plans = {}
         self._native = None
         self._ready_for = (self.qweight.data_ptr(), self.g_idx.data_ptr())

@@ -1,7 +1,8 @@
 """Host-side dispatch of QuantLinear.forward (no GPU): which entry point a given number of rows
 reaches.  The reference dispatches on M in TVMHandler.__call__ (tvm_untils/pycuda_warpper.py:138-189:
-m == 1 -> GEMV kernel, otherwise the padded GEMM buckets); here M <= 8 goes to the GEMV, more rows to
-the tensor-core GEMM for 3/4-bit layers and to GEMV passes of 8 rows for 2/8-bit layers."""
+m == 1 -> GEMV kernel, otherwise the padded GEMM buckets); here up to 16 rows (8 where groups cut 32-row blocks or a
+g_idx is kept) go to the GEMV, more rows to the tensor-core GEMM for every bit width, or, where it does not take the layout, to
+GEMV passes of 8 rows and from 65 rows on to one dequantisation and a dense product."""
 import pytest
 import torch
 
@@ -13,24 +14,31 @@ class _FakeCuda(torch.Tensor):
     is_cuda = property(lambda self: True)
 
 
-def _layer(bits, groupsize=128):
+def _layer(bits, groupsize=128, g_idx=None):
     m = ql.QuantLinear(bits, groupsize, 256, 64, False)
     m._ready = lambda: True
-    m._qweight_run, m._g_idx_run, m._x_perm = m.qweight, None, None
-    m._gemm_ok = bits in (3, 4) and groupsize % 32 == 0
+    m._qweight_run, m._g_idx_run, m._x_perm = m.qweight, g_idx, None
+    uniform = g_idx is None or bool((g_idx.view(-1, 32) == g_idx.view(-1, 32)[:, :1]).all())
+    m._gemm_ok, m._gemv_rows = ql.row_rules(256, m.groupsize, g_idx is not None, uniform)      # as post_init() has it
     return m
 
 
-@pytest.mark.parametrize("bits,M,want", [
-    (4, 1, ["gemv:1"]), (4, 8, ["gemv:8"]), (4, 9, ["gemm:9"]), (3, 16, ["gemm:16"]), (4, 2048, ["gemm:2048"]),
-    (8, 8, ["gemv:8"]), (8, 20, ["gemv:8", "gemv:8", "gemv:4"]), (2, 9, ["gemv:8", "gemv:1"]),
-    # a group size that cuts through 32-row blocks cannot use the tensor-core kernel (one group per block)
-    ((4, 16), 16, ["gemv:8", "gemv:8"]),
+BLOCKS = (torch.arange(256) // 32 * 3 % 8).to(torch.int32)      # one group per 32-row block, not k // group_size
+CUT = (torch.arange(256) // 16 * 3 % 16).to(torch.int32)        # groups that cut the blocks
+
+
+@pytest.mark.parametrize("bits", [2, 3, 4, 8])
+@pytest.mark.parametrize("groupsize,g_idx,M,want", [
+    (128, None, 1, ["plan:1"]), (128, None, 8, ["plan:8"]), (128, None, 9, ["plan:9"]), (128, None, 16, ["plan:16"]),
+    (128, None, 17, ["gemm:17"]), (128, None, 2048, ["gemm:2048"]),
+    (32, None, 16, ["plan:16"]), (32, None, 17, ["gemm:17"]), (-1, None, 16, ["plan:16"]), (-1, None, 17, ["gemm:17"]),
+    # a stored g_idx: the general kernel up to 8 rows, the tensor-core kernel with one group per block
+    (32, BLOCKS, 8, ["plan:8"]), (32, BLOCKS, 9, ["gemm:9"]), (32, BLOCKS, 65, ["gemm:65"]),
+    # groups that cut through 32-row blocks cannot use it
+    (16, None, 8, ["plan:8"]), (16, None, 9, ["gemv:8", "gemv:1"]), (16, None, 16, ["gemv:8", "gemv:8"]),
+    (16, None, 64, ["gemv:8"] * 8), (16, None, 65, ["dequantize"]), (16, CUT, 20, ["gemv:8", "gemv:8", "gemv:4"]), (16, CUT, 65, ["dequantize"]),
 ])
-def test_rows_decide_the_entry_point(monkeypatch, bits, M, want):
-    groupsize = 128
-    if isinstance(bits, tuple):
-        bits, groupsize = bits
+def test_rows_decide_the_entry_point(monkeypatch, bits, groupsize, g_idx, M, want):
     calls = []
 
     def fake(name):
@@ -39,20 +47,25 @@ def test_rows_decide_the_entry_point(monkeypatch, bits, M, want):
             return out if out is not None else torch.zeros((x.shape[0], 64), dtype=torch.float16)
         return f
 
-    class FakePlan:   # up to 8 rows go through a prepared launch (ops.GemvPlan)
+    def fake_dequantize(*args, **kw):
+        calls.append("dequantize")
+        return None, torch.zeros((256, 64), dtype=torch.float16)
+
+    class FakePlan:   # up to 16 rows go through a prepared launch (ops.GemvPlan)
         def __init__(self, *a, **k):
-            self._keep = (None,) * 6
+            pass
 
         def run(self, x, out=None):
-            return fake("gemv")(x, out=out)
+            return fake("plan")(x, out=out)
 
     monkeypatch.setattr(ql.ops, "GemvPlan", FakePlan)
     monkeypatch.setattr(ql.ops, "gemv", fake("gemv"))
     monkeypatch.setattr(ql.ops, "gemm", fake("gemm"))
+    monkeypatch.setattr(ql.ops, "dequantize", fake_dequantize)
     monkeypatch.setattr(torch.cuda, "device", lambda d: __import__("contextlib").nullcontext())
     monkeypatch.setattr(torch, "empty", lambda *a, device=None, **k: torch.zeros(*a, **k))
     x = torch.zeros((M, 256), dtype=torch.float16).as_subclass(_FakeCuda)
-    y = _layer(bits, groupsize).forward(x)
+    y = _layer(bits, groupsize, g_idx).forward(x)
     assert calls == want
     assert tuple(y.shape) == (M, 64)
 
