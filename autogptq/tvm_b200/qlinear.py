@@ -231,16 +231,17 @@ class QuantLinear(nn.Module):
         if not x2.is_contiguous():
             x2 = x2.contiguous()
         M = x2.shape[0]
-        kw = dict(bias=self.bias, x_perm=self._x_perm)
-        args = (self._qweight_run, self.qzeros, self.scales, self._g_idx_run, self.bits, self.groupsize)
+        now = self._constants()
+        qzeros, scales, bias = now[:3]
+        kw = dict(bias=bias, x_perm=self._x_perm)
+        args = (self._qweight_run, qzeros, scales, self._g_idx_run, self.bits, self.groupsize)
         if M <= self._gemv_rows:
-            now = self._constants()
             plan = self._plan(M, now)
             self._prepare_native(now, M, plan)
             with torch.cuda.device(x2.device):
                 y = plan.run(x2)
         elif self._gemm_ok:
-            self._prepare_native(self._constants())
+            self._prepare_native(now)
             # above that one tensor-core pass beats several GEMV passes
             y = ops.gemm(x2, *args, **kw)
         elif M > 64:
