@@ -232,7 +232,6 @@ __device__ __forceinline__ uint32_t zero_of(const uint8_t* row, int col) {
 
 struct PairArgs {
     int M, K, N, spg, groups_in_slot, TN, S, SW, acc_sets, splits;
-    int ahead;                           // fills of the weight ring in flight at most (ring_rules.h)
     int pairs, row_tiles, tiles;         // 256-column tiles, TN-row tiles, all tiles (with the runs of K)
     unsigned int spg_inv;                // ceil(2^32 / spg), spg = 32-row blocks per group
 };
@@ -316,20 +315,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
         //       be clipped to the arrays: the weight warps read scales and zero-points themselves.) =====
         const int rows_g = g_idx ? 0 : p.groups_in_slot;
         const uint32_t tx = pair_unit_bytes(BITS) + rows_g * (BN * 2 + pair_zero_words(BITS) * 4);
-        int s = 0, round = 0, left = p.ahead, ls = 0, lround = 0;     // the fill that has to have completed: slot ls
+        int s = 0, round = 0;
         bool ok = true;
         for (int t = cluster; t < p.tiles && ok; t += clusters) {
             const Tile v = tile_at(t);
             const int zn = v.n0 / 32 * BITS;
             for (int u = v.u0; u < v.u1; ++u) {
                 const int g0 = group_at(4 * u);
-                if (left > 0) {
-                    --left;
-                } else {                                              // (long done when a slot becomes free, as a rule)
-                    ok = mbar_wait(w_full(ls), lround & 1, &abort_flag);
-                    if (++ls == SW) { ls = 0; ++lround; }
-                }
-                if (round > 0) ok = ok && mbar_wait(w_empty(s), (round - 1) & 1, &abort_flag);
+                if (round > 0) ok = mbar_wait(w_empty(s), (round - 1) & 1, &abort_flag);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 if (elect_one()) {
@@ -403,11 +396,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
         int kt = wgroup, unit_base = 0;
         for (int t = cluster; t < p.tiles && ok; t += clusters) {
             const Tile v = tile_at(t);
-            for (; kt < v.KT; kt += kGroups) {
+            auto to_slot = [&] {
                 const int unit = unit_base + (kt >> 1);
                 ws += unit - at_unit;
                 at_unit = unit;
                 while (ws >= SW) { ws -= SW; ++wround; }
+            };
+            for (; kt < v.KT; kt += kGroups) {
+                to_slot();
                 const int rb = 2 * (v.kt0 + kt);
                 __half sc[2];
                 uint32_t z[2];
@@ -443,8 +439,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
                     }
                 }
                 __syncwarp();
-                // each slot is left by two k-tiles; the last k-tile of a tile may be alone in its slot
-                if (lane == 0 || (lane == 1 && kt + 1 == v.KT && !(kt & 1))) mbar_arrive(w_empty(ws));
+                if (lane == 0) mbar_arrive(w_empty(ws));   // (each slot is left by two turns)
                 if (round > 0) {
                     ok = mbar_wait(empty(s), (round - 1) & 1, &abort_flag);   // the products that read this buffer have retired
                     ok = __all_sync(0xffffffffu, ok);
@@ -464,8 +459,20 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
                 s += kGroups;
                 while (s >= S) { s -= S; ++round; }
             }
-            kt -= v.KT;                                   // this group's first k-tile of the next tile
+            const int turns = pair_turns(v.KT);
+            if (kt < turns && ok) {                       // the turn without a k-tile (ring_rules.h): seen and left
+                to_slot();
+                ok = mbar_wait(w_full(ws), wround & 1, &abort_flag);
+                ok = __all_sync(0xffffffffu, ok);
+                if (lane == 0) mbar_arrive(w_empty(ws));
+                kt += kGroups;
+                s += kGroups;
+            }
+            kt -= turns;                                  // this group's first k-tile of the next tile
             unit_base += v.u1 - v.u0;
+            s -= turns - v.KT;                            // (stages have no place for that turn)
+            while (s >= S) { s -= S; ++round; }
+            if (s < 0) { s += S; --round; }
         }
     } else if (warp >= kFirstEpiWarp) {
         // ===== accumulators (lane = column, tensor-memory column = row of x) -> y =====
@@ -618,17 +625,17 @@ int launch(const __half* x, const int32_t* qweight, const int32_t* qzeros, const
     a.spg_inv = (unsigned int)((0x100000000ULL + a.spg - 1) / a.spg);                 // (not used for 1)
     a.groups_in_slot = a.spg % 4 == 0 || groups == 1 ? 1 : (a.spg == 1 ? 4 : (a.spg == 2 ? 2 : 3));
     const int TN = a.TN = pick_rows(M, N, K, splits);
-    // (with K split every pair has one tile, so that no group meets the end of one)
-    const PairRings rings = pair_rings(BITS, a.groups_in_slot, TN, splits > 1 ? 2 : (K + BK - 1) / BK);
-    a.acc_sets = rings.acc_sets; a.S = rings.stages; a.SW = rings.slots; a.ahead = rings.ahead;
-    const int x_stage = TN / 2 * BK * 2, w_slot = pair_slot_bytes(BITS, a.groups_in_slot);
-    if (a.ahead < 1) return B200GPTQ_ERR_TOO_LARGE;
-    const int smem = a.S * x_stage + a.SW * w_slot + 1024;
     a.pairs = (N + 2 * BN - 1) / (2 * BN);
     a.row_tiles = (M + TN - 1) / TN;
     const long long tiles = (long long)a.pairs * a.row_tiles * splits;
     if (tiles > 0x7fffffff || (splits > 1 && 2LL * a.pairs * a.row_tiles >= kMaxCounters - 1)) return B200GPTQ_ERR_TOO_LARGE;
     a.tiles = (int)tiles;
+    const int pairs_of_sms = sm_count() / 2;
+    const PairRings rings = pair_rings(BITS, a.groups_in_slot, TN);
+    a.acc_sets = rings.acc_sets; a.S = rings.stages; a.SW = rings.slots;
+    const int x_stage = TN / 2 * BK * 2, w_slot = pair_slot_bytes(BITS, a.groups_in_slot);
+    if (a.SW < 4 || a.S < kPairMinStages) return B200GPTQ_ERR_TOO_LARGE;
+    const int smem = a.S * x_stage + a.SW * w_slot + 1024;
     auto map = [&](CUtensorMap* m, CUtensorMapDataType type, int rank, const void* ptr, const cuuint64_t* dims,
                    const cuuint64_t* strides, const cuuint32_t* box, CUtensorMapSwizzle swizzle) {
         const cuuint32_t estr[2] = {1, 1};
@@ -661,7 +668,6 @@ int launch(const __half* x, const int32_t* qweight, const int32_t* qzeros, const
     });
     if (result[dev] != 0) { set_last_cuda_error(result[dev]); return B200GPTQ_ERR_CUDA; }
     cudaLaunchConfig_t cfg = {};
-    const int pairs_of_sms = sm_count() / 2;
     cfg.gridDim = dim3(2 * (a.tiles < pairs_of_sms ? a.tiles : pairs_of_sms));
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = smem;

@@ -13,16 +13,13 @@ namespace b200gptq {
 // stages a stage always belongs to one group, which saw its previous fill itself.
 constexpr int ring_in_whole_turns(int stages, int groups) { return stages / groups * groups; }
 
-// Pairs of CTAs (gemm_pair.cu): a slot of the weight ring holds two k-tiles, four groups take k-tiles in turn, through tiles
-// of `k_tiles` whose last slot may hold one.  From one k-tile of a group to its next the slots move on by up to:
-constexpr int kPairGroups = 4;
-constexpr int pair_slot_step(int k_tiles) { return k_tiles == 1 ? kPairGroups : (k_tiles % 2 ? 3 : 2); }
-// Where that is always 2, an even number of slots gives every slot to the same two groups: each saw the previous fill itself.
-// Otherwise the warp that fills the ring starts a fill only when the one `ahead` before it has completed: a group that has
-// seen fill u complete then knows it of all fills up to u - ahead; its next wait is for u + step at most, and the previous
-// fill of that slot is u + step - slots.
-constexpr int kPairNoLimit = 1 << 30;
-constexpr int pair_fill_ahead(int slots, int step) { return step == 2 && slots % 2 == 0 ? kPairNoLimit : slots - step; }
+// Pairs of CTAs (gemm_pair.cu): a slot of the weight ring holds two k-tiles, four groups take k-tiles in turn, through one tile
+// after the other.  A tile with an odd number of k-tiles is walked as if it had one more, whose group sees the slot but does
+// nothing: a group then moves on by two slots at every turn, and with an even number of slots a slot always belongs to the same
+// two groups.  The stages (x and A) count real k-tiles only; a group's turns are at most eight of those apart, and a wait
+// for a stage knows that its products of two rounds before have retired if there are that many stages.
+constexpr int kPairGroups = 4, kPairMinStages = 8;
+constexpr int pair_turns(int k_tiles) { return (k_tiles + 1) & ~1; }
 
 constexpr int kPairColumns = 128, kPairKTile = 64;         // columns per CTA, rows of K per stage
 constexpr int kPairTmemCols = 512;                         // accumulators, then 32 columns of A per stage
@@ -38,18 +35,15 @@ struct PairRings {
     int acc_sets;      // sets of accumulators
     int stages;        // of x (shared memory) and A (tensor memory)
     int slots;         // of packed weights and constants
-    int ahead;         // fills of the weight ring in flight at most
 };
-inline PairRings pair_rings(int bits, int groups, int rows, int k_tiles) {      // rows of x per tile
+inline PairRings pair_rings(int bits, int groups, int rows) {      // rows of x per tile
     PairRings r;
     r.acc_sets = rows <= 128 ? 2 : 1;
     r.stages = (kPairTmemCols - r.acc_sets * rows) / 32;
     if (r.stages > kPairMaxStages) r.stages = kPairMaxStages;
     r.slots = (kPairSmem - 1024 - r.stages * (rows / 2 * kPairKTile * 2)) / pair_slot_bytes(bits, groups);
     if (r.slots > kPairMaxSlots) r.slots = kPairMaxSlots;
-    const int step = pair_slot_step(k_tiles);
-    if (step == 2) r.slots &= ~1;
-    r.ahead = pair_fill_ahead(r.slots, step);
+    r.slots &= ~1;
     return r;
 }
 
