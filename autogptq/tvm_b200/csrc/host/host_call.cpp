@@ -41,8 +41,10 @@ struct GemvEntry {
 struct Layer {
     PyObject_HEAD
     int K, N, bits, group_size, device;
-    // the buffers this object was prepared for: addresses of qweight / g_idx, identity and addresses of the others
+    // the buffers this object was prepared for: addresses of qweight / g_idx, identity and addresses of the others, and how
+    // often the weights, scales and zero-points had been written to
     const void *qweight_at, *g_idx_at;
+    uint32_t writes;
     PyObject *qzeros, *scales, *bias, *tuning;
     GemvEntry gemv[kMaxGemvRows + 1];
     // run-time layout for the GEMM (gemm_ok false: no tensor-core kernel for this layer)
@@ -76,8 +78,12 @@ const c10::DispatchKeySet kNotPlain({c10::DispatchKey::Python, c10::DispatchKey:
 inline const void* tensor_address(PyObject* t) {
     return t && t != Py_None && THPVariable_Check(t) ? THPVariable_Unpack(t).unsafeGetTensorImpl()->data() : nullptr;
 }
-inline bool address_is(PyObject* dict, PyObject* key, const void* at) {
-    PyObject* t = PyDict_GetItem(dict, key);
+// Writes in place to a tensor so far (tensors of inference mode do not count them).
+inline uint32_t writes_to(PyObject* t) {
+    c10::TensorImpl* impl = THPVariable_Unpack(t).unsafeGetTensorImpl();
+    return impl->is_inference() ? 0u : impl->version_counter().current_version();
+}
+inline bool lies_at(PyObject* t, const void* at) {
     return t && THPVariable_Check(t) && THPVariable_Unpack(t).unsafeGetTensorImpl()->data() == at;
 }
 
@@ -110,8 +116,9 @@ PyObject* run_prepared(Layer* self, PyObject* px, PyObject* dict) {
     if (M < 1) Py_RETURN_NONE;
     // the module's buffers are the ones this object was prepared for
     PyObject* buffers = PyDict_GetItem(dict, s_buffers);
-    if (!buffers || !address_is(buffers, s_qweight, self->qweight_at) || !address_is(buffers, s_g_idx, self->g_idx_at))
-        Py_RETURN_NONE;
+    if (!buffers) Py_RETURN_NONE;
+    PyObject *qweight = PyDict_GetItem(buffers, s_qweight), *g_idx = PyDict_GetItem(buffers, s_g_idx);
+    if (!lies_at(qweight, self->qweight_at) || !lies_at(g_idx, self->g_idx_at)) Py_RETURN_NONE;
     PyObject* bias = PyDict_GetItem(buffers, s_bias);
     if (!bias) bias = PyDict_GetItem(dict, s_bias);
     if ((bias ? bias : Py_None) != self->bias || PyDict_GetItem(buffers, s_qzeros) != self->qzeros ||
@@ -122,6 +129,8 @@ PyObject* run_prepared(Layer* self, PyObject* px, PyObject* dict) {
     if (at(self->qzeros) != self->qzeros_run || at(self->scales) != self->scales_run ||
         (self->bias_run && at(self->bias) != self->bias_run))
         Py_RETURN_NONE;
+    // (weights that have been written to: the Python route re-orders them anew, or sees to it that they can be read early)
+    if (writes_to(qweight) + writes_to(g_idx) + writes_to(self->qzeros) + writes_to(self->scales) != self->writes) Py_RETURN_NONE;
     const bool gemv = M <= self->gemv_rows;
     const GemvEntry* e = gemv ? &self->gemv[M] : nullptr;
     if (gemv ? (!e->plan || PyDict_GetItem(dict, s_gemv_tuning) != self->tuning) : !self->gemm_ok) Py_RETURN_NONE;
@@ -195,7 +204,7 @@ PyObject* make_layer(PyTypeObject* type, PyObject* args) {
     PyObject* bias = PyDict_GetItem(buffers, s_bias);
     if (!bias) bias = PyDict_GetItem(dict, s_bias);
     PyObject* tuning = PyDict_GetItem(dict, s_gemv_tuning);
-    if (!pq || !pg || !pz || !ps || !THPVariable_Check(pz) || !THPVariable_Check(ps) ||
+    if (!pq || !pg || !pz || !ps || !THPVariable_Check(pq) || !THPVariable_Check(pg) || !THPVariable_Check(pz) || !THPVariable_Check(ps) ||
         (bias && bias != Py_None && !THPVariable_Check(bias))) {
         PyErr_SetString(PyExc_TypeError, "the module lacks a buffer");
         return nullptr;
@@ -206,6 +215,7 @@ PyObject* make_layer(PyTypeObject* type, PyObject* args) {
     Layer* self = reinterpret_cast<Layer*>(type->tp_alloc(type, 0));
     if (!self) { Py_DECREF(keep); return nullptr; }
     self->K = K; self->N = N; self->bits = bits; self->group_size = group_size; self->device = device;
+    self->writes = writes_to(pq) + writes_to(pg) + writes_to(pz) + writes_to(ps);
     self->qweight_at = tensor_address(pq);
     self->g_idx_at = tensor_address(pg);
     self->qzeros = pz; self->scales = ps; self->bias = bias ? bias : Py_None; self->tuning = tuning;

@@ -57,6 +57,14 @@ def get_workspace(device: torch.device, nbytes: int) -> torch.Tensor:
 _lib._host.set_scratch_source(lambda index, nbytes: get_workspace(torch.device("cuda", index), nbytes))
 
 
+def settle(device: torch.device) -> None:
+    """Let what follows on the current stream start only when everything before has completed and can be read, weights
+    included: an ordinary operation (it writes a word of the scratch that is zero anyway) where the library's own kernels
+    may start beside the one in front of them."""
+    with torch.cuda.device(device):
+        get_workspace(device, 16)[:16].zero_()
+
+
 def check_status(device=None) -> None:
     """Raise if any kernel that used this module's scratch buffers on ``device`` gave up a bounded wait (its results
     were then undefined).  Synchronises the streams it looks at; meant for tests, benchmarks and the end of a run."""

@@ -69,9 +69,14 @@ def row_rules(K: int, groupsize: int, has_g_idx: bool, uniform: bool):
     return gemm_ok, GEMV_WIDE_M if streams else GEMV_MAX_M
 
 
+def _version(t) -> int:
+    """Counts what is written in place to a tensor (tensors of inference mode do not count)."""
+    return 0 if t.is_inference() else t._version
+
+
 def _same(a, b) -> bool:
-    """Of two results of ``QuantLinear._constants``: the same tensors at the same addresses."""
-    return all(s is t for s, t in zip(a[:3], b[:3])) and a[3:] == b[3:]
+    """Of two results of ``QuantLinear._constants``: the same tensors, at the same addresses, with the same numbers in them."""
+    return a[0] is b[0] and a[1] is b[1] and a[2] is b[2] and a[3:] == b[3:]
 
 
 class QuantLinear(nn.Module):
@@ -97,6 +102,7 @@ class QuantLinear(nn.Module):
             self.bias = None
         # derived, non-persistent state built by post_init() on the device
         self._ready_for = None
+        self._settled = None       # the _constants that a launch may read without waiting
         self._qweight_run = None   # the weights the kernels read: qweight itself or its row-sorted copy
         self._g_idx_run = None     # None => rows use group k // groupsize
         self._x_perm = None        # None => no gather of x
@@ -192,15 +198,21 @@ class QuantLinear(nn.Module):
         self._gemm_ok, self._gemv_rows = row_rules(K, self.groupsize, g_run is not None, uniform)
         self._plans = {}
         self._native = None
-        self._ready_for = (self.qweight.data_ptr(), self.g_idx.data_ptr())
+        self._ready_for = self._stored()
+        self._settled = self._constants()    # (the look at g_idx above has waited for the stream)
+
+    def _stored(self):
+        """What the run-time view was built from: where the stored weights and groups lie, on whatever device, and how often
+        they have been written to (weights that the kernels read as stored may be)."""
+        q, g = self._buffers["qweight"], self._buffers["g_idx"]
+        return q.data_ptr(), g.data_ptr(), 0 if self._qweight_run is q else _version(q), _version(g)
 
     def _ready(self) -> bool:
-        b = self._buffers    # (a tensor on another device has another address, so the addresses say it all)
-        return self._ready_for == (b["qweight"].data_ptr(), b["g_idx"].data_ptr())
+        return self._ready_for == self._stored()
 
     def __getstate__(self):
         """For ``copy.deepcopy`` and ``torch.save``: prepared launches hold addresses of this process and are made anew."""
-        state = dict(self.__dict__, _plans={}, _native=None, _ready_for=None)
+        state = dict(self.__dict__, _plans={}, _native=None, _ready_for=None, _settled=None)
         for name in ("_native_state", "_native_tuning"):
             state.pop(name, None)
         return state
@@ -232,18 +244,21 @@ class QuantLinear(nn.Module):
             x2 = x2.contiguous()
         M = x2.shape[0]
         now = self._constants()
+        self._settle(now)
         qzeros, scales, bias = now[:3]
         kw = dict(bias=bias, x_perm=self._x_perm)
         args = (self._qweight_run, qzeros, scales, self._g_idx_run, self.bits, self.groupsize)
         if M <= self._gemv_rows:
             plan = self._plan(M, now)
-            self._prepare_native(now, M, plan)
-            with torch.cuda.device(x2.device):
-                y = plan.run(x2)
+            y = self._prepare_native(now, x2, M, plan)
+            if y is None:
+                with torch.cuda.device(x2.device):
+                    y = plan.run(x2)
         elif self._gemm_ok:
-            self._prepare_native(now)
             # above that one tensor-core pass beats several GEMV passes
-            y = ops.gemm(x2, *args, **kw)
+            y = self._prepare_native(now, x2)
+            if y is None:
+                y = ops.gemm(x2, *args, **kw)
         elif M > 64:
             # no tensor-core kernel for this layout and many rows: dequantise once with the library's kernel (the
             # reference's own dequantise-then-matmul order, qlinear.py:242-243) and let the dense product run on the
@@ -262,11 +277,19 @@ class QuantLinear(nn.Module):
         return y.reshape(out_shape)
 
     def _constants(self):
-        """What a prepared launch holds beside the rows themselves: these tensors, and where their numbers lie (``.data``
-        may have been replaced)."""
+        """What a prepared launch holds beside the rows themselves: these tensors, where their numbers lie (``.data`` may
+        have been replaced) and how often they have been written to."""
         b = self._buffers
         qzeros, scales, bias = b["qzeros"], b["scales"], b.get("bias", self.__dict__.get("bias"))
-        return qzeros, scales, bias, qzeros.data_ptr(), scales.data_ptr(), None if bias is None else bias.data_ptr()
+        return (qzeros, scales, bias, qzeros.data_ptr(), scales.data_ptr(), None if bias is None else bias.data_ptr(),
+                _version(qzeros), _version(scales), _version(b["qweight"]))
+
+    def _settle(self, now):
+        """The kernels read weights, scales and zero-points before the kernel in front of them has ended.  Where those are new since
+        the last call, what wrote them may be that kernel: something that waits for it comes in between."""
+        if self._settled is None or not _same(self._settled, now):
+            ops.settle(self._buffers["qweight"].device)
+            self._settled = now
 
     def _plan(self, rows: int, now, input_act: int = 0):
         """The prepared GEMV of this row count, made anew when a tensor that it points to is not the one in ``now``
@@ -279,11 +302,12 @@ class QuantLinear(nn.Module):
             made = self._plans[key] = (plan, now)
         return made[0]
 
-    def _prepare_native(self, now, rows: int = 0, plan=None):
-        """Make the native call object for the current buffers (once), and hand it the plan of one more row count."""
+    def _prepare_native(self, now, x2, rows: int = 0, plan=None):
+        """Make the native call object for the current buffers (once), hand it the plan of one more row count, and make the
+        call; None where it does not take it (a tensor that is not a plain one, another current device)."""
         device = self._buffers["qweight"].device
         if device.type != "cuda":
-            return
+            return None
         if self._native is None or not _same(self._native_state, now) or self._native_tuning is not self.gemv_tuning:
             self._native_state, self._native_tuning = now, self.gemv_tuning
             self._native = _lib._host.Layer(self.infeatures, self.outfeatures, self.bits, self.groupsize,
@@ -291,6 +315,7 @@ class QuantLinear(nn.Module):
                                             self._qweight_run, self._g_idx_run, self._x_perm)
         if plan is not None:
             self._native.set_gemv(rows, plan, plan._handle.value, plan._need)
+        return self._native.run(x2, self.__dict__)
 
     # ---- the element-wise kernel in front of this layer folded into its read of x (decode batches only) ----
     def can_fold(self, rows: int, input_act: int) -> bool:
@@ -310,7 +335,9 @@ class QuantLinear(nn.Module):
         if not u2.is_contiguous():
             u2 = u2.contiguous()
         M = u2.shape[0]
-        plan = self._plan(M, self._constants(), input_act)
+        now = self._constants()
+        self._settle(now)
+        plan = self._plan(M, now, input_act)
         with torch.cuda.device(u2.device):
             y = plan.run(u2)
         return y.reshape(u.shape[:-1] + (self.outfeatures,))
@@ -327,6 +354,7 @@ class QuantLinear(nn.Module):
         if not x2.is_contiguous():
             x2 = x2.contiguous()
         if x2.shape[0] <= GEMV_MAX_M:
+            self._settle(self._constants())
             y = ops.gemv_tp(x2, self._qweight_run, self.qzeros, self.scales, self._g_idx_run, self.bits, self.groupsize,
                             self.exchange, bias=self.tp_bias, x_perm=self._x_perm, tuning=self.gemv_tuning,
                             input_act=input_act)

@@ -66,7 +66,7 @@ def test_a_prepared_module_can_be_copied_and_saved():
     m._native = _lib._host.Layer(256, 64, 4, 128, 0, m.__dict__, True, 16, m.qweight, None, None)
     m._native_state, m._native_tuning = m._constants(), None
     m._plans = {(1, None, 0): (ctypes.c_void_p(1), m._constants())}
-    m._ready_for = (m.qweight.data_ptr(), m.g_idx.data_ptr())
+    m._ready_for = m._stored()
     f = io.BytesIO()
     torch.save(m, f)
     f.seek(0)

@@ -19,6 +19,7 @@ def _layer(bits, groupsize=128, g_idx=None):
     m._ready = lambda: True
     m._qweight_run, m._g_idx_run, m._x_perm = m.qweight, g_idx, None
     uniform = g_idx is None or bool((g_idx.view(-1, 32) == g_idx.view(-1, 32)[:, :1]).all())
+    m._settled = m._constants()
     m._gemm_ok, m._gemv_rows = ql.row_rules(256, m.groupsize, g_idx is not None, uniform)      # as post_init() has it
     return m
 

@@ -20,6 +20,15 @@ def _module(layer):
     return m
 
 
+def _counting(f):
+    calls = []
+
+    def g(*a):
+        calls.append(1)
+        return f(*a)
+    return g, calls
+
+
 def _fresh(mod):
     m = QuantLinear(BITS, GS, K, N, True)
     for name in ("qweight", "qzeros", "scales", "g_idx", "bias"):
@@ -28,7 +37,7 @@ def _fresh(mod):
     return m
 
 
-@pytest.mark.parametrize("how", ["new tensor", "data"])
+@pytest.mark.parametrize("how", ["new tensor", "data", "in place"])
 @pytest.mark.parametrize("name", ["scales", "qzeros", "bias", "qweight", "g_idx"])
 @pytest.mark.parametrize("act", [False, True])
 def test_replaced_tensors_are_the_ones_used(name, how, act):
@@ -41,6 +50,8 @@ def test_replaced_tensors_are_the_ones_used(name, how, act):
     new = getattr(b, name) if act or name != "g_idx" else torch.flip(a.g_idx, (0,)).contiguous()
     if how == "data":
         getattr(mod, name).data = new
+    elif how == "in place":
+        getattr(mod, name).copy_(new)               # as load_state_dict does
     else:
         setattr(mod, name, new)
     for _ in range(3):                              # prepared anew, then prepared
@@ -154,3 +165,21 @@ def test_copies_of_a_used_module(act):
     for c in (copy.deepcopy(mod), torch.load(f, weights_only=False)):
         for _ in range(2):
             assert all(torch.equal(c(x), w) for x, w in zip(xs, want))
+
+
+@pytest.mark.parametrize("M", [1, 32])
+@pytest.mark.parametrize("name", ["scales", "qzeros"])
+def test_new_constants_are_waited_for_once(monkeypatch, M, name):
+    """The kernels read scales and zero-points before the kernel in front of them has ended; the call after they were written
+    puts an ordinary operation in between, later ones and the first after post_init() do not."""
+    mod, x = _module(synth.make_layer(BITS, K, N, GS, False, bias=True, seed=1, device=DEV)), synth.make_x(M, K, seed=3, device=DEV)
+    settle, calls = _counting(ops.settle)
+    monkeypatch.setattr(ops, "settle", settle)
+    mod(x), mod(x)
+    assert not calls
+    getattr(mod, name).add_(1 if name == "qzeros" else 0.5)
+    mod(x), mod(x), mod(x)
+    assert len(calls) == 1
+    setattr(mod, name, getattr(mod, name) * 2)
+    mod(x), mod(x)
+    assert len(calls) == 2 and torch.equal(mod(x), _fresh(mod)(x))
