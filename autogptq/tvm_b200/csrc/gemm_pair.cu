@@ -596,7 +596,8 @@ EncodeTiledFn encode_tiled_fn() {
 }
 
 // Rows of x per tile: the shortest sum over waves of (k-tiles x clocks per k-tile + drain of the accumulators, where there is
-// one set).  A k-tile costs its four products (TN / 2 clk each, measured) but no less than the weight warps take.
+// one set).  A k-tile costs its four products (TN / 2 clk each, measured) but no less than the weight warps take: 370 clk, what the
+// choice was fitted with; about 450 have been measured since, and the choice has not been fitted again.
 int pick_rows(int M, int N, int K, int splits) {
     const long long pairs = (N + 2 * BN - 1) / (2 * BN), slots = sm_count() / 2;
     const long long kt = ((K + BK - 1) / BK + splits - 1) / splits;

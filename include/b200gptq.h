@@ -107,6 +107,12 @@ B200GPTQ_API int b200gptq_workspace_status(const void* workspace, void* stream, 
  * once at load time and pass NULL when it matches (act-order layers: re-order
  * with b200gptq_sort_rows() first, which usually yields k / group_size again).
  * b200gptq_gemv_path() tells which kernel a call will run.
+ *
+ * The kernels are launched with the programmatic dependent launch attribute and read what is constant for a layer --
+ * qweight, qzeros, scales, x_perm -- BEFORE the preceding kernel of the stream has ended (x, bias and g_idx after).  This
+ * holds for b200gptq_gemm, the plans, b200gptq_gemv_tp and, for w and beta, b200gptq_add_norm.  A caller that has these
+ * arrays written on the same stream (b200gptq_pack_linear, b200gptq_sort_rows, a copy) lets the writes complete first: a
+ * synchronisation or an event, or any ordinary operation of the stream (a memset will do) between the write and the call.
  */
 B200GPTQ_API int b200gptq_gemv(const void* x, const int32_t* qweight, const int32_t* qzeros, const void* scales,
                   const int32_t* g_idx, const int32_t* x_perm, const void* bias, void* y,
