@@ -13,10 +13,16 @@
 //   warp 1      TMA: this CTA's rows of x, into the stages; completion is counted in the first CTA of the pair
 //   warp 2      first CTA: issues tcgen05.mma for both (M = 256 columns, N = TN rows of x, K = 16); allocates tensor memory
 //   warps 4..11 epilogue: accumulators -> y
-//   warps 12..27  four groups of four that take 64-row k-tiles in turn: a thread owns one column, dequantises it to the exact
+//   warps 12..27  four groups of four that take units of 128 rows in turn: a thread owns one column, dequantises it to the exact
 //               fp16 values of the reference (auto_gptq/nn_modules/qlinear.py:242: one rounding) in the natural order of k and
-//               stores them into the stage's A buffer in tensor memory.  (A warp per 32-row block spent as many instructions
-//               on hand-overs as on weights: 790 clk per k-tile whatever the number of rows.)
+//               stores them into the stage's A buffer in tensor memory.
+//
+// Up to about 180 rows per tile the weight warps are what bounds a launch.  Of a turn's 1800 clk per 64 rows 190 went to each of two
+// barriers that were ready, 400 to the words and constants, 650 to the arithmetic (four warps share a scheduler), 250 to the rest of
+// the loop, and the threads that issue copies and products spent about 200 clk per 64 rows on barriers too.  So everything moves in
+// units of 128 rows, x and A (a stage) as well as the weights: half the hand-overs.  Clocks per 64 rows of K before and after:
+// 3 bits, 32 rows of 9216 x 9216 505 and 335; 4 bits in groups of 64, 77 rows of 11008 x 4096 465 and 360; 8 bits, 512 rows of
+// 4096 x 4096 550 and 480.  What is left is the arithmetic: without it 230, without the products 310.
 //
 // The pairs are persistent: the rings run on from one tile to the next, so only the drain of the accumulators stands
 // between two tiles (nothing, where two sets of accumulators fit: up to 128 rows).  A stage is released in both CTAs by one
@@ -40,7 +46,7 @@ constexpr int BK = kPairKTile;           // rows of K per stage
 constexpr int kGroups = kPairGroups, kGroupWarps = 4;
 constexpr int kFirstEpiWarp = 4, kEpiWarps = 8, kFirstWeightWarp = kFirstEpiWarp + kEpiWarps;
 constexpr int kThreads = 32 * (kFirstWeightWarp + kGroups * kGroupWarps);
-constexpr int kMaxStages = kPairMaxStages, kMaxW = kPairMaxSlots;
+constexpr int kMaxStages = kPairMaxStages / 2, kMaxW = kPairMaxSlots;
 constexpr int kTmemCols = kPairTmemCols; // accumulators in columns [0, TN), 32 columns of A per stage behind them
 constexpr int kSmemMax = kPairSmem;
 constexpr int kStatusWord = kMaxCounters - 1;
@@ -152,6 +158,9 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr) {
     return d;
 }
 
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
 __device__ __forceinline__ uint32_t lop3_and_or(uint32_t a, uint32_t mask, uint32_t magic) {
     uint32_t r;
     asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(a), "r"(mask), "r"(magic));
@@ -249,16 +258,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     __shared__ __align__(8) uint64_t bars[2 * kMaxW + 2 * kMaxStages + 4];
     __shared__ uint32_t tmem_base_holder;
     __shared__ volatile int abort_flag;
-    __shared__ unsigned int arrived;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rank = blockIdx.x & 1;             // cluster rank; 0 issues the products
     const int K = p.K, N = p.N, TN = p.TN, S = p.S, SW = p.SW, TH = TN / 2;
     const int RB = K / 32, KT_all = (K + BK - 1) / BK, U_all = (K + 127) / 128;
     const int cluster = blockIdx.x >> 1, clusters = gridDim.x >> 1;
-    const uint32_t x_bytes = (uint32_t)TH * BK * 2;
+    const uint32_t x_bytes = (uint32_t)TH * BK * 2;      // of a k-tile; a stage holds two
     const int w_slot = pair_slot_bytes(BITS, p.groups_in_slot);
-    const uint32_t w_off = S * x_bytes;
+    const uint32_t w_off = S * 2 * x_bytes;
 
     const uint32_t bar_base = smem_u32(bars);
     auto w_full = [&](int s) { return bar_base + 8u * s; };
@@ -268,9 +276,27 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     auto acc_full = [&](int a) { return bar_base + 8u * (2 * kMaxW + 2 * kMaxStages + a); };
     auto acc_empty = [&](int a) { return bar_base + 8u * (2 * kMaxW + 2 * kMaxStages + 2 + a); };
 
+    // A tile: 256 columns x TN rows x a run of 128-row units.
+    struct Tile { int n0, m0, z, u0, u1, kt0, KT; };
+    auto tile_at = [&](int t) {
+        Tile v;
+        const int pr = t % p.pairs, r = t / p.pairs, row = r % p.row_tiles;
+        v.z = r / p.row_tiles;
+        v.n0 = (2 * pr + rank) * BN;
+        v.m0 = row * TN;
+        v.u0 = v.z * U_all / p.splits;
+        v.u1 = (v.z + 1) * U_all / p.splits;
+        v.kt0 = 2 * v.u0;
+        v.KT = min(2 * v.u1, KT_all) - v.kt0;
+        return v;
+    };
+    // group of a 32-row block without a division (140 clk each, in the one warp that feeds every k-tile)
+    auto group_at = [&](int rb) { return p.spg == 1 ? rb : (int)__umulhi((unsigned int)rb, p.spg_inv); };
+    const int zwords = N / 32 * BITS;
+
     if (threadIdx.x == 0) {
         abort_flag = 0;
-        for (int s = 0; s < SW; ++s) { mbar_init(w_full(s), 1); mbar_init(w_empty(s), 2 * kGroupWarps); }   // two k-tiles
+        for (int s = 0; s < SW; ++s) { mbar_init(w_full(s), 1); mbar_init(w_empty(s), kGroupWarps); }
         for (int s = 0; s < S; ++s) {
             mbar_init(full(s), 1 + 2 * kGroupWarps);     // the first CTA's expect_tx arrive, a group of weight warps in each
             mbar_init(empty(s), 1);                      // tcgen05.commit
@@ -289,71 +315,75 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = tmem_base_holder, tmem_a = tmem_base + (uint32_t)(p.acc_sets * TN);
     asm volatile("griddepcontrol.launch_dependents;");
-    // what a preceding kernel may still be writing: x; what it may still be reading: y and the scratch
-    if (warp != 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+    // What a preceding kernel may still be writing: x; what it may still be reading: y and the scratch.  The weights are unpacked
+    // before the wait, as far as the stages go (77 rows of 11008 x 4096: the first product came 2.6 us after the wait, now 1.1).
+    if (warp != 0 && (warp < kFirstWeightWarp || g_idx)) asm volatile("griddepcontrol.wait;" ::: "memory");
 
-    // A tile: 256 columns x TN rows x a run of 128-row units.
-    struct Tile { int n0, m0, z, u0, u1, kt0, KT; };
-    auto tile_at = [&](int t) {
-        Tile v;
-        const int pr = t % p.pairs, r = t / p.pairs, row = r % p.row_tiles;
-        v.z = r / p.row_tiles;
-        v.n0 = (2 * pr + rank) * BN;
-        v.m0 = row * TN;
-        v.u0 = (int)(((long long)v.z * U_all) / p.splits);
-        v.u1 = (int)(((long long)(v.z + 1) * U_all) / p.splits);
-        v.kt0 = 2 * v.u0;
-        v.KT = min(2 * v.u1, KT_all) - v.kt0;
-        return v;
+    // ---- epilogue: a warp reads the accumulators of 32 columns (tensor-memory lanes), 16 rows of x at a time ----
+    const uint32_t lane_acc = tmem_base + ((uint32_t)(32 * (warp & 3)) << 16);
+    auto column_bias = [&](const Tile& v) -> float {
+        const int n = v.n0 + 32 * (warp & 3) + lane;
+        return bias && n < N ? __half2float(bias[n]) : 0.f;
     };
-    // group of a 32-row block without a division (140 clk each, in the one warp that feeds every k-tile)
-    auto group_at = [&](int rb) { return p.spg == 1 ? rb : (int)__umulhi((unsigned int)rb, p.spg_inv); };
-    const int zwords = N / 32 * BITS;
+    // two lanes exchange values so that each stores a pair of columns of every other row (N is a multiple of 32: whole warps)
+    auto store_rows = [&](const Tile& v, int m, float (&x)[16]) {
+        const int n = v.n0 + 32 * (warp & 3) + lane, left = n < N ? p.M - m - (lane & 1) : 0;
+        __half* dst = y + (size_t)(m + (lane & 1)) * N + (n & ~1);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float give = (lane & 1) ? x[2 * i] : x[2 * i + 1];
+            const float got = __shfl_xor_sync(0xffffffffu, give, 1);
+            const __half2 h = (lane & 1) ? __floats2half2_rn(got, x[2 * i + 1]) : __floats2half2_rn(x[2 * i], got);
+            if (2 * i < left) *reinterpret_cast<__half2*>(dst) = h;
+            dst += 2 * (size_t)N;
+        }
+    };
 
     if (warp == 0) {
         // ===== packed weights, scales, zero-points.  (With a g_idx the number of groups is not known here, so boxes could not
-        //       be clipped to the arrays: the weight warps read scales and zero-points themselves.) =====
-        const int rows_g = g_idx ? 0 : p.groups_in_slot;
-        const uint32_t tx = pair_unit_bytes(BITS) + rows_g * (BN * 2 + pair_zero_words(BITS) * 4);
-        int s = 0, round = 0;
-        bool ok = true;
-        for (int t = cluster; t < p.tiles && ok; t += clusters) {
-            const Tile v = tile_at(t);
-            const int zn = v.n0 / 32 * BITS;
-            for (int u = v.u0; u < v.u1; ++u) {
-                const int g0 = group_at(4 * u);
-                if (round > 0) ok = mbar_wait(w_empty(s), (round - 1) & 1, &abort_flag);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                if (elect_one()) {
+        //       be clipped to the arrays: the weight warps read scales and zero-points themselves.  The first boxes sent off before the
+        //       cluster has met: a launch 0.4 to 0.6 us longer, a box takes its thread 120 clk.) =====
+        if (elect_one()) {
+            const int rows_g = g_idx ? 0 : p.groups_in_slot;
+            const uint32_t tx = pair_unit_bytes(BITS) + rows_g * (BN * 2 + pair_zero_words(BITS) * 4);
+            int s = 0, round = 0;
+            bool ok = true;
+            for (int t = cluster; t < p.tiles && ok; t += clusters) {
+                const Tile v = tile_at(t);
+                const int zn = v.n0 / 32 * BITS;
+                for (int u = v.u0; u < v.u1; ++u) {
+                    const int g0 = group_at(4 * u);
+                    if (round > 0) ok = mbar_wait(w_empty(s), (round - 1) & 1, &abort_flag);
+                    if (!ok) break;
                     const uint32_t dst = base + w_off + s * w_slot, bar = w_full(s);
                     mbar_expect(bar, tx);
                     tma_2d(dst, &tmap_w, v.n0, u * 4 * BITS, bar);
                     if (rows_g) tma_2d(dst + pair_unit_bytes(BITS), &tmap_s, v.n0, g0, bar);
                     for (int r = 0; r < rows_g; ++r)
                         tma_1d(dst + pair_unit_bytes(BITS) + rows_g * BN * 2 + r * 128, &tmap_z, ((g0 + r) * zwords + zn) & ~3, bar);
+                    if (++s == SW) { s = 0; ++round; }
                 }
-                __syncwarp();
-                if (++s == SW) { s = 0; ++round; }
             }
         }
     } else if (warp == 1) {
         // ===== this CTA's rows of x =====
-        const uint32_t first_full = in_cta(full(0), 0);
-        int s = 0, round = 0;
-        bool ok = true;
-        for (int t = cluster; t < p.tiles && ok; t += clusters) {
-            const Tile v = tile_at(t);
-            for (int kt = 0; kt < v.KT; ++kt) {
-                if (round > 0) ok = mbar_wait(empty(s), (round - 1) & 1, &abort_flag);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                if (elect_one()) {
-                    if (rank == 0) mbar_expect(full(s), 2 * x_bytes);
-                    tma_2d_pair(base + s * x_bytes, &tmap_x, (v.kt0 + kt) * BK, v.m0 + rank * TH, first_full + 8u * s);
+        if (elect_one()) {
+            const uint32_t first_full = in_cta(full(0), 0);
+            int s = 0, round = 0;
+            bool ok = true;
+            for (int t = cluster; t < p.tiles && ok; t += clusters) {
+                const Tile v = tile_at(t);
+                for (int kt = 0; kt < v.KT; kt += 2) {
+                    if (round > 0) ok = mbar_wait(empty(s), (round - 1) & 1, &abort_flag);
+                    if (!ok) break;
+                    const uint32_t dst = base + s * 2 * x_bytes, bar = first_full + 8u * s;
+                    const int k = (v.kt0 + kt) * BK, m = v.m0 + rank * TH;
+                    const bool two = kt + 1 < v.KT;
+                    if (rank == 0) mbar_expect(full(s), two ? 4 * x_bytes : 2 * x_bytes);
+                    tma_2d_pair(dst, &tmap_x, k, m, bar);
+                    if (two) tma_2d_pair(dst + x_bytes, &tmap_x, k + BK, m, bar);
+                    if (++s == S) { s = 0; ++round; }
                 }
-                __syncwarp();
-                if (++s == S) { s = 0; ++round; }
             }
         }
     } else if (warp == 2) {
@@ -368,15 +398,21 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t acc = tmem_base + (uint32_t)(set * TN);
-                for (int kt = 0; kt < v.KT; ++kt) {
+                for (int kt = 0; kt < v.KT; kt += 2) {
                     ok = mbar_wait(full(s), round & 1, &abort_flag);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint64_t bdesc = make_smem_desc(base + s * x_bytes);
-                    const uint32_t a_addr = tmem_a + 32u * s;
+                    const uint64_t bdesc = make_smem_desc(base + s * 2 * x_bytes);
+                    const uint32_t a_addr = tmem_a + 64u * s;
 #pragma unroll
                     for (int k16 = 0; k16 < BK / 16; ++k16)
                         mma_pair(acc, a_addr + 8u * k16, bdesc + 2u * k16, idesc, (kt > 0 || k16 > 0) ? 1u : 0u);
+                    if (kt + 1 < v.KT) {
+                        const uint64_t second = bdesc + (x_bytes >> 4);
+#pragma unroll
+                        for (int k16 = 0; k16 < BK / 16; ++k16)
+                            mma_pair(acc, a_addr + 32u + 8u * k16, second + 2u * k16, idesc, 1u);
+                    }
                     mma_commit_pair(empty(s));
                     if (++s == S) { s = 0; ++round; }
                 }
@@ -386,143 +422,107 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
         }
     } else if (warp >= kFirstWeightWarp) {
         // ===== dequantisation =====
-        const int ww = warp - kFirstWeightWarp, quarter = warp & 3;   // tensor-memory lanes 32 * quarter .. + 31
-        const int wgroup = ww / kGroupWarps, col = 32 * quarter + lane;
+        const int quarter = warp & 3;                    // tensor-memory lanes 32 * quarter .. + 31
+        const int wgroup = (warp - kFirstWeightWarp) / kGroupWarps, col = 32 * quarter + lane;
         const uint32_t lane_a = tmem_a + ((uint32_t)(32 * quarter) << 16);
         const uint32_t first_full = in_cta(full(0), 0);
         const bool early_words = BITS % 4 != 0 && (zwords & 3);       // zero-point boxes may start early
         bool ok = true;
-        int s = wgroup % S, round = wgroup / S, ws = 0, wround = 0, at_unit = 0;   // slot ws holds the at_unit-th unit so far
-        int kt = wgroup, unit_base = 0;
+        // Stage s and slot ws of the group's unit; from one turn to the next it moves on by kGroups units.
+        int s = wgroup, round = 0, ws = wgroup, wround = 0, turn = wgroup;
         for (int t = cluster; t < p.tiles && ok; t += clusters) {
             const Tile v = tile_at(t);
-            auto to_slot = [&] {
-                const int unit = unit_base + (kt >> 1);
-                ws += unit - at_unit;
-                at_unit = unit;
-                while (ws >= SW) { ws -= SW; ++wround; }
-            };
-            for (; kt < v.KT; kt += kGroups) {
-                to_slot();
-                const int rb = 2 * (v.kt0 + kt);
-                __half sc[2];
-                uint32_t z[2];
-                if (g_idx) {
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const int grp = __ldg(g_idx + 32 * min(rb + h, RB - 1));
-                        sc[h] = __float2half(0.f);
-                        z[h] = 1;
-                        if (v.n0 + col < N) {
-                            sc[h] = __ldg(scales + (size_t)grp * N + v.n0 + col);
-                            z[h] = (uint32_t)zero_point<BITS>(qzeros + (size_t)grp * zwords, v.n0 + col);
-                        }
-                    }
-                }
-                ok = mbar_wait(w_full(ws), wround & 1, &abort_flag);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                const uint8_t* src = base_ptr + w_off + ws * w_slot;
-                const uint32_t* pw = reinterpret_cast<const uint32_t*>(src) + (kt & 1) * 2 * BITS * BN + col;
-                uint32_t w[2][BITS];
-#pragma unroll
-                for (int r = 0; r < 2 * BITS; ++r) w[r / BITS][r % BITS] = pw[r * BN];
-                if (!g_idx) {
-                    const int g0 = group_at(rb & ~3);
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        // (one group in the slot: both blocks read the same constants)
-                        const int r = p.groups_in_slot == 1 ? 0 : min(group_at(rb + h) - g0, p.groups_in_slot - 1);
-                        const int early = early_words ? ((g0 + r) * zwords + v.n0 / 32 * BITS) & 3 : 0;
-                        sc[h] = reinterpret_cast<const __half*>(src + pair_unit_bytes(BITS) + r * BN * 2)[col];
-                        z[h] = zero_of<BITS>(src + pair_unit_bytes(BITS) + p.groups_in_slot * BN * 2 + r * 128 + 4 * early, col);
-                    }
-                }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(w_empty(ws));   // (each slot is left by two turns)
-                if (round > 0) {
-                    ok = mbar_wait(empty(s), (round - 1) & 1, &abort_flag);   // the products that read this buffer have retired
+            const int units = pair_turns(v.KT) / 2;
+            for (; turn < units; turn += kGroups) {
+                while (s >= S) { s -= S; ++round; }
+                if (ws >= SW) { ws -= SW; ++wround; }
+                const int u = v.u0 + turn, blocks = min(4, 2 * (v.KT - 2 * turn));
+                // (an answer takes 190 clk: both questions are asked before the first answer is looked at)
+                const bool there = mbar_try(w_full(ws), wround & 1), free = round == 0 || mbar_try(empty(s), (round - 1) & 1);
+                if (!__all_sync(0xffffffffu, there && free)) {
+                    ok = mbar_wait(w_full(ws), wround & 1, &abort_flag);
+                    if (ok && round > 0) ok = mbar_wait(empty(s), (round - 1) & 1, &abort_flag);   // its products have retired
                     ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint8_t* src = base_ptr + w_off + ws * w_slot;
+                const uint32_t* pw = reinterpret_cast<const uint32_t*>(src) + col;
+                const int g0 = group_at(4 * u);
+                __half2 s2, z2;
+                auto constants = [&](int b, int r) {      // of 32-row block b of the unit, group r of the slot
+                    __half sc = __float2half(0.f);
+                    uint32_t z = 1;
+                    if (g_idx) {
+                        const int grp = __ldg(g_idx + 32 * min(4 * u + b, RB - 1));
+                        if (v.n0 + col < N) {
+                            sc = __ldg(scales + (size_t)grp * N + v.n0 + col);
+                            z = (uint32_t)zero_point<BITS>(qzeros + (size_t)grp * zwords, v.n0 + col);
+                        }
+                    } else {
+                        const int early = early_words ? ((g0 + r) * zwords + v.n0 / 32 * BITS) & 3 : 0;
+                        sc = reinterpret_cast<const __half*>(src + pair_unit_bytes(BITS) + r * BN * 2)[col];
+                        z = zero_of<BITS>(src + pair_unit_bytes(BITS) + p.groups_in_slot * BN * 2 + r * 128 + 4 * early, col);
+                    }
+                    s2 = __half2half2(sc);
+                    z2 = __half2half2(__ushort2half_rn((unsigned short)z));
+                };
+                uint32_t w[2][BITS];                      // this block's words and the next one's
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
+                for (int r = 0; r < BITS; ++r) w[0][r] = pw[r * BN];
+                int r_at = 0;
+#pragma unroll
+                for (int b = 0; b < 4; ++b) {
+                    if (b >= blocks) break;
+                    if (b == 0 || g_idx) {
+                        constants(b, 0);
+                    } else if (p.groups_in_slot != 1) {
+                        const int r = min(group_at(4 * u + b) - g0, p.groups_in_slot - 1);
+                        if (r != r_at) constants(b, r);
+                        r_at = r;
+                    }
+                    if (b + 1 < 4)
+#pragma unroll
+                        for (int r = 0; r < BITS; ++r) w[(b + 1) & 1][r] = pw[((b + 1) * BITS + r) * BN];
                     uint32_t out[16];
-                    Block<BITS>::run(w[h], __half2half2(sc[h]), __half2half2(__ushort2half_rn((unsigned short)z[h])), out);
-                    tmem_st16(lane_a + 32u * s + 16 * h, out);
+                    Block<BITS>::run(w[b & 1], s2, z2, out);
+                    tmem_st16(lane_a + 64u * s + 16 * b, out);
                 }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(w_empty(ws));
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) mbar_arrive_cluster(first_full + 8u * s);
                 s += kGroups;
-                while (s >= S) { s -= S; ++round; }
+                ws += kGroups;
             }
-            const int turns = pair_turns(v.KT);
-            if (kt < turns && ok) {                       // the turn without a k-tile (ring_rules.h): seen and left
-                to_slot();
-                ok = mbar_wait(w_full(ws), wround & 1, &abort_flag);
-                ok = __all_sync(0xffffffffu, ok);
-                if (lane == 0) mbar_arrive(w_empty(ws));
-                kt += kGroups;
-                s += kGroups;
-            }
-            kt -= turns;                                  // this group's first k-tile of the next tile
-            unit_base += v.u1 - v.u0;
-            s -= turns - v.KT;                            // (stages have no place for that turn)
-            while (s >= S) { s -= S; ++round; }
-            if (s < 0) { s += S; --round; }
+            turn -= units;                                // this group's first unit of the next tile
         }
     } else if (warp >= kFirstEpiWarp) {
         // ===== accumulators (lane = column, tensor-memory column = row of x) -> y =====
-        const int quarter = warp & 3, half = (warp - kFirstEpiWarp) >> 2, col = 32 * quarter + lane;
-        const uint32_t lane_acc = tmem_base + ((uint32_t)(32 * quarter) << 16);
+        const int half = (warp - kFirstEpiWarp) >> 2;
         const uint32_t first_empty = in_cta(acc_empty(0), 0);
-        const int M = p.M, rows_pad = p.row_tiles * TN;
         bool ok = true;
         int set = 0, used = 0;
-        for (int t = cluster; t < p.tiles; t += clusters) {
+        for (int t = cluster; t < p.tiles && p.splits == 1; t += clusters) {
             const Tile v = tile_at(t);
-            const int n = v.n0 + col;
-            const bool col_ok = v.n0 + 32 * quarter < N;     // (N is a multiple of 32: whole warps)
-            const float b = (bias && col_ok) ? __half2float(bias[n]) : 0.f;
-            // two lanes exchange values so that each stores a pair of columns of every other row
-            auto store_rows = [&](int m, float (&x)[16]) {
-                const int left = col_ok ? M - m - (lane & 1) : 0;
-                __half* dst = y + (size_t)(m + (lane & 1)) * N + (n & ~1);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const float give = (lane & 1) ? x[2 * i] : x[2 * i + 1];
-                    const float got = __shfl_xor_sync(0xffffffffu, give, 1);
-                    const __half2 h = (lane & 1) ? __floats2half2_rn(got, x[2 * i + 1]) : __floats2half2_rn(x[2 * i], got);
-                    if (2 * i < left) *reinterpret_cast<__half2*>(dst) = h;
-                    dst += 2 * (size_t)N;
-                }
-            };
+            const float b = column_bias(v);
             if (ok) ok = mbar_wait(acc_full(set), used & 1, &abort_flag);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            float* mine = partial + (size_t)v.z * rows_pad * N;
-            const int chunks = min(TN, M - v.m0 + 15) / 16;          // 16 rows each; the next one is loaded meanwhile
+            const int chunks = min(TN, p.M - v.m0 + 15) / 16;        // 16 rows each; the next one is loaded meanwhile
             const uint32_t acc = lane_acc + (uint32_t)(set * TN);
             uint32_t r[16], next[16] = {};
             if (half < chunks) { tmem_ld16(acc + 16u * half, r); tmem_wait_ld(r); }
 #pragma unroll 1
             for (int c = half; c < chunks; c += 2) {
                 if (c + 2 < chunks) tmem_ld16(acc + 16u * (c + 2), next);
-                const int m = v.m0 + 16 * c;
-                if (p.splits == 1) {
-                    float x[16];
+                float x[16];
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) x[i] = __uint_as_float(r[i]) + b;
-                    store_rows(m, x);
-                } else if (col_ok) {
-#pragma unroll
-                    for (int i = 0; i < 16; ++i)
-                        if (m + i < M) mine[(size_t)(m + i) * N + n] = __uint_as_float(r[i]);
-                }
+                for (int i = 0; i < 16; ++i) x[i] = __uint_as_float(r[i]) + b;
+                store_rows(v, v.m0 + 16 * c, x);
                 tmem_wait_ld(next);
 #pragma unroll
                 for (int i = 0; i < 16; ++i) r[i] = next[i];
@@ -532,41 +532,70 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
             if (lane == 0) mbar_arrive_cluster(first_empty + 8u * set);
             if (++set == p.acc_sets) { set = 0; ++used; }
         }
-        if (p.splits > 1) __threadfence();               // the fp32 sums, before this CTA is counted in below
     }
 
-    if (p.splits > 1) {
-        // ===== split K (one tile per pair): the last CTA of a tile to arrive adds the runs in order, with all its warps: a warp
-        //       takes rows, a lane four columns.  (One column per lane and only the epilogue warps: 13 us for 77 rows.)
-        //       Reached whatever happened before, so that the tile's counter returns to zero. =====
-        __syncthreads();
+    if (p.splits > 1 && warp >= kFirstEpiWarp) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        // ===== split K (one tile per pair): blocks of 16 rows x 32 columns, a warp each, all warps but the first four.  A warp puts its
+        //       run's sums of a block into the scratch and is counted in; the last of the block's warps, of whichever CTA, adds the
+        //       runs in order.  No warp waits for another.  The counting is done whatever happened before, so that every counter
+        //       returns to zero.  (The last CTA of a tile to arrive adding all of it: 5000 clk for the sums in, 5000 for the sum,
+        //       of the 40 000 of 77 rows of 11008 x 4096.) =====
         const Tile v = tile_at(cluster);
-        unsigned int* counter = status + (cluster % (p.pairs * p.row_tiles)) * 2 + rank;
-        if (threadIdx.x == 0) arrived = atomicAdd(counter, 1u);
-        __syncthreads();
-        if (arrived == (unsigned int)p.splits - 1u) {
-            __threadfence();
-            const int n = v.n0 + 4 * lane;
-            const int rows = n < N ? min(TN, p.M - v.m0) : 0;
-            float bf[4] = {0.f, 0.f, 0.f, 0.f};
-            if (bias && n < N)
+        bool ok = mbar_wait(acc_full(0), 0, &abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const int chunks = min(TN, p.M - v.m0 + 15) / 16, all_chunks = TN / 16;
+        const int strips = N / 32, strip = v.n0 / 32 + (warp & 3), row_tile = v.m0 / TN;
+        if (strip < strips) {
+            const float b = column_bias(v);
+            const size_t run = (size_t)p.row_tiles * strips * all_chunks * 512;          // floats of a run of K
+#pragma unroll 1
+            for (int c = (warp - kFirstEpiWarp) >> 2; c < chunks; c += (kThreads / 32 - kFirstEpiWarp) / 4) {
+                const int block = (row_tile * strips + strip) * all_chunks + c;
+                float* base_p = partial + (size_t)block * 512 + 4 * lane;       // [4 rows][column][row] of a block
+                uint32_t r[16] = {};
+                if (ok) { tmem_ld16(lane_acc + 16u * c, r); tmem_wait_ld(r); }
+                float x[16];
 #pragma unroll
-                for (int c = 0; c < 4; ++c) bf[c] = __half2float(bias[n + c]);
-            const size_t run = (size_t)p.row_tiles * TN * N;
-#pragma unroll 2
-            for (int i = warp; i < rows; i += kThreads / 32) {
-                const float* src = partial + (size_t)(v.m0 + i) * N + n;
-                float4 part[kMaxSplits];
+                for (int i = 0; i < 16; ++i) x[i] = __uint_as_float(r[i]);
 #pragma unroll
-                for (int z = 0; z < kMaxSplits; ++z)
-                    part[z] = z < p.splits ? __ldcg(reinterpret_cast<const float4*>(src + z * run)) : make_float4(0.f, 0.f, 0.f, 0.f);
-                float4 x = part[0];
+                for (int i = 0; i < 4; ++i)
+                    *reinterpret_cast<float4*>(base_p + v.z * run + 128 * i) = make_float4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]);
+                __syncwarp();
+                unsigned int before = 0;                  // one lane's fences serve the warp, which it has just met and meets again
+                if (lane == 0) {
+                    asm volatile("fence.acq_rel.gpu;" ::: "memory");
+                    asm volatile("atom.relaxed.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(status + block) : "memory");
+                    asm volatile("fence.acq_rel.gpu;" ::: "memory");
+                }
+                __syncwarp();
+                if (__shfl_sync(0xffffffffu, before, 0) != (unsigned int)p.splits - 1u) continue;
+                // the other runs' sums, all on their way at once, through the rings (nothing is in flight there any more; their
+                // 48 values do not fit beside the warp's own in registers, and in two parts they took two round trips)
+                float* others = reinterpret_cast<float*>(base_ptr) + ((warp - kFirstEpiWarp) * (kMaxSplits - 1)) * 512 + 4 * lane;
+                if (ok)
+                    for (int z = 0, at = 0; z < p.splits; ++z)
+                        if (z != v.z) {
 #pragma unroll
-                for (int z = 1; z < kMaxSplits; ++z) { x.x += part[z].x; x.y += part[z].y; x.z += part[z].z; x.w += part[z].w; }
-                __half2 h[2] = {__floats2half2_rn(x.x + bf[0], x.y + bf[1]), __floats2half2_rn(x.z + bf[2], x.w + bf[3])};
-                *reinterpret_cast<uint2*>(y + (size_t)(v.m0 + i) * N + n) = *reinterpret_cast<const uint2*>(h);
+                            for (int i = 0; i < 4; ++i) cp_async16(smem_u32(others + at * 512 + 128 * i), base_p + z * run + 128 * i);
+                            ++at;
+                        }
+                asm volatile("cp.async.wait_all;" ::: "memory");
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float4 mine = make_float4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]);
+                    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (int z = 0, at = 0; z < p.splits; ++z) {
+                        const float4 f = z == v.z ? mine : *reinterpret_cast<const float4*>(others + at * 512 + 128 * i);
+                        at += z != v.z;
+                        sum.x += f.x; sum.y += f.y; sum.z += f.z; sum.w += f.w;
+                    }
+                    x[4 * i] = sum.x + b; x[4 * i + 1] = sum.y + b; x[4 * i + 2] = sum.z + b; x[4 * i + 3] = sum.w + b;
+                }
+                store_rows(v, v.m0 + 16 * c, x);
+                if (lane == 0) status[block] = 0u;
             }
-            if (threadIdx.x == 0) *counter = 0u;
         }
     }
 
@@ -629,13 +658,14 @@ int launch(const __half* x, const int32_t* qweight, const int32_t* qzeros, const
     a.pairs = (N + 2 * BN - 1) / (2 * BN);
     a.row_tiles = (M + TN - 1) / TN;
     const long long tiles = (long long)a.pairs * a.row_tiles * splits;
-    if (tiles > 0x7fffffff || (splits > 1 && 2LL * a.pairs * a.row_tiles >= kMaxCounters - 1)) return B200GPTQ_ERR_TOO_LARGE;
+    if (tiles > 0x7fffffff || (splits > 1 && (long long)(N / 32) * a.row_tiles * (TN / 16) >= kMaxCounters - 1)) return B200GPTQ_ERR_TOO_LARGE;
     a.tiles = (int)tiles;
     const int pairs_of_sms = sm_count() / 2;
-    const PairRings rings = pair_rings(BITS, a.groups_in_slot, TN);
-    a.acc_sets = rings.acc_sets; a.S = rings.stages; a.SW = rings.slots;
-    const int x_stage = TN / 2 * BK * 2, w_slot = pair_slot_bytes(BITS, a.groups_in_slot);
-    if (a.SW < 4 || a.S < kPairMinStages) return B200GPTQ_ERR_TOO_LARGE;
+    // (a second set of accumulators only serves a pair that has another tile to go on with)
+    const PairRings rings = pair_rings(BITS, a.groups_in_slot, TN, a.tiles > pairs_of_sms);
+    a.acc_sets = rings.acc_sets; a.S = rings.stages / 2; a.SW = rings.slots;
+    const int x_stage = TN * BK * 2, w_slot = pair_slot_bytes(BITS, a.groups_in_slot);
+    if (a.SW < 4 || rings.stages < kPairMinStages) return B200GPTQ_ERR_TOO_LARGE;
     const int smem = a.S * x_stage + a.SW * w_slot + 1024;
     auto map = [&](CUtensorMap* m, CUtensorMapDataType type, int rank, const void* ptr, const cuuint64_t* dims,
                    const cuuint64_t* strides, const cuuint32_t* box, CUtensorMapSwizzle swizzle) {

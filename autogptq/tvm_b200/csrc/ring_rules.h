@@ -13,16 +13,16 @@ namespace b200gptq {
 // stages a stage always belongs to one group, which saw its previous fill itself.
 constexpr int ring_in_whole_turns(int stages, int groups) { return stages / groups * groups; }
 
-// Pairs of CTAs (gemm_pair.cu): a slot of the weight ring holds two k-tiles, four groups take k-tiles in turn, through one tile
-// after the other.  A tile with an odd number of k-tiles is walked as if it had one more, whose group sees the slot but does
-// nothing: a group then moves on by two slots at every turn, and with an even number of slots a slot always belongs to the same
-// two groups.  The stages (x and A) count real k-tiles only; a group's turns are at most eight of those apart, and a wait
-// for a stage knows that its products of two rounds before have retired if there are that many stages.
+// Pairs of CTAs (gemm_pair.cu): units of two k-tiles, through one tile after the other; a tile with an odd number of k-tiles ends in
+// a unit of one.  A slot of the weight ring holds a unit, and with a multiple of the groups a slot always belongs to one group, which
+// saw its previous fill itself.  A stage (x and A) holds a unit as well; `stages` counts its k-tiles.  A group's turns are four units
+// apart and products retire in order, so a wait for a stage knows that its products of two rounds before have retired if there are
+// four units or more.
 constexpr int kPairGroups = 4, kPairMinStages = 8;
 constexpr int pair_turns(int k_tiles) { return (k_tiles + 1) & ~1; }
 
 constexpr int kPairColumns = 128, kPairKTile = 64;         // columns per CTA, rows of K per stage
-constexpr int kPairTmemCols = 512;                         // accumulators, then 32 columns of A per stage
+constexpr int kPairTmemCols = 512;                         // accumulators, then 32 columns of A per k-tile of a stage
 constexpr int kPairSmem = 222 * 1024;
 constexpr int kPairMaxStages = 14, kPairMaxSlots = 16;
 
@@ -33,17 +33,21 @@ constexpr int pair_slot_bytes(int bits, int groups) { return pair_unit_bytes(bit
 
 struct PairRings {
     int acc_sets;      // sets of accumulators
-    int stages;        // of x (shared memory) and A (tensor memory)
+    int stages;        // of x (shared memory) and A (tensor memory), in k-tiles: an even number
     int slots;         // of packed weights and constants
 };
-inline PairRings pair_rings(int bits, int groups, int rows) {      // rows of x per tile
+inline PairRings pair_rings(int bits, int groups, int rows, bool several_tiles = true) {      // rows of x per tile
     PairRings r;
-    r.acc_sets = rows <= 128 ? 2 : 1;
+    r.acc_sets = rows <= 128 && several_tiles ? 2 : 1;
     r.stages = (kPairTmemCols - r.acc_sets * rows) / 32;
     if (r.stages > kPairMaxStages) r.stages = kPairMaxStages;
-    r.slots = (kPairSmem - 1024 - r.stages * (rows / 2 * kPairKTile * 2)) / pair_slot_bytes(bits, groups);
-    if (r.slots > kPairMaxSlots) r.slots = kPairMaxSlots;
-    r.slots &= ~1;
+    // A group of weight warps wants two slots, one to unpack and one to fill: a stage above the least gives way to that.
+    for (r.stages &= ~1;; r.stages -= 2) {
+        r.slots = (kPairSmem - 1024 - r.stages * (rows / 2 * kPairKTile * 2)) / pair_slot_bytes(bits, groups);
+        if (r.slots > kPairMaxSlots) r.slots = kPairMaxSlots;
+        r.slots = ring_in_whole_turns(r.slots, kPairGroups);
+        if (r.slots >= 2 * kPairGroups || r.stages <= kPairMinStages) break;
+    }
     return r;
 }
 

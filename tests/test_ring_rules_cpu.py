@@ -115,3 +115,29 @@ def test_stages_of_the_small_gemm_belong_to_one_group_each(lib):
     for stages in range(4, 24):
         s = lib.whole_turns(stages, 3)
         assert 3 <= s <= stages and all((kt - s) % 3 == kt % 3 for kt in range(s, 200))
+
+
+def test_pair_units_never_wait_blind(lib):
+    """Groups take whole units in turn, through one tile after the other (a tile with an odd number of k-tiles ends in a unit of one):
+    a slot's previous fill was the group's own, and a stage's products of two rounds before have retired."""
+    r = (ctypes.c_int * 3)()
+    for bits in (2, 3, 4, 8):
+        for groups in (1, 2, 3, 4):
+            for rows in range(32, 257, 32):
+                lib.rings(bits, groups, rows, r)
+                stages, slots = r[1] // 2, r[2]
+                assert r[1] % 2 == 0
+                for k_tiles in (1, 2, 3, 5, 64, 171):
+                    units = lib.turns(k_tiles) // 2
+                    for g in range(4):
+                        turn, base, seen, upto = g, 0, set(), -1
+                        for _ in range(200 // units + 2):
+                            while turn < units:
+                                u = base + turn
+                                assert u % 4 == g
+                                assert u < slots or u - slots in seen
+                                assert u < 2 * stages or u - 2 * stages <= upto
+                                seen.add(u)
+                                upto = u - stages
+                                turn += 4
+                            turn, base = turn - units, base + units
