@@ -666,7 +666,10 @@ int launch(const __half* x, const int32_t* qweight, const int32_t* qzeros, const
     a.acc_sets = rings.acc_sets; a.S = rings.stages / 2; a.SW = rings.slots;
     const int x_stage = TN * BK * 2, w_slot = pair_slot_bytes(BITS, a.groups_in_slot);
     if (a.SW < 4 || rings.stages < kPairMinStages) return B200GPTQ_ERR_TOO_LARGE;
-    const int smem = a.S * x_stage + a.SW * w_slot + 1024;
+    // (the sums of a split K pass through the rings: 6 KB per warp that adds them)
+    const int rings_bytes = a.S * x_stage + a.SW * w_slot;
+    const int sum_bytes = splits > 1 ? (kThreads / 32 - kFirstEpiWarp) * (kMaxSplits - 1) * 2048 : 0;
+    const int smem = (rings_bytes > sum_bytes ? rings_bytes : sum_bytes) + 1024;
     auto map = [&](CUtensorMap* m, CUtensorMapDataType type, int rank, const void* ptr, const cuuint64_t* dims,
                    const cuuint64_t* strides, const cuuint32_t* box, CUtensorMapSwizzle swizzle) {
         const cuuint32_t estr[2] = {1, 1};
