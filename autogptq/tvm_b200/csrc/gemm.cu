@@ -34,6 +34,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "gemm_pair.h"
 #include "ring_rules.h"
 
 namespace b200gptq {
@@ -590,9 +591,8 @@ int splits_for(int M, int tiles, int KT, int slots) {
     if (sp > kMaxSplits) sp = kMaxSplits;
     // Every run keeps enough k-tiles to pay for its own start-up and for the final sum: 16 (4096 x 4096, 16 rows: 33.5 -> 21 us
     // with four runs).  The taller the partial sums, the more they cost: above 64 rows two runs of 16 lose (2048 x 4096, 100
-    // rows: 12.5 -> 14.1 us) where four gain (4096 x 4096, 80 rows: 19.5 -> 14.4).  Above 96 rows a run keeps 40, a bound that
-    // was measured with one CTA per tile; with pairs four runs of 16 gain there too (128 rows of 4096 x 4096: 19.9 -> 16.6), but
-    // other sizes of 97 to 128 rows have not been measured.
+    // rows: 12.5 -> 14.1 us) where four gain (4096 x 4096, 80 rows: 19.5 -> 14.4).  Above 96 rows a run keeps 40: two tiles of 64 rows
+    // in one run are as fast as three runs of one tile (128 rows of 4096 x 4096 13.0 and 12.8).
     const int min_tiles = M <= 96 ? 16 : 40;
     while (sp > 1 && KT / sp < min_tiles) --sp;
     if (M > 64 && M <= 96 && sp < 3) return 1;
@@ -691,20 +691,15 @@ int launch_gemm(const __half* x_for_tma, const int32_t* qweight, const int32_t* 
 
 }  // namespace
 
-size_t gemm_pair_partial_bytes(int M, int K, int N, int splits);
-int gemm_pair_dispatch(const __half* x, const int32_t* qweight, const int32_t* qzeros, const __half* scales, const int32_t* g_idx,
-                       const __half* bias, __half* y, int M, int K, int N, int bits, int group_size, int splits,
-                       unsigned int* status, float* partial, cudaStream_t stream);
-
 // More than 16 rows, and the bit widths that only it has: the kernel for pairs of CTAs (gemm_pair.cu).  From 17 to 64 rows,
 // one CTA per tile against pairs: 4096 x 4096, 17 rows 16.4 and 11.2 us; 4096 x 12288, 64 rows 29.1 and 20.2; 11008 x 4096, 64
 // rows 35.2 and 20.6; 9216 x 9216, 3 bits, 24 rows 38.0 and 33.3; 9216 x 27648, 64 rows 106 and 84.  Up to 16 rows single
 // CTAs, two per SM, have stayed, though pairs took 11.2 us where they take 14 to 16 on 4096 x 4096: a layer's rows go to the
 // decode GEMV there, and what is left (direct calls, layers with a g_idx) has not been measured over sizes.
 static bool use_pair(int M, int bits) { return M > 16 || bits == 2 || bits == 8; }
-// (a tile per pair of SMs, so that the last CTA of a tile can add the runs with all its warps)
-static int pair_splits(int M, int N, int K) {
-    return splits_for(M, (N + 2 * BN - 1) / (2 * BN), (K + BK - 1) / BK, sm_count() / 2);
+// (up to 128 rows as many runs as here; above, gemm_pair_plan weighs them against the rows of a tile)
+static GemmPairPlan pair_plan(int M, int N, int K) {
+    return gemm_pair_plan(M, N, K, splits_for(M, (N + 2 * BN - 1) / (2 * BN), (K + BK - 1) / BK, sm_count() / 2));
 }
 
 // Scratch: the counter region (its last word is the sticky status word) and, when x has to be
@@ -712,14 +707,14 @@ static int pair_splits(int M, int N, int K) {
 size_t gemm_workspace_bytes(int M, int K, int N, int bits) {
     // counters | copy of x (gathered / permuted) | fp32 partial sums of a split-K launch
     return kCounterBytes + (((size_t)M * K * sizeof(__half) + 255) & ~(size_t)255) +
-           (use_pair(M, bits) ? gemm_pair_partial_bytes(M, K, N, pair_splits(M, N, K)) : split_partial_bytes(M, N, K));
+           (use_pair(M, bits) ? gemm_pair_partial_bytes(M, N, pair_plan(M, N, K)) : split_partial_bytes(M, N, K));
 }
 
 
 void gemm_split_query(int M, int K, int N, int bits, int* splits, int* ctas_per_sm) {
     GemmSplit g;
     if (use_pair(M, bits)) {
-        g.splits = pair_splits(M, N, K);
+        g.splits = pair_plan(M, N, K).splits;
         g.per_sm = 1;
     } else {
         g = pick_split(M, N, K);
@@ -761,8 +756,8 @@ int gemm_dispatch(const __half* x, const int32_t* qweight, const int32_t* qzeros
     float* partial = reinterpret_cast<float*>(reinterpret_cast<char*>(workspace) + kCounterBytes +
                                               (((size_t)M * K * sizeof(__half) + 255) & ~(size_t)255));
     if (pair)
-        return gemm_pair_dispatch(xt, qweight, qzeros, scales, g_idx, bias, y, M, K, N, bits, group_size, pair_splits(M, N, K),
-                                  status, partial, stream);
+        return gemm_pair_dispatch(xt, qweight, qzeros, scales, g_idx, bias, y, M, K, N, bits, group_size,
+                                  pair_plan(M, N, K), status, partial, stream);
     if (bits == 4) return launch_gemm<4>(xt, qweight, qzeros, scales, g_idx, bias, y, M, K, N, group_size, status, partial, stream);
     if (bits == 3) return launch_gemm<3>(xt, qweight, qzeros, scales, g_idx, bias, y, M, K, N, group_size, status, partial, stream);
     return B200GPTQ_ERR_BITS;

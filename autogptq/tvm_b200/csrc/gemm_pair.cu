@@ -8,7 +8,7 @@
 // a quarter of the products 152, without the dequantisation 166).  Here two CTAs of a cluster share a 256-column tile
 // (tcgen05 cta_group::2): each holds and dequantises its own 128 columns and HALF of the rows of x.
 //
-//   warp 0      TMA: packed weights, scales and zero-points of 128 rows of K, into a ring of their own that runs ahead of
+//   warps 0, 3  TMA: packed weights, scales and zero-points of 128 rows of K, into a ring of their own that runs ahead of
 //               the products as far as shared memory allows (they come from DRAM, x from L2)
 //   warp 1      TMA: this CTA's rows of x, into the stages; completion is counted in the first CTA of the pair
 //   warp 2      first CTA: issues tcgen05.mma for both (M = 256 columns, N = TN rows of x, K = 16); allocates tensor memory
@@ -35,6 +35,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "gemm_pair.h"
 #include "ring_rules.h"
 
 namespace b200gptq {
@@ -51,6 +52,7 @@ constexpr int kTmemCols = kPairTmemCols; // accumulators in columns [0, TN), 32 
 constexpr int kSmemMax = kPairSmem;
 constexpr int kStatusWord = kMaxCounters - 1;
 constexpr int kMaxSplits = 4;
+constexpr int kSumWarps = kThreads / 32 - kFirstEpiWarp;     // warps that add the runs of a split K
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ bool elect_one() {
@@ -317,7 +319,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     asm volatile("griddepcontrol.launch_dependents;");
     // What a preceding kernel may still be writing: x; what it may still be reading: y and the scratch.  The weights are unpacked
     // before the wait, as far as the stages go (77 rows of 11008 x 4096: the first product came 2.6 us after the wait, now 1.1).
-    if (warp != 0 && (warp < kFirstWeightWarp || g_idx)) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (warp != 0 && warp != 3 && (warp < kFirstWeightWarp || g_idx)) asm volatile("griddepcontrol.wait;" ::: "memory");
 
     // ---- epilogue: a warp reads the accumulators of 32 columns (tensor-memory lanes), 16 rows of x at a time ----
     const uint32_t lane_acc = tmem_base + ((uint32_t)(32 * (warp & 3)) << 16);
@@ -339,28 +341,32 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
         }
     };
 
-    if (warp == 0) {
+    if (warp == 0 || warp == 3) {
         // ===== packed weights, scales, zero-points.  (With a g_idx the number of groups is not known here, so boxes could not
         //       be clipped to the arrays: the weight warps read scales and zero-points themselves.  The first boxes sent off before the
         //       cluster has met: a launch 0.4 to 0.6 us longer, a box takes its thread 120 clk.) =====
+        //       Two warps, every other unit each: one thread takes 600 clk for a unit's barrier and boxes, and the weight warps had to wait
+        //       for it (8 bits, 128 rows per tile 480 clk per 64 rows of K, now 430; 3 bits, 32 rows 335, now 310).
         if (elect_one()) {
             const int rows_g = g_idx ? 0 : p.groups_in_slot;
             const uint32_t tx = pair_unit_bytes(BITS) + rows_g * (BN * 2 + pair_zero_words(BITS) * 4);
-            int s = 0, round = 0;
+            int s = 0, round = 0, mine = warp == 0;
             bool ok = true;
             for (int t = cluster; t < p.tiles && ok; t += clusters) {
                 const Tile v = tile_at(t);
                 const int zn = v.n0 / 32 * BITS;
-                for (int u = v.u0; u < v.u1; ++u) {
-                    const int g0 = group_at(4 * u);
-                    if (round > 0) ok = mbar_wait(w_empty(s), (round - 1) & 1, &abort_flag);
-                    if (!ok) break;
-                    const uint32_t dst = base + w_off + s * w_slot, bar = w_full(s);
-                    mbar_expect(bar, tx);
-                    tma_2d(dst, &tmap_w, v.n0, u * 4 * BITS, bar);
-                    if (rows_g) tma_2d(dst + pair_unit_bytes(BITS), &tmap_s, v.n0, g0, bar);
-                    for (int r = 0; r < rows_g; ++r)
-                        tma_1d(dst + pair_unit_bytes(BITS) + rows_g * BN * 2 + r * 128, &tmap_z, ((g0 + r) * zwords + zn) & ~3, bar);
+                for (int u = v.u0; u < v.u1; ++u, mine ^= 1) {
+                    if (mine) {
+                        const int g0 = group_at(4 * u);
+                        if (round > 0) ok = mbar_wait(w_empty(s), (round - 1) & 1, &abort_flag);
+                        if (!ok) break;
+                        const uint32_t dst = base + w_off + s * w_slot, bar = w_full(s);
+                        mbar_expect(bar, tx);
+                        tma_2d(dst, &tmap_w, v.n0, u * 4 * BITS, bar);
+                        if (rows_g) tma_2d(dst + pair_unit_bytes(BITS), &tmap_s, v.n0, g0, bar);
+                        for (int r = 0; r < rows_g; ++r)
+                            tma_1d(dst + pair_unit_bytes(BITS) + rows_g * BN * 2 + r * 128, &tmap_z, ((g0 + r) * zwords + zn) & ~3, bar);
+                    }
                     if (++s == SW) { s = 0; ++round; }
                 }
             }
@@ -536,65 +542,61 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
 
     if (p.splits > 1 && warp >= kFirstEpiWarp) {
         asm volatile("griddepcontrol.wait;" ::: "memory");
-        // ===== split K (one tile per pair): blocks of 16 rows x 32 columns, a warp each, all warps but the first four.  A warp puts its
-        //       run's sums of a block into the scratch and is counted in; the last of the block's warps, of whichever CTA, adds the
-        //       runs in order.  No warp waits for another.  The counting is done whatever happened before, so that every counter
-        //       returns to zero.  (The last CTA of a tile to arrive adding all of it: 5000 clk for the sums in, 5000 for the sum,
-        //       of the 40 000 of 77 rows of 11008 x 4096.) =====
+        // ===== split K (one tile per pair): a warp takes every sixth 16 rows of its 32 columns, all warps but the first four.  It puts its
+        //       run's sums of them into the scratch and is counted in; the last of the runs' warps, of whichever CTA, adds the runs in
+        //       order.  No warp waits for another.  The counting is done whatever happened before, so that every counter returns to
+        //       zero.  (The last CTA of a tile to arrive adding all of it: 5000 clk for the sums in, 5000 for the sum, of the 40 000
+        //       of 77 rows of 11008 x 4096.) =====
         const Tile v = tile_at(cluster);
         bool ok = mbar_wait(acc_full(0), 0, &abort_flag);
         ok = __all_sync(0xffffffffu, ok);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const int chunks = min(TN, p.M - v.m0 + 15) / 16, all_chunks = TN / 16;
-        const int strips = N / 32, strip = v.n0 / 32 + (warp & 3), row_tile = v.m0 / TN;
-        if (strip < strips) {
-            const float b = column_bias(v);
+        const int chunks = min(TN, p.M - v.m0 + 15) / 16, all_chunks = TN / 16, first = (warp - kFirstEpiWarp) >> 2;
+        const int strips = N / 32, strip = v.n0 / 32 + (warp & 3), column = (v.m0 / TN) * strips + strip;
+        if (strip < strips && first < chunks) {
             const size_t run = (size_t)p.row_tiles * strips * all_chunks * 512;          // floats of a run of K
+            float* sums = partial + (size_t)column * all_chunks * 512 + 4 * lane;        // [16 rows][4 of them][column][row]
 #pragma unroll 1
-            for (int c = (warp - kFirstEpiWarp) >> 2; c < chunks; c += (kThreads / 32 - kFirstEpiWarp) / 4) {
-                const int block = (row_tile * strips + strip) * all_chunks + c;
-                float* base_p = partial + (size_t)block * 512 + 4 * lane;       // [4 rows][column][row] of a block
+            for (int c = first; c < chunks; c += kSumWarps / 4) {
                 uint32_t r[16] = {};
                 if (ok) { tmem_ld16(lane_acc + 16u * c, r); tmem_wait_ld(r); }
-                float x[16];
-#pragma unroll
-                for (int i = 0; i < 16; ++i) x[i] = __uint_as_float(r[i]);
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
-                    *reinterpret_cast<float4*>(base_p + v.z * run + 128 * i) = make_float4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]);
-                __syncwarp();
-                unsigned int before = 0;                  // one lane's fences serve the warp, which it has just met and meets again
-                if (lane == 0) {
-                    asm volatile("fence.acq_rel.gpu;" ::: "memory");
-                    asm volatile("atom.relaxed.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(status + block) : "memory");
-                    asm volatile("fence.acq_rel.gpu;" ::: "memory");
-                }
-                __syncwarp();
-                if (__shfl_sync(0xffffffffu, before, 0) != (unsigned int)p.splits - 1u) continue;
-                // the other runs' sums, all on their way at once, through the rings (nothing is in flight there any more; their
-                // 48 values do not fit beside the warp's own in registers, and in two parts they took two round trips)
-                float* others = reinterpret_cast<float*>(base_ptr) + ((warp - kFirstEpiWarp) * (kMaxSplits - 1)) * 512 + 4 * lane;
-                if (ok)
-                    for (int z = 0, at = 0; z < p.splits; ++z)
-                        if (z != v.z) {
+                    *reinterpret_cast<uint4*>(sums + v.z * run + c * 512 + 128 * i) = make_uint4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
+            }
+            __syncwarp();
+            unsigned int before = 0;                      // one lane's fences serve the warp, which it has just met and meets again
+            if (lane == 0) {
+                unsigned int* counter = status + column * (kSumWarps / 4) + first;
+                asm volatile("fence.acq_rel.gpu;" ::: "memory");
+                asm volatile("atom.relaxed.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(counter) : "memory");
+                asm volatile("fence.acq_rel.gpu;" ::: "memory");
+                if (before == (unsigned int)p.splits - 1u) *counter = 0u;
+            }
+            __syncwarp();
+            if (__shfl_sync(0xffffffffu, before, 0) == (unsigned int)p.splits - 1u) {
+                const float b = column_bias(v);
+                // All runs' sums of 16 rows on their way at once, through the rings: nothing is in flight there any more, and 64 values
+                // do not fit in registers (in two parts they took two round trips).  A lane reads what it has copied itself.
+                float* copy = reinterpret_cast<float*>(base_ptr) + (warp - kFirstEpiWarp) * p.splits * 512 + 4 * lane;
+#pragma unroll 1
+                for (int c = first; c < chunks && ok; c += kSumWarps / 4) {
+                    for (int z = 0; z < p.splits; ++z)
 #pragma unroll
-                            for (int i = 0; i < 4; ++i) cp_async16(smem_u32(others + at * 512 + 128 * i), base_p + z * run + 128 * i);
-                            ++at;
+                        for (int i = 0; i < 4; ++i) cp_async16(smem_u32(copy + z * 512 + 128 * i), sums + z * run + c * 512 + 128 * i);
+                    asm volatile("cp.async.wait_all;" ::: "memory");
+                    float x[16];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        float4 sum = *reinterpret_cast<const float4*>(copy + 128 * i);
+                        for (int z = 1; z < p.splits; ++z) {
+                            const float4 f = *reinterpret_cast<const float4*>(copy + z * 512 + 128 * i);
+                            sum.x += f.x; sum.y += f.y; sum.z += f.z; sum.w += f.w;
                         }
-                asm volatile("cp.async.wait_all;" ::: "memory");
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float4 mine = make_float4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]);
-                    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-                    for (int z = 0, at = 0; z < p.splits; ++z) {
-                        const float4 f = z == v.z ? mine : *reinterpret_cast<const float4*>(others + at * 512 + 128 * i);
-                        at += z != v.z;
-                        sum.x += f.x; sum.y += f.y; sum.z += f.z; sum.w += f.w;
+                        x[4 * i] = sum.x + b; x[4 * i + 1] = sum.y + b; x[4 * i + 2] = sum.z + b; x[4 * i + 3] = sum.w + b;
                     }
-                    x[4 * i] = sum.x + b; x[4 * i + 1] = sum.y + b; x[4 * i + 2] = sum.z + b; x[4 * i + 3] = sum.w + b;
+                    store_rows(v, v.m0 + 16 * c, x);
                 }
-                store_rows(v, v.m0 + 16 * c, x);
-                if (lane == 0) status[block] = 0u;
             }
         }
     }
@@ -624,41 +626,50 @@ EncodeTiledFn encode_tiled_fn() {
     return fn;
 }
 
-// Rows of x per tile: the shortest sum over waves of (k-tiles x clocks per k-tile + drain of the accumulators, where there is
-// one set).  A k-tile costs its four products (TN / 2 clk each, measured) but no less than the weight warps take: 370 clk, what the
-// choice was fitted with; about 450 have been measured since, and the choice has not been fitted again.
-int pick_rows(int M, int N, int K, int splits) {
-    const long long pairs = (N + 2 * BN - 1) / (2 * BN), slots = sm_count() / 2;
-    const long long kt = ((K + BK - 1) / BK + splits - 1) / splits;
+}  // namespace
+
+// Rows of x per tile and runs of K.  In clocks, fitted to 4 bits, 100 to 1024 rows of 4096 x 4096, 4096 x 12288, 11008 x 4096,
+// 2048 x 8192 and 8192 x 2048 (within 10 % of what was measured; 3 and 8 bits come within 5 % of 4): a k-tile takes what kPerTile
+// says, the weight warps up to 128 rows and the products above; start-up and drain take longer the more SMs work; the sum over runs
+// grows with what goes through the scratch.  Several runs have a tile per pair of SMs, of eight units or more.  Up to 128 rows the
+// caller says how many runs (`few`), in one tile of rows.  Against the best tile without runs: 256 rows of 11008 x 4096 32.1 -> 24.9 us,
+// 256 rows of 8192 x 2048 23.3 -> 15.9, 512 rows 25.0 -> 21.2.
+GemmPairPlan gemm_pair_plan(int M, int N, int K, int few) {
+    constexpr int kPerTile[8] = {300, 310, 325, 340, 390, 470, 540, 610};      // 32, 64, .. 256 rows
+    const long long pairs = (N + 2 * BN - 1) / (2 * BN), slots = sm_count() / 2, units = (K + 127) / 128;
+    const int least = M <= 128 ? few : 1, most = M <= 128 ? few : kMaxSplits;
     long long best = -1;
-    int tn = 256;
-    for (int t = 256; t >= 32; t -= 32) {
-        if (splits > 1 && t < M && t < 256) break;       // (a tile per pair)
-        const long long rows = (M + t - 1) / t;
-        const long long per_kt = 2 * t + 8 > 370 ? 2 * t + 8 : 370;
-        const long long cost = ((pairs * rows * splits + slots - 1) / slots) * (kt * per_kt + (t > 128 ? 8 * t : 300)) + 12 * t;
-        if (best < 0 || cost < best) { best = cost; tn = t; }
-    }
-    return tn;
+    GemmPairPlan plan = {256, 1};
+    for (int splits = least; splits <= most; ++splits)
+        for (int t = 256; t >= 32; t -= 32) {
+            const long long rows = (M + t - 1) / t, tiles = pairs * rows * splits, waves = (tiles + slots - 1) / slots;
+            if (splits > 1 && (M <= 128 ? t < M : waves > 1 || units / splits < 8)) break;
+            const long long kt = 2 * ((units + splits - 1) / splits), busy = tiles < slots ? tiles : slots;
+            const long long cost = waves * kt * kPerTile[t / 32 - 1] + 2850 + 8200 * busy / slots + (splits > 1 ? 6500 + 8 * t * splits : 0);
+            if (best < 0 || cost < best) { best = cost; plan = {t, splits}; }
+        }
+    return plan;
 }
+
+namespace {
 
 template <int BITS>
 int launch(const __half* x, const int32_t* qweight, const int32_t* qzeros, const __half* scales, const int32_t* g_idx,
-           const __half* bias, __half* y, int M, int K, int N, int group_size, int splits, unsigned int* status,
+           const __half* bias, __half* y, int M, int K, int N, int group_size, GemmPairPlan plan, unsigned int* status,
            float* partial, cudaStream_t stream) {
     const EncodeTiledFn encode = encode_tiled_fn();
     if (!encode) { set_last_cuda_error((int)cudaErrorNotSupported); return B200GPTQ_ERR_CUDA; }
     const int groups = (K + group_size - 1) / group_size;
     PairArgs a = {};
-    a.M = M; a.K = K; a.N = N; a.splits = splits;
+    const int splits = plan.splits, TN = plan.rows;
+    a.M = M; a.K = K; a.N = N; a.splits = splits; a.TN = TN;
     a.spg = group_size >= K ? (K + 31) / 32 : (group_size >= 32 ? group_size / 32 : 1);
     a.spg_inv = (unsigned int)((0x100000000ULL + a.spg - 1) / a.spg);                 // (not used for 1)
     a.groups_in_slot = a.spg % 4 == 0 || groups == 1 ? 1 : (a.spg == 1 ? 4 : (a.spg == 2 ? 2 : 3));
-    const int TN = a.TN = pick_rows(M, N, K, splits);
     a.pairs = (N + 2 * BN - 1) / (2 * BN);
     a.row_tiles = (M + TN - 1) / TN;
     const long long tiles = (long long)a.pairs * a.row_tiles * splits;
-    if (tiles > 0x7fffffff || (splits > 1 && (long long)(N / 32) * a.row_tiles * (TN / 16) >= kMaxCounters - 1)) return B200GPTQ_ERR_TOO_LARGE;
+    if (tiles > 0x7fffffff || (splits > 1 && (long long)(N / 32) * a.row_tiles * (kSumWarps / 4) >= kMaxCounters - 1)) return B200GPTQ_ERR_TOO_LARGE;
     a.tiles = (int)tiles;
     const int pairs_of_sms = sm_count() / 2;
     // (a second set of accumulators only serves a pair that has another tile to go on with)
@@ -666,9 +677,8 @@ int launch(const __half* x, const int32_t* qweight, const int32_t* qzeros, const
     a.acc_sets = rings.acc_sets; a.S = rings.stages / 2; a.SW = rings.slots;
     const int x_stage = TN * BK * 2, w_slot = pair_slot_bytes(BITS, a.groups_in_slot);
     if (a.SW < 4 || rings.stages < kPairMinStages) return B200GPTQ_ERR_TOO_LARGE;
-    // (the sums of a split K pass through the rings: 6 KB per warp that adds them)
-    const int rings_bytes = a.S * x_stage + a.SW * w_slot;
-    const int sum_bytes = splits > 1 ? (kThreads / 32 - kFirstEpiWarp) * (kMaxSplits - 1) * 2048 : 0;
+    // (the sums of a split K pass through the rings: 2 KB per run and warp)
+    const int rings_bytes = a.S * x_stage + a.SW * w_slot, sum_bytes = splits > 1 ? kSumWarps * splits * 2048 : 0;
     const int smem = (rings_bytes > sum_bytes ? rings_bytes : sum_bytes) + 1024;
     auto map = [&](CUtensorMap* m, CUtensorMapDataType type, int rank, const void* ptr, const cuuint64_t* dims,
                    const cuuint64_t* strides, const cuuint32_t* box, CUtensorMapSwizzle swizzle) {
@@ -718,21 +728,20 @@ int launch(const __half* x, const int32_t* qweight, const int32_t* qzeros, const
 
 }  // namespace
 
-// fp32 partial sums of a launch whose k-tiles are cut into `splits` runs
-size_t gemm_pair_partial_bytes(int M, int K, int N, int splits) {
-    if (splits == 1) return 0;
-    const int tn = pick_rows(M, N, K, splits);
-    return (size_t)splits * ((M + tn - 1) / tn * tn) * N * sizeof(float);
+// fp32 partial sums of a launch whose k-tiles are cut into runs
+size_t gemm_pair_partial_bytes(int M, int N, GemmPairPlan plan) {
+    if (plan.splits == 1) return 0;
+    return (size_t)plan.splits * ((M + plan.rows - 1) / plan.rows * plan.rows) * N * sizeof(float);
 }
 
 int gemm_pair_dispatch(const __half* x, const int32_t* qweight, const int32_t* qzeros, const __half* scales, const int32_t* g_idx,
-                       const __half* bias, __half* y, int M, int K, int N, int bits, int group_size, int splits,
+                       const __half* bias, __half* y, int M, int K, int N, int bits, int group_size, GemmPairPlan plan,
                        unsigned int* status, float* partial, cudaStream_t stream) {
     switch (bits) {
-        case 2: return launch<2>(x, qweight, qzeros, scales, g_idx, bias, y, M, K, N, group_size, splits, status, partial, stream);
-        case 3: return launch<3>(x, qweight, qzeros, scales, g_idx, bias, y, M, K, N, group_size, splits, status, partial, stream);
-        case 4: return launch<4>(x, qweight, qzeros, scales, g_idx, bias, y, M, K, N, group_size, splits, status, partial, stream);
-        case 8: return launch<8>(x, qweight, qzeros, scales, g_idx, bias, y, M, K, N, group_size, splits, status, partial, stream);
+        case 2: return launch<2>(x, qweight, qzeros, scales, g_idx, bias, y, M, K, N, group_size, plan, status, partial, stream);
+        case 3: return launch<3>(x, qweight, qzeros, scales, g_idx, bias, y, M, K, N, group_size, plan, status, partial, stream);
+        case 4: return launch<4>(x, qweight, qzeros, scales, g_idx, bias, y, M, K, N, group_size, plan, status, partial, stream);
+        case 8: return launch<8>(x, qweight, qzeros, scales, g_idx, bias, y, M, K, N, group_size, plan, status, partial, stream);
     }
     return B200GPTQ_ERR_BITS;
 }

@@ -100,8 +100,9 @@ def test_registered_operator_has_a_shape_rule():
 
 
 def test_gemm_work_split_rule():
-    """b200gptq_gemm_split is host-only (without a device it plans for 148 SMs): K is split only for up to 128 rows
-    and while every run keeps 16 k-tiles (40 above 96 rows; from 65 rows on into no fewer than three); more than 16 rows, and 2 and
+    """b200gptq_gemm_split is host-only (without a device it plans for 148 SMs): K is split for up to 128 rows
+    while every run keeps 16 k-tiles (40 above 96 rows; from 65 rows on into no fewer than three), above that where it saves unpacking
+    the weights for another tile of rows; more than 16 rows, and 2 and
     8 bits, run on pairs of SMs, one CTA each; the second CTA per SM comes only below that and only where it shortens waves x
     k-tiles."""
     from autogptq.tvm_b200 import ops

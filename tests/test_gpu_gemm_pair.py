@@ -47,6 +47,19 @@ def test_gemm_against_dequantised_product(bits, K, N, gs, M, gather):
     ops.check_status(DEV)
 
 
+@pytest.mark.parametrize("bits,K,N,gs,M,gather,runs", [
+    (4, 11008, 4096, 64, 256, False, 2),      # runs over several tiles of rows
+    (8, 8192, 2048, -1, 200, True, 4),
+    (3, 8224, 2080, 32, 400, False, 2),       # a cut last unit, a part of a column tile, tiles of more than 96 rows
+    (4, 8192, 2048, 128, 129, False, 4),      # fewest rows that are weighed
+    (2, 8192, 2048, 128, 90, False, 4),       # rings smaller than the room that the sums need
+    (2, 1056, 9472, 32, 130, False, 1),
+])
+def test_runs_of_k(bits, K, N, gs, M, gather, runs):
+    assert ops.gemm_split(M, K, N, bits)[0] == runs
+    test_gemm_against_dequantised_product(bits, K, N, gs, M, gather)
+
+
 def test_split_of_the_cases_above():
     assert ops.gemm_split(77, 11008, 4096, 4)[0] == 4
     assert ops.gemm_split(128, 11008, 1056, 8)[0] == 4
