@@ -70,23 +70,27 @@ int gemv_strip_prepare(GemvStripPlan* p, const int32_t* qweight, const int32_t* 
     // a unit lies in one group when groups are whole units (or there is only one)
     const int sub = (s.spg % 4 == 0 || s.groups == 1) ? 1 : 4;
     s.units = (K + kUnit - 1) / kUnit;
-    const int nt = M <= 8 ? 1 : 2;
-    // One and two rows: planes of x where they pay and fit; one row: x kept whole.  Planes cost a CTA about a strip per row, of
-    // 3 bits (more pieces, picked row by row) two: 9216 x 9216, two strips per CTA, 15.8 us against 15.0 in fp16; two rows of
-    // 4096 x 11008, three strips, 12.7 against 9.5; 4096 x 22016, five, 15.3 against 16.4.
     s.strips = N / kStripCols;
     // One CTA per SM: each takes the same whole number of strips.
     s.per_cta = (s.strips + sm_count() - 1) / sm_count();
-    const int plane_bytes = (s.units * M * ((bits == 3 ? 5 : 4) * 128 + 8) + 15) / 16 * 16;
-    int mode = M <= 2 && bits != 8 && sub == 1 && s.per_cta > (bits == 3 ? 2 * M : M) && plane_bytes <= 96 * 1024 ? kInt
-             : (M == 1 && K <= 65536 ? kOne : kSeveral);
+    // One and two rows: planes of x where they pay and fit; one row: x kept whole.  Planes take a CTA longer to prepare than x in operand
+    // order and save on every strip and unit, so they pay from two strips on: 4 bits, two strips, one row 1.09 (4096 x 6144), 1.13
+    // (8192 x 8192) times as fast, groups of 32 1.02 and 1.02; 2 bits 1.15, 1.20; 3 bits, which have more pieces, 1.15, 1.10 and with
+    // rows picked one by one (a gather) 1.04, 1.00, 0.99 (9216 x 9216), two rows 1.00, 1.08, 0.92: three strips there (one row with
+    // a gather 1.08, two rows 1.10, 1.12, 0.93, 1.00).  One strip, 4 bits: one row of 4096 1.04, of 11008 1.11, with a gather 0.97 and 1.05,
+    // 2048 0.90; two rows with a gather 1.09 and 1.15, without 1.02 and 0.96.
+    const int plane_bytes = (s.units * M * 4 * int_factors(sub) + 15) / 16 * 16 + s.units * M * (bits == 3 ? 5 : 4) * 128;
+    const bool one_strip = bits == 4 && (M == 1 ? sub == 1 && s.units >= (gather ? 64 : 32) : gather && s.units >= 32);
+    const bool planes_pay = s.per_cta >= (bits != 3 || (M == 1 && !gather) ? 2 : 3) || one_strip;
+    int mode = M <= 2 && int_takes(bits, sub) && planes_pay && plane_bytes <= 96 * 1024 ? kInt : (M == 1 && K <= 65536 ? kOne : kSeveral);
+    const int nt = M <= 8 ? 1 : 2;
     s.rows_g = sub == 1 ? 1 : (s.spg == 1 ? 4 : (s.spg == 2 ? 2 : 3));
     // Strips of a pass for W warps: a unit costs about half a strip's work on top of its strips, and the last pass is a whole
     // one.  The rings take at least two slots and what is left of the shared memory.
     struct Choice { int W, T, ring, fixed, bufs, cost; };
     auto choose = [&](int W) {
         Choice c = {W, 0, 0, 0, 0, 1 << 30};
-        const int tmax = mode == kInt ? 4 : (sub == 1 && nt == 1 ? 3 : 2);
+        const int tmax = sub == 1 && nt == 1 ? (mode == kInt ? 4 : 3) : 2;
         // (a gather works from a copy of x that the sums overwrite: it needs every unit's x kept)
         // x that is not kept: as many units ahead as leave the weights three slots, one ahead being the least.  Nine rows and
         // more are fetched again in every pass rather than kept where that saves a pass (9216 x 9216, 2 bits, 9 rows: 24 ->
@@ -94,7 +98,7 @@ int gemv_strip_prepare(GemvStripPlan* p, const int32_t* qweight, const int32_t* 
         for (int bufs = 5; bufs >= (mode == kSeveral && !gather ? 2 : 5) && (nt == 2 || c.bufs != 5); --bufs)
             for (int t = 1; t <= tmax && t <= s.per_cta; ++t) {
                 const int slot = slot_bytes(bits, t) + const_bytes(bits, t, s.rows_g);
-                const int sums = W * M * t * kStripCols * 4, copy = gather || mode != kSeveral ? M * K * 2 : 0;
+                const int sums = W * M * t * kStripCols * 4, copy = gather || mode == kOne || (mode == kInt && bits != 4) ? M * K * 2 : 0;
                 const int x = mode == kInt ? plane_bytes
                             : (mode == kOne ? s.units * kUnit * 2 : (bufs == 5 ? s.units : bufs * W) * M * kXPitch * 2);
                 const int f = x + (sums > copy ? sums : copy) + 1024, r = (kSmemMax - f) / (W * slot);
@@ -152,11 +156,13 @@ int gemv_strip_prepare(GemvStripPlan* p, const int32_t* qweight, const int32_t* 
     const cuuint32_t wb[3] = {kStripCols, (cuuint32_t)(4 * bits), (cuuint32_t)T};
     const cuuint64_t sd[2] = {(cuuint64_t)N, (cuuint64_t)s.groups}, ss[1] = {(cuuint64_t)N * 2};
     const cuuint32_t sb[2] = {(cuuint32_t)(T * kStripCols), (cuuint32_t)s.rows_g};
-    const cuuint64_t zd[1] = {(cuuint64_t)s.groups * (N / 32 * bits)};
-    const cuuint32_t zb[1] = {(cuuint32_t)zero_words(bits, T)};
+    const bool rows_of_zeros = bits % 4 == 0;       // qzeros as [G, N/32*bits] where its rows are whole 16-byte pieces
+    const cuuint64_t zd[2] = {(cuuint64_t)(rows_of_zeros ? 1 : s.groups) * (N / 32 * bits), (cuuint64_t)s.groups};
+    const cuuint64_t zs[1] = {(cuuint64_t)(N / 32 * bits) * 4};
+    const cuuint32_t zb[2] = {(cuuint32_t)zero_words(bits, T), (cuuint32_t)s.rows_g};
     if (!map(&p->tmap_w, CU_TENSOR_MAP_DATA_TYPE_INT32, 3, qweight, wd, ws, wb, CU_TENSOR_MAP_SWIZZLE_128B) ||
         !map(&p->tmap_s, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, scales, sd, ss, sb, CU_TENSOR_MAP_SWIZZLE_NONE) ||
-        !map(&p->tmap_z, CU_TENSOR_MAP_DATA_TYPE_INT32, 1, qzeros, zd, ws, zb, CU_TENSOR_MAP_SWIZZLE_NONE)) {
+        !map(&p->tmap_z, CU_TENSOR_MAP_DATA_TYPE_INT32, rows_of_zeros ? 2 : 1, qzeros, zd, zs, zb, CU_TENSOR_MAP_SWIZZLE_NONE)) {
         set_last_cuda_error((int)cudaErrorInvalidValue);
         return B200GPTQ_ERR_CUDA;
     }

@@ -37,6 +37,8 @@
 
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace b200gptq {
@@ -273,11 +275,12 @@ constexpr unsigned long long pack8(const Bytes8& t) {
     return r;
 }
 
-template <int BITS> struct IntLayout;
+// WHOLE: a unit lies in one group; otherwise step s is rows 32 s .. 32 s + 31 (4 bits only).
+template <int BITS, bool WHOLE> struct IntLayout;
 
-template <> struct IntLayout<4> {                 // a word-row is a step: nibbles 0 2 4 6 (q) and 1 3 5 7 (q << 4)
+template <bool WHOLE> struct IntLayout<4, WHOLE> {  // a word-row is a step: nibbles 0 2 4 6 (q) and 1 3 5 7 (q << 4)
     static constexpr int kSteps = 4, kPre = 4, kLoads = 4;
-    __device__ static int load_row(int i, int j) { return 2 * j + (i & 1) + 8 * (i >> 1); }
+    __device__ static int load_row(int i, int j) { return WHOLE ? 2 * j + (i & 1) + 8 * (i >> 1) : 4 * i + j; }
     __device__ static void regs(const uint32_t (&w)[kLoads], uint32_t (&r)[2 * kSteps]) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) { r[2 * i] = w[i] & 0x0f0f0f0fu; r[2 * i + 1] = w[i] & 0xf0f0f0f0u; }
@@ -287,8 +290,8 @@ template <> struct IntLayout<4> {                 // a word-row is a step: nibbl
         for (int e = 0; e < 8; ++e) { row[e] = 8 * load_row(i, j) + 2 * (e & 3) + (e >> 2); pre[e] = e < 4 ? 4 : 0; }
     }
 };
-template <> struct IntLayout<8> : IntLayout<4> {};   // (not used: 8-bit fields need no unpacking in fp16 either)
-template <> struct IntLayout<2> {                 // a word-row is two steps: fields f, f + 4, f + 8, f + 12 (q << 2 f), f = 0 .. 3
+template <bool WHOLE> struct IntLayout<8, WHOLE> : IntLayout<4, WHOLE> {};   // (not used: 8-bit fields need no unpacking in fp16 either)
+template <> struct IntLayout<2, true> {                 // a word-row is two steps: fields f, f + 4, f + 8, f + 12 (q << 2 f), f = 0 .. 3
     static constexpr int kSteps = 4, kPre = 6, kLoads = 2;
     __device__ static int load_row(int i, int j) { return 2 * j + i; }
     __device__ static void regs(const uint32_t (&w)[kLoads], uint32_t (&r)[2 * kSteps]) {
@@ -314,7 +317,7 @@ template <> struct IntLayout<2> {                 // a word-row is two steps: fi
 //   R6 = (run >> 6)  : f2 p0, f5 p1, -, f10 p0    R7 = (run >> 38): f13 p1, -, f18 p0, f21 p1
 //   R8 = (run >> 70) : -, f26 p0, f29 p1, -
 // Step s multiplies (R[2s], R[2s+1]); the fifth step has only R8.
-template <> struct IntLayout<3> {
+template <> struct IntLayout<3, true> {
     static constexpr int kSteps = 5, kPre = 5, kLoads = 3;
     __device__ static int load_row(int i, int j) { return 3 * j + i; }
     static constexpr uint32_t m(int p0, int p1, int p2, int p3) {
@@ -345,8 +348,11 @@ template <> struct IntLayout<3> {
         }
     }
 };
-// bytes of one unit's B operands for M rows of x, [step][quad lane][4 row + plane][b0, b1], and of its factors
-template <int BITS> __host__ __device__ constexpr int int_unit_bytes(int M) { return IntLayout<BITS>::kSteps * 128 * M; }
+// Byte planes of M rows of x: a unit's B operands [step][quad lane][4 row + plane][b0, b1], and per unit and row its factor and the
+// sums of x of its groups (floats).
+template <int BITS> __host__ __device__ constexpr int int_unit_bytes(int M) { return (BITS == 3 ? 5 : 4) * 128 * M; }
+__host__ __device__ constexpr int int_factors(int sub) { return sub == 1 ? 2 : 8; }
+__host__ __device__ constexpr bool int_takes(int bits, int sub) { return bits == 4 || (bits != 8 && sub == 1); }
 
 // How x meets the weights: several rows in fp16, one row in fp16, one or two rows as byte planes.
 enum { kSeveral = 0, kOne = 1, kInt = 2 };
@@ -368,12 +374,13 @@ struct StripPlan {
 };
 
 // A slot: weights (1024-byte aligned for the swizzle), and in a second ring the scales [group][32 T] and the zero-point
-// words of each group.  A group's words start anywhere in qzeros: for 2 and 3 bits the box starts up to three words early.
+// words of each group.  Rows of qzeros of 4 and 8 bits are whole 16-byte pieces: one box holds every group's.  Of 2 and 3 bits a
+// group's words start anywhere, a box per group starts up to three words early.
 __host__ __device__ constexpr int slot_bytes(int bits, int T) { return (4 * bits * 128 * T + 1023) & ~1023; }
 __host__ __device__ constexpr int zero_words(int bits, int T) { return bits % 4 == 0 ? T * bits : (T * bits + 3 + 3) & ~3; }
-__host__ __device__ constexpr int zero_pitch(int bits, int T) { return (zero_words(bits, T) * 4 + 127) & ~127; }
+__host__ __device__ constexpr int zero_pitch(int bits, int T) { return bits % 4 == 0 ? T * bits * 4 : (zero_words(bits, T) * 4 + 127) & ~127; }
 __host__ __device__ constexpr int scale_bytes(int T, int rows) { return (rows * T * 64 + 127) & ~127; }
-__host__ __device__ constexpr int const_bytes(int bits, int T, int rows) { return scale_bytes(T, rows) + rows * zero_pitch(bits, T); }
+__host__ __device__ constexpr int const_bytes(int bits, int T, int rows) { return scale_bytes(T, rows) + ((rows * zero_pitch(bits, T) + 127) & ~127); }
 
 // The two activations folded into the read of x, rounded exactly like the stand-alone kernel (b200gptq_act).
 __device__ __forceinline__ uint32_t act_relu2(uint32_t v) {
@@ -396,15 +403,15 @@ __device__ __forceinline__ uint32_t act_swiglu2(uint32_t gv, uint32_t uv) {
 // started when a CTA ended, and the next product's weights after that: 22 us against 16.6 (and 14.3 against 14.1 where
 // nothing is gathered).
 template <int BITS, int SUB, int NT, int MODE, int T, int W>
-__global__ void __maxnreg__(W == 16 ? 120 : NT == 1 ? 128 : 224)
+__global__ void __maxnreg__(W == 16 ? 120 : NT == 1 ? 168 : 224)
 gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_s,
                   const __grid_constant__ CUtensorMap tmap_z, const __half* __restrict__ x,
                   const int32_t* __restrict__ x_perm, const __half* __restrict__ bias, __half* __restrict__ y, int M_rows, int K, int N, const StripPlan plan,
                   unsigned int* __restrict__ status) {
     using L = Layout<BITS, SUB == 1>;
-    using I = IntLayout<BITS>;
+    using I = IntLayout<BITS, SUB == 1 || BITS != 4>;
     constexpr bool ONE = MODE == kOne, INT = MODE == kInt, ROWS = MODE == kSeveral;
-    static_assert(!INT || (SUB == 1 && NT == 1 && BITS != 8), "the integer path takes whole units of one or two rows");
+    static_assert(!INT || (NT == 1 && int_takes(BITS, SUB)), "not a case of the integer path");
     constexpr int STRIP_BYTES = L::kRows * 128, STEPS = 4 / SUB, SLOT = slot_bytes(BITS, T);
     constexpr int NC = ROWS ? 2 : 1;             // rows of x per lane and n-tile that exist
     constexpr int COLS = T * kStripCols;
@@ -433,8 +440,9 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     const int unit_x = ONE ? kUnit * 2 : (INT ? int_unit_bytes<BITS>(M) : M * kXPitch * 2);
     const int x_units = ROWS && !plan.kept ? plan.x_bufs * W : plan.units;
     uint8_t* p_x = base_x + (size_t)(ROWS && !plan.kept ? plan.x_bufs * warp : u_begin) * unit_x;
-    float2* p_f = reinterpret_cast<float2*>(base_x + (size_t)plan.units * unit_x) + (size_t)u_begin * M;
-    uint8_t* base_r = base_x + (size_t)x_units * unit_x + (INT ? (plan.units * M * 8 + 15) / 16 * 16 : 0);
+    constexpr int FACTORS = int_factors(SUB);
+    float* p_f = reinterpret_cast<float*>(base_x + (size_t)plan.units * unit_x) + (size_t)u_begin * M * FACTORS;
+    uint8_t* base_r = base_x + (size_t)x_units * unit_x + (INT ? (plan.units * M * FACTORS * 4 + 15) / 16 * 16 : 0);
     float* red = reinterpret_cast<float*>(base_r);                                 // [warp][m][column of the pass]
     unsigned short* raw = reinterpret_cast<unsigned short*>(base_r);               // [m][k]
     const uint32_t bar0 = smem_u32(bars) + 8u * (warp * kMaxRing);
@@ -460,11 +468,17 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
             asm volatile(
                 "cp.async.bulk.tensor.2d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                 ::"r"(cst), "l"(&tmap_s), "r"(strip * kStripCols), "r"(grp), "r"(bar) : "memory");
-            for (int r = 0; r < plan.rows_g; ++r)
+            if constexpr (BITS % 4 == 0) {
                 asm volatile(
-                    "cp.async.bulk.tensor.1d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2}], [%3];"
-                    ::"r"(cst + scale_bytes(T, plan.rows_g) + r * zero_pitch(BITS, T)), "l"(&tmap_z),
-                      "r"(((grp + r) * zwords + strip * BITS) & ~3), "r"(bar) : "memory");
+                    "cp.async.bulk.tensor.2d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                    ::"r"(cst + scale_bytes(T, plan.rows_g)), "l"(&tmap_z), "r"(strip * BITS), "r"(grp), "r"(bar) : "memory");
+            } else {
+                for (int r = 0; r < plan.rows_g; ++r)
+                    asm volatile(
+                        "cp.async.bulk.tensor.1d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2}], [%3];"
+                        ::"r"(cst + scale_bytes(T, plan.rows_g) + r * zero_pitch(BITS, T)), "l"(&tmap_z),
+                          "r"(((grp + r) * zwords + strip * BITS) & ~3), "r"(bar) : "memory");
+            }
         }
         ++q_w;
         if (++u_w == nu) { u_w = 0; win_w = min(win_w + T, last_window); }
@@ -479,27 +493,61 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     for (int i = 0; i < R && i < total; ++i) request();
 
     const bool gather = plan.gather != 0;
-    // What does not need x is done before the wait.  Byte planes: a lane's rows of a 128-row unit, and where they lie in x for its
-    // first two units (3 bits, 4096 x 11008 with a gather 9.4 -> 8.2 us, without 8.5 -> 7.9).  3 bits in fp16: where its four rows
-    // of the first units lie.
-    int row[8], pre[8], first[2][8];
+    // What does not need x is done before the wait.  Byte planes: which rows of a 128-row unit a lane takes.  A gather: where these,
+    // or the rows of an item of the other modes, lie in x, in the bytes that the item itself (planes: its unit) is written to.  Looked
+    // up after the wait, two units at a time, they were a round trip to L2 each: 9 units per warp, 9216 x 36864, 3 bits, 34.2 us
+    // against 29.7.  Planes: the first two units' in registers, the others' copied without waiting; a CTA that starts late is on its
+    // way to x meanwhile (3 bits, 4096 x 11008, two units per warp, through shared memory 8.6 against 8.4).
+    int row[8], pre[8], first[8];
+    auto index_slot = [&](int i) { return reinterpret_cast<uint4*>(INT ? p_x + (i >> 4) * unit_x + (i & 15) * 32 : p_x + i * 16); };
+    auto pack2 = [](int a, int b) { return (uint32_t)a | ((uint32_t)b << 16); };
     if constexpr (INT) {
         I::item((lane >> 2) & 3, lane & 3, row, pre);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            const int k = (u_begin + (lane >> 4)) * kUnit + row[e];
-            first[0][e] = !gather || k >= K ? min(k, K - 1) : __ldg(x_perm + k);
-            asm volatile("" : "+r"(row[e]), "+r"(pre[e]), "+r"(first[0][e]));
-        }
-        if (gather && nu > 2) {
+        for (int e = 0; e < 8; ++e) asm volatile("" : "+r"(row[e]), "+r"(pre[e]));
+        if (gather) {
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                first[1][e] = __ldg(x_perm + min((u_begin + 2 + (lane >> 4)) * kUnit + row[e], K - 1));
-                asm volatile("" : "+r"(first[1][e]));
+            for (int e = 0; e < 8; ++e) first[e] = __ldg(x_perm + min((u_begin + (lane >> 4)) * kUnit + row[e], K - 1));
+            for (int i = lane + 32; i < nu * 16; i += 32) {
+                const int k0 = (u_begin + (i >> 4)) * kUnit;
+                const uint32_t dst = smem_u32(index_slot(i));
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + 4 * e), "l"(x_perm + min(k0 + row[e], K - 1)) : "memory");
             }
+#pragma unroll
+            for (int e = 0; e < 8; ++e) asm volatile("" : "+r"(first[e]));
         }
     }
     constexpr bool BLOCKS = ONE && BITS == 3 && SUB == 1;
+    // the two runs of four rows of item i of one row in fp16
+    auto item_rows = [&](int i, int& ka, int& kb) {
+        const int k = (u_begin + (i >> 4)) * kUnit, jj = (i >> 2) & 3, st = i & 3;
+        if constexpr (BITS == 8) {
+            ka = k + 4 * L::load_row(2 * st, jj); kb = k + 4 * L::load_row(2 * st + 1, jj);
+        } else if constexpr (BITS != 3 || SUB != 1) {
+            ka = k + L::x_first(st, jj); kb = ka + 4;
+        }
+    };
+    if constexpr (ONE && !BLOCKS)
+        if (gather) {
+#pragma unroll 2
+            for (int i = lane; i < nu * 16; i += 32) {
+                int ka = 0, kb = 0;
+                item_rows(i, ka, kb);
+                const int4 a = __ldg(reinterpret_cast<const int4*>(x_perm + min(ka, K - 4)));
+                const int4 b = __ldg(reinterpret_cast<const int4*>(x_perm + min(kb, K - 4)));
+                *index_slot(i) = make_uint4(pack2(a.x, a.y), pack2(a.z, a.w), pack2(b.x, b.y), pack2(b.z, b.w));
+            }
+        }
+    if constexpr (ROWS)
+        if (gather) {                              // of several rows: in the place of the first row's four values
+#pragma unroll 2
+            for (int i = lane; i < nu * 32; i += 32) {
+                const int4 a = __ldg(reinterpret_cast<const int4*>(x_perm + min(u_begin * kUnit + 4 * i, K - 4)));
+                *reinterpret_cast<uint2*>(p_x + (size_t)(i >> 5) * unit_x + 8 * lane) = make_uint2(pack2(a.x, a.y), pack2(a.z, a.w));
+            }
+        }
     constexpr int EARLY = 4;
     uint4 first4[EARLY];
     if (BLOCKS && gather) {
@@ -514,9 +562,9 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     if (gather)                                   // all of x, by all warps
         for (int i = tid; i < M * K / 8; i += 32 * W)
             cp_async16(smem_u32(raw + 8 * (size_t)i), x + 8 * (size_t)i, true);
-    // One or two rows: the warp's slice of x is copied first (`raw`), so that its rows can be picked in any order without
-    // 2-byte requests from every CTA to the same few L2 lines (they cost 7 us at 9216 rows).
-    const bool staged = gather || (!ROWS && plan.xact != 1);
+    // One row, and planes of 2 and 3 bits: the warp's slice of x is copied first (`raw`), so that its rows can be picked in any order
+    // without 2-byte requests from every CTA to the same few L2 lines (they cost 7 us at 9216 rows).
+    const bool staged = gather || (!ROWS && !(INT && BITS == 4) && plan.xact != 1);
     if (!ROWS && !gather && staged) {
         const int k0 = u_begin * kUnit, count = min(nu * kUnit, K - k0) / 8;
         for (int m = 0; m < M; ++m)
@@ -555,16 +603,9 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         }
         return v;
     };
-    auto load_half = [&](int m, int k) -> unsigned short {
-        if (k >= K) return 0;
-        uint32_t v;
-        if (staged) {
-            v = raw[(size_t)m * K + (gather ? __ldg(x_perm + k) : k)];
-        } else {
-            const unsigned short* px = reinterpret_cast<const unsigned short*>(x) + (size_t)m * 2 * K + k;
-            return (unsigned short)act_swiglu2(__ldcg(px), __ldcg(px + K));
-        }
-        return (unsigned short)(plan.xact ? act_relu2(v) : v);
+    auto load_swiglu = [&](int m, int k) -> uint32_t {
+        const unsigned short* px = reinterpret_cast<const unsigned short*>(x) + (size_t)m * 2 * K + k;
+        return act_swiglu2(__ldcg(px), __ldcg(px + K)) & 0xffffu;
     };
     const bool async_x = ROWS && !gather && plan.xact == 0;
     auto fetch_x = [&](int u, int buf) {          // several rows, as they lie in memory
@@ -575,20 +616,21 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    if (async_x && plan.kept) {
+    if (async_x && plan.kept)                      // (waited for unit by unit, in the first pass)
         for (int u = 0; u < nu; ++u) fetch_x(u, u);
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncwarp();
-    }
     if (gather || (!ROWS && staged)) {
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         if (gather) __syncthreads();
         else __syncwarp();
     }
     if (ROWS && !async_x && plan.kept) {
-        for (int i = lane; i < nu * 32; i += 32)
+        for (int i = lane; i < nu * 32; i += 32) {
+            uint2* to = reinterpret_cast<uint2*>(p_x + (size_t)(i >> 5) * unit_x + 8 * lane);
+            const int k = u_begin * kUnit + 4 * i;
+            const uint2 at = *to;                  // (where a gather finds them)
             for (int m = 0; m < M; ++m)
-                *reinterpret_cast<uint2*>(p_x + (size_t)(i >> 5) * unit_x + m * kXPitch * 2 + 8 * lane) = load4(m, u_begin * kUnit + 4 * i);
+                to[m * kXPitch / 4] = gather ? pick4(m, k, make_uint4(at.x & 0xffffu, at.x >> 16, at.y & 0xffffu, at.y >> 16)) : load4(m, k);
+        }
         __syncwarp();
     }
     if constexpr (ONE) {
@@ -620,13 +662,20 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         } else {
 #pragma unroll 2
             for (int i = lane; i < nu * 16; i += 32) {
-                const int u = i >> 4, jj = (i >> 2) & 3, s = i & 3, k = (u_begin + u) * kUnit;
+                int ka = 0, kb = 0;
+                item_rows(i, ka, kb);
+                uint2 v, w;
+                if (gather) {
+                    const uint4 at = *index_slot(i);
+                    v = pick4(0, ka, make_uint4(at.x & 0xffffu, at.x >> 16, at.y & 0xffffu, at.y >> 16));
+                    w = pick4(0, kb, make_uint4(at.z & 0xffffu, at.z >> 16, at.w & 0xffffu, at.w >> 16));
+                } else {
+                    v = load4(0, ka); w = load4(0, kb);
+                }
                 uint32_t b[4];
                 if constexpr (BITS == 8) {
-                    const uint2 v = load4(0, k + 4 * L::load_row(2 * s, jj)), w = load4(0, k + 4 * L::load_row(2 * s + 1, jj));
                     b[0] = v.x; b[1] = v.y; b[2] = w.x; b[3] = w.y;
                 } else {
-                    const uint2 v = load4(0, k + L::x_first(s, jj)), w = load4(0, k + L::x_first(s, jj) + 4);
                     L::b_regs(make_uint4(v.x, v.y, w.x, w.y), b);
                 }
                 *reinterpret_cast<uint4*>(p_x + i * 16) = make_uint4(b[0], b[1], b[2], b[3]);
@@ -635,84 +684,114 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         __syncwarp();
     }
     if constexpr (INT) {
-        // fixed point per unit, four signed byte planes; the 16 items of a unit sit in 16 adjacent lanes
-        for (int m = 0; m < M; ++m)
-#pragma unroll 2
-            for (int q0 = 0; q0 < nu * 16; q0 += 32) {
-                const int q = q0 + lane, u = q >> 4, jq = q & 3, iq = (q >> 2) & 3;
-                const bool active = q < nu * 16;
-                const int k0 = (u_begin + u) * kUnit;
-                unsigned short h[8];
-                if (staged && (q0 == 0 || (gather && q0 == 32)) && (BITS != 4 || gather)) {
+        // Fixed point per unit, four signed byte planes; the 16 items of a unit sit in 16 adjacent lanes.  V pairs of units at a time,
+        // or each waits out the other's latencies.
+        auto planes = [&](int q0, auto count) {
+            constexpr int V = decltype(count)::value;
+            const int jq = lane & 3, iq = (lane >> 2) & 3;
+            uint4 at[V][2];
+            bool active[V];
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                active[v] = q0 + 32 * v + lane < nu * 16;
+                at[v][0] = at[v][1] = make_uint4(0u, 0u, 0u, 0u);
+                if (gather && v == 0 && q0 == 0) {
+                    at[0][0] = make_uint4(first[0], first[1], first[2], first[3]); at[0][1] = make_uint4(first[4], first[5], first[6], first[7]);
+                } else if (gather && active[v]) { at[v][0] = index_slot(q0 + 32 * v + lane)[0]; at[v][1] = index_slot(q0 + 32 * v + lane)[1]; }
+            }
+            __syncwarp();
+            for (int m = 0; m < M; ++m) {
+                uint32_t h[V][8], mx[V];
+#pragma unroll
+                for (int v = 0; v < V; ++v) {
+                    const int k0 = (u_begin + ((q0 + 32 * v + lane) >> 4)) * kUnit;
+                    const uint32_t idx[8] = {at[v][0].x, at[v][0].y, at[v][0].z, at[v][0].w, at[v][1].x, at[v][1].y, at[v][1].z, at[v][1].w};
+                    if (gather || (BITS != 4 && staged)) {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) {
+                            const uint32_t from = gather ? idx[e] : k0 + row[e];
+                            h[v][e] = active[v] && k0 + row[e] < K ? raw[(size_t)m * K + from] : 0u;
+                            if (plan.xact) h[v][e] = act_relu2(h[v][e]) & 0xffffu;
+                        }
+                    } else if constexpr (BITS == 4) {          // a run of eight rows
+                        uint2 a = make_uint2(0u, 0u), b = a;
+                        if (active[v]) { a = load4(m, k0 + row[0]); b = load4(m, k0 + row[0] + 4); }
+                        const uint32_t x4[4] = {a.x, a.y, b.x, b.y};
+#pragma unroll
+                        for (int e = 0; e < 8; ++e)
+                            h[v][e] = e < 4 ? x4[e & 3] & 0xffffu : x4[e & 3] >> 16;
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) h[v][e] = active[v] && k0 + row[e] < K ? load_swiglu(m, k0 + row[e]) : 0u;
+                    }
+                    mx[v] = 0u;
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) mx[v] = max(mx[v], h[v][e] & 0x7fffu);    // the order of non-negative fp16 numbers
+                }
+                float scale[V];
+                int ex[V], sum[V];
+                bool bad[V];
+#pragma unroll
+                for (int v = 0; v < V; ++v) {
+                    const uint32_t lo = __reduce_max_sync(0xffffffffu, lane < 16 ? mx[v] : 0u), hi = __reduce_max_sync(0xffffffffu, lane < 16 ? 0u : mx[v]);
+                    // 2^ex > max |x| of the unit; X = x * 2^(148 - ex) has |X| < 2^22.  A unit of zeros takes any scale; a
+                    // unit with an infinity or a NaN gets a NaN factor, so that its columns come out as NaN.
+                    mx[v] = lane < 16 ? lo : hi;
+                    ex[v] = (int)(__float_as_uint(__half2float(__ushort_as_half((unsigned short)mx[v]))) >> 23);
+                    bad[v] = mx[v] >= 0x7c00u;
+                    if (mx[v] == 0u || bad[v]) ex[v] = 127;
+                    scale[v] = __uint_as_float((uint32_t)(275 - ex[v]) << 23);
+                }
+                uint32_t dg[V][8];
+#pragma unroll
+                for (int v = 0; v < V; ++v) {
+                    sum[v] = 0;
 #pragma unroll
                     for (int e = 0; e < 8; ++e) {
-                        h[e] = active && k0 + row[e] < K ? raw[(size_t)m * K + (q0 == 0 ? first[0][e] : first[1][e])] : (unsigned short)0;
-                        if (plan.xact) h[e] = (unsigned short)act_relu2(h[e]);
+                        // round to nearest through the fp32 adder: |x * scale| <= 2^22
+                        const int X = __float_as_int(fmaf(__half2float(__ushort_as_half((unsigned short)h[v][e])), scale[v], 12582912.f)) - 0x4B400000;
+                        sum[v] += X;
+                        dg[v][e] = (uint32_t)((X << pre[e]) + 0x00808080) ^ 0x00808080u;   // four signed base-256 digits
                     }
-                } else if constexpr (BITS == 4) {      // a run of eight rows
-                    uint2 v = make_uint2(0u, 0u), w = v;
-                    if (active) { v = load4(m, k0 + row[0]); w = load4(m, k0 + row[0] + 4); }
-                    const uint32_t x4[4] = {v.x, v.y, w.x, w.y};
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) h[e] = (unsigned short)(x4[e & 3] >> (16 * (e >> 2)));
-                } else {
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) h[e] = active ? load_half(m, k0 + row[e]) : (unsigned short)0;
-                }
-                float xf[8];
-                unsigned int mx = 0u;   // bits of the largest |x|: the order of non-negative floats, NaN above infinity
-#pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    xf[e] = __half2float(__ushort_as_half(h[e]));
-                    mx = max(mx, __float_as_uint(fabsf(xf[e])));
                 }
 #pragma unroll
-                for (int o = 1; o < 16; o <<= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-                // 2^ex > max |x| of the unit; X = x * 2^(148 - ex) has |X| < 2^22.  A unit of zeros takes any scale; a
-                // unit with an infinity or a NaN gets a NaN factor, so that its columns come out as NaN.
-                int ex = (int)(mx >> 23);
-                const bool bad = ex == 255;
-                if (ex == 0 || bad) ex = 127;
-                const float scale = __uint_as_float((uint32_t)(275 - ex) << 23);
-                int sum = 0;
-                uint32_t dg[8];
+                for (int o = 1; o < (SUB == 1 ? 16 : 4); o <<= 1)
 #pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    // round to nearest through the fp32 adder: |x * scale| <= 2^22
-                    const int X = __float_as_int(fmaf(xf[e], scale, 12582912.f)) - 0x4B400000;
-                    sum += X;
-                    dg[e] = (uint32_t)((X << pre[e]) + 0x00808080) ^ 0x00808080u;   // four signed base-256 digits
-                }
+                    for (int v = 0; v < V; ++v) sum[v] += __shfl_xor_sync(0xffffffffu, sum[v], o);
 #pragma unroll
-                for (int o = 1; o < 16; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-                if (active) {
-                    if ((lane & 15) == 0) {
-                        const float delta = __uint_as_float((uint32_t)(ex - 21) << 23);   // 2^(ex - 148)
-                        float cq = __uint_as_float((uint32_t)(ex - 21 - I::kPre) << 23);
-                        if (bad) cq = __uint_as_float(0x7fc00000u);
-                        p_f[u * M + m] = make_float2(cq, -delta * (float)sum);   // (factor of the planes, -sum of x)
-                    }
-                    uint8_t* dst = p_x + (size_t)u * unit_x + (jq * M + m) * 32;
+                for (int v = 0; v < V; ++v) {
+                    if (!active[v]) continue;
+                    const int u = (q0 + 32 * v + lane) >> 4;
+                    // the factor of the planes, then minus the sum of x of every group (32 rows each where they are scaled apart)
+                    const float delta = __uint_as_float((uint32_t)(ex[v] - 21) << 23);   // 2^(ex - 148)
+                    float* f = p_f + (u * M + m) * FACTORS;
+                    if ((lane & 15) == 0) f[0] = bad[v] ? __uint_as_float(0x7fc00000u) : __uint_as_float((uint32_t)(ex[v] - 21 - I::kPre) << 23);
+                    if (SUB == 1 ? (lane & 15) == 0 : jq == 0) f[1 + (SUB == 1 ? 0 : iq)] = -delta * (float)sum[v];
+                    uint8_t* dst = p_x + (size_t)u * unit_x + jq * (32 * M) + m * 32;
                     auto store = [&](int step, const uint32_t (&lo)[4], const uint32_t (&hi)[4]) {
-                        uint4* d = reinterpret_cast<uint4*>(dst + step * 128 * M);
+                        uint4* d = reinterpret_cast<uint4*>(dst + step * 4 * (32 * M));
                         d[0] = make_uint4(lo[0], hi[0], lo[1], hi[1]);
                         d[1] = make_uint4(lo[2], hi[2], lo[3], hi[3]);
                     };
                     uint32_t lo[4], hi[4];
                     if (BITS != 3 || iq < 3) {
-                        planes_of(dg[0], dg[1], dg[2], dg[3], lo);
-                        planes_of(dg[4], dg[5], dg[6], dg[7], hi);
+                        planes_of(dg[v][0], dg[v][1], dg[v][2], dg[v][3], lo);
+                        planes_of(dg[v][4], dg[v][5], dg[v][6], dg[v][7], hi);
                         store(iq, lo, hi);
                     } else {
-                        planes_of(dg[0], dg[1], 0, dg[2], lo);
-                        planes_of(dg[3], 0, dg[4], dg[5], hi);
+                        planes_of(dg[v][0], dg[v][1], 0, dg[v][2], lo);
+                        planes_of(dg[v][3], 0, dg[v][4], dg[v][5], hi);
                         store(3, lo, hi);
-                        planes_of(0, dg[6], dg[7], 0, lo);
+                        planes_of(0, dg[v][6], dg[v][7], 0, lo);
                         hi[0] = hi[1] = hi[2] = hi[3] = 0u;
                         store(4, lo, hi);
                     }
                 }
             }
+        };
+        int q0 = 0;
+        for (; q0 + 32 < nu * 16; q0 += 64) planes(q0, std::integral_constant<int, 2>{});
+        if (q0 < nu * 16) planes(q0, std::integral_constant<int, 1>{});
         __syncwarp();
     }
     // planes: quad lane j holds planes 2j, 2j+1 of row j >> 1 ... of one row only j < 2; the zero-point term goes to one lane
@@ -755,8 +834,11 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                     bx[s] = make_uint2(0u, 0u);
                     if (g < 4 * M) bx[s] = *reinterpret_cast<const uint2*>(p_x + (size_t)u * unit_x + (s * 4 + j) * (32 * M) + g * 8);
                 }
-                const float2 f = p_f[u * M + (M == 2 ? j >> 1 : 0)];
-                const float cf = f.x * plane_weight, sx = f.y * sum_weight;
+                const float* f = p_f + (u * M + (M == 2 ? j >> 1 : 0)) * FACTORS;
+                const float cf = f[0] * plane_weight;
+                float sx[SUB];
+#pragma unroll
+                for (int sub = 0; sub < SUB; ++sub) sx[sub] = f[1 + sub] * sum_weight;
                 mbar_wait(bar0 + 8u * slot, parity, ok);
 #pragma unroll
                 for (int t = 0; t < T; ++t) {
@@ -766,26 +848,35 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                         const uint4 v = *reinterpret_cast<const uint4*>(src + read_at(t, I::load_row(i, j)));
                         w[0][i] = v.x; w[1][i] = v.y; w[2][i] = v.z; w[3][i] = v.w;
                     }
-                    const uint2 sv = *reinterpret_cast<const uint2*>(csc + t * 64);
-                    const float2 s01 = __half22float2(*reinterpret_cast<const __half2*>(&sv.x));
-                    const float2 s23 = __half22float2(*reinterpret_cast<const __half2*>(&sv.y));
-                    const float sf[4] = {s01.x, s01.y, s23.x, s23.y};
-                    const uint32_t zv = load_zeros<BITS>(zero_at(0, t), 4 * g);
+                    constexpr int SSTEPS = I::kSteps / SUB;
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        uint32_t ra[2 * I::kSteps], rb[2 * I::kSteps];
-                        I::regs(w[2 * h], ra);
-                        I::regs(w[2 * h + 1], rb);
-                        // the sums start at the bits of 1.5 * 2^23: |sum| < 2^22, so they end as floats with that offset
-                        constexpr int kBias = 0x4B400000;
-                        int d[4] = {kBias, kBias, kBias, kBias};
+                    for (int sub = 0; sub < SUB; ++sub) {
+                        const int r = SUB == 1 ? 0 : group_at(step0 + sub) - grp0;
+                        const uint2 sv = *reinterpret_cast<const uint2*>(csc + (r * T + t) * 64);
+                        const float2 s01 = __half22float2(*reinterpret_cast<const __half2*>(&sv.x));
+                        const float2 s23 = __half22float2(*reinterpret_cast<const __half2*>(&sv.y));
+                        const float sf[4] = {s01.x, s01.y, s23.x, s23.y};
+                        const uint32_t zv = load_zeros<BITS>(zero_at(r, t), 4 * g);
 #pragma unroll
-                        for (int s = 0; s < I::kSteps; ++s) imma(d, d, ra[2 * s], rb[2 * s], ra[2 * s + 1], rb[2 * s + 1], bx[s].x, bx[s].y);
+                        for (int h = 0; h < 2; ++h) {
+                            uint32_t ra[2 * I::kSteps], rb[2 * I::kSteps];
+                            I::regs(w[2 * h], ra);
+                            I::regs(w[2 * h + 1], rb);
+                            float zf[2];
 #pragma unroll
-                        for (int c = 0; c < 2; ++c) {
-                            const float lo = __int_as_float(d[2 * c]) - 12582912.f, hi = __int_as_float(d[2 * c + 1]) - 12582912.f;
-                            const float zf = __uint_as_float(0x4B000000u | ((zv >> (BITS * (2 * h + c))) & ((1u << BITS) - 1u))) - 8388607.f;
-                            out[t][0][2 * h + c][0] = fmaf(sf[2 * h + c], fmaf(fmaf(256.f, hi, lo), cf, zf * sx), out[t][0][2 * h + c][0]);
+                            for (int c = 0; c < 2; ++c)
+                                zf[c] = __uint_as_float(0x4B000000u | ((zv >> (BITS * (2 * h + c))) & ((1u << BITS) - 1u))) - 8388607.f;
+                            // the sums start at the bits of 1.5 * 2^23: |sum| < 2^22, so they end as floats with that offset
+                            constexpr int kBias = 0x4B400000;
+                            int d[4] = {kBias, kBias, kBias, kBias};
+#pragma unroll
+                            for (int s = sub * SSTEPS; s < (sub + 1) * SSTEPS; ++s)
+                                imma(d, d, ra[2 * s], rb[2 * s], ra[2 * s + 1], rb[2 * s + 1], bx[s].x, bx[s].y);
+#pragma unroll
+                            for (int c = 0; c < 2; ++c) {
+                                const float lo = __int_as_float(d[2 * c]) - 12582912.f, hi = __int_as_float(d[2 * c + 1]) - 12582912.f;
+                                out[t][0][2 * h + c][0] = fmaf(sf[2 * h + c], fmaf(fmaf(256.f, hi, lo), cf, zf[c] * sx[sub]), out[t][0][2 * h + c][0]);
+                            }
                         }
                     }
                 }
@@ -801,7 +892,18 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                 }
             } else {
                 __half* xs = reinterpret_cast<__half*>(p_x + (size_t)(plan.kept ? u : buf) * unit_x);
-                if (!plan.kept) {
+                if (plan.kept) {
+                    if (async_x && p == 0) {
+                        // this unit's x; the copies of those behind it go on (8 rows of 4096 x 12288: all of x first 10.1 us, so 9.2)
+                        const int behind = nu - 1 - u;
+                        if (behind >= 4) asm volatile("cp.async.wait_group 4;" ::: "memory");
+                        else if (behind == 3) asm volatile("cp.async.wait_group 3;" ::: "memory");
+                        else if (behind == 2) asm volatile("cp.async.wait_group 2;" ::: "memory");
+                        else if (behind == 1) asm volatile("cp.async.wait_group 1;" ::: "memory");
+                        else asm volatile("cp.async.wait_group 0;" ::: "memory");
+                        __syncwarp();
+                    }
+                } else {
                     if (async_x) {
                         if (plan.x_bufs == 4) asm volatile("cp.async.wait_group 2;" ::: "memory");
                         else if (plan.x_bufs == 3) asm volatile("cp.async.wait_group 1;" ::: "memory");
@@ -989,13 +1091,13 @@ const void* strip_kernel_t(int T) {
     if (T == 2) return reinterpret_cast<const void*>(gemv_strip_kernel<BITS, SUB, NT, MODE, 2, W>);
     if constexpr (NT == 1 && SUB == 1)
         if (T == 3) return reinterpret_cast<const void*>(gemv_strip_kernel<BITS, SUB, NT, MODE, 3, W>);
-    if constexpr (MODE == kInt)
+    if constexpr (MODE == kInt && SUB == 1)
         if (T == 4) return reinterpret_cast<const void*>(gemv_strip_kernel<BITS, SUB, NT, MODE, 4, W>);
     return nullptr;
 }
 template <int BITS, int SUB, int W>
 const void* strip_kernel_m(int mode, int nt, int T) {
-    if constexpr (SUB == 1 && BITS != 8)
+    if constexpr (int_takes(BITS, SUB))
         if (mode == kInt) return strip_kernel_t<BITS, SUB, 1, kInt, W>(T);
     if (mode == kOne) return strip_kernel_t<BITS, SUB, 1, kOne, W>(T);
     if (nt == 1) return strip_kernel_t<BITS, SUB, 1, kSeveral, W>(T);

@@ -60,6 +60,20 @@ def test_gemv_vs_oracle(bits, K, N, gs, gather, M):
     ops.check_status(DEV)
 
 
+@pytest.mark.parametrize("bits,K,N,gs,gather", [
+    # planes with groups inside a unit (4 bits, from two strips per CTA on): of one, two and three blocks, cut units
+    (4, 992, 4832, 32, False), (4, 1120, 9632, 64, True), (4, 2080, 4832, 96, True), (4, 96, 4832, 32, True),
+    # planes of one strip per CTA: one long row, rows with a gather
+    (4, 8224, 96, 128, True), (4, 4128, 64, 128, True), (4, 4096, 4096, 128, False),
+    # more pairs of units than one per warp, rows picked one by one
+    (2, 5152, 9632, 128, True), (3, 9248, 14432, 128, True), (3, 4128, 14432, -1, False), (2, 4128, 4832, 160, False),
+])
+@pytest.mark.parametrize("M", [1, 2])
+def test_byte_planes_vs_oracle(bits, K, N, gs, gather, M):
+    """(test_gemv_vs_oracle's bound)"""
+    test_gemv_vs_oracle(bits, K, N, gs, gather, M)
+
+
 @pytest.mark.parametrize("bits,K,N,gs,gather", [(2, 544, 96, 32, True), (3, 1152, 4832, 128, False), (3, 1184, 64, 64, True),
                                                 (4, 4096, 4800, 128, True), (4, 992, 32, 32, False), (8, 288, 9632, -1, False),
                                                 # x does not fit: places in turn, three and four of them, several passes
