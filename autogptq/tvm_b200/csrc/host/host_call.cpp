@@ -7,7 +7,10 @@
 // device, other buffers, a row count without a plan, a tensor subclass); the caller then takes the Python route,
 // which prepares what is missing.  Nothing here launches kernels of its own: the work goes through the C ABI.
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAException.h>
 #include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
+#include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -20,8 +23,9 @@ namespace {
 constexpr int kMaxGemvRows = 16;
 
 // Scratch buffers by (device, stream), registered by ops.get_workspace.  Read and written under the GIL; `owner` is the
-// tensor, held while it is registered and by a call that works without the GIL.
-struct Scratch { PyObject* owner; void* ptr; size_t bytes; };
+// tensor, held while it is registered and by a call that works without the GIL.  in_graph: it was handed out while its stream
+// was being captured, so a graph may hold its address for good.
+struct Scratch { PyObject* owner; void* ptr; size_t bytes; bool in_graph; };
 struct KeyHash {
     size_t operator()(const std::pair<int, void*>& k) const {
         return std::hash<void*>()(k.second) * 31u + (size_t)k.first;
@@ -87,8 +91,16 @@ inline bool lies_at(PyObject* t, const void* at) {
     return t && THPVariable_Check(t) && THPVariable_Unpack(t).unsafeGetTensorImpl()->data() == at;
 }
 
+// (the legacy default stream cannot be captured)
+bool is_capturing(cudaStream_t stream) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (stream) C10_CUDA_CHECK(cudaStreamIsCapturing(stream, &status));
+    return status != cudaStreamCaptureStatusNone;
+}
+
 bool scratch_for(int device, cudaStream_t stream, size_t need, Scratch* out) {
     auto it = g_scratch->find({device, (void*)stream});
+    if (it != g_scratch->end() && !it->second.in_graph) it->second.in_graph = is_capturing(stream);
     if (it == g_scratch->end() || it->second.bytes < need) {
         PyObject* r = PyObject_CallFunction(g_get_workspace, "in", device, (Py_ssize_t)need);
         if (!r) return false;
@@ -254,12 +266,12 @@ PyMethodDef layer_methods[] = {
 };
 PyTypeObject LayerType = {PyVarObject_HEAD_INIT(nullptr, 0) "autogptq.tvm_b200._host.Layer", sizeof(Layer)};
 
-// set_scratch(device, stream, tensor, bytes)
+// set_scratch(device, stream, tensor, bytes, in_graph)
 PyObject* set_scratch(PyObject*, PyObject* args) {
-    int device;
+    int device, in_graph;
     unsigned long long stream, bytes;
     PyObject* tensor;
-    if (!PyArg_ParseTuple(args, "iKOK", &device, &stream, &tensor, &bytes)) return nullptr;
+    if (!PyArg_ParseTuple(args, "iKOKp", &device, &stream, &tensor, &bytes, &in_graph)) return nullptr;
     const void* address = nullptr;
     try {
         address = tensor_address(tensor);
@@ -269,9 +281,48 @@ PyObject* set_scratch(PyObject*, PyObject* args) {
     Scratch& s = (*g_scratch)[{device, (void*)(uintptr_t)stream}];
     PyObject* before = s.owner;
     Py_INCREF(tensor);
-    s = Scratch{tensor, const_cast<void*>(address), (size_t)bytes};
+    s = Scratch{tensor, const_cast<void*>(address), (size_t)bytes, in_graph != 0};
     Py_XDECREF(before);
     Py_RETURN_NONE;
+}
+// scratch_use(device, stream): notes that the stream's scratch is handed out; (the stream is being captured, a graph may hold the
+// address of the scratch)
+PyObject* scratch_use(PyObject*, PyObject* args) {
+    int device;
+    unsigned long long stream;
+    if (!PyArg_ParseTuple(args, "iK", &device, &stream)) return nullptr;
+    bool capturing = false;
+    try {
+        capturing = is_capturing((cudaStream_t)(uintptr_t)stream);
+    } catch (const std::exception& e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what());
+        return nullptr;
+    }
+    auto it = g_scratch->find({device, (void*)(uintptr_t)stream});
+    if (it != g_scratch->end()) it->second.in_graph = it->second.in_graph || capturing;
+    return Py_BuildValue("(NN)", PyBool_FromLong(capturing), PyBool_FromLong(it != g_scratch->end() && it->second.in_graph));
+}
+// zeros_outside_capture(device, bytes): zeroed memory that exists now, while a stream of this thread is being captured.  (An ordinary
+// allocation would come from the graph's own memory, and be zeroed by the graph.)
+PyObject* zeros_outside_capture(PyObject*, PyObject* args) {
+    int device;
+    long long bytes;
+    if (!PyArg_ParseTuple(args, "iL", &device, &bytes)) return nullptr;
+    try {
+        const c10::cuda::CUDAGuard on((c10::DeviceIndex)device);
+        const c10::cuda::CUDAStreamCaptureModeGuard relaxed{cudaStreamCaptureModeRelaxed};
+        // (streams of the pool are handed out in turn: one of them may be the one that is captured)
+        c10::cuda::CUDAStream side = c10::cuda::getStreamFromPool(false, (c10::DeviceIndex)device);
+        for (int i = 0; i < 64 && is_capturing(side.stream()); ++i) side = c10::cuda::getStreamFromPool(false, (c10::DeviceIndex)device);
+        const c10::cuda::CUDAStreamGuard beside(side);
+        at::Tensor t = at::detail::empty_cuda({bytes}, at::kByte, at::Device(at::kCUDA, (c10::DeviceIndex)device), std::nullopt);
+        C10_CUDA_CHECK(cudaMemsetAsync(t.mutable_data_ptr(), 0, (size_t)bytes, side.stream()));
+        C10_CUDA_CHECK(cudaStreamSynchronize(side.stream()));
+        return THPVariable_Wrap(std::move(t));
+    } catch (const std::exception& e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what());
+        return nullptr;
+    }
 }
 PyObject* set_scratch_source(PyObject*, PyObject* fn) {
     Py_INCREF(fn);
@@ -282,6 +333,8 @@ PyObject* set_scratch_source(PyObject*, PyObject* fn) {
 PyMethodDef module_methods[] = {
     {"set_scratch", set_scratch, METH_VARARGS, nullptr},
     {"set_scratch_source", set_scratch_source, METH_O, nullptr},
+    {"scratch_use", scratch_use, METH_VARARGS, nullptr},
+    {"zeros_outside_capture", zeros_outside_capture, METH_VARARGS, nullptr},
     {nullptr, nullptr, 0, nullptr},
 };
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, module_methods};

@@ -13,7 +13,8 @@ import torch
 
 from . import _lib
 
-_workspaces = {}
+_workspaces = {}     # (device, stream) -> scratch
+_held = {}           # (device, stream) -> scratch that larger one has replaced and that a CUDA graph may hold the address of
 
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
@@ -39,18 +40,28 @@ def get_workspace(device: torch.device, nbytes: int) -> torch.Tensor:
 
     The kernels restore the scratch to its zero state, so one buffer serves every layer as long as calls are
     ordered on a stream; calls on different streams may overlap on the GPU and therefore get different buffers.
-    A buffer that has to grow is replaced (its sticky status word travels to the new one).
+    A buffer that has to grow is replaced (its sticky status word travels to the new one).  A CUDA graph holds the address of
+    what was handed out while its stream was captured: such a buffer stays for good, and its successor has at least twice its
+    size, so that all that stay are smaller than the one in use.  What is allocated during a capture exists beside the graph,
+    zeroed at once: it also serves graphs that are captured later, on their own.
     """
     index = device.index if device.index is not None else torch.cuda.current_device()
-    key = (index, torch._C._cuda_getCurrentRawStream(index))
+    key = (index, _stream(device))
+    capturing, in_graph = _lib._host.scratch_use(*key)
     ws = _workspaces.get(key)
     if ws is None or ws.numel() < nbytes:
-        size = max(nbytes, 1 << 20)
-        new = torch.zeros(size, dtype=torch.uint8, device=device)
-        if ws is not None:
+        keep = ws is not None and (capturing or in_graph)
+        size = max(nbytes, 1 << 20, 2 * ws.numel() if keep else 0)
+        if capturing:
+            new = _lib._host.zeros_outside_capture(index, size)
+        else:
+            new = torch.zeros(size, dtype=torch.uint8, device=device)
+        if keep:
+            _held.setdefault(key, []).append(ws)
+        elif ws is not None:
             new[16380:16384].copy_(ws[16380:16384])
         ws = _workspaces[key] = new
-        _lib._host.set_scratch(index, key[1], new, size)
+        _lib._host.set_scratch(index, key[1], new, size, capturing)
     return ws
 
 
@@ -69,7 +80,7 @@ def check_status(device=None) -> None:
     """Raise if any kernel that used this module's scratch buffers on ``device`` gave up a bounded wait (its results
     were then undefined).  Synchronises the streams it looks at; meant for tests, benchmarks and the end of a run."""
     import ctypes
-    for (index, stream), ws in list(_workspaces.items()):
+    for (index, stream), ws in [*_workspaces.items(), *((key, ws) for key, old in _held.items() for ws in old)]:
         if device is not None and torch.device(device).index not in (None, index):
             continue
         word = ctypes.c_uint(0)
