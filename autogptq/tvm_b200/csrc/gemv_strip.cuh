@@ -348,10 +348,13 @@ template <> struct IntLayout<3, true> {
         }
     }
 };
-// Byte planes of M rows of x: a unit's B operands [step][quad lane][4 row + plane][b0, b1], and per unit and row its factor and the
-// sums of x of its groups (floats).
+// Byte planes of M rows of x: a unit's B operands [step][quad lane][4 row + plane][b0, b1], and per unit and row its factors and the
+// sums of x, of the unit or of each 32 rows where these are scaled apart (floats).
 template <int BITS> __host__ __device__ constexpr int int_unit_bytes(int M) { return (BITS == 3 ? 5 : 4) * 128 * M; }
 __host__ __device__ constexpr int int_factors(int sub) { return sub == 1 ? 2 : 8; }
+// Bits of |X|.  Shifted by up to kPre, X has to fit in four signed bytes: 30 - kPre at most.  4 bits take all of them, their fp16 form
+// being exact products summed in fp32.  2 and 3 bits keep 22: their fp16 form subtracts sums of up to 1024 times x and is off by more.
+__host__ __device__ constexpr int int_x_bits(int bits) { return bits == 4 ? 26 : 22; }
 __host__ __device__ constexpr bool int_takes(int bits, int sub) { return bits == 4 || (bits != 8 && sub == 1); }
 
 // How x meets the weights: several rows in fp16, one row in fp16, one or two rows as byte planes.
@@ -728,19 +731,25 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
 #pragma unroll
                     for (int e = 0; e < 8; ++e) mx[v] = max(mx[v], h[v][e] & 0x7fffu);    // the order of non-negative fp16 numbers
                 }
+                constexpr int XB = int_x_bits(BITS);
                 float scale[V];
                 int ex[V], sum[V];
                 bool bad[V];
 #pragma unroll
                 for (int v = 0; v < V; ++v) {
-                    const uint32_t lo = __reduce_max_sync(0xffffffffu, lane < 16 ? mx[v] : 0u), hi = __reduce_max_sync(0xffffffffu, lane < 16 ? 0u : mx[v]);
-                    // 2^ex > max |x| of the unit; X = x * 2^(148 - ex) has |X| < 2^22.  A unit of zeros takes any scale; a
-                    // unit with an infinity or a NaN gets a NaN factor, so that its columns come out as NaN.
-                    mx[v] = lane < 16 ? lo : hi;
+                    // 2^ex > max |x| of the rows that share a factor; X = x * 2^(126 + XB - ex) has |X| < 2^XB.  Rows of zeros take any
+                    // scale; rows with an infinity or a NaN get a NaN factor, so that their columns come out as NaN.
+                    if constexpr (SUB == 1) {
+                        const uint32_t lo = __reduce_max_sync(0xffffffffu, lane < 16 ? mx[v] : 0u), hi = __reduce_max_sync(0xffffffffu, lane < 16 ? 0u : mx[v]);
+                        mx[v] = lane < 16 ? lo : hi;
+                    } else {
+#pragma unroll
+                        for (int o = 1; o < 4; o <<= 1) mx[v] = max(mx[v], __shfl_xor_sync(0xffffffffu, mx[v], o));
+                    }
                     ex[v] = (int)(__float_as_uint(__half2float(__ushort_as_half((unsigned short)mx[v]))) >> 23);
                     bad[v] = mx[v] >= 0x7c00u;
                     if (mx[v] == 0u || bad[v]) ex[v] = 127;
-                    scale[v] = __uint_as_float((uint32_t)(275 - ex[v]) << 23);
+                    scale[v] = __uint_as_float((uint32_t)(253 + XB - ex[v]) << 23);
                 }
                 uint32_t dg[V][8];
 #pragma unroll
@@ -748,25 +757,37 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                     sum[v] = 0;
 #pragma unroll
                     for (int e = 0; e < 8; ++e) {
-                        // round to nearest through the fp32 adder: |x * scale| <= 2^22
-                        const int X = __float_as_int(fmaf(__half2float(__ushort_as_half((unsigned short)h[v][e])), scale[v], 12582912.f)) - 0x4B400000;
+                        const float xf = __half2float(__ushort_as_half((unsigned short)h[v][e]));
+                        // round to nearest; up to 22 bits through the fp32 adder
+                        const int X = XB > 22 ? __float2int_rn(xf * scale[v]) : __float_as_int(fmaf(xf, scale[v], 12582912.f)) - 0x4B400000;
                         sum[v] += X;
                         dg[v][e] = (uint32_t)((X << pre[e]) + 0x00808080) ^ 0x00808080u;   // four signed base-256 digits
                     }
                 }
+                // (the X of 128 rows of 22 bits, or of 32 rows of 26, add up to less than 2^31)
+                constexpr int WHOLE_SUM = SUB == 4 || XB > 22 ? 4 : 16;
 #pragma unroll
-                for (int o = 1; o < (SUB == 1 ? 16 : 4); o <<= 1)
+                for (int o = 1; o < WHOLE_SUM; o <<= 1)
 #pragma unroll
                     for (int v = 0; v < V; ++v) sum[v] += __shfl_xor_sync(0xffffffffu, sum[v], o);
+                float sumf[V];
+#pragma unroll
+                for (int v = 0; v < V; ++v) sumf[v] = (float)sum[v];
+#pragma unroll
+                for (int o = WHOLE_SUM; o < (SUB == 1 ? 16 : 4); o <<= 1)
+#pragma unroll
+                    for (int v = 0; v < V; ++v) sumf[v] += __shfl_xor_sync(0xffffffffu, sumf[v], o);
 #pragma unroll
                 for (int v = 0; v < V; ++v) {
                     if (!active[v]) continue;
                     const int u = (q0 + 32 * v + lane) >> 4;
-                    // the factor of the planes, then minus the sum of x of every group (32 rows each where they are scaled apart)
-                    const float delta = __uint_as_float((uint32_t)(ex[v] - 21) << 23);   // 2^(ex - 148)
+                    const float delta = __uint_as_float((uint32_t)(ex[v] + 1 - XB) << 23);   // 2^(ex - 126 - XB)
+                    const float factor = bad[v] ? __uint_as_float(0x7fc00000u) : __uint_as_float((uint32_t)(ex[v] + 1 - XB - I::kPre) << 23);
                     float* f = p_f + (u * M + m) * FACTORS;
-                    if ((lane & 15) == 0) f[0] = bad[v] ? __uint_as_float(0x7fc00000u) : __uint_as_float((uint32_t)(ex[v] - 21 - I::kPre) << 23);
-                    if (SUB == 1 ? (lane & 15) == 0 : jq == 0) f[1 + (SUB == 1 ? 0 : iq)] = -delta * (float)sum[v];
+                    if (SUB == 1 ? (lane & 15) == 0 : jq == 0) {       // factor of the planes and minus the sum of x, or four of each
+                        f[SUB == 1 ? 0 : iq] = factor;
+                        f[SUB == 1 ? 1 : 4 + iq] = -delta * sumf[v];
+                    }
                     uint8_t* dst = p_x + (size_t)u * unit_x + jq * (32 * M) + m * 32;
                     auto store = [&](int step, const uint32_t (&lo)[4], const uint32_t (&hi)[4]) {
                         uint4* d = reinterpret_cast<uint4*>(dst + step * 4 * (32 * M));
@@ -835,10 +856,15 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                     if (g < 4 * M) bx[s] = *reinterpret_cast<const uint2*>(p_x + (size_t)u * unit_x + (s * 4 + j) * (32 * M) + g * 8);
                 }
                 const float* f = p_f + (u * M + (M == 2 ? j >> 1 : 0)) * FACTORS;
-                const float cf = f[0] * plane_weight;
-                float sx[SUB];
-#pragma unroll
-                for (int sub = 0; sub < SUB; ++sub) sx[sub] = f[1 + sub] * sum_weight;
+                float cf[SUB], sx[SUB];
+                if constexpr (SUB == 1) {
+                    const float2 v = *reinterpret_cast<const float2*>(f);
+                    cf[0] = v.x * plane_weight; sx[0] = v.y * sum_weight;
+                } else {
+                    const float4 c = *reinterpret_cast<const float4*>(f), v = *reinterpret_cast<const float4*>(f + 4);
+                    cf[0] = c.x * plane_weight; cf[1] = c.y * plane_weight; cf[2] = c.z * plane_weight; cf[3] = c.w * plane_weight;
+                    sx[0] = v.x * sum_weight; sx[1] = v.y * sum_weight; sx[2] = v.z * sum_weight; sx[3] = v.w * sum_weight;
+                }
                 mbar_wait(bar0 + 8u * slot, parity, ok);
 #pragma unroll
                 for (int t = 0; t < T; ++t) {
@@ -875,7 +901,7 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
 #pragma unroll
                             for (int c = 0; c < 2; ++c) {
                                 const float lo = __int_as_float(d[2 * c]) - 12582912.f, hi = __int_as_float(d[2 * c + 1]) - 12582912.f;
-                                out[t][0][2 * h + c][0] = fmaf(sf[2 * h + c], fmaf(fmaf(256.f, hi, lo), cf, zf[c] * sx[sub]), out[t][0][2 * h + c][0]);
+                                out[t][0][2 * h + c][0] = fmaf(sf[2 * h + c], fmaf(fmaf(256.f, hi, lo), cf[sub], zf[c] * sx[sub]), out[t][0][2 * h + c][0]);
                             }
                         }
                     }

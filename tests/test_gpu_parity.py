@@ -209,11 +209,13 @@ def test_single_row_gemv_vs_oracle(bits, K, N, gs, act, bias):
     ops.check_status(DEV)
 
 
-def test_single_row_value_ranges():
-    """On the integer tensor path x is converted to fixed point per 128 rows of K: rows of zeros, a wide dynamic
-    range inside a unit, values at the ends of the fp16 range and a NaN must all come out as fp32 accumulation
+@pytest.mark.parametrize("bits,N,gs", [(3, 4736, 128),                                     # one strip of columns per CTA: fp16
+                                       (3, 14432, 128), (2, 9632, 128), (4, 9632, 128), (4, 9632, 32)])   # several: byte planes
+def test_single_row_value_ranges(bits, N, gs):
+    """On the integer tensor path x is converted to fixed point per 128 rows of K, or per 32 that are scaled apart: rows of zeros, a
+    wide dynamic range inside a unit, values at the ends of the fp16 range and a NaN must all come out as fp32 accumulation
     would give them."""
-    bits, K, N, gs = 3, 4096, 4736, 128
+    K = 4096
     layer = synth.make_layer(bits, K, N, gs, False, seed=99)
     _, _, W = O.dequantize(*_layer_np(layer), bits)
     d = layer.to(DEV)

@@ -74,6 +74,74 @@ def test_byte_planes_vs_oracle(bits, K, N, gs, gather, M):
     test_gemv_vs_oracle(bits, K, N, gs, gather, M)
 
 
+def _bound_of_planes(bits, x, w, a, rows):
+    """What fixed point per `rows` rows of x and fp32 sums may be off by, for x [M, K], exact weights w and a = scale * (field + zero):
+    X is rounded at 2^-26 of a power of two above the largest |x| (4 bits; 2^-22 for 2 and 3), uniformly, seven standard deviations
+    for 1e5 outputs; every unit's sums are rounded half a dozen times and added over up to 16 units and 16 warps (2^-24 each)."""
+    M, K = x.shape
+    var, top = 0.0, 0.0
+    for k in range(0, K, rows):
+        m = np.abs(x[:, k:k + rows]).max(axis=1, keepdims=True)
+        e = np.where(m > 0, np.floor(np.log2(np.maximum(m, 2.0 ** -24))) + 1, -30.0)
+        step = 2.0 ** (e - (26 if bits == 4 else 22))
+        var = var + step ** 2 / 12 * (w[k:k + rows] ** 2).sum(axis=0, keepdims=True)
+        top = top + np.abs(x[:, k:k + rows]) @ a[k:k + rows]
+    return 7 * np.sqrt(var) + 38 * 2.0 ** -24 * top
+
+
+def _run_and_exact(layer, x):
+    """The kernel's result, and the result, weights and scale * (field + zero) in 64 bits (no rounding of the weights)."""
+    q, z, _ = O.dequantize(layer.qweight.numpy(), layer.qzeros.numpy(), layer.scales.numpy(), layer.g_idx.numpy(), layer.bits)
+    g = layer.g_idx.numpy().astype(np.int64)
+    s, q, z = layer.scales.numpy().astype(np.float64)[g], q.astype(np.float64), z.astype(np.float64)[g]
+    w = s * (q - z)
+    d = layer.to(DEV)
+    y = ops.gemv(x.to(DEV), d.qweight, d.qzeros, d.scales, None, layer.bits, layer.group_size).cpu().numpy().astype(np.float64)
+    ops.check_status(DEV)
+    return y, x.numpy().astype(np.float64) @ w, w, s * (q + z)
+
+
+@pytest.mark.parametrize("bits,K,N,gs", [(4, 4128, 9632, 32), (4, 4160, 9632, 64), (4, 4128, 9632, 96), (4, 4224, 9632, 128),
+                                         (3, 4224, 9632, 128), (2, 4224, 9632, 128)])
+@pytest.mark.parametrize("M", [1, 2])
+def test_groups_of_other_magnitudes_keep_their_bits(bits, K, N, gs, M):
+    """Neighbouring groups whose x differs by up to 2^27 and whose scales make up for it, on byte planes: the small ones count as much
+    as the large ones.  (A fixed point shared by groups that are scaled apart loses them.)"""
+    layer = synth.make_layer(bits, K, N, gs, False, seed=K + bits)
+    G = layer.scales.shape[0]
+    mag = 2.0 ** torch.tensor([[-14, 13, -9, 4, 0, -12][g % 6] for g in range(G)], dtype=torch.float64)
+    gen = torch.Generator().manual_seed(5)
+    layer.scales = ((1 + torch.rand((G, N), generator=gen)) / mag[:, None]).half()
+    x = torch.randn((M, K), generator=gen).double() * mag[layer.g_idx.long()]
+    x[:, 128:256] = 0.0                                    # a unit of zeros
+    x[:, 300:416:3] = 0.0
+    x = x.clamp(-60000, 60000).half()
+    y, ref, w, a = _run_and_exact(layer, x)
+    bound = _bound_of_planes(bits, x.numpy().astype(np.float64), w, a, 32 if gs % 128 else 128) + 2.0 ** -11 * np.abs(ref) + 2.0 ** -24
+    assert np.all(np.abs(y - ref) <= bound), (np.abs(y - ref) / bound).max()
+
+
+@pytest.mark.parametrize("M", [1, 2])
+def test_small_values_beside_outliers_keep_their_bits(M):
+    """4 bits, every 128 rows with two values 4e6 times the others that cancel exactly (rows of equal weights): what is left shows in
+    how many bits the others were held."""
+    K, N = 4096, 9632
+    layer = synth.make_layer(4, K, N, 128, False, seed=9)
+    first = layer.qweight[0::16]
+    layer.qweight[0::16] = (first & ~0xf0) | ((first & 0xf) << 4)          # row 1 of every unit like row 0
+    x = torch.randn((M, K), generator=torch.Generator().manual_seed(6)) * 2.0 ** -7
+    x[:, 0::128], x[:, 1::128] = 30000.0, -30000.0
+    x = x.half()
+    y, ref, w, a = _run_and_exact(layer, x)
+    rest = np.abs(x.numpy().astype(np.float64))
+    rest[:, 0::128] = rest[:, 1::128] = 0.0
+    xs = x.numpy().astype(np.float64)
+    w[0::128] = w[1::128] = 0.0                            # (exact in fixed point: integers of 11 bits)
+    a[0::128] = a[1::128] = 0.0
+    bound = _bound_of_planes(4, xs, w, a, 128) + 2.0 ** -11 * np.abs(ref) + 2.0 ** -24
+    assert np.all(np.abs(y - ref) <= bound), (np.abs(y - ref) / bound).max()
+
+
 @pytest.mark.parametrize("bits,K,N,gs,gather", [(2, 544, 96, 32, True), (3, 1152, 4832, 128, False), (3, 1184, 64, 64, True),
                                                 (4, 4096, 4800, 128, True), (4, 992, 32, 32, False), (8, 288, 9632, -1, False),
                                                 # x does not fit: places in turn, three and four of them, several passes
