@@ -318,7 +318,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     const uint32_t tmem_base = tmem_base_holder, tmem_a = tmem_base + (uint32_t)(p.acc_sets * TN);
     asm volatile("griddepcontrol.launch_dependents;");
     // What a preceding kernel may still be writing: x; what it may still be reading: y and the scratch.  The weights are unpacked
-    // before the wait, as far as the stages go (77 rows of 11008 x 4096: the first product came 2.6 us after the wait, now 1.1).
+    // before the wait, as far as the stages go (77 rows of 11008 x 4096: the first product came 2.6 us after the wait, now 1.1).  From
+    // there on what a warp waits for comes after the products, and these after x: it lets the preceding kernel end before
+    // it starts the clock of a bounded wait (a sum over ranks may take its time).
     if (warp != 0 && warp != 3 && (warp < kFirstWeightWarp || g_idx)) asm volatile("griddepcontrol.wait;" ::: "memory");
 
     // ---- epilogue: a warp reads the accumulators of 32 columns (tensor-memory lanes), 16 rows of x at a time ----
@@ -358,7 +360,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
                 for (int u = v.u0; u < v.u1; ++u, mine ^= 1) {
                     if (mine) {
                         const int g0 = group_at(4 * u);
-                        if (round > 0) ok = mbar_wait(w_empty(s), (round - 1) & 1, &abort_flag);
+                        if (round > 0 && !mbar_try(w_empty(s), (round - 1) & 1)) {
+                            asm volatile("griddepcontrol.wait;" ::: "memory");
+                            ok = mbar_wait(w_empty(s), (round - 1) & 1, &abort_flag);
+                        }
                         if (!ok) break;
                         const uint32_t dst = base + w_off + s * w_slot, bar = w_full(s);
                         mbar_expect(bar, tx);
@@ -446,6 +451,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
                 // (an answer takes 190 clk: both questions are asked before the first answer is looked at)
                 const bool there = mbar_try(w_full(ws), wround & 1), free = round == 0 || mbar_try(empty(s), (round - 1) & 1);
                 if (!__all_sync(0xffffffffu, there && free)) {
+                    if (round > 0 || wround > 0) asm volatile("griddepcontrol.wait;" ::: "memory");
                     ok = mbar_wait(w_full(ws), wround & 1, &abort_flag);
                     if (ok && round > 0) ok = mbar_wait(empty(s), (round - 1) & 1, &abort_flag);   // its products have retired
                     ok = __all_sync(0xffffffffu, ok);

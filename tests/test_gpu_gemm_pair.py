@@ -1,13 +1,16 @@
 """The tensor-core kernel for pairs of SMs (more than 16 rows; 2 and 8 bits at any number) at the edges of its split: column
 tiles with one CTA or part of one beyond the layer, cut k-tiles and units, one to four groups per unit, more tiles than pairs
 (persistent), one and two sets of accumulators, and K split over pairs."""
+import ctypes
+from types import SimpleNamespace
+
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
 
 if torch.cuda.is_available():
-    from autogptq.tvm_b200 import ops, synth
+    from autogptq.tvm_b200 import _lib, ops, synth
     DEV = torch.device("cuda:0")
 
 CASES = [
@@ -66,3 +69,24 @@ def test_split_of_the_cases_above():
     assert ops.gemm_split(33, 4096, 4128, 3) == (4, 1)
     assert ops.gemm_split(64, 2048, 19232, 4) == (1, 1)
     assert ops.gemm_split(96, 4064, 64, 3)[0] == 4
+
+
+@pytest.mark.parametrize("K", [4096, 384])       # more units of K than there are stages, and fewer
+def test_a_kernel_in_front_that_takes_longer_than_a_bounded_wait(K):
+    """The kernel unpacks weights while the one in front of it still runs; the time it waits for that one is not its own.  In front: an
+    all-reduce whose peer never comes, which gives up after 2.4e9 clocks (the GEMM's own waits end after 2e9)."""
+    d = synth.make_layer(4, K, 1056, 128, False, seed=K, device=DEV)
+    x = synth.make_x(77, K, seed=1, device=DEV)
+    run = lambda: ops.gemm(x, d.qweight, d.qzeros, d.scales, None, 4, 128)
+    want = run()
+    buffers = [torch.zeros(int(_lib.lib.b200gptq_tp_buffer_bytes()), dtype=torch.uint8, device=DEV) for _ in range(2)]
+    exchange = SimpleNamespace(rank=0, world=2, peer_table=(ctypes.c_void_p * 2)(*(b.data_ptr() for b in buffers)),
+                               timeout_cycles=2_400_000_000)
+    y = torch.zeros((1, 256), dtype=torch.float16, device=DEV)
+    torch.cuda.synchronize()
+    ops.tp_allreduce(y, exchange)
+    got = run()
+    torch.cuda.synchronize()
+    assert int(buffers[0][:4].view(torch.int32)) == 2       # the all-reduce did run out of time
+    assert torch.equal(got, want)
+    ops.check_status(DEV)
