@@ -37,6 +37,7 @@ size_t gemv_generic_workspace_bytes(int M, int K, int N);
 bool gemv_stream_supported(int M, int K, int N, int bits, int group_size);
 size_t gemv_stream_workspace_bytes(int M, int K, int N, int bits);
 size_t gemm_workspace_bytes(int M, int K, int N, int bits);
+size_t gemm_workspace_least(int M, int K, int N, int bits);
 void gemm_split_query(int M, int K, int N, int bits, int* splits, int* ctas_per_sm);
 int gemm_dispatch(const __half*, const int32_t*, const int32_t*, const __half*, const int32_t*, const int32_t*,
                   const __half*, __half*, int, int, int, int, int, void*, size_t, cudaStream_t);
@@ -307,7 +308,7 @@ int b200gptq_gemm(const void* x, const int32_t* qweight, const int32_t* qzeros, 
     if (!g_idx && group_size % 32 != 0) return B200GPTQ_ERR_GROUPS;
     if (!aligned16(qweight) || !aligned16(x) || !aligned16(y) || !aligned16(scales) || !aligned16(qzeros))
         return B200GPTQ_ERR_ALIGNMENT;
-    const size_t need = b200gptq_workspace_bytes(B200GPTQ_OP_GEMM, M, K, N, bits);
+    const size_t need = gemm_workspace_least(M, K, N, bits);
     if (need && (!workspace || workspace_bytes < need)) return B200GPTQ_ERR_WORKSPACE;
     if (workspace && !aligned16(workspace)) return B200GPTQ_ERR_ALIGNMENT;
     return gemm_dispatch(static_cast<const __half*>(x), qweight, qzeros, static_cast<const __half*>(scales), g_idx,

@@ -709,7 +709,13 @@ size_t gemm_workspace_bytes(int M, int K, int N, int bits) {
     return kCounterBytes + (((size_t)M * K * sizeof(__half) + 255) & ~(size_t)255) +
            (use_pair(M, bits) ? gemm_pair_partial_bytes(M, N, pair_plan(M, N, K)) : split_partial_bytes(M, N, K));
 }
-
+// What a call is taken with: more than 128 rows run without cutting K where there is no room for the sums of its runs.  (A scratch
+// that was made for a longer prompt may be smaller than what a shorter one would like: 16.8 MB for 1024 rows of 8192 x 2048,
+// 18.4 for 400.)
+size_t gemm_workspace_least(int M, int K, int N, int bits) {
+    if (M <= 128 || !use_pair(M, bits)) return gemm_workspace_bytes(M, K, N, bits);
+    return kCounterBytes + (((size_t)M * K * sizeof(__half) + 255) & ~(size_t)255);
+}
 
 void gemm_split_query(int M, int K, int N, int bits, int* splits, int* ctas_per_sm) {
     GemmSplit g;
@@ -744,7 +750,6 @@ int gather_x_dispatch(const __half* x, const int32_t* x_perm, __half* xp, int M,
 int gemm_dispatch(const __half* x, const int32_t* qweight, const int32_t* qzeros, const __half* scales,
                   const int32_t* g_idx, const int32_t* x_perm, const __half* bias, __half* y, int M, int K, int N,
                   int bits, int group_size, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
-    (void)workspace_bytes;
     unsigned int* status = reinterpret_cast<unsigned int*>(workspace);
     const __half* xt = x;
     const bool pair = use_pair(M, bits);
@@ -755,9 +760,13 @@ int gemm_dispatch(const __half* x, const int32_t* qweight, const int32_t* qzeros
     }
     float* partial = reinterpret_cast<float*>(reinterpret_cast<char*>(workspace) + kCounterBytes +
                                               (((size_t)M * K * sizeof(__half) + 255) & ~(size_t)255));
-    if (pair)
-        return gemm_pair_dispatch(xt, qweight, qzeros, scales, g_idx, bias, y, M, K, N, bits, group_size,
-                                  pair_plan(M, N, K), status, partial, stream);
+    if (pair) {
+        GemmPairPlan plan = pair_plan(M, N, K);
+        if (gemm_workspace_least(M, K, N, bits) + gemm_pair_partial_bytes(M, N, plan) > workspace_bytes && M > 128)
+            plan = gemm_pair_plan(M, N, K, 1, true);
+        return gemm_pair_dispatch(xt, qweight, qzeros, scales, g_idx, bias, y, M, K, N, bits, group_size, plan, status, partial,
+                                  stream);
+    }
     if (bits == 4) return launch_gemm<4>(xt, qweight, qzeros, scales, g_idx, bias, y, M, K, N, group_size, status, partial, stream);
     if (bits == 3) return launch_gemm<3>(xt, qweight, qzeros, scales, g_idx, bias, y, M, K, N, group_size, status, partial, stream);
     return B200GPTQ_ERR_BITS;

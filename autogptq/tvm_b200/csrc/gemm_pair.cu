@@ -639,11 +639,11 @@ EncodeTiledFn encode_tiled_fn() {
 // says, the weight warps up to 128 rows and the products above; start-up and drain take longer the more SMs work; the sum over runs
 // grows with what goes through the scratch.  Several runs have a tile per pair of SMs, of eight units or more.  Up to 128 rows the
 // caller says how many runs (`few`), in one tile of rows.  Against the best tile without runs: 256 rows of 11008 x 4096 32.1 -> 24.9 us,
-// 256 rows of 8192 x 2048 23.3 -> 15.9, 512 rows 25.0 -> 21.2.
-GemmPairPlan gemm_pair_plan(int M, int N, int K, int few) {
+// 256 rows of 8192 x 2048 23.3 -> 15.9, 512 rows 25.0 -> 21.2.  one_run: more than 128 rows without runs (no room for their sums).
+GemmPairPlan gemm_pair_plan(int M, int N, int K, int few, bool one_run) {
     constexpr int kPerTile[8] = {300, 310, 325, 340, 390, 470, 540, 610};      // 32, 64, .. 256 rows
     const long long pairs = (N + 2 * BN - 1) / (2 * BN), slots = sm_count() / 2, units = (K + 127) / 128;
-    const int least = M <= 128 ? few : 1, most = M <= 128 ? few : kMaxSplits;
+    const int least = M <= 128 ? few : 1, most = M <= 128 ? few : one_run ? 1 : kMaxSplits;
     long long best = -1;
     GemmPairPlan plan = {256, 1};
     for (int splits = least; splits <= most; ++splits)

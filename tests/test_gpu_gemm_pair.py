@@ -90,3 +90,22 @@ def test_a_kernel_in_front_that_takes_longer_than_a_bounded_wait(K):
     assert int(buffers[0][:4].view(torch.int32)) == 2       # the all-reduce did run out of time
     assert torch.equal(got, want)
     ops.check_status(DEV)
+
+
+def test_scratch_of_a_longer_prompt_serves_a_shorter_one():
+    """More than 128 rows are taken with any scratch that holds the counters and a copy of x; without room for the sums of several runs
+    of K there is one run."""
+    bits, K, N, gs = 4, 8192, 2048, 128
+    d = synth.make_layer(bits, K, N, gs, False, seed=4, device=DEV)
+    x = synth.make_x(400, K, seed=5, device=DEV)
+    need = lambda M: _lib.workspace_bytes(_lib.OP_GEMM, M, K, N, bits)
+    assert ops.gemm_split(400, K, N, bits)[0] > 1 and need(1024) < need(400)
+    _, W = ops.dequantize(d.qweight, d.qzeros, d.scales, d.g_idx, bits, gs, want_q=False)
+    ref, size = x.double() @ W.double(), x.double().abs() @ W.double().abs()
+    for nbytes in (need(400), need(1024), 16384 + 2 * 400 * K):
+        ws = torch.zeros(nbytes, dtype=torch.uint8, device=DEV)
+        y = ops.gemm(x, d.qweight, d.qzeros, d.scales, None, bits, gs, workspace=ws)
+        assert bool(((y.double() - ref).abs() <= 2.0 ** -11 * ref.abs() + K * 2.0 ** -23 * size + 2.0 ** -24).all())
+        assert not bool(ws[:16384].any())
+    with pytest.raises((RuntimeError, ValueError)):
+        ops.gemm(x, d.qweight, d.qzeros, d.scales, None, bits, gs, workspace=ws[:-16])
