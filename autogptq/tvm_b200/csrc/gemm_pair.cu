@@ -636,7 +636,9 @@ EncodeTiledFn encode_tiled_fn() {
 
 // Rows of x per tile and runs of K.  In clocks, fitted to 4 bits, 100 to 1024 rows of 4096 x 4096, 4096 x 12288, 11008 x 4096,
 // 2048 x 8192 and 8192 x 2048 (within 10 % of what was measured; 3 and 8 bits come within 5 % of 4): a k-tile takes what kPerTile
-// says, the weight warps up to 128 rows and the products above; start-up and drain take longer the more SMs work; the sum over runs
+// says, the weight warps up to 128 rows and the products above; tiles of 160 rows, bound by the weight warps and with one set of
+// accumulators, take 25 more where one follows another, their drain (2048 rows of 11008 x 4096 in groups of 32 139 us in such tiles,
+// 129 in tiles of 256); start-up and drain take longer the more SMs work; the sum over runs
 // grows with what goes through the scratch.  Several runs have a tile per pair of SMs, of eight units or more.  Up to 128 rows the
 // caller says how many runs (`few`), in one tile of rows.  Against the best tile without runs: 256 rows of 11008 x 4096 32.1 -> 24.9 us,
 // 256 rows of 8192 x 2048 23.3 -> 15.9, 512 rows 25.0 -> 21.2.  one_run: more than 128 rows without runs (no room for their sums).
@@ -651,7 +653,7 @@ GemmPairPlan gemm_pair_plan(int M, int N, int K, int few, bool one_run) {
             const long long rows = (M + t - 1) / t, tiles = pairs * rows * splits, waves = (tiles + slots - 1) / slots;
             if (splits > 1 && (M <= 128 ? t < M : waves > 1 || units / splits < 8)) break;
             const long long kt = 2 * ((units + splits - 1) / splits), busy = tiles < slots ? tiles : slots;
-            const long long cost = waves * kt * kPerTile[t / 32 - 1] + 2850 + 8200 * busy / slots + (splits > 1 ? 6500 + 8 * t * splits : 0);
+            const long long cost = waves * kt * (kPerTile[t / 32 - 1] + (t == 160 && waves > 1 ? 25 : 0)) + 2850 + 8200 * busy / slots + (splits > 1 ? 6500 + 8 * t * splits : 0);
             if (best < 0 || cost < best) { best = cost; plan = {t, splits}; }
         }
     return plan;
