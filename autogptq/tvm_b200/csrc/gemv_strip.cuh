@@ -377,13 +377,13 @@ struct StripPlan {
 };
 
 // A slot: weights (1024-byte aligned for the swizzle), and in a second ring the scales [group][32 T] and the zero-point
-// words of each group.  Rows of qzeros of 4 and 8 bits are whole 16-byte pieces: one box holds every group's.  Of 2 and 3 bits a
-// group's words start anywhere, a box per group starts up to three words early.
+// words of each group.  Rows of qzeros of 4 and 8 bits are whole 16-byte pieces: one box holds every group's, unless `apart` asks for a
+// box per group (the host says when).  Of 2 and 3 bits a group's words start anywhere, a box per group starts up to three words early.
 __host__ __device__ constexpr int slot_bytes(int bits, int T) { return (4 * bits * 128 * T + 1023) & ~1023; }
 __host__ __device__ constexpr int zero_words(int bits, int T) { return bits % 4 == 0 ? T * bits : (T * bits + 3 + 3) & ~3; }
-__host__ __device__ constexpr int zero_pitch(int bits, int T) { return bits % 4 == 0 ? T * bits * 4 : (zero_words(bits, T) * 4 + 127) & ~127; }
+__host__ __device__ constexpr int zero_pitch(int bits, int T, bool apart) { return bits % 4 == 0 && !apart ? T * bits * 4 : (zero_words(bits, T) * 4 + 127) & ~127; }
 __host__ __device__ constexpr int scale_bytes(int T, int rows) { return (rows * T * 64 + 127) & ~127; }
-__host__ __device__ constexpr int const_bytes(int bits, int T, int rows) { return scale_bytes(T, rows) + ((rows * zero_pitch(bits, T) + 127) & ~127); }
+__host__ __device__ constexpr int const_bytes(int bits, int T, int rows, bool apart) { return scale_bytes(T, rows) + ((rows * zero_pitch(bits, T, apart) + 127) & ~127); }
 
 // The two activations folded into the read of x, rounded exactly like the stand-alone kernel (b200gptq_act).
 __device__ __forceinline__ uint32_t act_relu2(uint32_t v) {
@@ -401,11 +401,15 @@ __device__ __forceinline__ uint32_t act_swiglu2(uint32_t gv, uint32_t uv) {
 
 // SUB: groups of a unit that are scaled apart (1: a group is a whole number of units).  NT: rows of x / 8.
 // MODE: kSeveral, kOne, kInt.  T: strips of a pass.  W: warps of a CTA.
-// Registers: two CTAs of eight warps fit on an SM; sixteen warps, or sixteen rows of x, leave 4096 or 8192 of an SM's for the
-// kernel that comes next.  With all of them taken, the gather of x between two products of 8 rows, 9216 x 9216, 3 bits, only
+// Registers: what an SM has beside a CTA of eight warps (22 528 at 168) takes no second one, mostly.  With 128 two fit where K is short,
+// and the next launch's weights arrive beside the current one: 1024 x 7168 alone, 3 bits, two rows 3.1 us for 3.5, but 1024 x 3072 in
+// groups of 32, three rows with a gather 3.3 for 2.9 (two share an SM while others idle), a step of a decoder with hidden size 1024, batches of 4
+// and 8, 253 and 241 us for 237 and 232, and 9216 x 36864 6 % longer.  Sixteen warps, or sixteen rows of x, leave 4096 or 8192 of an SM's for
+// the kernel that comes next.  With all of them taken, the gather of x between two products of 8 rows, 9216 x 9216, 3 bits, only
 // started when a CTA ended, and the next product's weights after that: 22 us against 16.6 (and 14.3 against 14.1 where
 // nothing is gathered).
-template <int BITS, int SUB, int NT, int MODE, int T, int W>
+// APART: a box for the zero-points of each group.
+template <int BITS, int SUB, int NT, int MODE, int T, int W, bool APART>
 __global__ void __maxnreg__(W == 16 ? 120 : NT == 1 ? 168 : 224)
 gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_s,
                   const __grid_constant__ CUtensorMap tmap_z, const __half* __restrict__ x,
@@ -434,7 +438,7 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
 
     // shared memory: rings | x | sums of the warps, and in the same bytes: x as it lies in memory
     uint8_t* aligned = dsm + ((1024u - (smem_u32(dsm) & 1023u)) & 1023u);
-    const int cbytes = const_bytes(BITS, T, plan.rows_g);
+    const int cbytes = const_bytes(BITS, T, plan.rows_g, APART);
     uint8_t* p_ring = aligned + (size_t)warp * R * SLOT;
     uint8_t* p_const = aligned + (size_t)W * R * SLOT + (size_t)warp * R * cbytes;
     uint8_t* base_x = aligned + (size_t)W * R * (SLOT + cbytes);
@@ -471,7 +475,7 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
             asm volatile(
                 "cp.async.bulk.tensor.2d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                 ::"r"(cst), "l"(&tmap_s), "r"(strip * kStripCols), "r"(grp), "r"(bar) : "memory");
-            if constexpr (BITS % 4 == 0) {
+            if constexpr (!APART) {
                 asm volatile(
                     "cp.async.bulk.tensor.2d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                     ::"r"(cst + scale_bytes(T, plan.rows_g)), "l"(&tmap_z), "r"(strip * BITS), "r"(grp), "r"(bar) : "memory");
@@ -479,7 +483,7 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                 for (int r = 0; r < plan.rows_g; ++r)
                     asm volatile(
                         "cp.async.bulk.tensor.1d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2}], [%3];"
-                        ::"r"(cst + scale_bytes(T, plan.rows_g) + r * zero_pitch(BITS, T)), "l"(&tmap_z),
+                        ::"r"(cst + scale_bytes(T, plan.rows_g) + r * zero_pitch(BITS, T, APART)), "l"(&tmap_z),
                           "r"(((grp + r) * zwords + strip * BITS) & ~3), "r"(bar) : "memory");
             }
         }
@@ -758,7 +762,8 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
 #pragma unroll
                     for (int e = 0; e < 8; ++e) {
                         const float xf = __half2float(__ushort_as_half((unsigned short)h[v][e]));
-                        // round to nearest; up to 22 bits through the fp32 adder
+                        // round to nearest; up to 22 bits through the fp32 adder.  (26 bits through it, in two steps: more code, 0.1 to 0.5 us
+                        // a launch longer)
                         const int X = XB > 22 ? __float2int_rn(xf * scale[v]) : __float_as_int(fmaf(xf, scale[v], 12582912.f)) - 0x4B400000;
                         sum[v] += X;
                         dg[v][e] = (uint32_t)((X << pre[e]) + 0x00808080) ^ 0x00808080u;   // four signed base-256 digits
@@ -846,7 +851,7 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
             const uint8_t* cze = p_const + slot * cbytes + scale_bytes(T, plan.rows_g);
             auto zero_at = [&](int r, int t) {
                 const int early = BITS % 4 == 0 ? 0 : ((grp0 + r) * zwords + (strip0 + win) * BITS) & 3;
-                return cze + r * zero_pitch(BITS, T) + 4 * early + t * BITS * 4;
+                return cze + r * zero_pitch(BITS, T, APART) + 4 * early + t * BITS * 4;
             };
             if constexpr (INT) {
                 uint2 bx[I::kSteps];
@@ -1109,31 +1114,35 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     if (!ok) atomicExch(status + kStatusWord, 1u);
 }
 
-// The instantiation for (groups scaled apart in a unit, mode, rows of x / 8, strips of a pass, warps), nullptr where there
-// is none.
+// The instantiation for (groups scaled apart in a unit, mode, rows of x / 8, strips of a pass, warps, zero-points in a box each), nullptr
+// where there is none.
 template <int BITS, int SUB, int NT, int MODE, int W>
-const void* strip_kernel_t(int T) {
-    if (T == 1) return reinterpret_cast<const void*>(gemv_strip_kernel<BITS, SUB, NT, MODE, 1, W>);
-    if (T == 2) return reinterpret_cast<const void*>(gemv_strip_kernel<BITS, SUB, NT, MODE, 2, W>);
+const void* strip_kernel_t(int T, bool apart) {
+    constexpr bool APART = BITS % 4 != 0;
+    if constexpr (BITS == 4 && SUB == 4)
+        if (T == 1 && apart) return reinterpret_cast<const void*>(gemv_strip_kernel<BITS, SUB, NT, MODE, 1, W, true>);
+    if (apart != APART) return nullptr;
+    if (T == 1) return reinterpret_cast<const void*>(gemv_strip_kernel<BITS, SUB, NT, MODE, 1, W, APART>);
+    if (T == 2) return reinterpret_cast<const void*>(gemv_strip_kernel<BITS, SUB, NT, MODE, 2, W, APART>);
     if constexpr (NT == 1 && SUB == 1)
-        if (T == 3) return reinterpret_cast<const void*>(gemv_strip_kernel<BITS, SUB, NT, MODE, 3, W>);
+        if (T == 3) return reinterpret_cast<const void*>(gemv_strip_kernel<BITS, SUB, NT, MODE, 3, W, APART>);
     if constexpr (MODE == kInt && SUB == 1)
-        if (T == 4) return reinterpret_cast<const void*>(gemv_strip_kernel<BITS, SUB, NT, MODE, 4, W>);
+        if (T == 4) return reinterpret_cast<const void*>(gemv_strip_kernel<BITS, SUB, NT, MODE, 4, W, APART>);
     return nullptr;
 }
 template <int BITS, int SUB, int W>
-const void* strip_kernel_m(int mode, int nt, int T) {
+const void* strip_kernel_m(int mode, int nt, int T, bool apart) {
     if constexpr (int_takes(BITS, SUB))
-        if (mode == kInt) return strip_kernel_t<BITS, SUB, 1, kInt, W>(T);
-    if (mode == kOne) return strip_kernel_t<BITS, SUB, 1, kOne, W>(T);
-    if (nt == 1) return strip_kernel_t<BITS, SUB, 1, kSeveral, W>(T);
-    if constexpr (W == 8) return strip_kernel_t<BITS, SUB, 2, kSeveral, W>(T);
+        if (mode == kInt) return strip_kernel_t<BITS, SUB, 1, kInt, W>(T, apart);
+    if (mode == kOne) return strip_kernel_t<BITS, SUB, 1, kOne, W>(T, apart);
+    if (nt == 1) return strip_kernel_t<BITS, SUB, 1, kSeveral, W>(T, apart);
+    if constexpr (W == 8) return strip_kernel_t<BITS, SUB, 2, kSeveral, W>(T, apart);
     return nullptr;
 }
 template <int BITS>
-const void* strip_kernel_bits(int sub, int mode, int nt, int T, int warps) {
-    if (warps == 8) return sub == 1 ? strip_kernel_m<BITS, 1, 8>(mode, nt, T) : strip_kernel_m<BITS, 4, 8>(mode, nt, T);
-    return sub == 1 ? strip_kernel_m<BITS, 1, 16>(mode, nt, T) : strip_kernel_m<BITS, 4, 16>(mode, nt, T);
+const void* strip_kernel_bits(int sub, int mode, int nt, int T, int warps, bool apart) {
+    if (warps == 8) return sub == 1 ? strip_kernel_m<BITS, 1, 8>(mode, nt, T, apart) : strip_kernel_m<BITS, 4, 8>(mode, nt, T, apart);
+    return sub == 1 ? strip_kernel_m<BITS, 1, 16>(mode, nt, T, apart) : strip_kernel_m<BITS, 4, 16>(mode, nt, T, apart);
 }
 
 }  // namespace

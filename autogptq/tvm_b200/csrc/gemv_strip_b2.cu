@@ -2,7 +2,7 @@
 #include "gemv_strip.cuh"
 
 namespace b200gptq {
-const void* gemv_strip_kernel_b2(int sub, int mode, int nt, int T, int warps) {
-    return strip_kernel_bits<2>(sub, mode, nt, T, warps);
+const void* gemv_strip_kernel_b2(int sub, int mode, int nt, int T, int warps, bool apart) {
+    return strip_kernel_bits<2>(sub, mode, nt, T, warps, apart);
 }
 }  // namespace b200gptq
