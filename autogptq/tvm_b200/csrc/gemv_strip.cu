@@ -74,14 +74,23 @@ int gemv_strip_prepare(GemvStripPlan* p, const int32_t* qweight, const int32_t* 
     // One CTA per SM: each takes the same whole number of strips.
     s.per_cta = (s.strips + sm_count() - 1) / sm_count();
     // One and two rows: planes of x where they pay and fit; one row: x kept whole.  Planes take a CTA longer to prepare than x in operand
-    // order and save on every strip and unit, so they pay from two strips on: 4 bits, two strips, one row 1.09 (4096 x 6144), 1.13
-    // (8192 x 8192) times as fast, groups of 32 1.02 and 1.02; 2 bits 1.15, 1.20; 3 bits, which have more pieces, 1.15, 1.10 and with
-    // rows picked one by one (a gather) 1.04, 1.00, 0.99 (9216 x 9216), two rows 1.00, 1.08, 0.92: three strips there (one row with
-    // a gather 1.08, two rows 1.10, 1.12, 0.93, 1.00).  One strip, 4 bits: one row of 4096 1.04, of 11008 1.11, with a gather 0.97 and 1.05,
-    // 2048 0.90; two rows with a gather 1.09 and 1.15, without 1.02 and 0.96.
+    // order and save on every strip and unit, so they pay where a warp has several units, or several strips of one.  Times as fast as
+    // fp16, in a chain of such layers and with a small kernel before each, as in a decode step:
+    //   two strips   K from 3072 on 1.00 to 1.24, but two rows in groups of 32 without a gather 0.87 to 0.98 for 8192 and 9216 (planes leave
+    //                room for eight warps, not sixteen); 2048 0.87 to 1.08, 1536 0.85 to 1.10, 1024 0.74 to 0.97; one row of 2 bits there
+    //                0.95 to 0.99, 1.00 to 1.18, 0.86 to 1.11; 3 bits, which have more pieces, one row 1.00 to 1.24, with rows picked one
+    //                by one (a gather) 0.99 to 1.04, two rows 0.92 to 1.08
+    //   three, more  K from 2048 on one row 0.93 to 1.53, two rows of 2 and 4 bits 0.96 to 1.46; 1024 0.86 to 1.15.  Two rows of 3 bits 0.79 to
+    //                0.97 up to K = 2048 and 1.02 to 1.16 above, but a step of a decoder (three layers, hidden size 4096, batch 2) takes 191 us with
+    //                three strips on planes and 182 without, and 201 with seven on planes and 206 without
+    //   one strip    4 bits, one row of 4096 1.02 and 1.03, of 11008 1.11, with a gather of 8192 1.07 and 4096 0.97 and 0.99; two rows with a
+    //                gather 1.05 to 1.11, without 1.02 and 0.96
     const int plane_bytes = (s.units * M * 4 * int_factors(sub) + 15) / 16 * 16 + s.units * M * (bits == 3 ? 5 : 4) * 128;
     const bool one_strip = bits == 4 && (M == 1 ? sub == 1 && s.units >= (gather ? 64 : 32) : gather && s.units >= 32);
-    const bool planes_pay = s.per_cta >= (bits != 3 || (M == 1 && !gather) ? 2 : 3) || one_strip;
+    const bool two_strips = bits == 3 ? M == 1 && !gather
+                          : (bits == 2 && M == 1) || (s.units > 16 && !(sub == 4 && M == 2 && !gather && s.units > 32));
+    const bool more_strips = bits == 3 ? M == 1 || s.per_cta > 4 : (bits == 2 && M == 1) || s.units >= 16;
+    const bool planes_pay = s.per_cta == 1 ? one_strip : (s.per_cta == 2 ? two_strips : more_strips);
     int mode = M <= 2 && int_takes(bits, sub) && planes_pay && plane_bytes <= 96 * 1024 ? kInt : (M == 1 && K <= 65536 ? kOne : kSeveral);
     const int nt = M <= 8 ? 1 : 2;
     s.rows_g = sub == 1 ? 1 : (s.spg == 1 ? 4 : (s.spg == 2 ? 2 : 3));
