@@ -694,8 +694,9 @@ int launch_gemm(const __half* x_for_tma, const int32_t* qweight, const int32_t* 
 // More than 16 rows, and the bit widths that only it has: the kernel for pairs of CTAs (gemm_pair.cu).  From 17 to 64 rows,
 // one CTA per tile against pairs: 4096 x 4096, 17 rows 16.4 and 11.2 us; 4096 x 12288, 64 rows 29.1 and 20.2; 11008 x 4096, 64
 // rows 35.2 and 20.6; 9216 x 9216, 3 bits, 24 rows 38.0 and 33.3; 9216 x 27648, 64 rows 106 and 84.  Up to 16 rows single
-// CTAs, two per SM, have stayed, though pairs took 11.2 us where they take 14 to 16 on 4096 x 4096: a layer's rows go to the
-// decode GEMV there, and what is left (direct calls, layers with a g_idx) has not been measured over sizes.
+// CTAs, two per SM, have stayed, though pairs take 9.1 us (32 rows) where they take 14 to 16 on 4096 x 4096: a layer's rows go to the
+// decode GEMV there, and what is left (direct calls, layers with a g_idx) has not been measured over sizes.  (These are times of
+// the pair kernel before it moved in units of 128 rows; it is faster now, 64 rows of 4096 x 12288 14.2.)
 static bool use_pair(int M, int bits) { return M > 16 || bits == 2 || bits == 8; }
 // (up to 128 rows as many runs as here; above, gemm_pair_plan weighs them against the rows of a tile)
 static GemmPairPlan pair_plan(int M, int N, int K) {

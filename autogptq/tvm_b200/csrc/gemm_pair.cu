@@ -22,7 +22,8 @@
 // the loop, and the threads that issue copies and products spent about 200 clk per 64 rows on barriers too.  So everything moves in
 // units of 128 rows, x and A (a stage) as well as the weights: half the hand-overs.  Clocks per 64 rows of K before and after:
 // 3 bits, 32 rows of 9216 x 9216 505 and 335; 4 bits in groups of 64, 77 rows of 11008 x 4096 465 and 360; 8 bits, 512 rows of
-// 4096 x 4096 550 and 480.  What is left is the arithmetic: without it 230, without the products 310.
+// 4096 x 4096 550 and 480 (with a second warp for the weights 310, 340 and 430).  What is left is the arithmetic: without it 230,
+// without the products 310.
 //
 // The pairs are persistent: the rings run on from one tile to the next, so only the drain of the accumulators stands
 // between two tiles (nothing, where two sets of accumulators fit: up to 128 rows).  A stage is released in both CTAs by one
@@ -43,12 +44,12 @@ namespace b200gptq {
 namespace {
 
 constexpr int BN = kPairColumns;         // columns per CTA
-constexpr int BK = kPairKTile;           // rows of K per stage
+constexpr int BK = kPairKTile;           // rows of K of a k-tile; a stage holds two
 constexpr int kGroups = kPairGroups, kGroupWarps = 4;
 constexpr int kFirstEpiWarp = 4, kEpiWarps = 8, kFirstWeightWarp = kFirstEpiWarp + kEpiWarps;
 constexpr int kThreads = 32 * (kFirstWeightWarp + kGroups * kGroupWarps);
 constexpr int kMaxStages = kPairMaxStages / 2, kMaxW = kPairMaxSlots;
-constexpr int kTmemCols = kPairTmemCols; // accumulators in columns [0, TN), 32 columns of A per stage behind them
+constexpr int kTmemCols = kPairTmemCols; // accumulators in columns [0, TN) of a set, 64 columns of A per stage behind them
 constexpr int kSmemMax = kPairSmem;
 constexpr int kStatusWord = kMaxCounters - 1;
 constexpr int kMaxSplits = 4;

@@ -12,18 +12,18 @@
 //    word-rows, strips} (128-byte swizzle), of the unit's scales and of its zero-points, one mbarrier per slot, no barrier of
 //    the CTA.  (16-byte cp.async by the lanes instead of the weight boxes: 13.0 against 7.0 us on 4096 x 12288, 4 bits;
 //    scales and zero-points loaded one unit ahead: 38 against 32 us without them on 9216 x 36864, 3 bits.)  The ring is
-//    filled before griddepcontrol.wait; with eight warps the footprint is half an SM, so under programmatic dependent
-//    launch the next launch's weights arrive while this one computes.
+//    filled before griddepcontrol.wait.  Eight warps with one or two strips leave room for a second CTA where K is short, so that under
+//    programmatic dependent launch the next launch's weights arrive while this one computes.
 //  * One row of x: a warp puts its whole slice of x into shared memory in the order of the B registers, once.  Several
 //    rows: copied with cp.async and permuted as they are read; all of x at once where it fits, else one to three units ahead
 //    (one unit ahead is an L2 latency per unit: 16 rows, 9216 x 9216, 3 bits 29 us, two ahead 21).  Which k a lane multiplies
 //    is free as long as x is read in the same order.
-//  * One or two rows, 2 to 4 bits, whole units per group: products on the integer tensor path.  A byte of weights is q << p, one
-//    AND per four fields and no shift; x is fixed point per unit (|X| < 2^22: exact for every
-//    element within 2^-12 of the unit's largest), shifted by what its weight byte lacks and split into four signed byte
-//    planes, which are columns of the B operand.  mma.sync m16n8k32 u8 x s8 costs what m16n8k16 f16 does and does twice
-//    the products; the fp16 form below needs 2.3 times the instructions (9216 x 36864, 3 bits: 35 against 42 us).  It
-//    is used where a CTA has more strips than rows of x: the planes take each CTA about as long as a strip saves.
+//  * One or two rows, 2 to 4 bits, whole units per group (4 bits: any groups): products on the integer tensor path.  A byte of weights
+//    is q << p, one AND per four fields and no shift; x is fixed point per unit, or per step where the groups of a unit are scaled apart
+//    (4 bits |X| < 2^26, exact for every element within 2^-16 of the largest; 2 and 3 bits 2^22 and 2^-12), shifted by what
+//    its weight byte lacks and split into four signed byte planes, which are columns of the B operand.  mma.sync m16n8k32
+//    u8 x s8 costs what m16n8k16 f16 does and does twice the products; the fp16 form below needs 2.3 times the instructions.
+//    Used where K is long enough for what the planes take to prepare (the plan in gemv_strip.cu has the measurements).
 //  * Otherwise fp16.  4- and 8-bit fields are used as fp16 subnormals: a field masked in place at bit p of its half IS q * 2^(p - 24), so
 //    unpacking is one AND (4 bits: and one shift per two words); the two positions of a nibble go to different
 //    accumulators and the power of two is applied to the result.  2- and 3-bit fields are ORed into the mantissa of a

@@ -21,7 +21,7 @@ constexpr int ring_in_whole_turns(int stages, int groups) { return stages / grou
 constexpr int kPairGroups = 4, kPairMinStages = 8;
 constexpr int pair_turns(int k_tiles) { return (k_tiles + 1) & ~1; }
 
-constexpr int kPairColumns = 128, kPairKTile = 64;         // columns per CTA, rows of K per stage
+constexpr int kPairColumns = 128, kPairKTile = 64;         // columns per CTA, rows of K of a k-tile (a stage holds two)
 constexpr int kPairTmemCols = 512;                         // accumulators, then 32 columns of A per k-tile of a stage
 constexpr int kPairSmem = 222 * 1024;
 constexpr int kPairMaxStages = 14, kPairMaxSlots = 16;

@@ -60,8 +60,8 @@ def row_rules(K: int, groupsize: int, has_g_idx: bool, uniform: bool):
     block; ``uniform`` says so of a ``g_idx``), and the largest batch that goes through the GEMV in one pass.
 
     9 to 16 rows: one pass of the streaming GEMV, where it takes the layer, beats the tensor-core kernel's 16-row tile, whose
-    weight warps are the bottleneck (9216 x 9216, 3 bits: 20 against 40 us; 4096 x 4096, 4 bits: 8.3 against 16.6).  It is also
-    where results change by a rounding: the GEMM multiplies the reference's fp16 ``scale * (q - zero)``, the GEMV the exact field
+    weight warps are the bottleneck (9216 x 9216, 3 bits: 21 against 40 us; 4096 x 4096, 4 bits: 7.9 against 16.6).  The kernel for
+    pairs of SMs has not been set against it (it takes 19.9 us for 32 rows of 9216 x 9216).  It is also where results change by a rounding: the GEMM multiplies the reference's fp16 ``scale * (q - zero)``, the GEMV the exact field
     and the scale in fp32 (2.1e-4 against 2.8e-4 from the exact product)."""
     whole_blocks = groupsize % 32 == 0
     gemm_ok = uniform if has_g_idx else whole_blocks

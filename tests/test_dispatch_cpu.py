@@ -116,7 +116,33 @@ def test_gemm_work_split_rule():
     assert ops.gemm_split(16, 9216, 27648, 3) == (1, 2)       # 216 tiles: one wave of two per SM instead of two waves
     assert ops.gemm_split(16, 4096, 12288, 8)[1] == 1         # 8 bits: pairs at any number of rows
     assert ops.gemm_split(16, 9216, 9216, 3)[0] > 1
-    assert ops.gemm_split(256, 4096, 4096, 4) == (1, 1)       # more than one row tile: never split
+    assert ops.gemm_split(256, 4096, 4096, 4) == (1, 1)       # more than one row tile: split where pairs of SMs stand idle
+    assert ops.gemm_split(256, 11008, 4096, 4) == (2, 1)
+    assert ops.gemm_split(129, 8192, 2048, 4) == (4, 1)
     assert ops.gemm_split(2048, 4096, 12288, 4) == (1, 1)
     with pytest.raises(ValueError):
         ops.gemm_split(16, 4095, 4096, 4)
+
+
+def test_runs_of_a_long_prompt_fit_their_pairs_and_their_scratch():
+    """Above 128 rows a split product has a tile per pair of SMs (the kernel's sum over runs takes one), runs of eight units of 128 rows or
+    more, and room for the sums of every run in the scratch; without runs only the counters and a copy of x are asked for."""
+    from autogptq.tvm_b200 import _lib, ops
+    split = 0
+    for K in (1024, 2048, 2080, 4096, 8192, 11008):
+        for N in (32, 1024, 2048, 4096, 6176, 12288):
+            for M in (129, 160, 200, 256, 257, 300, 448, 512, 700, 1024, 2048):
+                runs, per_sm = ops.gemm_split(M, K, N, 4)
+                base = 16384 + -(-2 * M * K // 256) * 256
+                extra = _lib.workspace_bytes(_lib.OP_GEMM, M, K, N, 4) - base
+                assert per_sm == 1 and 1 <= runs <= 4
+                if runs == 1:
+                    assert extra == 0
+                    continue
+                split += 1
+                rows = extra // (runs * N * 4)             # padded to whole tiles
+                assert extra == runs * rows * N * 4 and M <= rows < M + 256 and rows % 32 == 0
+                assert -(-K // 128) // runs >= 8
+                # the fewest tiles that so many padded rows can be (256 rows each) fit, with all their runs
+                assert -(-N // 256) * -(-rows // 256) * runs <= 74
+    assert split > 20

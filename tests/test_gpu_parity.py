@@ -174,8 +174,8 @@ def test_streaming_gemv_vs_oracle(bits, K, N, gs, bias, M):
 
 
 SINGLE_ROW_CASES = [
-    # bits, K, N, gs, act, bias : one row of x; the 3-bit ones run on the integer tensor path (x in fixed point per
-    # 128 rows of K, four byte planes), the 4-bit ones on fp16 fragments
+    # bits, K, N, gs, act, bias : one row of x; several strips of columns per CTA run on the integer tensor path (x in fixed
+    # point per 128 rows of K, four byte planes), the others on fp16 fragments
     (3, 4096, 11008, 128, True, False),      # config 1
     (3, 4096, 11008, 128, False, True),
     (4, 4096, 12288, 128, True, False),      # fused q|k|v
