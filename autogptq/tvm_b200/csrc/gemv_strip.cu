@@ -11,7 +11,7 @@ const void* gemv_strip_kernel_b4(int sub, int mode, int nt, int T, int warps, bo
 const void* gemv_strip_kernel_b8(int sub, int mode, int nt, int T, int warps, bool apart);
 
 struct GemvStripPlan {
-    int M, K, N, smem, warps;
+    int M, K, N, smem, warps;          // of a CTA: shared memory, warps (with idle ones)
     StripPlan plan;
     CUtensorMap tmap_w, tmap_s, tmap_z;
     const void* kernel;
@@ -144,12 +144,12 @@ int gemv_strip_prepare(GemvStripPlan* p, const int32_t* qweight, const int32_t* 
     if (!c.T) return B200GPTQ_ERR_TOO_LARGE;
     const int W = c.W, T = c.T;
     s.passes = (s.per_cta + T - 1) / T;
-    s.kept = c.bufs == 5;
-    s.x_bufs = s.kept ? 2 : c.bufs;
+    s.x_bufs = c.bufs == 5 ? 2 : c.bufs;
+    if (c.bufs != 5) mode = kTurns;
     const int longest = ((s.units + W - 1) / W) * s.passes;
     s.ring = c.ring < longest ? c.ring : longest;
     if (s.ring > kMaxRing) s.ring = kMaxRing;
-    p->warps = W;
+    p->warps = W + idle_warps(W, mode == kSeveral, nt);
     const bool apart = zeros_apart(T);
     p->smem = W * s.ring * (slot_bytes(bits, T) + const_bytes(bits, T, s.rows_g, apart)) + c.fixed;
     p->kernel = strip_kernel(bits, sub, mode, nt, T, W, apart);

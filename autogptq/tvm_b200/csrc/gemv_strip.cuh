@@ -357,8 +357,9 @@ __host__ __device__ constexpr int int_factors(int sub) { return sub == 1 ? 2 : 8
 __host__ __device__ constexpr int int_x_bits(int bits) { return bits == 4 ? 26 : 22; }
 __host__ __device__ constexpr bool int_takes(int bits, int sub) { return bits == 4 || (bits != 8 && sub == 1); }
 
-// How x meets the weights: several rows in fp16, one row in fp16, one or two rows as byte planes.
-enum { kSeveral = 0, kOne = 1, kInt = 2 };
+// How x meets the weights: several rows in fp16, every unit's x kept or a few units at a time in turn; one row in fp16; one or two rows as
+// byte planes.  (The first two in one form, with a branch per unit, were 3 % slower for nine rows and more.)
+enum { kSeveral = 0, kOne = 1, kInt = 2, kTurns = 3 };
 
 struct StripPlan {
     int units;        // units of 128 rows along K (the last one may be cut)
@@ -370,8 +371,7 @@ struct StripPlan {
     int groups;
     unsigned int spg_inv;   // ceil(2^32 / spg)
     int rows_g;       // groups whose constants a slot holds
-    int kept;         // several rows: every unit's x has a place of its own
-    int x_bufs;       // otherwise: places of a warp, 2..4, used in turn
+    int x_bufs;       // several rows of which x is not kept: places of a warp, 2..4, used in turn
     int gather;       // x is picked through x_perm from a copy of it in shared memory
     int xact;         // activation applied to x as it is read: 0 none, 1 SwiGLU, 2 ReLU
 };
@@ -400,14 +400,16 @@ __device__ __forceinline__ uint32_t act_swiglu2(uint32_t gv, uint32_t uv) {
 }
 
 // SUB: groups of a unit that are scaled apart (1: a group is a whole number of units).  NT: rows of x / 8.
-// MODE: kSeveral, kOne, kInt.  T: strips of a pass.  W: warps of a CTA.
-// Registers: what an SM has beside a CTA of eight warps (22 528 at 168) takes no second one, mostly.  With 128 two fit where K is short,
-// and the next launch's weights arrive beside the current one: 1024 x 7168 alone, 3 bits, two rows 3.1 us for 3.5, but 1024 x 3072 in
-// groups of 32, three rows with a gather 3.3 for 2.9 (two share an SM while others idle), a step of a decoder with hidden size 1024, batches of 4
-// and 8, 253 and 241 us for 237 and 232, and 9216 x 36864 6 % longer.  Sixteen warps, or sixteen rows of x, leave 4096 or 8192 of an SM's for
-// the kernel that comes next.  With all of them taken, the gather of x between two products of 8 rows, 9216 x 9216, 3 bits, only
-// started when a CTA ended, and the next product's weights after that: 22 us against 16.6 (and 14.3 against 14.1 where
-// nothing is gathered).
+// MODE: kSeveral, kTurns, kOne, kInt.  T: strips of a pass.  W: warps of a CTA.
+// Registers: a second CTA of eight warps would fit on an SM where K is short and two to eight rows of x leave registers (128 and less), and
+// the next launch's weights would arrive beside the current one.  That serves such a layer alone (1024 x 7168, 3 bits, two rows 3.1 us for
+// 3.5), but two CTAs share an SM while others idle (1024 x 3072, 2 bits, three rows 2.6 us for 2.4), and with a small kernel before each layer,
+// as in a decode step, it loses: 1024 x 7424, 4 bits, 8 rows 4.8 us for 4.1; a step of a decoder with hidden size 1024, batches of 4 and 8,
+// 253 and 241 us for 237 and 232.  So these launches carry warps that end at once, for the registers they hold.  Sixteen warps, or
+// sixteen rows of x, leave 4096 or 8192 of an SM's for the kernel that comes next.  With all of them taken, the gather of x between
+// two products of 8 rows, 9216 x 9216, 3 bits, only started when a CTA ended, and the next product's weights after that: 22 us
+// against 16.6 (and 14.3 against 14.1 where nothing is gathered).
+__host__ __device__ constexpr int idle_warps(int W, bool kept, int nt) { return W == 8 && kept && nt == 1 ? 3 : 0; }
 // APART: a box for the zero-points of each group.
 template <int BITS, int SUB, int NT, int MODE, int T, int W, bool APART>
 __global__ void __maxnreg__(W == 16 ? 120 : NT == 1 ? 168 : 224)
@@ -417,7 +419,7 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                   unsigned int* __restrict__ status) {
     using L = Layout<BITS, SUB == 1>;
     using I = IntLayout<BITS, SUB == 1 || BITS != 4>;
-    constexpr bool ONE = MODE == kOne, INT = MODE == kInt, ROWS = MODE == kSeveral;
+    constexpr bool ONE = MODE == kOne, INT = MODE == kInt, KEPT = MODE == kSeveral, TURNS = MODE == kTurns, ROWS = KEPT || TURNS;
     static_assert(!INT || (NT == 1 && int_takes(BITS, SUB)), "not a case of the integer path");
     constexpr int STRIP_BYTES = L::kRows * 128, STEPS = 4 / SUB, SLOT = slot_bytes(BITS, T);
     constexpr int NC = ROWS ? 2 : 1;             // rows of x per lane and n-tile that exist
@@ -427,6 +429,7 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
 
     const int M = ONE ? 1 : M_rows;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, j = lane & 3;
+    if (idle_warps(W, KEPT, NT) && warp >= W) return;     // (before any barrier)
     const int R = plan.ring;
     // The runs start evenly over the columns and all have per_cta strips: neighbours may share a strip, both then write
     // the same bits.  (A grid of fewer, disjoint runs left SMs idle, and the next launch, which becomes resident beside
@@ -445,8 +448,8 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     // one row: [unit][quad lane][16 registers]; planes: [unit][step]..., then (factor, sum) [unit][row]; several rows:
     // [unit][row][natural halves], or a few units in turn per warp
     const int unit_x = ONE ? kUnit * 2 : (INT ? int_unit_bytes<BITS>(M) : M * kXPitch * 2);
-    const int x_units = ROWS && !plan.kept ? plan.x_bufs * W : plan.units;
-    uint8_t* p_x = base_x + (size_t)(ROWS && !plan.kept ? plan.x_bufs * warp : u_begin) * unit_x;
+    const int x_units = TURNS ? plan.x_bufs * W : plan.units;
+    uint8_t* p_x = base_x + (size_t)(TURNS ? plan.x_bufs * warp : u_begin) * unit_x;
     constexpr int FACTORS = int_factors(SUB);
     float* p_f = reinterpret_cast<float*>(base_x + (size_t)plan.units * unit_x) + (size_t)u_begin * M * FACTORS;
     uint8_t* base_r = base_x + (size_t)x_units * unit_x + (INT ? (plan.units * M * FACTORS * 4 + 15) / 16 * 16 : 0);
@@ -547,7 +550,7 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                 *index_slot(i) = make_uint4(pack2(a.x, a.y), pack2(a.z, a.w), pack2(b.x, b.y), pack2(b.z, b.w));
             }
         }
-    if constexpr (ROWS)
+    if constexpr (KEPT)
         if (gather) {                              // of several rows: in the place of the first row's four values
 #pragma unroll 2
             for (int i = lane; i < nu * 32; i += 32) {
@@ -623,14 +626,14 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    if (async_x && plan.kept)                      // (waited for unit by unit, in the first pass)
+    if (KEPT && async_x)                      // (waited for unit by unit, in the first pass)
         for (int u = 0; u < nu; ++u) fetch_x(u, u);
     if (gather || (!ROWS && staged)) {
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         if (gather) __syncthreads();
         else __syncwarp();
     }
-    if (ROWS && !async_x && plan.kept) {
+    if (KEPT && !async_x) {
         for (int i = lane; i < nu * 32; i += 32) {
             uint2* to = reinterpret_cast<uint2*>(p_x + (size_t)(i >> 5) * unit_x + 8 * lane);
             const int k = u_begin * kUnit + 4 * i;
@@ -839,7 +842,7 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     static_assert(L::kRows % 4 == 0, "strips start on lines 0 or 4 of the swizzle pattern");
 
     int slot = 0, parity = 0, buf = 0;
-    if (ROWS && async_x && !plan.kept && nu > 0)          // x that is not kept: x_bufs - 1 units (no more than nu) ahead
+    if (TURNS && async_x && nu > 0)          // x that is not kept: x_bufs - 1 units (no more than nu) ahead
         for (int i = 0; i < plan.x_bufs - 1; ++i) fetch_x(i, i);
     for (int p = 0, win = 0; p < plan.passes; ++p, win = min(win + T, last_window)) {
 #pragma unroll 1
@@ -922,8 +925,8 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                     b[0][4 * s] = v.x; b[0][4 * s + 1] = v.y; b[0][4 * s + 2] = v.z; b[0][4 * s + 3] = v.w;
                 }
             } else {
-                __half* xs = reinterpret_cast<__half*>(p_x + (size_t)(plan.kept ? u : buf) * unit_x);
-                if (plan.kept) {
+                __half* xs = reinterpret_cast<__half*>(p_x + (size_t)(KEPT ? u : buf) * unit_x);
+                if constexpr (KEPT) {
                     if (async_x && p == 0) {
                         // this unit's x; the copies of those behind it go on (8 rows of 4096 x 12288: all of x first 10.1 us, so 9.2)
                         const int behind = nu - 1 - u;
@@ -1135,8 +1138,10 @@ const void* strip_kernel_m(int mode, int nt, int T, bool apart) {
     if constexpr (int_takes(BITS, SUB))
         if (mode == kInt) return strip_kernel_t<BITS, SUB, 1, kInt, W>(T, apart);
     if (mode == kOne) return strip_kernel_t<BITS, SUB, 1, kOne, W>(T, apart);
-    if (nt == 1) return strip_kernel_t<BITS, SUB, 1, kSeveral, W>(T, apart);
-    if constexpr (W == 8) return strip_kernel_t<BITS, SUB, 2, kSeveral, W>(T, apart);
+    if (nt == 1)
+        return mode == kTurns ? strip_kernel_t<BITS, SUB, 1, kTurns, W>(T, apart) : strip_kernel_t<BITS, SUB, 1, kSeveral, W>(T, apart);
+    if constexpr (W == 8)
+        return mode == kTurns ? strip_kernel_t<BITS, SUB, 2, kTurns, W>(T, apart) : strip_kernel_t<BITS, SUB, 2, kSeveral, W>(T, apart);
     return nullptr;
 }
 template <int BITS>
