@@ -12,8 +12,7 @@
 //    word-rows, strips} (128-byte swizzle), of the unit's scales and of its zero-points, one mbarrier per slot, no barrier of
 //    the CTA.  (16-byte cp.async by the lanes instead of the weight boxes: 13.0 against 7.0 us on 4096 x 12288, 4 bits;
 //    scales and zero-points loaded one unit ahead: 38 against 32 us without them on 9216 x 36864, 3 bits.)  The ring is
-//    filled before griddepcontrol.wait.  Eight warps with one or two strips leave room for a second CTA where K is short, so that under
-//    programmatic dependent launch the next launch's weights arrive while this one computes.
+//    filled before griddepcontrol.wait: under programmatic dependent launch while the kernel in front ends, where that leaves the SM room.
 //  * One row of x: a warp puts its whole slice of x into shared memory in the order of the B registers, once.  Several
 //    rows: copied with cp.async and permuted as they are read; all of x at once where it fits, else one to three units ahead
 //    (one unit ahead is an L2 latency per unit: 16 rows, 9216 x 9216, 3 bits 29 us, two ahead 21).  Which k a lane multiplies
