@@ -61,8 +61,27 @@ _SIGNATURES = {
     "b200gptq_dense_gemv": (_c_int, [_c_void_p] * 3 + [_c_int] * 3 + [_c_void_p]),
     "b200gptq_pick_local": (_c_int, [_c_void_p, _c_int, _c_int, _c_int, ctypes.c_longlong, _c_int, _c_int, _c_void_p,
                                      _c_void_p, ctypes.c_longlong, _c_void_p, _c_void_p]),
+    "b200gptq_step_plan_bytes": (_c_size_t, [_c_void_p]),
+    "b200gptq_step_table_bytes": (_c_size_t, [_c_int]),
+    "b200gptq_step_plan_create": (_c_int, [_c_void_p] * 4),
+    "b200gptq_step_plan_run": (_c_int, [_c_void_p] * 5),
+    "b200gptq_step_plan_destroy": (None, [_c_void_p]),
     "b200gptq_pick_final": (_c_int, [_c_void_p, _c_int, _c_int, _c_void_p, ctypes.c_longlong, _c_void_p, _c_void_p]),
 }
+
+
+class StepLinear(ctypes.Structure):
+    _fields_ = [(n, _c_void_p) for n in ("qweight", "qzeros", "scales", "bias", "x_perm")]
+
+
+class StepLayer(ctypes.Structure):
+    _fields_ = [("linear", StepLinear * 4), ("norm_w", _c_void_p * 2), ("norm_b", _c_void_p * 2), ("k_cache", _c_void_p),
+                ("v_cache", _c_void_p)]
+
+
+class StepShape(ctypes.Structure):
+    _fields_ = ([(n, _c_int) for n in ("layers", "batch", "hidden", "heads", "inter", "max_seq", "bits", "group_size", "gated", "rms", "rope")]
+                + [("eps", ctypes.c_float), ("scale", ctypes.c_float)] + [(n, _c_void_p) for n in ("cos_t", "sin_t", "pos")])
 
 
 def _load() -> ctypes.CDLL:

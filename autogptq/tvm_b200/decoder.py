@@ -202,6 +202,9 @@ class GPTQDecoder:
         self.tokens = torch.zeros(batch, dtype=torch.long, device=dev)
         self.positions = torch.arange(cfg.max_seq, device=dev)
         self.graph: Optional[torch.cuda.CUDAGraph] = None
+        self.one_launch = True       # False: the kernels of a decode step's layers are launched one by one
+        self._plan = None            # (what it was made from, ops.StepPlan or None)
+        self._graph_plan = None      # the one whose memory the captured step uses
         self._pos_host = 0   # host copy of the position, for range checks
 
     # ---- pieces ----
@@ -363,15 +366,56 @@ class GPTQDecoder:
         self.tokens.copy_(self._sample(x[:, -1]))
         self.pos.add_(1)
 
+    def _step_plan(self) -> Optional[ops.StepPlan]:
+        """The layers of a decode step as one launch, for one sequence on one GPU and layers that the kernel takes; None where the
+        kernels of a layer are launched one by one.  Everything that the plan points to is looked at in every step that is not replayed."""
+        cfg = self.cfg
+        if self.world > 1 or self.batch != 1 or not self.one_launch:
+            return None
+        key, layers = [], []
+
+        def plain(t, *shape):
+            return t is not None and t.dtype is torch.float16 and t.shape == shape and t.is_contiguous() and t.device == self.pos.device
+
+        H, rms = cfg.hidden, cfg.arch == "llama"
+        sizes = ((H, 3 * H), (H, H), (H, (2 if rms else 1) * cfg.inter), (cfg.inter, H))
+        for L in self.layers:
+            linears = []
+            for m, (K, N) in zip((L.qkv, L.o, L.up, L.down), sizes):
+                if (type(m) is not QuantLinear or m._forward_hooks or m._forward_pre_hooks or m.gemv_tuning is not None
+                        or m.exchange is not None or (m.bits, m.groupsize, m.infeatures, m.outfeatures) != (cfg.bits, cfg.group_size, K, N)):
+                    return None
+                if not m._ready():
+                    m.post_init()
+                if m._g_idx_run is not None:
+                    return None
+                linears.append((m._qweight_run, m.qzeros, m.scales, m.bias, m._x_perm))
+            cache = (1, cfg.heads, cfg.max_seq, cfg.head_dim)
+            norms = (L.norm1_w, L.norm2_w) + (() if rms else (L.norm1_b, L.norm2_b))
+            if not (all(plain(t, H) for t in norms) and plain(L.k_cache, *cache) and plain(L.v_cache, *cache)):
+                return None
+            layers.append((linears, norms[:2], (None, None) if rms else norms[2:], L.k_cache, L.v_cache))
+            key.extend(None if t is None else t.data_ptr() for t in sum(linears, ()) + norms + (L.k_cache, L.v_cache))
+        key.extend(t.data_ptr() for t in (self.cos, self.sin, self.pos))
+        if self._plan is None or self._plan[0] != key:
+            if torch.cuda.is_current_stream_capturing():
+                return None                        # (a plan is made outside)
+            self._plan = (key, ops.StepPlan.make(layers, H, cfg.heads, cfg.inter, cfg.bits, cfg.group_size, rms, 1e-6 if rms else 1e-5,
+                                                 self.cos, self.sin, self.pos))
+        return self._plan[1]
+
     def _decode_step_fused(self):
-        """One token per sequence with the fused helper kernels: per layer 5 small launches + 4 linears."""
+        """One token per sequence: all layers in one launch where :meth:`_step_plan` has one, else the fused helper kernels, per
+        layer 5 small launches + 4 linears."""
         cfg, B = self.cfg, self.batch
         hd, rms = cfg.head_dim, cfg.arch == "llama"
         eps = 1e-6 if rms else 1e-5
         x = self._embed(self.tokens, self.pos).reshape(B, cfg.hidden).contiguous()
         h = torch.empty_like(x)
         delta = None   # output of the previous row-parallel linear, added to the residual by the next norm
-        for L in self.layers:
+        plan = self._step_plan()
+        done = plan is not None and plan.run(x)
+        for L in () if done else self.layers:
             ops.add_norm(x, delta, L.norm1_w, L.norm1_b, h, eps, rms)
             qkv = L.qkv(h)
             att = torch.empty((B, L.heads_local * hd), dtype=torch.float16, device=self.device)
@@ -422,6 +466,7 @@ class GPTQDecoder:
         self.graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(self.graph):
             self._decode_step()
+        self._graph_plan = self._plan
         self.pos.copy_(saved_pos)
         self.tokens.copy_(saved_tok)
 

@@ -467,3 +467,58 @@ def dense_gemv(x, w, out=None):
         st = _lib.lib.b200gptq_dense_gemv(_ptr(x), _ptr(w), _ptr(out), x.shape[0], x.shape[1], w.shape[0], _stream(x.device))
     _lib.check(st, "b200gptq_dense_gemv")
     return out
+
+
+class StepPlan:
+    """The decoder layers of one decode step of one sequence as one launch (``b200gptq_step_plan_*``), prepared for fixed tensors, which
+    it keeps."""
+
+    def __init__(self, handle: int, memory, keep):
+        self._handle, self._memory, self._keep = handle, memory, keep
+
+    @classmethod
+    def make(cls, layers, hidden: int, heads: int, inter: int, bits: int, group_size: int, llama: bool, eps: float, cos, sin, pos):
+        """``layers``: per layer ``(linears, norm_w, norm_b, k_cache, v_cache)``, four linears ``(qweight, qzeros, scales, bias, x_perm)`` in their
+        run-time layout.  None for shapes that the kernel does not take."""
+        import ctypes
+        device, max_seq, hd = pos.device, layers[0][3].shape[2], hidden // heads
+        shape = _lib.StepShape(len(layers), 1, hidden, heads, inter, max_seq, bits, group_size, int(llama), int(llama), int(llama), eps,
+                               1.0 / (hd ** 0.5), _ptr(cos), _ptr(sin), _ptr(pos))
+        need = _lib.lib.b200gptq_step_plan_bytes(ctypes.byref(shape))
+        if need == 0:
+            return None
+        table = (_lib.StepLayer * len(layers))()
+        for to, (linears, norm_w, norm_b, k_cache, v_cache) in zip(table, layers):
+            for i, tensors in enumerate(linears):
+                to.linear[i] = _lib.StepLinear(*(_ptr(t) for t in tensors))
+            for i in range(2):
+                to.norm_w[i], to.norm_b[i] = _ptr(norm_w[i]), _ptr(norm_b[i])
+            to.k_cache, to.v_cache = _ptr(k_cache), _ptr(v_cache)
+        host = torch.zeros(_lib.lib.b200gptq_step_table_bytes(len(layers)), dtype=torch.uint8)
+        handle = ctypes.c_void_p()
+        with torch.cuda.device(device):
+            st = _lib.lib.b200gptq_step_plan_create(ctypes.byref(shape), table, host.data_ptr(), ctypes.byref(handle))
+            if st in (-4, -8):       # (a tensor that is not aligned, a device that cannot hold a CTA per SM)
+                return None
+            _lib.check(st, "b200gptq_step_plan_create")
+            plan = cls(handle.value, torch.zeros(need, dtype=torch.uint8, device=device), (layers, cos, sin, pos))
+            plan._memory[:host.numel()].copy_(host)
+        return plan
+
+    def run(self, x) -> bool:
+        """``x`` fp16 ``[1, hidden]``: the residual stream, in place.  False where the device cannot hold all CTAs now; nothing was
+        launched."""
+        _need_cuda("x", x, torch.float16)
+        ws = get_workspace(x.device, 1)
+        with torch.cuda.device(x.device):
+            st = _lib.lib.b200gptq_step_plan_run(self._handle, self._memory.data_ptr(), _ptr(x), _ptr(ws), _stream(x.device))
+        if st == -8:
+            return False
+        _lib.check(st, "b200gptq_step_plan_run")
+        return True
+
+    def __reduce__(self):            # (it holds addresses of this process: a copy makes its own)
+        return type(None), ()
+
+    def __del__(self):
+        _lib.lib.b200gptq_step_plan_destroy(self._handle)

@@ -423,6 +423,48 @@ B200GPTQ_API int b200gptq_pick_local(const void* logits, int rows, int ld, int v
 B200GPTQ_API int b200gptq_pick_final(const void* slots, int rows, int world, long long* tokens, long long max_token,
                                      long long* pos_inc, void* stream);
 
+/*
+ * The decoder layers of one decode step of one sequence as ONE cooperative launch: per layer norm, q|k|v, rotary embedding +
+ * cache write + attention, output projection, residual sum, norm, first FFN linear, activation, second FFN linear, residual sum: the
+ * arithmetic of the helpers above and of b200gptq_gemv.  The reference has no counterpart (its loop is transformers' generate(),
+ * end2end/autogptq-generation-inference-benchmark.py:26-49).
+ *
+ * shape     layers, batch (1), hidden = heads * {64, 128} (up to 6144) and inter, both multiples of 128, bits 2, 3 or 4, group_size a
+ *           multiple of 128 or at least K; gated: SwiGLU with the first FFN linear [gate | up], else ReLU; rms: RMSNorm, else
+ *           LayerNorm; rope: rotary embedding with cos_t / sin_t [max_seq, hd / 2]; pos: device int64, the position of the token (outside the
+ *           caches: they are left alone and the attention's output is zero).
+ * layers    per layer linear[4] = q|k|v, output projection, first and second FFN linear in their run-time layout (group k / group_size;
+ *           x_perm[k]: the row of x that row k multiplies, NULL where rows are not re-ordered, which those of the second FFN linear never
+ *           are), norm weights (and offsets, LayerNorm), caches [1, heads, max_seq, hd].
+ *   b200gptq_step_plan_bytes    device bytes that a plan needs (0: not a shape of this kernel)
+ *   b200gptq_step_table_bytes   host bytes of the layer table that b200gptq_step_plan_create fills; the caller copies it to the start of
+ *                               the plan's device memory (256-byte aligned, otherwise zero)
+ *   b200gptq_step_plan_run      x fp16 [hidden] in place.  `workspace`: scratch whose status word a wait that runs out raises
+ *                               (b200gptq_workspace_status).  B200GPTQ_ERR_TOO_LARGE: the device cannot hold a CTA per SM for this
+ *                               process, nothing was launched.  Launches of one plan must be ordered: they share its memory.
+ */
+typedef struct {
+    const void *qweight, *qzeros, *scales, *bias;
+    const int32_t* x_perm;
+} b200gptq_step_linear;
+typedef struct {
+    b200gptq_step_linear linear[4];
+    const void *norm_w[2], *norm_b[2];
+    void *k_cache, *v_cache;
+} b200gptq_step_layer;
+typedef struct {
+    int layers, batch, hidden, heads, inter, max_seq, bits, group_size, gated, rms, rope;
+    float eps, scale;
+    const void *cos_t, *sin_t, *pos;
+} b200gptq_step_shape;
+typedef struct b200gptq_step_plan b200gptq_step_plan;
+B200GPTQ_API size_t b200gptq_step_plan_bytes(const b200gptq_step_shape* shape);
+B200GPTQ_API size_t b200gptq_step_table_bytes(int layers);
+B200GPTQ_API int b200gptq_step_plan_create(const b200gptq_step_shape* shape, const b200gptq_step_layer* layers, void* table,
+                                           b200gptq_step_plan** out);
+B200GPTQ_API int b200gptq_step_plan_run(const b200gptq_step_plan* plan, void* memory, void* x, void* workspace, void* stream);
+B200GPTQ_API void b200gptq_step_plan_destroy(b200gptq_step_plan* plan);
+
 #ifdef __cplusplus
 }
 #endif

@@ -1,0 +1,128 @@
+"""The decoder layers of a step in one launch (``b200gptq_step_plan_*``) against the kernels launched one by one."""
+import copy
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+if torch.cuda.is_available():
+    from autogptq.tvm_b200 import decoder, ops
+    DEV = torch.device("cuda:0")
+
+
+def _model(arch, bits, act, layers, hidden, heads, inter, prompt, group=128, batch=1, max_seq=None):
+    cfg = decoder.DecoderConfig(arch=arch, layers=layers, hidden=hidden, heads=heads, inter=inter, vocab=1000, bits=bits,
+                                group_size=group, desc_act=act, max_seq=max_seq or prompt + 8)
+    text = torch.randint(0, cfg.vocab, (batch, prompt + 4), generator=torch.Generator().manual_seed(prompt)).to(DEV)
+    return decoder.GPTQDecoder(cfg, batch=batch, device=DEV), text
+
+
+def _steps(m, text, prompt, one_launch, steps=4):
+    m.one_launch = one_launch
+    m.prefill(text[:, :prompt].contiguous())
+    logits = []
+    for i in range(steps):
+        m.tokens.copy_(text[:, prompt + i])
+        m._decode_step()
+        logits.append(m.last_logits.double().clone())
+    ops.check_status(DEV)
+    return torch.stack(logits), [(L.k_cache.clone(), L.v_cache.clone()) for L in m.layers]
+
+
+def _close(got, want, layers):
+    """Both round to fp16 at the same places, some eight per layer, and sum in fp32 in another order: a rounding may go the other way, by
+    2^-11 of the value, each on its own."""
+    assert float((got - want).norm() / want.norm()) <= (8 * layers) ** 0.5 * 2.0 ** -11
+
+
+@pytest.mark.parametrize("shape", [
+    ("llama", 4, False, 2, 256, 2, 512, 12),             # units for two of the eight warps
+    ("llama", 4, False, 3, 1024, 8, 2816, 40),           # half a slot; 22 units, the second slot cut
+    ("llama", 4, True, 2, 4096, 32, 11008, 2),           # gather of x; pairs of strips, three per CTA
+    ("llama", 4, False, 2, 6144, 48, 6272, 9),           # as many slots as are read at once; an odd number of units
+    ("llama", 3, True, 2, 2048, 16, 5504, 400),          # three CTAs per head; three slots
+    ("llama", 3, False, 2, 512, 8, 1024, 193),           # zero-points that start inside a 16-byte piece; two CTAs per head, 64 dims
+    ("llama", 2, True, 2, 1024, 8, 1152, 30),
+    ("opt", 3, True, 2, 1024, 16, 4096, 1),
+    ("opt", 4, False, 2, 1024, 8, 2048, 700, 256),       # two units per group; four CTAs per head
+    ("opt", 4, True, 2, 768, 12, 3072, 65, 384),         # three units per group
+    ("opt", 2, False, 1, 512, 4, 640, 5),
+])
+def test_one_launch_computes_what_the_kernels_compute(shape):
+    prompt, layers = shape[7], shape[3]
+    m, text = _model(*shape)
+    want, caches = _steps(m, text, prompt, False)
+    got, own = _steps(m, text, prompt, True)
+    assert m._plan is not None and m._plan[1] is not None, "a shape that the kernel takes"
+    _close(got, want, layers)
+    for (k0, v0), (k1, v1) in zip(caches, own):
+        _close(k1.double(), k0.double(), layers)
+        _close(v1.double(), v0.double(), layers)
+        assert torch.equal(k0[:, :, prompt + 4:], k1[:, :, prompt + 4:])
+    again, _ = _steps(m, text, prompt, True)
+    assert torch.equal(again, got), "the same bits every time"
+    # captured, and several steps in a row on the caller's stream
+    m.prefill(text[:, :prompt].contiguous())
+    m.capture()
+    for i in range(4):
+        m.tokens.copy_(text[:, prompt + i])
+        m.graph.replay()
+        assert torch.equal(m.last_logits.double(), got[i])
+
+
+def test_what_the_kernel_does_not_take_goes_kernel_by_kernel():
+    for args, kw in ((("llama", 4, False, 1, 256, 2, 512, 12), dict(batch=2)), (("llama", 8, False, 1, 256, 2, 512, 12), {}),
+                     (("opt", 3, False, 1, 320, 5, 512, 12), dict(group=64))):
+        m, text = _model(*args, **kw)
+        m.prefill(text[:, :12].contiguous())
+        m._decode_step()
+        assert m._step_plan() is None
+    # a hook sees every call of its layer; without it the plan is back
+    m, text = _model("llama", 4, False, 2, 256, 2, 512, 12)
+    want, _ = _steps(m, text, 12, True)
+    calls = []
+    hook = m.layers[1].o.register_forward_hook(lambda *a: calls.append(1))
+    _steps(m, text, 12, True)
+    assert len(calls) == 5                               # the prompt and four steps
+    hook.remove()
+    got, _ = _steps(m, text, 12, True)
+    assert torch.equal(got, want)
+
+
+def test_replaced_tensors_are_followed():
+    m, text = _model("llama", 4, True, 2, 512, 4, 1024, 20)
+    first, _ = _steps(m, text, 20, True)
+    kept = m._plan[1]
+    m.layers[0].down.scales = m.layers[0].down.scales * 2
+    m.layers[1].norm1_w = m.layers[1].norm1_w * 0.5
+    want, _ = _steps(m, text, 20, False)
+    got, _ = _steps(m, text, 20, True)
+    assert m._plan[1] is not kept and not torch.equal(got, first)
+    _close(got, want, 2)
+    m.layers[1].up.qzeros.zero_()                        # in place: read as it is
+    want, _ = _steps(m, text, 20, False)
+    got, _ = _steps(m, text, 20, True)
+    _close(got, want, 2)
+
+
+def test_a_copy_makes_a_plan_of_its_own():
+    m, text = _model("llama", 4, False, 2, 512, 4, 1024, 20)
+    want, _ = _steps(m, text, 20, True)
+    c = copy.deepcopy(m)
+    assert c._plan[1] is None
+    assert torch.equal(_steps(c, text, 20, True)[0], want) and c._plan[1] is not m._plan[1]
+
+
+def test_a_position_outside_the_caches_writes_none():
+    m, text = _model("llama", 4, False, 2, 256, 2, 512, 12)
+    _steps(m, text, 12, True)
+    before = [(L.k_cache.clone(), L.v_cache.clone()) for L in m.layers]
+    for pos in (m.cfg.max_seq, -1):
+        m.pos.fill_(pos)
+        x = torch.ones(1, 256, dtype=torch.float16, device=DEV)
+        assert m._step_plan().run(x)
+        for L, (k, v) in zip(m.layers, before):
+            assert torch.equal(L.k_cache, k) and torch.equal(L.v_cache, v)
+        assert bool(torch.isfinite(x).all())
+    ops.check_status(DEV)
