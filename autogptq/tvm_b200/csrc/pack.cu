@@ -14,6 +14,7 @@
 #include <cuda_bf16.h>
 
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -136,6 +137,42 @@ __device__ __noinline__ void pack_divided(const T* row, const int* gr, const flo
     for (int i = 0; i < BITS; ++i) out[(size_t)i * N] = (int32_t)w[i];
 }
 
+// scales_out and qzeros of one strip of 32 columns.  smem: 2 * 128 * kPackPitch floats
+template <int BITS, int THREADS>
+__device__ __forceinline__ void pack_constants(const float* __restrict__ scales, const float* __restrict__ zeros, int G, int N, int strip,
+                                               int32_t* __restrict__ qzeros, __half* __restrict__ scales_out, unsigned char* smem) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n0 = strip * kPackCols, n = n0 + lane;
+    // scales and zero-points of the strip, 128 groups at a time: read along the groups, written along the columns
+    constexpr int GT = 128;
+    float* st = reinterpret_cast<float*>(smem);
+    float* zt = st + GT * kPackPitch;
+    for (int g0 = 0; g0 < G; g0 += GT) {
+        const int count = min(GT, G - g0);
+        for (int g = lane; g < count; g += 32)
+#pragma unroll
+            for (int r = 0; r < kPackCols; r += THREADS / 32) {
+                const size_t at = (size_t)(n0 + r + warp) * G + g0 + g;
+                st[g * kPackPitch + r + warp] = scales[at];
+                zt[g * kPackPitch + r + warp] = zeros[at];
+            }
+        __syncthreads();
+        for (int g = warp; g < count; g += THREADS / 32)
+            scales_out[(size_t)(g0 + g) * N + n] = __float2half_rn(st[g * kPackPitch + lane]);
+        for (int g = threadIdx.x; g < count; g += THREADS) {
+            uint32_t w[BITS];
+#pragma unroll
+            for (int i = 0; i < BITS; ++i) w[i] = 0u;
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+                pack_insert<BITS>(w, j, (uint32_t)(long long)(zt[g * kPackPitch + j] - 1.f));
+#pragma unroll
+            for (int i = 0; i < BITS; ++i)
+                qzeros[(size_t)(g0 + g) * (N / 32 * BITS) + strip * BITS + i] = (int32_t)w[i];
+        }
+        __syncthreads();
+    }
+}
+
 template <int BITS, typename T>
 __global__ void __launch_bounds__(kPackThreads, kPackCtas)
 pack_linear_kernel(const T* __restrict__ weight, const float* __restrict__ scales, const float* __restrict__ zeros,
@@ -169,35 +206,7 @@ pack_linear_kernel(const T* __restrict__ weight, const float* __restrict__ scale
         return k < K ? min(max(__ldg(g_idx + k), 0), G - 1) : 0;
     };
     if (blockIdx.y == gridDim.y - 1) {
-        // scales and zero-points of the strip, 128 groups at a time: read along the groups, written along the columns
-        constexpr int GT = 128;
-        float* st = reinterpret_cast<float*>(pack_smem);
-        float* zt = st + GT * kPackPitch;
-        for (int g0 = 0; g0 < G; g0 += GT) {
-            const int count = min(GT, G - g0);
-            for (int g = lane; g < count; g += 32)
-#pragma unroll
-                for (int r = 0; r < kPackCols; r += kPackThreads / 32) {
-                    const size_t at = (size_t)(n0 + r + warp) * G + g0 + g;
-                    st[g * kPackPitch + r + warp] = scales[at];
-                    zt[g * kPackPitch + r + warp] = zeros[at];
-                }
-            __syncthreads();
-            for (int g = warp; g < count; g += kPackThreads / 32)
-                scales_out[(size_t)(g0 + g) * N + n] = __float2half_rn(st[g * kPackPitch + lane]);
-            for (int g = threadIdx.x; g < count; g += kPackThreads) {
-                uint32_t w[BITS];
-#pragma unroll
-                for (int i = 0; i < BITS; ++i) w[i] = 0u;
-#pragma unroll
-                for (int j = 0; j < 32; ++j)
-                    pack_insert<BITS>(w, j, (uint32_t)(long long)(zt[g * kPackPitch + j] - 1.f));
-#pragma unroll
-                for (int i = 0; i < BITS; ++i)
-                    qzeros[(size_t)(g0 + g) * (N / 32 * BITS) + blockIdx.x * BITS + i] = (int32_t)w[i];
-            }
-            __syncthreads();
-        }
+        pack_constants<BITS, kPackThreads>(scales, zeros, G, N, blockIdx.x, qzeros, scales_out, pack_smem);
         return;
     }
     fetch(c_begin, 0);
@@ -283,10 +292,205 @@ pack_linear_kernel(const T* __restrict__ weight, const float* __restrict__ scale
     }
 }
 
+// fp16 weights, 2 to 4 bits: two columns at a time in fp16.  t = w / s + z' with 1 / s and z' = zero * scale / s rounded to fp16, u = t + 1.5 *
+// 2^10 the integer in the low bits of a half, d = t - (u - 1.5 * 2^10).  For an integer in the range of the fields and |z'| <= 32 (a table
+// entry beyond that, or with 1 / s out of the normal numbers, is NaN) t is within 2^-11 (|w / s| + |z'|) + 2^-8 < 0.05 of the quotient,
+// |w / s| being less than 16 + |z'|; so where |d| <= 0.4375 the quotient is within 0.49 of that integer, and fp32 rounds it to the same.
+// Everything else (a half nearby, out of range, NaN, infinity) is redone with the division.
+//
+// A thread takes columns c and c + 16 of a 32-row block, a half-warp a block: both columns' rows lie in one group, so that (1 / s, z') of
+// both are one 8-byte look-up, and fields pile up in the two halves of a register.  (A column per thread, in fp32 17 instructions per
+// element, in fp16 with two rows at a time 16.)  Two chunks are on their way from the start, while the table is made.  us, fp32 -> here:
+// 4096 x 11008, 4 bits, groups of 128 in act-order 35.1 -> 26.0, in order 29.7 -> 24.7 (its bytes at the copy rate: 17.8, the start of the
+// CTAs 4); 11008 x 4096, groups of 32 in act-order 106 -> 45.7 (344 groups: the table counts); 4096 x 4096, one group 13.8 -> 11.3; 2 bits, groups
+// of 64 17.8 -> 13.1; 1024 x 1024 3.7 -> 2.8.  Chunks of 512 rows (1 KB of a row) instead of 256: 29.3; of 128: 37.9.
+constexpr int kPairThreads = 128, kPairChunk = 2 * kPairThreads, kPairCtas = 6;
+constexpr int kPairPitch = 17;                         // pairs of columns in a row of the table
+constexpr uint32_t kHalfRound2 = 0x66006600u;          // 1.5 * 2^10 twice
+constexpr uint32_t kHalfFar = 0x3700u;                 // 0.4375
+
+template <int BITS>
+__global__ void __launch_bounds__(kPairThreads, kPairCtas)
+pack_pairs_kernel(const __half* __restrict__ weight, const float* __restrict__ scales, const float* __restrict__ zeros,
+                  const int32_t* __restrict__ g_idx, int K, int N, int G, int chunks_per_cta, int32_t* __restrict__ qweight,
+                  int32_t* __restrict__ qzeros, __half* __restrict__ scales_out) {
+    constexpr int PITCH = kPairChunk + 8, TILE = kPackCols * PITCH;
+    extern __shared__ __align__(16) unsigned char pack_smem[];
+    __half* tiles = reinterpret_cast<__half*>(pack_smem);          // two of [32][PITCH]
+    int* groups = reinterpret_cast<int*>(pack_smem + 2 * sizeof(__half) * TILE);   // two of: groups of the chunk's rows
+    uint2* table = reinterpret_cast<uint2*>(groups + 2 * kPairChunk);              // [G][17]: 1 / s of both columns, z' of both
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n0 = blockIdx.x * kPackCols;
+    if (blockIdx.y == gridDim.y - 1) {
+        pack_constants<BITS, kPairThreads>(scales, zeros, G, N, blockIdx.x, qzeros, scales_out, pack_smem);
+        return;
+    }
+    const int c_begin = blockIdx.y * chunks_per_cta, c_end = min((K + kPairChunk - 1) / kPairChunk, c_begin + chunks_per_cta);
+    auto fetch = [&](int c, int buf) {
+        // (whole rows of the tile by as many threads as they have pieces)
+        constexpr int PIECES = kPairChunk / 8, STEP = kPairThreads / PIECES;
+        const int k = c * kPairChunk + 8 * (threadIdx.x % PIECES), r0 = threadIdx.x / PIECES;
+        if (k < K) {
+            const __half* src = weight + (size_t)(n0 + r0) * K + k;
+            uint32_t dst = (uint32_t)__cvta_generic_to_shared(tiles + buf * TILE + r0 * PITCH + 8 * (threadIdx.x % PIECES));
+#pragma unroll
+            for (int r = 0; r < kPackCols; r += STEP) {
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+                src += (size_t)STEP * K;
+                dst += STEP * PITCH * 2;
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto group_of = [&](int c, int i) {                            // (an index outside the groups is refused by the host when the layer is used)
+        const int k = c * kPairChunk + threadIdx.x + i * kPairThreads;
+        return k < K ? min(max(__ldg(g_idx + k), 0), G - 1) : 0;
+    };
+    fetch(c_begin, 0);
+    if (c_begin + 1 < c_end) fetch(c_begin + 1, 1);
+    int g_next[2] = {group_of(c_begin, 0), group_of(c_begin, 1)};
+    auto entry = [&](size_t at) -> uint32_t {                      // (1 / s, z')
+        const float sf = scales[at];
+        float r;
+        asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(__half2float(__float2half_rn(sf))));
+        const float z = zeros[at] * sf * r;
+        if (!(fabsf(z) <= 32.f && fabsf(r) >= 0.0001220703125f && fabsf(r) <= 32768.f)) return 0x7fff7fffu;
+        const __half2 h = __floats2half2_rn(r, z);
+        return *reinterpret_cast<const uint32_t*>(&h);
+    };
+    for (int g = lane; g < G; g += 32)
+#pragma unroll
+        for (int r = 0; r < 16; r += kPairThreads / 32) {
+            const uint32_t a = entry((size_t)(n0 + r + warp) * G + g), b = entry((size_t)(n0 + r + warp + 16) * G + g);
+            table[g * kPairPitch + r + warp] = make_uint2(__byte_perm(a, b, 0x5410), __byte_perm(a, b, 0x7632));
+        }
+    auto as_h2 = [](uint32_t v) { return *reinterpret_cast<const __half2*>(&v); };
+    auto as_u = [](__half2 v) { return *reinterpret_cast<const uint32_t*>(&v); };
+    const int col = lane & 15, block = 2 * warp + (lane >> 4);
+    for (int c = c_begin; c < c_end; ++c) {
+        const int buf = (c - c_begin) & 1;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) groups[buf * kPairChunk + threadIdx.x + i * kPairThreads] = g_next[i];
+        if (c + 1 < c_end) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) g_next[i] = group_of(c + 1, i);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+        const int rb = c * (kPairChunk / kRowsPerBlock) + block;
+        const int* gr = groups + buf * kPairChunk + block * kRowsPerBlock;
+        const int g_first = gr[0];
+        const bool one_group = __all_sync(0xffffffffu, gr[col] == g_first && gr[col + 16] == g_first);   // rows in order, groups of whole blocks
+        if (rb * kRowsPerBlock < K) {
+            const __half* row = tiles + buf * TILE + col * PITCH + block * kRowsPerBlock;
+            constexpr int PER = BITS == 4 ? 4 : (BITS == 2 ? 8 : 5), SUMS = (32 + PER - 1) / PER;        // fields of a half
+            uint32_t sum[SUMS], any = 0u, far = 0u;                // all integers or'ed; largest distances from one
+            const uint2* at = table + col;
+            auto rows = [&](auto look_up) {
+#pragma unroll
+                for (int j0 = 0; j0 < kRowsPerBlock; j0 += 8) {
+                    const uint4 a = *reinterpret_cast<const uint4*>(row + j0), b = *reinterpret_cast<const uint4*>(row + 16 * PITCH + j0);
+                    const uint32_t pa[4] = {a.x, a.y, a.z, a.w}, pb[4] = {b.x, b.y, b.z, b.w};
+                    uint2 e[8];
+                    look_up(j0, e);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const int j = j0 + i;
+                        const __half2 x = as_h2(__byte_perm(pa[i >> 1], pb[i >> 1], i & 1 ? 0x7632 : 0x5410));
+                        const __half2 t = __hfma2(x, as_h2(e[i].x), as_h2(e[i].y)), u = __hadd2(t, as_h2(kHalfRound2));
+                        far = as_u(__hmax2(as_h2(far), __habs2(__hsub2(t, __hsub2(u, as_h2(kHalfRound2))))));
+                        const uint32_t q = as_u(u) ^ kHalfRound2;
+                        any |= q;
+                        sum[j / PER] = j % PER == 0 ? q : sum[j / PER] + (q << (BITS * (j % PER)));
+                    }
+                }
+            };
+            if (one_group) {
+                const uint2 one = at[g_first * kPairPitch];
+                rows([&](int, uint2 (&e)[8]) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) e[i] = one;
+                });
+            } else {
+                rows([&](int j0, uint2 (&e)[8]) {
+                    const int4 lo = *reinterpret_cast<const int4*>(gr + j0), hi = *reinterpret_cast<const int4*>(gr + j0 + 4);
+                    const int g[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) e[i] = at[g[i] * kPairPitch];
+                });
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int n = n0 + col + 16 * h;
+                int32_t* out = qweight + (size_t)rb * BITS * N + n;
+                const uint32_t beyond = (h ? any >> 16 : any & 0xffffu) >> BITS, most = h ? far >> 16 : far & 0xffffu;
+                if (beyond != 0u || most > kHalfFar) {
+                    pack_divided<BITS, __half>(row + h * 16 * PITCH, gr, scales + (size_t)n * G, zeros + (size_t)n * G, out, N);
+                } else if constexpr (BITS == 3) {                  // seven pieces of 15 bits
+                    uint32_t v[SUMS];
+#pragma unroll
+                    for (int i = 0; i < SUMS; ++i) v[i] = h ? sum[i] >> 16 : sum[i] & 0xffffu;
+                    out[0] = (int32_t)(v[0] | (v[1] << 15) | (v[2] << 30));
+                    out[N] = (int32_t)((v[2] >> 2) | (v[3] << 13) | (v[4] << 28));
+                    out[2 * (size_t)N] = (int32_t)((v[4] >> 4) | (v[5] << 11) | (v[6] << 26));
+                } else {
+#pragma unroll
+                    for (int i = 0; i < BITS; ++i)
+                        out[(size_t)i * N] = (int32_t)__byte_perm(sum[2 * i], sum[2 * i + 1], h ? 0x7632 : 0x5410);
+                }
+            }
+        }
+        __syncthreads();
+        if (c + 2 < c_end) fetch(c + 2, buf);
+    }
+}
+
+// Chunks of K per CTA, so that the waves of the grid are full and short: a CTA costs its chunks, the start of its pipeline and its table
+// (an entry about as much as four elements).
+int pack_split(int chunks, int strips, int resident, int G) {
+    int per = chunks;
+    long long best = -1;
+    for (int p = 1; p <= chunks; ++p) {
+        const int c = (chunks + p - 1) / p, ctas = strips * ((chunks + c - 1) / c);
+        const long long cost = (long long)((ctas + resident - 1) / resident) * (64 * (c + 1) + G);
+        if (best < 0 || cost < best) { best = cost; per = c; }
+    }
+    return per;
+}
+
+template <int BITS>
+int launch_pack_pairs(const void* weight, const float* scales, const float* zeros, const int32_t* g_idx, int K, int N, int G,
+                      int32_t* qweight, int32_t* qzeros, __half* scales_out, cudaStream_t stream) {
+    const int chunks = (K + kPairChunk - 1) / kPairChunk, strips = N / kPackCols;
+    const size_t used = 2 * (sizeof(__half) * kPackCols * (kPairChunk + 8) + kPairChunk * sizeof(int)) + (size_t)G * kPairPitch * sizeof(uint2);
+    const size_t constants = 2 * 128 * kPackPitch * sizeof(float), smem = used > constants ? used : constants;
+    static std::once_flag once[64];
+    static int result[64];
+    int dev = 0;
+    B200GPTQ_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return B200GPTQ_ERR_TOO_LARGE;
+    std::call_once(once[dev], [dev] {
+        result[dev] = (int)cudaFuncSetAttribute(pack_pairs_kernel<BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    });
+    if (result[dev] != 0) { set_last_cuda_error(result[dev]); return B200GPTQ_ERR_CUDA; }
+    const int fit = (int)(220 * 1024 / (smem + 1024));
+    const int per = pack_split(chunks, strips, sm_count() * (fit < kPairCtas ? fit : kPairCtas), G);
+    dim3 grid(strips, (chunks + per - 1) / per + 1);
+    pack_pairs_kernel<BITS><<<grid, kPairThreads, smem, stream>>>(static_cast<const __half*>(weight), scales, zeros, g_idx, K, N, G, per,
+                                                                      qweight, qzeros, scales_out);
+    B200GPTQ_CUDA_TRY(cudaGetLastError());
+    return B200GPTQ_OK;
+}
+
 template <int BITS, typename T>
 int launch_pack_linear(const void* weight, const float* scales, const float* zeros, const int32_t* g_idx, int K, int N,
                        int G, int32_t* qweight, int32_t* qzeros, __half* scales_out, cudaStream_t stream) {
     const int chunks = (K + kPackChunk - 1) / kPackChunk, strips = N / kPackCols;
+    // fp16 weights of 2 to 4 bits whose table fits; 8 bits have no room for their integers in a half
+    if constexpr (std::is_same<T, __half>::value && BITS != 8)
+        if ((long long)G * kPairPitch * (int)sizeof(uint2) <= kPackTableMax)
+            return launch_pack_pairs<BITS>(weight, scales, zeros, g_idx, K, N, G, qweight, qzeros, scales_out, stream);
     const long long table = (long long)G * kPackPitch * sizeof(float2);
     const int use_table = table <= kPackTableMax;
     const size_t smem = 2 * (sizeof(T) * kPackCols * (kPackChunk + 16 / sizeof(T)) + kPackChunk * sizeof(int)) + (use_table ? table : 0);
@@ -300,16 +504,8 @@ int launch_pack_linear(const void* weight, const float* scales, const float* zer
                                                 200 * 1024);
     });
     if (result[dev] != 0) { set_last_cuda_error(result[dev]); return B200GPTQ_ERR_CUDA; }
-    // K is cut so that the waves of the grid are full and short: a CTA costs its chunks, the start of its pipeline and its
-    // table (an entry about as much as four elements).
     const int resident = sm_count() * (smem * kPackCtas <= 220 * 1024 ? kPackCtas : (int)(220 * 1024 / smem));
-    int per = chunks;
-    long long best = -1;
-    for (int p = 1; p <= chunks; ++p) {
-        const int c = (chunks + p - 1) / p, ctas = strips * ((chunks + c - 1) / c);
-        const long long cost = (long long)((ctas + resident - 1) / resident) * (64 * (c + 1) + G);
-        if (best < 0 || cost < best) { best = cost; per = c; }
-    }
+    const int per = pack_split(chunks, strips, resident, G);
     dim3 grid(strips, (chunks + per - 1) / per + 1);
     pack_linear_kernel<BITS, T><<<grid, kPackThreads, smem, stream>>>(static_cast<const T*>(weight), scales, zeros, g_idx, K, N,
                                                                       G, per, use_table, qweight, qzeros, scales_out);

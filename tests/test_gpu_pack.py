@@ -130,3 +130,33 @@ def test_one_launch_pack_in_order_and_out_of_range(bits, K, N, gs):
     assert torch.equal(a.qweight, b.qweight.cpu())
     assert torch.equal(a.qzeros, b.qzeros.cpu())
     assert torch.equal(a.scales, b.scales.cpu())
+
+
+@pytest.mark.parametrize("bits", [2, 3, 4])
+@pytest.mark.parametrize("K,N,gs", [(32, 32, 32), (288, 64, 16), (544, 32, -1), (4480, 96, 64), (16384, 32, 16)])
+def test_fp16_weights_equal_the_cpu_packer(bits, K, N, gs):
+    """fp16 weights of 2 to 4 bits are rounded in fp16 where that gives the quotient's integer for certain: any fraction, with quotients on
+    both sides of the line (0.4375 from an integer) and of a half, zero-points and scales past the ones that fp16 takes (|zero * scale / s|
+    > 32, 1 / s no normal number), negative scales, groups that cut 32-row blocks, more groups than the
+    table holds (16384 rows in groups of 16)."""
+    gen = torch.Generator().manual_seed(bits + K)
+    size = gs if gs != -1 else K
+    G, top = -(-K // size), 2 ** bits - 1
+    scales = torch.rand(N, G, generator=gen) * 0.02 + 1e-3
+    zeros = torch.randint(1, top + 2, (N, G), generator=gen).float()
+    zeros[3::8], zeros[4::8] = 31.99, 33.0
+    scales[5::8], scales[6::8], scales[7::8] = 2.0 ** -15.5, 20000.0, -scales[7::8]
+    g_idx = (torch.randperm(K, generator=gen) // size).to(torch.int32)
+    sel = g_idx.long()
+    frac = torch.tensor([0.0, 0.43, 0.4375, 0.45, 0.4999, 0.5, 0.5001, -0.43, -0.4375, -0.45, -0.5, -0.5001])
+    q = torch.randint(0, top + 1, (N, K), generator=gen) + frac[torch.randint(0, len(frac), (N, K), generator=gen)]
+    q[0] = torch.rand(K, generator=gen) * (top + 2) - 1
+    W = ((q - zeros[:, sel]) * scales[:, sel]).clamp(-6e4, 6e4).half()     # (finite: what an infinity becomes as an integer is nobody's)
+    lin = nn.Linear(K, N, bias=False)
+    lin.weight.data = W
+    a, b = QuantLinear(bits, gs, K, N, False), QuantLinear(bits, gs, K, N, False).to(DEV)
+    a.pack(lin, scales, zeros, g_idx)
+    b.pack(lin.to(DEV), scales.to(DEV), zeros.to(DEV), g_idx.to(DEV))
+    assert torch.equal(a.qweight, b.qweight.cpu())
+    assert torch.equal(a.qzeros, b.qzeros.cpu())
+    assert torch.equal(a.scales, b.scales.cpu())
