@@ -764,21 +764,29 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                 uint32_t dg[V][8];
 #pragma unroll
                 for (int v = 0; v < V; ++v) {
-                    int X[8];
                     sum[v] = 0;
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) {
+                    // round to nearest; up to 22 bits through the fp32 adder.  (26 bits through it, in two steps: more code, 0.1 to 0.5 us
+                    // a launch longer)
+                    auto fixed = [&](int e) {
                         const float xf = __half2float(__ushort_as_half((unsigned short)h[v][e]));
-                        // round to nearest; up to 22 bits through the fp32 adder.  (26 bits through it, in two steps: more code, 0.1 to 0.5 us
-                        // a launch longer)
-                        X[e] = XB > 22 ? __float2int_rn(xf * scale[v]) : __float_as_int(fmaf(xf, scale[v], 12582912.f)) - 0x4B400000;
-                        sum[v] += X[e];
-                    }
+                        return XB > 22 ? __float2int_rn(xf * scale[v]) : __float_as_int(fmaf(xf, scale[v], 12582912.f)) - 0x4B400000;
+                    };
+                    auto digits = [](int X) { return (uint32_t)(X + 0x00808080) ^ 0x00808080u; };   // four signed base-256 digits
+                    if constexpr (BITS == 4 && SUB == 1) {
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) {
-                        // (4 bits, whole units: |16 X - X'| < 2^30 + 2^26, which four digits hold)
-                        const int shifted = BITS == 4 && SUB == 1 ? (e < 4 ? X[e] * 16 - X[e | 4] : X[e]) : X[e] << pre[e];
-                        dg[v][e] = (uint32_t)(shifted + 0x00808080) ^ 0x00808080u;         // four signed base-256 digits
+                        for (int e = 0; e < 4; ++e) {              // (|16 X - X'| < 2^30 + 2^26, which four digits hold)
+                            const int lo = fixed(e), hi = fixed(e + 4);
+                            sum[v] += lo + hi;
+                            dg[v][e] = digits(lo * 16 - hi);
+                            dg[v][e + 4] = digits(hi);
+                        }
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) {
+                            const int X = fixed(e);
+                            sum[v] += X;
+                            dg[v][e] = digits(X << pre[e]);
+                        }
                     }
                 }
                 // (the X of 128 rows of 22 bits, or of 32 rows of 26, add up to less than 2^31)
