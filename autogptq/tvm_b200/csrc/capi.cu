@@ -28,7 +28,7 @@ int dequant_dispatch(const int32_t*, const int32_t*, const __half*, const int32_
                      __half*, cudaStream_t);
 int pack_fields_dispatch(const int32_t*, int, int, int, int32_t*, cudaStream_t);
 int pack_linear_dispatch(const void*, int, const float*, const float*, const int32_t*, int, int, int, int, int32_t*,
-                         int32_t*, __half*, cudaStream_t);
+                         int32_t*, __half*, int32_t*, cudaStream_t);
 int sort_rows_dispatch(const int32_t*, const int32_t*, const int32_t*, int, int, int, int32_t*, int32_t*,
                        cudaStream_t);
 int gemv_generic_dispatch(const __half*, const int32_t*, const int32_t*, const __half*, const int32_t*,
@@ -112,13 +112,19 @@ int b200gptq_pack_fields(const int32_t* vals, int R, int C, int bits, int32_t* o
 int b200gptq_pack_linear(const void* weight, int dtype, const float* scales, const float* zeros, const int32_t* g_idx,
                          int K, int N, int G, int bits, int32_t* qweight, int32_t* qzeros, void* scales_out,
                          void* stream) {
+    return b200gptq_pack_linear_ex(weight, dtype, scales, zeros, g_idx, K, N, G, bits, qweight, qzeros, scales_out, nullptr, stream);
+}
+
+int b200gptq_pack_linear_ex(const void* weight, int dtype, const float* scales, const float* zeros, const int32_t* g_idx,
+                            int K, int N, int G, int bits, int32_t* qweight, int32_t* qzeros, void* scales_out,
+                            int32_t* g_idx_out, void* stream) {
     if (!weight || !scales || !zeros || !g_idx || !qweight || !qzeros || !scales_out) return B200GPTQ_ERR_NULL_POINTER;
     int gs = K;
     if (int st = check_layer(K, N, bits, &gs)) return st;
     if (G < 1 || dtype < B200GPTQ_F16 || dtype > B200GPTQ_F32) return B200GPTQ_ERR_SHAPE;
     if (!aligned16(weight)) return B200GPTQ_ERR_ALIGNMENT;
     return pack_linear_dispatch(weight, dtype, scales, zeros, g_idx, K, N, G, bits, qweight, qzeros,
-                                static_cast<__half*>(scales_out), static_cast<cudaStream_t>(stream));
+                                static_cast<__half*>(scales_out), g_idx_out, static_cast<cudaStream_t>(stream));
 }
 
 int b200gptq_sort_rows(const int32_t* qweight, const int32_t* g_idx, const int32_t* perm, int K, int N, int bits,

@@ -324,6 +324,60 @@ PyObject* zeros_outside_capture(PyObject*, PyObject* args) {
         return nullptr;
     }
 }
+// pack(weight, scales, zeros, g_idx, bits, copy_g_idx): QuantLinear.pack's (qweight, qzeros, scales, copy of g_idx or None) in one launch, or None
+// where the Python route has more to do (another type, order, device or shape).
+PyObject* pack_prepared(PyObject* const* args, Py_ssize_t nargs) {
+    if (nargs != 6) { PyErr_SetString(PyExc_TypeError, "pack(weight, scales, zeros, g_idx, bits, copy_g_idx)"); return nullptr; }
+    const at::Tensor* t[4];
+    for (int i = 0; i < 4; ++i) {
+        if (!THPVariable_Check(args[i])) Py_RETURN_NONE;
+        t[i] = &THPVariable_Unpack(args[i]);
+        if (t[i]->key_set().has_any(kNotPlain) || !t[i]->is_cuda() || !t[i]->is_contiguous()) Py_RETURN_NONE;
+    }
+    const at::Tensor &w = *t[0], &scales = *t[1], &zeros = *t[2], &g_idx = *t[3];
+    const int bits = (int)PyLong_AsLong(args[4]), copy = PyObject_IsTrue(args[5]);
+    if (PyErr_Occurred()) return nullptr;
+    const auto type = w.scalar_type();
+    const int dtype = type == at::kHalf ? B200GPTQ_F16 : (type == at::kBFloat16 ? B200GPTQ_BF16 : (type == at::kFloat ? B200GPTQ_F32 : -1));
+    const int device = w.get_device();
+    if (dtype < 0 || w.dim() != 2 || scales.dim() != 2 || scales.scalar_type() != at::kFloat || zeros.scalar_type() != at::kFloat ||
+        g_idx.scalar_type() != at::kInt || g_idx.dim() != 1 || scales.get_device() != device || zeros.get_device() != device ||
+        g_idx.get_device() != device || c10::cuda::current_device() != device)
+        Py_RETURN_NONE;
+    const int64_t N = w.size(0), K = w.size(1), G = scales.size(1);
+    const void* wp = w.unsafeGetTensorImpl()->data();
+    if (scales.size(0) != N || zeros.sizes() != scales.sizes() || g_idx.numel() != K || G < 1 || K < 32 || K % 32 || N < 32 || N % 32 ||
+        K > INT32_MAX || N > INT32_MAX || ((uintptr_t)wp & 15u))
+        Py_RETURN_NONE;
+    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream();
+    const at::Device on(at::kCUDA, (c10::DeviceIndex)device);
+    at::Tensor qweight, qzeros, scales16, g_copy;
+    int st;
+    {
+        const WithoutGil released;
+        qweight = at::detail::empty_cuda({K / 32 * bits, N}, at::kInt, on, std::nullopt);
+        qzeros = at::detail::empty_cuda({G, N / 32 * bits}, at::kInt, on, std::nullopt);
+        scales16 = at::detail::empty_cuda({G, N}, at::kHalf, on, std::nullopt);
+        if (copy) g_copy = at::detail::empty_cuda({K}, at::kInt, on, std::nullopt);
+        auto ints = [](at::Tensor& x) { return static_cast<int32_t*>(x.unsafeGetTensorImpl()->mutable_data()); };
+        st = b200gptq_pack_linear_ex(wp, dtype, static_cast<const float*>(scales.unsafeGetTensorImpl()->data()),
+                                     static_cast<const float*>(zeros.unsafeGetTensorImpl()->data()),
+                                     static_cast<const int32_t*>(g_idx.unsafeGetTensorImpl()->data()), (int)K, (int)N, (int)G, bits,
+                                     ints(qweight), ints(qzeros), scales16.unsafeGetTensorImpl()->mutable_data(),
+                                     copy ? ints(g_copy) : nullptr, stream);
+    }
+    if (st != B200GPTQ_OK) Py_RETURN_NONE;   // the Python route repeats the call and reports the status
+    PyObject* out[4] = {THPVariable_Wrap(std::move(qweight)), THPVariable_Wrap(std::move(qzeros)), THPVariable_Wrap(std::move(scales16)),
+                        copy ? THPVariable_Wrap(std::move(g_copy)) : Py_NewRef(Py_None)};
+    return Py_BuildValue("(NNNN)", out[0], out[1], out[2], out[3]);
+}
+PyObject* pack(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    try {
+        return pack_prepared(args, nargs);
+    } catch (const std::exception&) {        // out of memory: met again by the Python route, which raises it with its own type
+        Py_RETURN_NONE;
+    }
+}
 PyObject* set_scratch_source(PyObject*, PyObject* fn) {
     Py_INCREF(fn);
     Py_XSETREF(g_get_workspace, fn);
@@ -331,6 +385,7 @@ PyObject* set_scratch_source(PyObject*, PyObject* fn) {
 }
 
 PyMethodDef module_methods[] = {
+    {"pack", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(pack)), METH_FASTCALL, nullptr},
     {"set_scratch", set_scratch, METH_VARARGS, nullptr},
     {"set_scratch_source", set_scratch_source, METH_O, nullptr},
     {"scratch_use", scratch_use, METH_VARARGS, nullptr},

@@ -140,7 +140,10 @@ __device__ __noinline__ void pack_divided(const T* row, const int* gr, const flo
 // scales_out and qzeros of one strip of 32 columns.  smem: 2 * 128 * kPackPitch floats
 template <int BITS, int THREADS>
 __device__ __forceinline__ void pack_constants(const float* __restrict__ scales, const float* __restrict__ zeros, int G, int N, int strip,
-                                               int32_t* __restrict__ qzeros, __half* __restrict__ scales_out, unsigned char* smem) {
+                                               int32_t* __restrict__ qzeros, __half* __restrict__ scales_out, unsigned char* smem,
+                                               const int32_t* __restrict__ g_idx, int K, int32_t* __restrict__ g_idx_out) {
+    if (g_idx_out)                                                 // a copy, 32 of every 32 * strips by each strip
+        for (int k = strip * 32 + (threadIdx.x & 31); k < K && threadIdx.x < 32; k += 32 * gridDim.x) g_idx_out[k] = g_idx[k];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n0 = strip * kPackCols, n = n0 + lane;
     // scales and zero-points of the strip, 128 groups at a time: read along the groups, written along the columns
     constexpr int GT = 128;
@@ -177,7 +180,7 @@ template <int BITS, typename T>
 __global__ void __launch_bounds__(kPackThreads, kPackCtas)
 pack_linear_kernel(const T* __restrict__ weight, const float* __restrict__ scales, const float* __restrict__ zeros,
                    const int32_t* __restrict__ g_idx, int K, int N, int G, int chunks_per_cta, int use_table,
-                   int32_t* __restrict__ qweight, int32_t* __restrict__ qzeros, __half* __restrict__ scales_out) {
+                   int32_t* __restrict__ qweight, int32_t* __restrict__ qzeros, __half* __restrict__ scales_out, int32_t* __restrict__ g_idx_out) {
     constexpr int VEC = 16 / (int)sizeof(T);                       // elements of one 16-byte read
     constexpr int PITCH = kPackChunk + VEC;                        // elements of a tile row: 16 bytes of padding
     constexpr int TILE = kPackCols * PITCH;
@@ -206,7 +209,7 @@ pack_linear_kernel(const T* __restrict__ weight, const float* __restrict__ scale
         return k < K ? min(max(__ldg(g_idx + k), 0), G - 1) : 0;
     };
     if (blockIdx.y == gridDim.y - 1) {
-        pack_constants<BITS, kPackThreads>(scales, zeros, G, N, blockIdx.x, qzeros, scales_out, pack_smem);
+        pack_constants<BITS, kPackThreads>(scales, zeros, G, N, blockIdx.x, qzeros, scales_out, pack_smem, g_idx, K, g_idx_out);
         return;
     }
     fetch(c_begin, 0);
@@ -313,7 +316,7 @@ template <int BITS>
 __global__ void __launch_bounds__(kPairThreads, kPairCtas)
 pack_pairs_kernel(const __half* __restrict__ weight, const float* __restrict__ scales, const float* __restrict__ zeros,
                   const int32_t* __restrict__ g_idx, int K, int N, int G, int chunks_per_cta, int32_t* __restrict__ qweight,
-                  int32_t* __restrict__ qzeros, __half* __restrict__ scales_out) {
+                  int32_t* __restrict__ qzeros, __half* __restrict__ scales_out, int32_t* __restrict__ g_idx_out) {
     constexpr int PITCH = kPairChunk + 8, TILE = kPackCols * PITCH;
     extern __shared__ __align__(16) unsigned char pack_smem[];
     __half* tiles = reinterpret_cast<__half*>(pack_smem);          // two of [32][PITCH]
@@ -321,7 +324,7 @@ pack_pairs_kernel(const __half* __restrict__ weight, const float* __restrict__ s
     uint2* table = reinterpret_cast<uint2*>(groups + 2 * kPairChunk);              // [G][17]: 1 / s of both columns, z' of both
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n0 = blockIdx.x * kPackCols;
     if (blockIdx.y == gridDim.y - 1) {
-        pack_constants<BITS, kPairThreads>(scales, zeros, G, N, blockIdx.x, qzeros, scales_out, pack_smem);
+        pack_constants<BITS, kPairThreads>(scales, zeros, G, N, blockIdx.x, qzeros, scales_out, pack_smem, g_idx, K, g_idx_out);
         return;
     }
     const int c_begin = blockIdx.y * chunks_per_cta, c_end = min((K + kPairChunk - 1) / kPairChunk, c_begin + chunks_per_cta);
@@ -461,7 +464,7 @@ int pack_split(int chunks, int strips, int resident, int G) {
 
 template <int BITS>
 int launch_pack_pairs(const void* weight, const float* scales, const float* zeros, const int32_t* g_idx, int K, int N, int G,
-                      int32_t* qweight, int32_t* qzeros, __half* scales_out, cudaStream_t stream) {
+                      int32_t* qweight, int32_t* qzeros, __half* scales_out, int32_t* g_idx_out, cudaStream_t stream) {
     const int chunks = (K + kPairChunk - 1) / kPairChunk, strips = N / kPackCols;
     const size_t used = 2 * (sizeof(__half) * kPackCols * (kPairChunk + 8) + kPairChunk * sizeof(int)) + (size_t)G * kPairPitch * sizeof(uint2);
     const size_t constants = 2 * 128 * kPackPitch * sizeof(float), smem = used > constants ? used : constants;
@@ -478,19 +481,19 @@ int launch_pack_pairs(const void* weight, const float* scales, const float* zero
     const int per = pack_split(chunks, strips, sm_count() * (fit < kPairCtas ? fit : kPairCtas), G);
     dim3 grid(strips, (chunks + per - 1) / per + 1);
     pack_pairs_kernel<BITS><<<grid, kPairThreads, smem, stream>>>(static_cast<const __half*>(weight), scales, zeros, g_idx, K, N, G, per,
-                                                                      qweight, qzeros, scales_out);
+                                                                      qweight, qzeros, scales_out, g_idx_out);
     B200GPTQ_CUDA_TRY(cudaGetLastError());
     return B200GPTQ_OK;
 }
 
 template <int BITS, typename T>
 int launch_pack_linear(const void* weight, const float* scales, const float* zeros, const int32_t* g_idx, int K, int N,
-                       int G, int32_t* qweight, int32_t* qzeros, __half* scales_out, cudaStream_t stream) {
+                       int G, int32_t* qweight, int32_t* qzeros, __half* scales_out, int32_t* g_idx_out, cudaStream_t stream) {
     const int chunks = (K + kPackChunk - 1) / kPackChunk, strips = N / kPackCols;
     // fp16 weights of 2 to 4 bits whose table fits; 8 bits have no room for their integers in a half
     if constexpr (std::is_same<T, __half>::value && BITS != 8)
         if ((long long)G * kPairPitch * (int)sizeof(uint2) <= kPackTableMax)
-            return launch_pack_pairs<BITS>(weight, scales, zeros, g_idx, K, N, G, qweight, qzeros, scales_out, stream);
+            return launch_pack_pairs<BITS>(weight, scales, zeros, g_idx, K, N, G, qweight, qzeros, scales_out, g_idx_out, stream);
     const long long table = (long long)G * kPackPitch * sizeof(float2);
     const int use_table = table <= kPackTableMax;
     const size_t smem = 2 * (sizeof(T) * kPackCols * (kPackChunk + 16 / sizeof(T)) + kPackChunk * sizeof(int)) + (use_table ? table : 0);
@@ -508,7 +511,7 @@ int launch_pack_linear(const void* weight, const float* scales, const float* zer
     const int per = pack_split(chunks, strips, resident, G);
     dim3 grid(strips, (chunks + per - 1) / per + 1);
     pack_linear_kernel<BITS, T><<<grid, kPackThreads, smem, stream>>>(static_cast<const T*>(weight), scales, zeros, g_idx, K, N,
-                                                                      G, per, use_table, qweight, qzeros, scales_out);
+                                                                      G, per, use_table, qweight, qzeros, scales_out, g_idx_out);
     B200GPTQ_CUDA_TRY(cudaGetLastError());
     return B200GPTQ_OK;
 }
@@ -516,15 +519,15 @@ int launch_pack_linear(const void* weight, const float* scales, const float* zer
 }  // namespace
 
 int pack_linear_dispatch(const void* weight, int dtype, const float* scales, const float* zeros, const int32_t* g_idx,
-                         int K, int N, int G, int bits, int32_t* qweight, int32_t* qzeros, __half* scales_out,
+                         int K, int N, int G, int bits, int32_t* qweight, int32_t* qzeros, __half* scales_out, int32_t* g_idx_out,
                          cudaStream_t stream) {
-#define B200GPTQ_PACK(B)                                                                                               \
-    (dtype == B200GPTQ_F16    ? launch_pack_linear<B, __half>(weight, scales, zeros, g_idx, K, N, G, qweight, qzeros,  \
-                                                              scales_out, stream)                                      \
-     : dtype == B200GPTQ_BF16 ? launch_pack_linear<B, __nv_bfloat16>(weight, scales, zeros, g_idx, K, N, G, qweight,   \
-                                                                     qzeros, scales_out, stream)                       \
-                              : launch_pack_linear<B, float>(weight, scales, zeros, g_idx, K, N, G, qweight, qzeros,   \
-                                                             scales_out, stream))
+#define B200GPTQ_PACK(B)                                                                                                             \
+    (dtype == B200GPTQ_F16    ? launch_pack_linear<B, __half>(weight, scales, zeros, g_idx, K, N, G, qweight, qzeros, scales_out,    \
+                                                              g_idx_out, stream)                                                     \
+     : dtype == B200GPTQ_BF16 ? launch_pack_linear<B, __nv_bfloat16>(weight, scales, zeros, g_idx, K, N, G, qweight, qzeros,         \
+                                                                     scales_out, g_idx_out, stream)                                  \
+                              : launch_pack_linear<B, float>(weight, scales, zeros, g_idx, K, N, G, qweight, qzeros, scales_out,     \
+                                                             g_idx_out, stream))
     switch (bits) {
         case 2: return B200GPTQ_PACK(2);
         case 3: return B200GPTQ_PACK(3);

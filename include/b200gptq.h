@@ -250,6 +250,10 @@ B200GPTQ_API int b200gptq_pack_fields(const int32_t* vals, int R, int C, int bit
 B200GPTQ_API int b200gptq_pack_linear(const void* weight, int dtype, const float* scales, const float* zeros,
                                       const int32_t* g_idx, int K, int N, int G, int bits, int32_t* qweight,
                                       int32_t* qzeros, void* scales_out, void* stream);
+/* The same with a copy of g_idx (g_idx_out int32 [K], may be NULL), which the reference's pack keeps. */
+B200GPTQ_API int b200gptq_pack_linear_ex(const void* weight, int dtype, const float* scales, const float* zeros,
+                                         const int32_t* g_idx, int K, int N, int G, int bits, int32_t* qweight,
+                                         int32_t* qzeros, void* scales_out, int32_t* g_idx_out, void* stream);
 
 /*
  * Re-order the rows of a packed layer so that rows of one group are adjacent

@@ -160,3 +160,36 @@ def test_fp16_weights_equal_the_cpu_packer(bits, K, N, gs):
     assert torch.equal(a.qweight, b.qweight.cpu())
     assert torch.equal(a.qzeros, b.qzeros.cpu())
     assert torch.equal(a.scales, b.scales.cpu())
+
+
+def test_pack_in_one_native_call_keeps_what_the_python_route_has():
+    """The native call and the Python route (taken here because of a scale that is not contiguous, an int64 g_idx, a CPU g_idx) store the
+    same buffers; the caller's g_idx is copied, the module's own kept where none is given, and hooks on buffers see every one."""
+    K, N, gs = 256, 64, 64
+    gen = torch.Generator().manual_seed(3)
+    lin = nn.Linear(K, N, bias=True)
+    lin.weight.data = torch.randn(N, K, generator=gen).half() * 0.05
+    lin = lin.to(DEV)
+    scales, zeros = (torch.rand(N, K // gs, generator=gen) * 0.02 + 1e-3).to(DEV), torch.randint(1, 16, (N, K // gs), generator=gen).float().to(DEV)
+    g_idx = (torch.randperm(K, generator=gen) // gs).to(torch.int32).to(DEV)
+    want = QuantLinear(4, gs, K, N, True).to(DEV)
+    want.pack(lin, scales, zeros, g_idx)
+    assert want.g_idx.data_ptr() != g_idx.data_ptr() and want.g_idx.dtype == torch.int32 and torch.equal(want.g_idx, g_idx)
+    for kw in (dict(scales=scales.t().contiguous().t()), dict(g_idx=g_idx.long()), dict(g_idx=g_idx.cpu())):
+        m = QuantLinear(4, gs, K, N, True).to(DEV)
+        m.pack(lin, kw.get("scales", scales), zeros, kw.get("g_idx", g_idx))
+        for name in ("qweight", "qzeros", "scales", "bias"):
+            assert torch.equal(getattr(m, name), getattr(want, name)), name
+        assert torch.equal(m.g_idx.to(DEV), g_idx.to(m.g_idx.dtype)) and m.g_idx.dtype == kw.get("g_idx", g_idx).dtype
+    m = QuantLinear(4, gs, K, N, True).to(DEV)
+    own = m.g_idx
+    seen = []
+    hook = torch.nn.modules.module.register_module_buffer_registration_hook(lambda mod, name, b: seen.append(name))
+    try:
+        m.pack(lin, scales, zeros)
+    finally:
+        hook.remove()
+    assert m.g_idx is own and {"qweight", "qzeros", "scales"} <= set(seen)
+    assert set(m.state_dict()) == {"qweight", "qzeros", "scales", "g_idx", "bias"}
+    with pytest.raises(ValueError):
+        m.pack(lin, scales[:, :2].contiguous(), zeros, g_idx)
