@@ -45,10 +45,10 @@ int gemm_dispatch(const __half*, const int32_t*, const int32_t*, const __half*, 
 struct GemvStripPlan;
 bool gemv_strip_supported(int M, int K, int N, int bits, int group_size);
 bool gemv_strip_gathers(int M, int K);
-GemvStripPlan* gemv_strip_plan_create(const int32_t*, const int32_t*, const __half*, bool, int, int, int, int, int, int, int, int*);
+GemvStripPlan* gemv_strip_plan_create(const int32_t*, const int32_t*, const __half*, bool, bool, int, int, int, int, int, int, int, int*);
 int gemv_strip_run(const GemvStripPlan*, const __half*, const int32_t*, const __half*, __half*, void*, cudaStream_t);
 void gemv_strip_plan_destroy(GemvStripPlan*);
-int gemv_strip_dispatch(const __half*, const int32_t*, const int32_t*, const __half*, const int32_t*, const __half*, __half*,
+int gemv_strip_dispatch(const __half*, const int32_t*, const int32_t*, const __half*, const int32_t*, bool, const __half*, __half*,
                         int, int, int, int, int, void*, int, int, cudaStream_t);
 int gather_x_dispatch(const __half*, const int32_t*, __half*, int, int, int, cudaStream_t);
 
@@ -227,8 +227,9 @@ int b200gptq_gemv_ex(const void* x, const int32_t* qweight, const int32_t* qzero
     if (!act_supported(input_act, streams, x_perm)) return B200GPTQ_ERR_SHAPE;
     if (!g_idx && gemv_strip_supported(M, K, N, bits, group_size)) {
         const __half* xh = static_cast<const __half*>(x);
+        const bool permuted = x_perm != nullptr;
         if (int e = gather_first(&xh, &x_perm, M, K, workspace, st)) return e;
-        return gemv_strip_dispatch(xh, qweight, qzeros, static_cast<const __half*>(scales), x_perm,
+        return gemv_strip_dispatch(xh, qweight, qzeros, static_cast<const __half*>(scales), x_perm, permuted,
                                    static_cast<const __half*>(bias), static_cast<__half*>(y), M, K, N, bits, group_size,
                                    workspace, ctas_per_sm, input_act, st);
     }
@@ -274,7 +275,7 @@ int b200gptq_gemv_plan_create_ex(b200gptq_gemv_plan** out, const int32_t* qweigh
     if (!g_idx && gemv_strip_supported(M, K, N, bits, group_size)) {
         int st = B200GPTQ_OK;
         const bool gather = x_perm != nullptr && gemv_strip_gathers(M, K) && aligned16(x_perm);
-        p->strip = gemv_strip_plan_create(qweight, qzeros, p->scales, gather, M, K, N, bits, group_size, ctas_per_sm, input_act, &st);
+        p->strip = gemv_strip_plan_create(qweight, qzeros, p->scales, gather, x_perm != nullptr, M, K, N, bits, group_size, ctas_per_sm, input_act, &st);
         if (!p->strip) { delete p; return st; }
     }
     *out = p;

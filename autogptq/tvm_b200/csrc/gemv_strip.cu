@@ -5,10 +5,10 @@
 
 namespace b200gptq {
 
-const void* gemv_strip_kernel_b2(int sub, int mode, int nt, int T, int warps, bool apart);
-const void* gemv_strip_kernel_b3(int sub, int mode, int nt, int T, int warps, bool apart);
-const void* gemv_strip_kernel_b4(int sub, int mode, int nt, int T, int warps, bool apart);
-const void* gemv_strip_kernel_b8(int sub, int mode, int nt, int T, int warps, bool apart);
+const void* gemv_strip_kernel_b2(int sub, int mode, int nt, int T, int warps, bool apart, bool split);
+const void* gemv_strip_kernel_b3(int sub, int mode, int nt, int T, int warps, bool apart, bool split);
+const void* gemv_strip_kernel_b4(int sub, int mode, int nt, int T, int warps, bool apart, bool split);
+const void* gemv_strip_kernel_b8(int sub, int mode, int nt, int T, int warps, bool apart, bool split);
 
 struct GemvStripPlan {
     int M, K, N, smem, warps;          // of a CTA: shared memory, warps (with idle ones)
@@ -37,12 +37,12 @@ EncodeTiledFn encode_tiled_fn() {
     return fn;
 }
 
-const void* strip_kernel(int bits, int sub, int mode, int nt, int T, int warps, bool apart) {
+const void* strip_kernel(int bits, int sub, int mode, int nt, int T, int warps, bool apart, bool split) {
     switch (bits) {
-        case 2: return gemv_strip_kernel_b2(sub, mode, nt, T, warps, apart);
-        case 3: return gemv_strip_kernel_b3(sub, mode, nt, T, warps, apart);
-        case 4: return gemv_strip_kernel_b4(sub, mode, nt, T, warps, apart);
-        case 8: return gemv_strip_kernel_b8(sub, mode, nt, T, warps, apart);
+        case 2: return gemv_strip_kernel_b2(sub, mode, nt, T, warps, apart, split);
+        case 3: return gemv_strip_kernel_b3(sub, mode, nt, T, warps, apart, split);
+        case 4: return gemv_strip_kernel_b4(sub, mode, nt, T, warps, apart, split);
+        case 8: return gemv_strip_kernel_b8(sub, mode, nt, T, warps, apart, split);
     }
     return nullptr;
 }
@@ -58,7 +58,7 @@ bool gemv_strip_supported(int M, int K, int N, int bits, int group_size) {
 bool gemv_strip_gathers(int M, int K) { return (size_t)M * K * 2 <= kRawMax; }
 
 int gemv_strip_prepare(GemvStripPlan* p, const int32_t* qweight, const int32_t* qzeros,
-                       const __half* scales, bool gather, int M, int K, int N, int bits, int group_size,
+                       const __half* scales, bool gather, bool permuted, int M, int K, int N, int bits, int group_size,
                        int ctas_per_sm, int xact) {
     p->M = M; p->K = K; p->N = N;
     StripPlan& s = p->plan;
@@ -73,6 +73,20 @@ int gemv_strip_prepare(GemvStripPlan* p, const int32_t* qweight, const int32_t* 
     s.strips = N / kStripCols;
     // One CTA per SM: each takes the same whole number of strips.
     s.per_cta = (s.strips + sm_count() - 1) / sm_count();
+    // Fewer strips than half the SMs: clusters of two or four CTAs share one, where the units of K that a CTA is spared take longer than
+    // the cluster's sum.  Hundredths of a us, from layers of 1024 to 2304 columns one behind the other, 1 to 16 rows of 1024 to 11008 values
+    // (600 of them): a unit takes 6 (one row) to 18, the cluster 150 and more with the number of strips, with a gather (every CTA copies x)
+    // and 8 bits.  us, unsplit -> split: 4 bits, 11008 x 1024, one row 6.6 -> 4.4, 8 rows 9.4 -> 4.9, 16 rows 17.2 -> 6.4; 11008 x 2304, one row
+    // 6.9 -> 6.4, 8 rows 9.9 -> 7.5, 16 rows 17.1 -> 10.4; 8192 x 1536, 3 bits act-order, 4 rows 8.0 -> 6.3.  Below the line 4096 x 1536, one
+    // row would be 3.1 -> 3.6 and 1024 x 1024 2.2 -> 2.8; rows in act-order gain less than they vary by from 57 strips on.
+    s.split = 1;
+    if (ctas_per_sm == 0 && !(permuted && M <= 8 && s.strips > 56))
+        for (int split = 4; split > 1 && s.split == 1; split /= 2) {
+            const int unit = M == 1 ? 6 : (M <= 8 ? 7 : 14), many = s.strips > 48 ? s.strips - 48 : 0;
+            const int cluster = 150 + many + (gather ? 60 + 2 * many : 0) + (bits == 8 ? 60 : 0);
+            if (s.strips * split <= sm_count() && 10 * unit * (s.units - s.units / split) > 11 * cluster) s.split = split;
+        }
+    s.cta_units = (s.units + s.split - 1) / s.split;
     // One and two rows: planes of x where they pay and fit; one row: x kept whole.  Planes take a CTA longer to prepare than x in operand
     // order and save on every strip and unit, so they pay where a warp has several units, or several strips of one.  Times as fast as
     // fp16, in a chain of such layers and with a small kernel before each, as in a decode step:
@@ -85,11 +99,11 @@ int gemv_strip_prepare(GemvStripPlan* p, const int32_t* qweight, const int32_t* 
     //                three strips on planes and 182 without, and 201 with seven on planes and 206 without
     //   one strip    4 bits, one row of 4096 1.02 and 1.03, of 11008 1.11, with a gather of 8192 1.07 and 4096 0.97 and 0.99; two rows with a
     //                gather 1.05 to 1.11, without 1.02 and 0.96
-    const int plane_bytes = (s.units * M * 4 * int_factors(sub) + 15) / 16 * 16 + s.units * M * (bits == 3 ? 5 : 4) * 128;
-    const bool one_strip = bits == 4 && (M == 1 ? sub == 1 && s.units >= (gather ? 64 : 32) : gather && s.units >= 32);
+    const int plane_bytes = (s.cta_units * M * 4 * int_factors(sub) + 15) / 16 * 16 + s.cta_units * M * (bits == 3 ? 5 : 4) * 128;
+    const bool one_strip = bits == 4 && (M == 1 ? sub == 1 && s.cta_units >= (gather ? 64 : 32) : gather && s.cta_units >= 32);
     const bool two_strips = bits == 3 ? M == 1 && !gather
-                          : (bits == 2 && M == 1) || (s.units > 16 && !(sub == 4 && M == 2 && !gather && s.units > 32));
-    const bool more_strips = bits == 3 ? M == 1 || s.per_cta > 4 : (bits == 2 && M == 1) || s.units >= 16;
+                          : (bits == 2 && M == 1) || (s.cta_units > 16 && !(sub == 4 && M == 2 && !gather && s.cta_units > 32));
+    const bool more_strips = bits == 3 ? M == 1 || s.per_cta > 4 : (bits == 2 && M == 1) || s.cta_units >= 16;
     const bool planes_pay = s.per_cta == 1 ? one_strip : (s.per_cta == 2 ? two_strips : more_strips);
     int mode = M <= 2 && int_takes(bits, sub) && planes_pay && plane_bytes <= 96 * 1024 ? kInt : (M == 1 && K <= 65536 ? kOne : kSeveral);
     const int nt = M <= 8 ? 1 : 2;
@@ -99,7 +113,7 @@ int gemv_strip_prepare(GemvStripPlan* p, const int32_t* qweight, const int32_t* 
     // Zero-points of several groups: one box is 3 to 5 % faster (4 bits in groups of 32, 4096 x 4096 4.68 -> 4.46 us; 8 bits, 16 rows of 4096 x
     // 12288 27.5 -> 22.1).  4 bits in several passes of one strip, 16 bytes of a row at a time: a box each is faster up to K = 5120 (4096 x 12288, one
     // row 12.1 -> 10.5, three rows 15.0 -> 13.4; 5120 x 10240 15.2 -> 14.6), slower for 11008 x 12288 (23.6 -> 25.7).
-    auto zeros_apart = [&](int t) { return bits % 4 != 0 || (bits == 4 && s.rows_g > 1 && t == 1 && s.per_cta > 1 && s.units <= 64); };
+    auto zeros_apart = [&](int t) { return bits % 4 != 0 || (bits == 4 && s.rows_g > 1 && t == 1 && s.per_cta > 1 && s.cta_units <= 64); };
     struct Choice { int W, T, ring, fixed, bufs, cost; };
     auto choose = [&](int W) {
         Choice c = {W, 0, 0, 0, 0, 1 << 30};
@@ -111,13 +125,13 @@ int gemv_strip_prepare(GemvStripPlan* p, const int32_t* qweight, const int32_t* 
         for (int bufs = 5; bufs >= (mode == kSeveral && !gather ? 2 : 5) && (nt == 2 || c.bufs != 5); --bufs)
             for (int t = 1; t <= tmax && t <= s.per_cta; ++t) {
                 const int slot = slot_bytes(bits, t) + const_bytes(bits, t, s.rows_g, zeros_apart(t));
-                const int sums = W * M * t * kStripCols * 4, copy = gather || mode == kOne || (mode == kInt && bits != 4) ? M * K * 2 : 0;
+                const int others = (s.split - 1) * M * kStripCols * 4, sums = W * M * t * kStripCols * 4, copy = gather || mode == kOne || (mode == kInt && bits != 4) ? M * K * 2 : 0;
                 const int x = mode == kInt ? plane_bytes
-                            : (mode == kOne ? s.units * kUnit * 2 : (bufs == 5 ? s.units : bufs * W) * M * kXPitch * 2);
-                const int f = x + (sums > copy ? sums : copy) + 1024, r = (kSmemMax - f) / (W * slot);
+                            : (mode == kOne ? s.cta_units * kUnit * 2 : (bufs == 5 ? s.cta_units : bufs * W) * M * kXPitch * 2);
+                const int f = x + (sums > copy ? sums : copy) + others + 1024, r = (kSmemMax - f) / (W * slot);
                 const int cost = ((s.per_cta + t - 1) / t) * (2 * t + 1);
                 const int least = bufs == 3 || bufs == 4 ? 3 : 2;
-                if (bufs != 5 && bufs > 2 && s.units / W < bufs - 1) continue;
+                if (bufs != 5 && bufs > 2 && s.cta_units / W < bufs - 1) continue;
                 if (f < kSmemMax && r >= least && (cost < c.cost || (cost == c.cost && bufs == c.bufs))) c = {W, t, r, f, bufs, cost};
             }
         return c;
@@ -138,7 +152,7 @@ int gemv_strip_prepare(GemvStripPlan* p, const int32_t* qweight, const int32_t* 
     }
     if (nt == 1 && ctas_per_sm <= 1) {
         const Choice w = choose(16);
-        const bool pays = s.units >= 16 && 10 * w.cost <= 11 * c.cost && (mode != kOne || K <= 16384);
+        const bool pays = s.cta_units >= 16 && 10 * w.cost <= 11 * c.cost && (mode != kOne || K <= 16384);
         if (w.T && (ctas_per_sm == 1 || !c.T || pays)) c = w;
     }
     if (!c.T) return B200GPTQ_ERR_TOO_LARGE;
@@ -146,13 +160,15 @@ int gemv_strip_prepare(GemvStripPlan* p, const int32_t* qweight, const int32_t* 
     s.passes = (s.per_cta + T - 1) / T;
     s.x_bufs = c.bufs == 5 ? 2 : c.bufs;
     if (c.bufs != 5) mode = kTurns;
-    const int longest = ((s.units + W - 1) / W) * s.passes;
+    const int longest = ((s.cta_units + W - 1) / W) * s.passes;
+    const int sums = W * M * T * kStripCols * 4, copy = gather || mode == kOne || (mode == kInt && bits != 4) ? M * K * 2 : 0;
+    s.others = sums > copy ? sums : copy;
     s.ring = c.ring < longest ? c.ring : longest;
     if (s.ring > kMaxRing) s.ring = kMaxRing;
     p->warps = W + idle_warps(W, mode == kSeveral, nt);
     const bool apart = zeros_apart(T);
     p->smem = W * s.ring * (slot_bytes(bits, T) + const_bytes(bits, T, s.rows_g, apart)) + c.fixed;
-    p->kernel = strip_kernel(bits, sub, mode, nt, T, W, apart);
+    p->kernel = strip_kernel(bits, sub, mode, nt, T, W, apart, s.split > 1);
     if (!p->kernel) return B200GPTQ_ERR_SHAPE;
     // (only the one that is used: raising the limit loads a kernel, and there are a hundred)
     B200GPTQ_CUDA_TRY(cudaFuncSetAttribute(p->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
@@ -187,15 +203,18 @@ int gemv_strip_run(const GemvStripPlan* p, const __half* x, const int32_t* x_per
                    const __half* bias, __half* y, void* workspace, cudaStream_t stream) {
     unsigned int* status = reinterpret_cast<unsigned int*>(workspace);
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(p->plan.strips < sm_count() ? p->plan.strips : sm_count());
+    cfg.gridDim = dim3(p->plan.split > 1 ? p->plan.strips * p->plan.split : (p->plan.strips < sm_count() ? p->plan.strips : sm_count()));
     cfg.blockDim = dim3(32 * p->warps);
     cfg.dynamicSmemBytes = p->smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = p->plan.split;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = p->plan.split > 1 ? 2 : 1;
     int M = p->M, K = p->K, N = p->N;
     void* args[] = {const_cast<CUtensorMap*>(&p->tmap_w), const_cast<CUtensorMap*>(&p->tmap_s),
                     const_cast<CUtensorMap*>(&p->tmap_z), &x, &x_perm, &bias, &y, &M, &K, &N,
@@ -204,21 +223,21 @@ int gemv_strip_run(const GemvStripPlan* p, const __half* x, const int32_t* x_per
     return B200GPTQ_OK;
 }
 
-GemvStripPlan* gemv_strip_plan_create(const int32_t* qweight, const int32_t* qzeros, const __half* scales, bool gather, int M, int K, int N, int bits, int group_size,
+GemvStripPlan* gemv_strip_plan_create(const int32_t* qweight, const int32_t* qzeros, const __half* scales, bool gather, bool permuted, int M, int K, int N, int bits, int group_size,
                                       int ctas_per_sm, int xact, int* status_out) {
     GemvStripPlan* p = new (std::nothrow) GemvStripPlan;
     if (!p) { *status_out = B200GPTQ_ERR_CUDA; return nullptr; }
-    *status_out = gemv_strip_prepare(p, qweight, qzeros, scales, gather, M, K, N, bits, group_size, ctas_per_sm, xact);
+    *status_out = gemv_strip_prepare(p, qweight, qzeros, scales, gather, permuted, M, K, N, bits, group_size, ctas_per_sm, xact);
     if (*status_out != B200GPTQ_OK) { delete p; return nullptr; }
     return p;
 }
 void gemv_strip_plan_destroy(GemvStripPlan* p) { delete p; }
 
 int gemv_strip_dispatch(const __half* x, const int32_t* qweight, const int32_t* qzeros, const __half* scales,
-                        const int32_t* x_perm, const __half* bias, __half* y, int M, int K, int N, int bits, int group_size,
+                        const int32_t* x_perm, bool permuted, const __half* bias, __half* y, int M, int K, int N, int bits, int group_size,
                         void* workspace, int ctas_per_sm, int xact, cudaStream_t stream) {
     GemvStripPlan p;
-    if (int st = gemv_strip_prepare(&p, qweight, qzeros, scales, x_perm != nullptr, M, K, N, bits, group_size, ctas_per_sm, xact)) return st;
+    if (int st = gemv_strip_prepare(&p, qweight, qzeros, scales, x_perm != nullptr, permuted, M, K, N, bits, group_size, ctas_per_sm, xact)) return st;
     return gemv_strip_run(&p, x, x_perm, bias, y, workspace, stream);
 }
 

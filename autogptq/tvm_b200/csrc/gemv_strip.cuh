@@ -377,6 +377,9 @@ struct StripPlan {
     int x_bufs;       // several rows of which x is not kept: places of a warp, 2..4, used in turn
     int gather;       // x is picked through x_perm from a copy of it in shared memory
     int xact;         // activation applied to x as it is read: 0 none, 1 SwiGLU, 2 ReLU
+    int split;        // CTAs (a cluster) that share a strip, a run of units each
+    int cta_units;    // units of a CTA, at most
+    int others;       // where the first of them keeps the others' sums (bytes behind the place of its own)
 };
 
 // A slot: weights (1024-byte aligned for the swizzle), and in a second ring the scales [group][32 T] and the zero-point
@@ -414,7 +417,9 @@ __device__ __forceinline__ uint32_t act_swiglu2(uint32_t gv, uint32_t uv) {
 // against 16.6 (and 14.3 against 14.1 where nothing is gathered).
 __host__ __device__ constexpr int idle_warps(int W, bool kept, int nt) { return W == 8 && kept && nt == 1 ? 3 : 0; }
 // APART: a box for the zero-points of each group.
-template <int BITS, int SUB, int NT, int MODE, int T, int W, bool APART>
+// SPLIT: the layer has fewer strips than half the SMs, so that clusters of plan.split CTAs share one, a run of K each; they push their sums
+// into the first one's shared memory, which adds them in their order.
+template <int BITS, int SUB, int NT, int MODE, int T, int W, bool APART, bool SPLIT = false>
 __global__ void __maxnreg__(W == 16 ? 120 : NT == 1 ? 168 : 224)
 gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_s,
                   const __grid_constant__ CUtensorMap tmap_z, const __half* __restrict__ x,
@@ -437,9 +442,15 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     // The runs start evenly over the columns and all have per_cta strips: neighbours may share a strip, both then write
     // the same bits.  (A grid of fewer, disjoint runs left SMs idle, and the next launch, which becomes resident beside
     // this one, put two of its CTAs on each of those: up to twice the time.)
-    const int strip0 = min((int)(((long long)blockIdx.x * plan.strips) / gridDim.x), plan.strips - plan.per_cta);
+    uint32_t rank = 0;
+    if constexpr (SPLIT) {
+        asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+        asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");     // (waited for before the sums are pushed: all have started)
+    }
+    const int strip0 = SPLIT ? (int)blockIdx.x / plan.split : min((int)(((long long)blockIdx.x * plan.strips) / gridDim.x), plan.strips - plan.per_cta);
     const int last_window = plan.per_cta - T;     // (so is the last pass's window)
-    const int u_begin = (warp * plan.units) / W, nu = ((warp + 1) * plan.units) / W - u_begin;
+    const int u_cta = SPLIT ? (int)rank * plan.units / plan.split : 0, n_cta = SPLIT ? ((int)rank + 1) * plan.units / plan.split - u_cta : plan.units;
+    const int u_begin = u_cta + (warp * n_cta) / W, nu = u_cta + ((warp + 1) * n_cta) / W - u_begin;
     const int total = plan.passes * nu;           // boxes of this warp
 
     // shared memory: rings | x | sums of the warps, and in the same bytes: x as it lies in memory
@@ -451,11 +462,12 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     // one row: [unit][quad lane][16 registers]; planes: [unit][step]..., then (factor, sum) [unit][row]; several rows:
     // [unit][row][natural halves], or a few units in turn per warp
     const int unit_x = ONE ? kUnit * 2 : (INT ? int_unit_bytes<BITS>(M) : M * kXPitch * 2);
-    const int x_units = TURNS ? plan.x_bufs * W : plan.units;
-    uint8_t* p_x = base_x + (size_t)(TURNS ? plan.x_bufs * warp : u_begin) * unit_x;
+    const int cta_units = SPLIT ? plan.cta_units : plan.units;
+    const int x_units = TURNS ? plan.x_bufs * W : cta_units;
+    uint8_t* p_x = base_x + (size_t)(TURNS ? plan.x_bufs * warp : u_begin - u_cta) * unit_x;
     constexpr int FACTORS = int_factors(SUB);
-    float* p_f = reinterpret_cast<float*>(base_x + (size_t)plan.units * unit_x) + (size_t)u_begin * M * FACTORS;
-    uint8_t* base_r = base_x + (size_t)x_units * unit_x + (INT ? (plan.units * M * FACTORS * 4 + 15) / 16 * 16 : 0);
+    float* p_f = reinterpret_cast<float*>(base_x + (size_t)cta_units * unit_x) + (size_t)(u_begin - u_cta) * M * FACTORS;
+    uint8_t* base_r = base_x + (size_t)x_units * unit_x + (INT ? (cta_units * M * FACTORS * 4 + 15) / 16 * 16 : 0);
     float* red = reinterpret_cast<float*>(base_r);                                 // [warp][m][column of the pass]
     unsigned short* raw = reinterpret_cast<unsigned short*>(base_r);               // [m][k]
     const uint32_t bar0 = smem_u32(bars) + 8u * (warp * kMaxRing);
@@ -1115,6 +1127,28 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                 }
         __syncthreads();
         const int n0 = (strip0 + win) * kStripCols;
+        float2* others = nullptr;
+        if constexpr (SPLIT) {
+            // (one pass) the sums of the cluster's other CTAs, [CTA - 1][m][column]
+            others = reinterpret_cast<float2*>(base_r + plan.others);
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+            if (rank != 0)
+                for (int i = tid; i < M * (COLS / 2); i += 32 * W) {
+                    const int m = i / (COLS / 2), c = 2 * (i % (COLS / 2));
+                    float2 v = make_float2(0.f, 0.f);
+#pragma unroll
+                    for (int w = 0; w < W; ++w) {
+                        const float2 r = *reinterpret_cast<const float2*>(red + ((size_t)w * M + m) * COLS + c);
+                        v.x += r.x; v.y += r.y;
+                    }
+                    uint32_t to;
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(smem_u32(others + (rank - 1) * M * (COLS / 2) + i)), "r"(0));
+                    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(to), "f"(v.x), "f"(v.y) : "memory");
+                }
+            asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+            if (rank != 0) break;
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        }
         for (int i = tid; i < M * (COLS / 2); i += 32 * W) {
             const int m = i / (COLS / 2), c = 2 * (i % (COLS / 2));
             float2 v = make_float2(0.f, 0.f);
@@ -1123,6 +1157,11 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                 const float2 r = *reinterpret_cast<const float2*>(red + ((size_t)w * M + m) * COLS + c);
                 v.x += r.x; v.y += r.y;
             }
+            if constexpr (SPLIT)
+                for (int r = 0; r < plan.split - 1; ++r) {
+                    const float2 o = others[r * M * (COLS / 2) + i];
+                    v.x += o.x; v.y += o.y;
+                }
             if (!INT) { v.x *= L::kScale; v.y *= L::kScale; }
             if (bias) {
                 v.x += __half2float(bias[n0 + c]);
@@ -1134,14 +1173,15 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     if (!ok) atomicExch(status + kStatusWord, 1u);
 }
 
-// The instantiation for (groups scaled apart in a unit, mode, rows of x / 8, strips of a pass, warps, zero-points in a box each), nullptr
-// where there is none.
+// The instantiation for (groups scaled apart in a unit, mode, rows of x / 8, strips of a pass, warps, zero-points in a box each, CTAs that share a
+// strip), nullptr where there is none.
 template <int BITS, int SUB, int NT, int MODE, int W>
-const void* strip_kernel_t(int T, bool apart) {
+const void* strip_kernel_t(int T, bool apart, bool split) {
     constexpr bool APART = BITS % 4 != 0;
     if constexpr (BITS == 4 && SUB == 4)
-        if (T == 1 && apart) return reinterpret_cast<const void*>(gemv_strip_kernel<BITS, SUB, NT, MODE, 1, W, true>);
+        if (T == 1 && apart && !split) return reinterpret_cast<const void*>(gemv_strip_kernel<BITS, SUB, NT, MODE, 1, W, true>);
     if (apart != APART) return nullptr;
+    if (split) return T == 1 ? reinterpret_cast<const void*>(gemv_strip_kernel<BITS, SUB, NT, MODE, 1, W, APART, true>) : nullptr;
     if (T == 1) return reinterpret_cast<const void*>(gemv_strip_kernel<BITS, SUB, NT, MODE, 1, W, APART>);
     if (T == 2) return reinterpret_cast<const void*>(gemv_strip_kernel<BITS, SUB, NT, MODE, 2, W, APART>);
     if constexpr (NT == 1 && SUB == 1)
@@ -1151,20 +1191,20 @@ const void* strip_kernel_t(int T, bool apart) {
     return nullptr;
 }
 template <int BITS, int SUB, int W>
-const void* strip_kernel_m(int mode, int nt, int T, bool apart) {
+const void* strip_kernel_m(int mode, int nt, int T, bool apart, bool split) {
     if constexpr (int_takes(BITS, SUB))
-        if (mode == kInt) return strip_kernel_t<BITS, SUB, 1, kInt, W>(T, apart);
-    if (mode == kOne) return strip_kernel_t<BITS, SUB, 1, kOne, W>(T, apart);
+        if (mode == kInt) return strip_kernel_t<BITS, SUB, 1, kInt, W>(T, apart, split);
+    if (mode == kOne) return strip_kernel_t<BITS, SUB, 1, kOne, W>(T, apart, split);
     if (nt == 1)
-        return mode == kTurns ? strip_kernel_t<BITS, SUB, 1, kTurns, W>(T, apart) : strip_kernel_t<BITS, SUB, 1, kSeveral, W>(T, apart);
+        return mode == kTurns ? strip_kernel_t<BITS, SUB, 1, kTurns, W>(T, apart, split) : strip_kernel_t<BITS, SUB, 1, kSeveral, W>(T, apart, split);
     if constexpr (W == 8)
-        return mode == kTurns ? strip_kernel_t<BITS, SUB, 2, kTurns, W>(T, apart) : strip_kernel_t<BITS, SUB, 2, kSeveral, W>(T, apart);
+        return mode == kTurns ? strip_kernel_t<BITS, SUB, 2, kTurns, W>(T, apart, split) : strip_kernel_t<BITS, SUB, 2, kSeveral, W>(T, apart, split);
     return nullptr;
 }
 template <int BITS>
-const void* strip_kernel_bits(int sub, int mode, int nt, int T, int warps, bool apart) {
-    if (warps == 8) return sub == 1 ? strip_kernel_m<BITS, 1, 8>(mode, nt, T, apart) : strip_kernel_m<BITS, 4, 8>(mode, nt, T, apart);
-    return sub == 1 ? strip_kernel_m<BITS, 1, 16>(mode, nt, T, apart) : strip_kernel_m<BITS, 4, 16>(mode, nt, T, apart);
+const void* strip_kernel_bits(int sub, int mode, int nt, int T, int warps, bool apart, bool split) {
+    if (warps == 8) return sub == 1 ? strip_kernel_m<BITS, 1, 8>(mode, nt, T, apart, split) : strip_kernel_m<BITS, 4, 8>(mode, nt, T, apart, split);
+    return sub == 1 ? strip_kernel_m<BITS, 1, 16>(mode, nt, T, apart, split) : strip_kernel_m<BITS, 4, 16>(mode, nt, T, apart, split);
 }
 
 }  // namespace

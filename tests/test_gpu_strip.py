@@ -176,3 +176,32 @@ def test_folded_activation_equals_the_kernel_in_front(bits, K, gated, M):
     args = (layer.qweight, layer.qzeros, layer.scales, None, bits, 128)
     assert torch.equal(ops.gemv(u, *args, input_act=1 if gated else 2), ops.gemv(a, *args))
     ops.check_status(DEV)
+
+
+@pytest.mark.parametrize("bits,K,N,gs,gather,M", [
+    # four CTAs per strip (up to 37 strips): the shortest K of one row and of sixteen; units that do not divide; a cut last unit
+    (4, 4864, 32, 128, False, 1), (4, 8032, 1184, 32, False, 2), (3, 8064, 1024, 128, True, 8), (2, 11008, 1024, 128, False, 16),
+    (8, 10496, 1152, 128, False, 5), (4, 2176, 1024, 128, False, 16), (4, 2208, 992, 96, True, 9), (3, 10272, 64, -1, False, 3),
+    # two CTAs (up to 74 strips); the largest and smallest number of them
+    (4, 9856, 1856, 64, False, 2), (4, 11008, 2368, 128, False, 8), (3, 8992, 1216, 128, True, 1), (8, 7168, 2304, 128, False, 12),
+    (2, 8192, 1536, 64, False, 4), (4, 40960, 1536, 128, False, 1),
+    # one strip more, or a little less K: unsplit
+    (4, 11008, 2400, 128, False, 8), (4, 4608, 1024, 128, False, 1), (4, 11008, 1824, 128, True, 4),
+])
+def test_layers_of_few_strips_vs_oracle(bits, K, N, gs, gather, M):
+    """Clusters of CTAs that share a strip, against the oracle (test_gemv_vs_oracle's bound), and the same bits every time."""
+    layer = synth.make_layer(bits, K, N, gs, False, bias=N % 96 == 0, seed=K + N + bits)
+    _, _, W = O.dequantize(layer.qweight.numpy(), layer.qzeros.numpy(), layer.scales.numpy(), layer.g_idx.numpy(), bits)
+    x = synth.make_x(M, K, seed=M)
+    perm = torch.randperm(K, generator=torch.Generator().manual_seed(K)).to(torch.int32) if gather else None
+    xg = x if perm is None else x[:, perm.long()]
+    d = layer.to(DEV)
+    plan = ops.GemvPlan(d.qweight, d.qzeros, d.scales, None, None if perm is None else perm.to(DEV), d.bias, M, bits,
+                        gs if gs != -1 else K, None, 0)
+    y = plan.run(x.to(DEV))
+    assert torch.equal(y, plan.run(x.to(DEV)))
+    ops.check_status(DEV)
+    ref = O.forward_fp64(xg.numpy(), W, None if layer.bias is None else layer.bias.numpy())
+    err = np.abs(y.cpu().numpy().astype(np.float64) - ref)
+    bound = 2.0 ** -11 * np.abs(ref) + 2.0 ** -11 * np.linalg.norm(xg.numpy().astype(np.float64), axis=1)[:, None] * np.abs(W.astype(np.float64)).max()
+    assert np.all(err <= bound), (err / bound).max()
