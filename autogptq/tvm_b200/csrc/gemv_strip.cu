@@ -100,11 +100,14 @@ int gemv_strip_prepare(GemvStripPlan* p, const int32_t* qweight, const int32_t* 
     //   one strip    4 bits, one row of 4096 1.02 and 1.03, of 11008 1.11, with a gather of 8192 1.07 and 4096 0.97 and 0.99; two rows with a
     //                gather 1.05 to 1.11, without 1.02 and 0.96
     const int plane_bytes = (s.cta_units * M * 4 * int_factors(sub) + 15) / 16 * 16 + s.cta_units * M * (bits == 3 ? 5 : 4) * 128;
-    const bool one_strip = bits == 4 && (M == 1 ? sub == 1 && s.cta_units >= (gather ? 64 : 32) : gather && s.cta_units >= 32);
+    const bool one_strip = bits == 4 && (M == 1 ? s.cta_units >= (gather ? 64 : 32) : gather && s.cta_units >= 32);
     const bool two_strips = bits == 3 ? M == 1 && !gather
                           : (bits == 2 && M == 1) || (s.cta_units > 16 && !(sub == 4 && M == 2 && !gather && s.cta_units > 32));
     const bool more_strips = bits == 3 ? M == 1 || s.per_cta > 4 : (bits == 2 && M == 1) || s.cta_units >= 16;
-    const bool planes_pay = s.per_cta == 1 ? one_strip : (s.per_cta == 2 ? two_strips : more_strips);
+    // One row in groups scaled apart, two groups to a product (gemv_strip.cuh): one strip, K from 3072 on 1.08 to 1.18 (11008 x 4096 9.05 -> 7.95 us),
+    // 2048 0.96 to 1.02; more strips, K from 1536 on 1.10 to 1.33 (8192 x 8192 9.9 -> 8.1, 4096 x 12288 9.8 -> 8.5), 1024 1.07 to 1.19.
+    const bool paired = bits == 4 && sub == 4 && M == 1;
+    const bool planes_pay = paired ? s.cta_units > (s.per_cta == 1 ? 16 : 7) : s.per_cta == 1 ? one_strip : (s.per_cta == 2 ? two_strips : more_strips);
     int mode = M <= 2 && int_takes(bits, sub) && planes_pay && plane_bytes <= 96 * 1024 ? kInt : (M == 1 && K <= 65536 ? kOne : kSeveral);
     const int nt = M <= 8 ? 1 : 2;
     s.rows_g = sub == 1 ? 1 : (s.spg == 1 ? 4 : (s.spg == 2 ? 2 : 3));
@@ -160,6 +163,7 @@ int gemv_strip_prepare(GemvStripPlan* p, const int32_t* qweight, const int32_t* 
     s.passes = (s.per_cta + T - 1) / T;
     s.x_bufs = c.bufs == 5 ? 2 : c.bufs;
     if (c.bufs != 5) mode = kTurns;
+    if (mode == kInt && paired) mode = kIntOne;
     const int longest = ((s.cta_units + W - 1) / W) * s.passes;
     const int sums = W * M * T * kStripCols * 4, copy = gather || mode == kOne || (mode == kInt && bits != 4) ? M * K * 2 : 0;
     s.others = sums > copy ? sums : copy;

@@ -22,6 +22,8 @@
 //    (4 bits |X| < 2^26, exact for every element within 2^-16 of the largest; 2 and 3 bits 2^22 and 2^-12), shifted by what
 //    its weight byte lacks and split into four signed byte planes, which are columns of the B operand.  mma.sync m16n8k32
 //    u8 x s8 costs what m16n8k16 f16 does and does twice the products; the fp16 form below needs 2.3 times the instructions.
+//    One row with groups of 32, 64 or 96 rows: a product serves two groups, so that scaling their sums, four times a unit, is done by all
+//    lanes (half of them had zeros: 4 bits, 8192 x 8192 9.9 -> 8.1 us, 11008 x 12288 23.6 -> 20.0).
 //    Used where K is long enough for what the planes take to prepare (the plan in gemv_strip.cu has the measurements).
 //  * Otherwise fp16.  4- and 8-bit fields are used as fp16 subnormals: a field masked in place at bit p of its half IS q * 2^(p - 24), so
 //    unpacking is one AND (4 bits: and one shift per two words); the two positions of a nibble go to different
@@ -361,8 +363,9 @@ __host__ __device__ constexpr int int_x_bits(int bits) { return bits == 4 ? 26 :
 __host__ __device__ constexpr bool int_takes(int bits, int sub) { return bits == 4 || (bits != 8 && sub == 1); }
 
 // How x meets the weights: several rows in fp16, every unit's x kept or a few units at a time in turn; one row in fp16; one or two rows as
-// byte planes.  (The first two in one form, with a branch per unit, were 3 % slower for nine rows and more.)
-enum { kSeveral = 0, kOne = 1, kInt = 2, kTurns = 3 };
+// byte planes, one row with groups scaled apart in a form of its own.  (The first two in one form, with a branch per unit, were 3 % slower for
+// nine rows and more; the last two 6 % for two rows.)
+enum { kSeveral = 0, kOne = 1, kInt = 2, kTurns = 3, kIntOne = 4 };
 
 struct StripPlan {
     int units;        // units of 128 rows along K (the last one may be cut)
@@ -427,15 +430,16 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                   unsigned int* __restrict__ status) {
     using L = Layout<BITS, SUB == 1>;
     using I = IntLayout<BITS, SUB == 1 || BITS != 4>;
-    constexpr bool ONE = MODE == kOne, INT = MODE == kInt, KEPT = MODE == kSeveral, TURNS = MODE == kTurns, ROWS = KEPT || TURNS;
+    constexpr bool ONE = MODE == kOne, PAIRED = MODE == kIntOne, INT = MODE == kInt || PAIRED, KEPT = MODE == kSeveral, TURNS = MODE == kTurns, ROWS = KEPT || TURNS;
     static_assert(!INT || (NT == 1 && int_takes(BITS, SUB)), "not a case of the integer path");
+    static_assert(!PAIRED || (BITS == 4 && SUB == 4), "not a case of paired groups");
     constexpr int STRIP_BYTES = L::kRows * 128, STEPS = 4 / SUB, SLOT = slot_bytes(BITS, T);
     constexpr int NC = ROWS ? 2 : 1;             // rows of x per lane and n-tile that exist
     constexpr int COLS = T * kStripCols;
     extern __shared__ __align__(1024) uint8_t dsm[];
     __shared__ __align__(8) uint64_t bars[W * kMaxRing];
 
-    const int M = ONE ? 1 : M_rows;
+    const int M = ONE || PAIRED ? 1 : M_rows;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, j = lane & 3;
     if (idle_warps(W, KEPT, NT) && warp >= W) return;     // (before any barrier)
     const int R = plan.ring;
@@ -885,7 +889,57 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                 const int early = BITS % 4 == 0 ? 0 : ((grp0 + r) * zwords + (strip0 + win) * BITS) & 3;
                 return cze + r * zero_pitch(BITS, T, APART) + 4 * early + t * BITS * 4;
             };
-            if constexpr (INT) {
+            if constexpr (PAIRED) {
+                // One row, groups of 32 rows scaled apart: its planes are four of the eight columns of B.  Two groups share a product: the
+                // first one's planes are columns 0..3 and lie along its first 16 rows of K, the second one's 4..7 and along the others,
+                // zeros elsewhere; A has half of each group's rows.  As many products, and what follows them is done for two groups
+                // at once, by lanes that had nothing to do: quad lanes 0, 1 hold the first group's planes, 2, 3 the second one's.
+                uint2 bq[2];
+                float cf[2], sx[2];
+                int r[2];
+                const float* f = p_f + u * FACTORS;
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    bq[q] = *reinterpret_cast<const uint2*>(p_x + (size_t)u * unit_x + ((2 * q + (g >> 2)) * 4 + j) * 32 + (g & 3) * 8);
+                    const int sub = 2 * q + (j >> 1);
+                    cf[q] = j & 1 ? f[sub] * 65536.f : f[sub];
+                    sx[q] = j & 1 ? 0.f : f[4 + sub];
+                    r[q] = group_at(step0 + sub) - grp0;
+                }
+                mbar_wait(bar0 + 8u * slot, parity, ok);
+#pragma unroll
+                for (int t = 0; t < T; ++t) {
+                    uint32_t w[4][I::kLoads];
+#pragma unroll
+                    for (int i = 0; i < I::kLoads; ++i) {
+                        const uint4 v = *reinterpret_cast<const uint4*>(src + read_at(t, I::load_row(i, j)));
+                        w[0][i] = v.x; w[1][i] = v.y; w[2][i] = v.z; w[3][i] = v.w;
+                    }
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) {
+                        const uint2 sv = *reinterpret_cast<const uint2*>(csc + (r[q] * T + t) * 64);
+                        const float2 s01 = __half22float2(*reinterpret_cast<const __half2*>(&sv.x));
+                        const float2 s23 = __half22float2(*reinterpret_cast<const __half2*>(&sv.y));
+                        const float sf[4] = {s01.x, s01.y, s23.x, s23.y};
+                        const uint32_t zv = load_zeros<BITS>(zero_at(r[q], t), 4 * g);
+                        const uint32_t lo0 = g < 4 ? bq[q].x : 0u, lo1 = g < 4 ? 0u : bq[q].x, hi0 = g < 4 ? bq[q].y : 0u, hi1 = g < 4 ? 0u : bq[q].y;
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            constexpr int kBias = 0x4B400000;
+                            int d[4] = {kBias, kBias, kBias, kBias};
+                            const uint32_t a0 = w[2 * h][2 * q], a1 = w[2 * h + 1][2 * q], a2 = w[2 * h][2 * q + 1], a3 = w[2 * h + 1][2 * q + 1];
+                            imma(d, d, a0 & 0x0f0f0f0fu, a1 & 0x0f0f0f0fu, a2 & 0x0f0f0f0fu, a3 & 0x0f0f0f0fu, lo0, lo1);
+                            imma(d, d, a0 & 0xf0f0f0f0u, a1 & 0xf0f0f0f0u, a2 & 0xf0f0f0f0u, a3 & 0xf0f0f0f0u, hi0, hi1);
+#pragma unroll
+                            for (int c = 0; c < 2; ++c) {
+                                const float zf = __uint_as_float(0x4B000000u | ((zv >> (BITS * (2 * h + c))) & ((1u << BITS) - 1u))) - 8388607.f;
+                                const float lo = __int_as_float(d[2 * c]) - 12582912.f, hi = __int_as_float(d[2 * c + 1]) - 12582912.f;
+                                out[t][0][2 * h + c][0] = fmaf(sf[2 * h + c], fmaf(fmaf(256.f, hi, lo), cf[q], zf * sx[q]), out[t][0][2 * h + c][0]);
+                            }
+                        }
+                    }
+                }
+            } else if constexpr (INT) {
                 uint2 bx[I::kSteps];
 #pragma unroll
                 for (int s = 0; s < I::kSteps; ++s) {
@@ -1105,6 +1159,7 @@ gemv_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     v[c] = out[t][0][c][0] + __shfl_xor_sync(0xffffffffu, out[t][0][c][0], 1);   // the row's other planes
+                    if (PAIRED) v[c] += __shfl_xor_sync(0xffffffffu, v[c], 2);         // the other groups
                     out[t][0][c][0] = 0.f;
                 }
                 if (!(j & 1) && (j >> 1) < M)
@@ -1194,6 +1249,8 @@ template <int BITS, int SUB, int W>
 const void* strip_kernel_m(int mode, int nt, int T, bool apart, bool split) {
     if constexpr (int_takes(BITS, SUB))
         if (mode == kInt) return strip_kernel_t<BITS, SUB, 1, kInt, W>(T, apart, split);
+    if constexpr (BITS == 4 && SUB == 4)
+        if (mode == kIntOne) return strip_kernel_t<BITS, SUB, 1, kIntOne, W>(T, apart, split);
     if (mode == kOne) return strip_kernel_t<BITS, SUB, 1, kOne, W>(T, apart, split);
     if (nt == 1)
         return mode == kTurns ? strip_kernel_t<BITS, SUB, 1, kTurns, W>(T, apart, split) : strip_kernel_t<BITS, SUB, 1, kSeveral, W>(T, apart, split);

@@ -205,3 +205,38 @@ def test_layers_of_few_strips_vs_oracle(bits, K, N, gs, gather, M):
     err = np.abs(y.cpu().numpy().astype(np.float64) - ref)
     bound = 2.0 ** -11 * np.abs(ref) + 2.0 ** -11 * np.linalg.norm(xg.numpy().astype(np.float64), axis=1)[:, None] * np.abs(W.astype(np.float64)).max()
     assert np.all(err <= bound), (err / bound).max()
+
+
+@pytest.mark.parametrize("K,N,gs,gather", [
+    (2080, 32, 32, False), (2208, 96, 96, True), (3104, 2048, 64, False), (11008, 4096, 32, True),      # one strip per CTA, the shortest K; cut units
+    (2048, 4096, 32, True),                                                                              # a little less: fp16
+    (928, 9632, 32, False), (1024, 4832, 64, True), (1056, 14432, 96, False), (2144, 19008, 32, True),   # more strips; seven units: fp16
+    (8192, 1024, 32, False), (7968, 1536, 64, True),                                                     # in clusters
+])
+def test_two_groups_to_a_product_vs_64_bits(K, N, gs, gather):
+    """One row, 4 bits, groups scaled apart: within the rounding of the result and what fixed point per 32 rows and fp32 sums may be off by,
+    where neighbouring groups differ by up to 2^23 in x and the scales make up for it (so that no group counts less than another, and
+    one that met the other's scale, zero-point or factor would show)."""
+    layer = synth.make_layer(4, K, N, gs, False, seed=K + N)
+    G = layer.scales.shape[0]
+    mag = 2.0 ** torch.tensor([[-10, 13, -9, 4, 0, -8, 7][g % 7] for g in range(G)], dtype=torch.float64)
+    gen = torch.Generator().manual_seed(6)
+    layer.scales = ((1 + torch.rand((G, N), generator=gen)) / mag[:, None]).half()
+    xs = (torch.randn((1, K), generator=gen).double() * mag[layer.g_idx.long()]).clamp(-60000, 60000).half()
+    perm = torch.randperm(K, generator=gen).to(torch.int32) if gather else None
+    x = xs.clone()
+    if gather:
+        x[:, perm.long()] = xs                              # row k of the layer multiplies x[perm[k]]
+    q, z, _ = O.dequantize(layer.qweight.numpy(), layer.qzeros.numpy(), layer.scales.numpy(), layer.g_idx.numpy(), 4)
+    g = layer.g_idx.numpy().astype(np.int64)
+    s, q, z = layer.scales.numpy().astype(np.float64)[g], q.astype(np.float64), z.astype(np.float64)[g]
+    d = layer.to(DEV)
+    plan = ops.GemvPlan(d.qweight, d.qzeros, d.scales, None, None if perm is None else perm.to(DEV), None, 1, 4, gs, None, 0)
+    y = plan.run(x.to(DEV))
+    assert torch.equal(y, plan.run(x.to(DEV)))
+    ops.check_status(DEV)
+    x64 = xs.numpy().astype(np.float64)
+    ref = x64 @ (s * (q - z))
+    bound = _bound_of_planes(4, x64, s * (q - z), s * (q + z), 32) + 2.0 ** -11 * np.abs(ref) + 2.0 ** -24
+    err = np.abs(y.cpu().numpy().astype(np.float64) - ref)
+    assert np.all(err <= bound), (err / bound).max()
