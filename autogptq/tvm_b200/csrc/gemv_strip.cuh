@@ -4,10 +4,11 @@
 //
 // One layer is 2..130 MB and lasts a few microseconds, so what counts is the chain of latencies of one launch as much as
 // bandwidth: start-up, the wait for the previous kernel, x, the products, the sum over K.  The split below has no
-// cluster, no scratch and no traffic between CTAs:
+// scratch and, from 75 strips of columns on, no cluster and no traffic between CTAs:
 //
 //  * The columns are cut into strips of 32; a CTA owns a run of strips over ALL of K, one CTA per SM.  Its warps split K
-//    in units of 128 rows and are added up through shared memory at the end.
+//    in units of 128 rows and are added up through shared memory at the end.  Where the strips would leave half the SMs
+//    idle and K is long, clusters of two or four CTAs share one (the rule and its figures: gemv_strip.cu).
 //  * Every warp streams its own units through its own ring: cp.async.bulk.tensor boxes of {32 columns, the unit's
 //    word-rows, strips} (128-byte swizzle), of the unit's scales and of its zero-points, one mbarrier per slot, no barrier of
 //    the CTA.  (16-byte cp.async by the lanes instead of the weight boxes: 13.0 against 7.0 us on 4096 x 12288, 4 bits;
@@ -18,7 +19,7 @@
 //    (one unit ahead is an L2 latency per unit: 16 rows, 9216 x 9216, 3 bits 29 us, two ahead 21).  Which k a lane multiplies
 //    is free as long as x is read in the same order.
 //  * One or two rows, 2 to 4 bits, whole units per group (4 bits: any groups): products on the integer tensor path.  A byte of weights
-//    is q << p, one AND per four fields and no shift; x is fixed point per unit, or per step where the groups of a unit are scaled apart
+//    is q << p, one AND per four fields and no shift (4 bits, whole units: no AND in one of the two products); x is fixed point per unit, or per step where the groups of a unit are scaled apart
 //    (4 bits |X| < 2^26, exact for every element within 2^-16 of the largest; 2 and 3 bits 2^22 and 2^-12), shifted by what
 //    its weight byte lacks and split into four signed byte planes, which are columns of the B operand.  mma.sync m16n8k32
 //    u8 x s8 costs what m16n8k16 f16 does and does twice the products; the fp16 form below needs 2.3 times the instructions.

@@ -73,8 +73,9 @@ int launch_pack(const int32_t* vals, int R, int C, int32_t* out, cudaStream_t st
 // writes its words, 128 bytes per warp and word-row.  (zero * scale, 1 / scale) of the 32 columns x all groups sit in
 // shared memory, column fastest, so that a look-up by any g_idx is one conflict-free 8-byte read; the rows are one entry
 // longer than the columns, so that the table is written without conflicts from coalesced reads of [N, G] too.  scales and
-// qzeros are left to CTAs of their own.  4096 x 11008, 4 bits, groups of 128 in act-order: 35 us; in order, where a row
-// block is one group and needs no look-ups, 31 us.
+// qzeros (and the copy of g_idx) are left to CTAs of their own.  4096 x 11008, 4 bits, groups of 128 in act-order: 35 us from fp16; in
+// order, where a row block is one group and needs no look-ups, 30 us.  fp16 weights of 2 to 4 bits have pack_pairs_kernel (26 and 25 us)
+// unless its table is too large; this kernel packs 8 bits, bf16 and fp32.
 //
 // What remains is the start of a CTA (its table) and the instructions of an element, 20 of them once (25 us at full issue):
 // - No IEEE division.  With r = 1 / s rounded, a * r is within a relative 2^-24 of a / s and the rounded quotient within

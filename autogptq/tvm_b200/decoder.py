@@ -27,6 +27,7 @@ from typing import List, Optional
 import torch
 import torch.distributed as dist
 import torch.nn.functional as F
+from torch.nn.modules import module as _module
 
 from . import _lib, ops, synth, tp
 from .qlinear import QuantLinear
@@ -370,25 +371,28 @@ class GPTQDecoder:
         """The layers of a decode step as one launch, for one sequence on one GPU and layers that the kernel takes; None where the
         kernels of a layer are launched one by one.  Everything that the plan points to is looked at in every step that is not replayed."""
         cfg = self.cfg
-        if self.world > 1 or self.batch != 1 or not self.one_launch:
+        if self.world > 1 or self.batch != 1 or not self.one_launch or _module._global_forward_hooks or _module._global_forward_pre_hooks:
             return None
         key, layers = [], []
 
-        def plain(t, *shape):
-            return t is not None and t.dtype is torch.float16 and t.shape == shape and t.is_contiguous() and t.device == self.pos.device
+        def plain(t, *shape, dtype=torch.float16):
+            return t is not None and t.dtype is dtype and t.shape == shape and t.is_contiguous() and t.device == self.pos.device
 
         H, rms = cfg.hidden, cfg.arch == "llama"
         sizes = ((H, 3 * H), (H, H), (H, (2 if rms else 1) * cfg.inter), (cfg.inter, H))
         for L in self.layers:
             linears = []
             for m, (K, N) in zip((L.qkv, L.o, L.up, L.down), sizes):
-                if (type(m) is not QuantLinear or m._forward_hooks or m._forward_pre_hooks or m.gemv_tuning is not None
+                if (type(m) is not QuantLinear or m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__ or m.gemv_tuning is not None
                         or m.exchange is not None or (m.bits, m.groupsize, m.infeatures, m.outfeatures) != (cfg.bits, cfg.group_size, K, N)):
                     return None
                 if not m._ready():
                     m.post_init()
-                if m._g_idx_run is not None:
-                    return None
+                groups = -(-K // m.groupsize)
+                if (m._g_idx_run is not None or not plain(m._qweight_run, K // 32 * m.bits, N, dtype=torch.int32)
+                        or not plain(m.qzeros, groups, N // 32 * m.bits, dtype=torch.int32) or not plain(m.scales, groups, N)
+                        or not (m.bias is None or plain(m.bias, N))):
+                    return None                    # (the layer's own call says what is wrong with them)
                 linears.append((m._qweight_run, m.qzeros, m.scales, m.bias, m._x_perm))
             cache = (1, cfg.heads, cfg.max_seq, cfg.head_dim)
             norms = (L.norm1_w, L.norm2_w) + (() if rms else (L.norm1_b, L.norm2_b))

@@ -473,7 +473,7 @@ class StepPlan:
     """The decoder layers of one decode step of one sequence as one launch (``b200gptq_step_plan_*``), prepared for fixed tensors, which
     it keeps."""
 
-    def __init__(self, handle: int, memory, keep):
+    def __init__(self, handle, memory, keep):
         self._handle, self._memory, self._keep = handle, memory, keep
 
     @classmethod
@@ -501,7 +501,7 @@ class StepPlan:
             if st in (-4, -8):       # (a tensor that is not aligned, a device that cannot hold a CTA per SM)
                 return None
             _lib.check(st, "b200gptq_step_plan_create")
-            plan = cls(handle.value, torch.zeros(need, dtype=torch.uint8, device=device), (layers, cos, sin, pos))
+            plan = cls(handle, torch.zeros(need, dtype=torch.uint8, device=device), (layers, cos, sin, pos))
             plan._memory[:host.numel()].copy_(host)
         return plan
 
@@ -511,6 +511,8 @@ class StepPlan:
         _need_cuda("x", x, torch.float16)
         ws = get_workspace(x.device, 1)
         with torch.cuda.device(x.device):
+            if not torch.cuda.is_current_stream_capturing():     # (a graph's owner keeps the plan)
+                self._memory.record_stream(torch.cuda.current_stream())
             st = _lib.lib.b200gptq_step_plan_run(self._handle, self._memory.data_ptr(), _ptr(x), _ptr(ws), _stream(x.device))
         if st == -8:
             return False
@@ -520,5 +522,7 @@ class StepPlan:
     def __reduce__(self):            # (it holds addresses of this process: a copy makes its own)
         return type(None), ()
 
-    def __del__(self):
-        _lib.lib.b200gptq_step_plan_destroy(self._handle)
+    def __del__(self, _finalizing=sys.is_finalizing):
+        h, self._handle = getattr(self, "_handle", None), None
+        if h and not _finalizing():
+            _lib.lib.b200gptq_step_plan_destroy(h)

@@ -106,6 +106,35 @@ def test_replaced_tensors_are_followed():
     _close(got, want, 2)
 
 
+@pytest.mark.parametrize("name,change,error", [
+    ("scales", lambda t: t.float(), TypeError), ("qzeros", lambda t: t.cpu(), RuntimeError), ("scales", lambda t: t.cpu(), RuntimeError)])
+def test_tensors_that_the_layers_refuse_are_refused(name, change, error):
+    m, text = _model("llama", 4, False, 2, 256, 2, 512, 12)
+    _steps(m, text, 12, True)
+    o = m.layers[1].o
+    setattr(o, name, change(getattr(o, name)))
+    assert m._step_plan() is None
+    for m.one_launch in (False, True):
+        with pytest.raises(error):
+            m._decode_step()
+
+
+def test_a_forward_of_one_layer_or_a_hook_of_all_is_called():
+    m, text = _model("llama", 4, False, 2, 256, 2, 512, 12)
+    want, _ = _steps(m, text, 12, True)
+    o, calls = m.layers[1].o, []
+    o.forward = lambda x: (calls.append(1), type(o).forward(o, x))[1]
+    _close(_steps(m, text, 12, True)[0], want, 2)
+    assert len(calls) == 5                               # the prompt and four steps
+    del o.forward
+    hook = torch.nn.modules.module.register_module_forward_hook(lambda mod, *a: calls.append(1) if mod is o else None)
+    try:
+        _steps(m, text, 12, True)
+    finally:
+        hook.remove()
+    assert len(calls) == 10 and m._step_plan() is not None
+
+
 def test_a_copy_makes_a_plan_of_its_own():
     m, text = _model("llama", 4, False, 2, 512, 4, 1024, 20)
     want, _ = _steps(m, text, 20, True)
