@@ -191,6 +191,7 @@ pack_linear_kernel(const T* __restrict__ weight, const float* __restrict__ scale
     float2* table = reinterpret_cast<float2*>(groups + 2 * kPackChunk);            // [G][33] (zero * scale, 1 / scale)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int n0 = blockIdx.x * kPackCols, n = n0 + lane;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int c_begin = blockIdx.y * chunks_per_cta, c_end = min((K + kPackChunk - 1) / kPackChunk, c_begin + chunks_per_cta);
     auto fetch = [&](int c, int buf) {
         const int k0 = c * kPackChunk;
@@ -324,6 +325,7 @@ pack_pairs_kernel(const __half* __restrict__ weight, const float* __restrict__ s
     int* groups = reinterpret_cast<int*>(pack_smem + 2 * sizeof(__half) * TILE);   // two of: groups of the chunk's rows
     uint2* table = reinterpret_cast<uint2*>(groups + 2 * kPairChunk);              // [G][17]: 1 / s of both columns, z' of both
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n0 = blockIdx.x * kPackCols;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     if (blockIdx.y == gridDim.y - 1) {
         pack_constants<BITS, kPairThreads>(scales, zeros, G, N, blockIdx.x, qzeros, scales_out, pack_smem, g_idx, K, g_idx_out);
         return;
@@ -463,6 +465,24 @@ int pack_split(int chunks, int strips, int resident, int G) {
     return per;
 }
 
+// Launched while the kernel in front ends (both kernels wait for it before they touch memory, and let none start before they have ended
+// themselves): layers one behind the other 28.8 -> 26.3 us for 4096 x 11008, 16.6 -> 14.9 for 1664 x 10720 in groups of 32.
+template <typename... P, typename... A>
+int launch_pack_early(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    B200GPTQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+    return B200GPTQ_OK;
+}
+
 template <int BITS>
 int launch_pack_pairs(const void* weight, const float* scales, const float* zeros, const int32_t* g_idx, int K, int N, int G,
                       int32_t* qweight, int32_t* qzeros, __half* scales_out, int32_t* g_idx_out, cudaStream_t stream) {
@@ -481,10 +501,8 @@ int launch_pack_pairs(const void* weight, const float* scales, const float* zero
     const int fit = (int)(220 * 1024 / (smem + 1024));
     const int per = pack_split(chunks, strips, sm_count() * (fit < kPairCtas ? fit : kPairCtas), G);
     dim3 grid(strips, (chunks + per - 1) / per + 1);
-    pack_pairs_kernel<BITS><<<grid, kPairThreads, smem, stream>>>(static_cast<const __half*>(weight), scales, zeros, g_idx, K, N, G, per,
-                                                                      qweight, qzeros, scales_out, g_idx_out);
-    B200GPTQ_CUDA_TRY(cudaGetLastError());
-    return B200GPTQ_OK;
+    return launch_pack_early(pack_pairs_kernel<BITS>, grid, kPairThreads, smem, stream, static_cast<const __half*>(weight), scales, zeros,
+                             g_idx, K, N, G, per, qweight, qzeros, scales_out, g_idx_out);
 }
 
 template <int BITS, typename T>
@@ -511,10 +529,8 @@ int launch_pack_linear(const void* weight, const float* scales, const float* zer
     const int resident = sm_count() * (smem * kPackCtas <= 220 * 1024 ? kPackCtas : (int)(220 * 1024 / smem));
     const int per = pack_split(chunks, strips, resident, G);
     dim3 grid(strips, (chunks + per - 1) / per + 1);
-    pack_linear_kernel<BITS, T><<<grid, kPackThreads, smem, stream>>>(static_cast<const T*>(weight), scales, zeros, g_idx, K, N,
-                                                                      G, per, use_table, qweight, qzeros, scales_out, g_idx_out);
-    B200GPTQ_CUDA_TRY(cudaGetLastError());
-    return B200GPTQ_OK;
+    return launch_pack_early(pack_linear_kernel<BITS, T>, grid, kPackThreads, smem, stream, static_cast<const T*>(weight), scales, zeros,
+                             g_idx, K, N, G, per, use_table, qweight, qzeros, scales_out, g_idx_out);
 }
 
 }  // namespace
