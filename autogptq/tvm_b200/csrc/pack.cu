@@ -301,7 +301,7 @@ pack_linear_kernel(const T* __restrict__ weight, const float* __restrict__ scale
 // 2^10 the integer in the low bits of a half, d = t - (u - 1.5 * 2^10).  For an integer in the range of the fields and |z'| <= 32 (a table
 // entry beyond that, or with 1 / s out of the normal numbers, is NaN) t is within 2^-11 (|w / s| + |z'|) + 2^-8 < 0.05 of the quotient,
 // |w / s| being less than 16 + |z'|; so where |d| <= 0.4375 the quotient is within 0.49 of that integer, and fp32 rounds it to the same.
-// Everything else (a half nearby, out of range, NaN, infinity) is redone with the division.
+// Everything else (a half nearby, out of range, NaN, infinity) is redone with the division, and so is column c + 16 where column c is out of range.
 //
 // A thread takes columns c and c + 16 of a 32-row block, a half-warp a block: both columns' rows lie in one group, so that (1 / s, z') of
 // both are one 8-byte look-up, and fields pile up in the two halves of a register.  (A column per thread, in fp32 17 instructions per
@@ -430,7 +430,8 @@ pack_pairs_kernel(const __half* __restrict__ weight, const float* __restrict__ s
             for (int h = 0; h < 2; ++h) {
                 const int n = n0 + col + 16 * h;
                 int32_t* out = qweight + (size_t)rb * BITS * N + n;
-                const uint32_t beyond = (h ? any >> 16 : any & 0xffffu) >> BITS, most = h ? far >> 16 : far & 0xffffu;
+                // (a field of the lower half that is out of range has been added to the upper half's sums as well)
+                const uint32_t beyond = (h ? (any >> 16) | (any & 0xffffu) : any & 0xffffu) >> BITS, most = h ? far >> 16 : far & 0xffffu;
                 if (beyond != 0u || most > kHalfFar) {
                     pack_divided<BITS, __half>(row + h * 16 * PITCH, gr, scales + (size_t)n * G, zeros + (size_t)n * G, out, N);
                 } else if constexpr (BITS == 3) {                  // seven pieces of 15 bits

@@ -110,9 +110,10 @@ def test_one_launch_pack_equals_the_cpu_packer(bits, K, N, gs, dtype):
     assert torch.equal(a.scales, b.scales.cpu())
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
 @pytest.mark.parametrize("bits", [2, 3, 4, 8])
 @pytest.mark.parametrize("K,N,gs", [(288, 32, 32), (4480, 64, 32)])     # (140 groups: more than one tile of the zero-points)
-def test_one_launch_pack_in_order_and_out_of_range(bits, K, N, gs):
+def test_one_launch_pack_in_order_and_out_of_range(bits, K, N, gs, dtype):
     """Rows in group order take no table; fields outside 0..2^bits-1 spill into their neighbours as the CPU route has them."""
     gen = torch.Generator().manual_seed(bits + K)
     G = K // gs
@@ -123,7 +124,8 @@ def test_one_launch_pack_in_order_and_out_of_range(bits, K, N, gs):
     for i, wrong in enumerate([-1., 2. ** bits, 300., -4194304., -9437184., 2.**24]):
         q[3 + i, 17 * i + 9] = wrong
     lin = nn.Linear(K, N, bias=False)
-    lin.weight.data = (q - zeros[:, sel]) * scales[:, sel]
+    W = (q - zeros[:, sel]) * scales[:, sel]
+    lin.weight.data = W if dtype is torch.float32 else W.clamp(-6e4, 6e4).to(dtype)          # (finite)
     a, b = QuantLinear(bits, gs, K, N, False), QuantLinear(bits, gs, K, N, False).to(DEV)
     a.pack(lin, scales, zeros)
     b.pack(lin.to(DEV), scales.to(DEV), zeros.to(DEV))
@@ -160,6 +162,45 @@ def test_fp16_weights_equal_the_cpu_packer(bits, K, N, gs):
     assert torch.equal(a.qweight, b.qweight.cpu())
     assert torch.equal(a.qzeros, b.qzeros.cpu())
     assert torch.equal(a.scales, b.scales.cpu())
+
+
+@pytest.mark.parametrize("act", [False, True])
+@pytest.mark.parametrize("wrong", [-1.0, "above", 300.0, "tiny scale", "huge scale", "zero-point"])
+@pytest.mark.parametrize("bits", [2, 3, 4])
+def test_fp16_columns_beside_one_that_is_redone(bits, wrong, act):
+    """Columns c and c + 16 of a strip are packed in the two halves of a register.  Every field is an integer in the range, so that no block
+    is redone, but for one field or one group's constants of columns c < 16 that send column c to the division: at each row of a block once, and
+    in each group; column c + 16, which is not redone, must not notice."""
+    K, N, gs = 1024, 96, 64
+    gen = torch.Generator().manual_seed(bits)
+    G, top = K // gs, 2 ** bits - 1
+    scales = 2.0 ** torch.randint(-8, -3, (N, G), generator=gen).float()
+    zeros = torch.randint(1, top + 1, (N, G), generator=gen).float()
+    g_idx = torch.arange(K) // gs
+    if act:
+        g_idx = g_idx[torch.randperm(K, generator=gen)]
+    q = torch.randint(0, top + 1, (N, K), generator=gen).float()
+    bad = [(32 * (g % 2) + g % 16, g) for g in range(G)]                   # columns 0..15 and 32..47, a group each
+    for n, g in bad:
+        if wrong == "tiny scale":
+            scales[n, g] = 2.0 ** -15.5
+        elif wrong == "huge scale":
+            scales[n, g], zeros[n, g] = 16384.0, 1.0
+            q[n, g_idx == g] = q[n, g_idx == g].clamp(max=3)
+        elif wrong == "zero-point":
+            zeros[n, g] = 40.0
+    if wrong not in ("tiny scale", "huge scale", "zero-point"):
+        for j in range(K // 32):                                           # row j of block j
+            q[32 * (j % 2) + j // 2, 32 * j + j] = top + 1.0 if wrong == "above" else wrong
+    sel = g_idx.long()
+    lin = nn.Linear(K, N, bias=False)
+    lin.weight.data = ((q - zeros[:, sel]) * scales[:, sel]).half()
+    a, b = QuantLinear(bits, gs, K, N, False), QuantLinear(bits, gs, K, N, False).to(DEV)
+    a.pack(lin, scales, zeros, g_idx.to(torch.int32))
+    b.pack(lin.to(DEV), scales.to(DEV), zeros.to(DEV), g_idx.to(torch.int32).to(DEV))
+    differ = (a.qweight != b.qweight.cpu()).any(dim=0).nonzero().flatten().tolist()
+    assert not differ, f"columns {differ}"
+    assert torch.equal(a.qzeros, b.qzeros.cpu()) and torch.equal(a.scales, b.scales.cpu())
 
 
 def test_pack_in_one_native_call_keeps_what_the_python_route_has():
