@@ -87,6 +87,7 @@ struct StepParams {
     LinearShape lin[4];
     int slots;                             // of the ring
     int off_const, off_x, off_red;         // shared memory (from the aligned base)
+    int sums_bytes;                        // of one of the two places at off_red; a power of two
     int warp_bytes;                        // what a warp keeps of x
     int off_factors, off_planes;           // within them: factors and sums per unit; planes
     int off_natural;                       // x in natural order, behind the planes of the normalised linears
@@ -225,7 +226,7 @@ decode_layers_kernel(const StepParams p) {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kMoreRegs));
     const int H = p.hidden;
     const uint32_t tag0 = *p.tag + 1;                       // (not 0, which new memory holds)
-    int slot = 0, parity = 0;
+    int slot = 0, parity = 0, sums_at = 0;
     const long long p64 = p.pos[0];
     const bool in_range = p64 >= 0 && p64 < p.max_seq;      // (a position outside the caches: no attention, as in b200gptq_attn_step)
     const int P = in_range ? (int)p64 : 0;
@@ -244,7 +245,6 @@ decode_layers_kernel(const StepParams p) {
     // A linear: this CTA's strips (pairs of strips) one after the other.
     auto linear = [&](const StepPointers& layer, int ph, uint32_t tag, bool last) {
         const int g = lane >> 2, j = lane & 3;
-        float* red = reinterpret_cast<float*>(base + p.off_red);                // [strip of the item][warp][32]
         uint8_t* own = base + p.off_x + warp * p.warp_bytes;
         __half* own_x = reinterpret_cast<__half*>(own);                         // (of two units, as it lies in memory)
         float* own_f = reinterpret_cast<float*>(own + p.off_factors);
@@ -622,6 +622,7 @@ decode_layers_kernel(const StepParams p) {
                 }
                 if (residual) xr = p.x[n];
             }
+            float* red;                                          // [strip of the item][warp][32]
             {
                 // a pair of strips: both strips' slot i, with the same x; else two slots of the strip
                 float out[2][4] = {};
@@ -637,7 +638,10 @@ decode_layers_kernel(const StepParams p) {
                         if (second) pass_slot();
                     }
                 }
-                if (it > begin) consumers_meet();                // (the sums of the item before have been read)
+                // Two places for the sums, in turn over all items of this CTA whatever linear they belong to: the warp that reads them joins
+                // the next item's meeting after it has read, and no warp is past that meeting when it writes this place again.
+                red = reinterpret_cast<float*>(base + p.off_red + sums_at);
+                sums_at ^= p.sums_bytes;
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     if (!pair) out[0][c] += out[1][c];
@@ -988,8 +992,8 @@ bool plan_step(const b200gptq_step_shape& q, StepPlan* plan) {
     if (p.warp_bytes < p.off_planes + 2 * n_max * plane_bytes) p.warp_bytes = p.off_planes + 2 * n_max * plane_bytes;
     if (p.warp_bytes < hd * 4) p.warp_bytes = hd * 4;
     p.warp_bytes = (p.warp_bytes + 15) / 16 * 16;
-    const int red = (q.gated ? 2 : 1) * kLayerWarps * 32 * 4;
-    const int fixed = 1024 + kLayerWarps * p.warp_bytes + red, slot = slot_weights(q.bits) + slot_consts(q.bits);
+    p.sums_bytes = (q.gated ? 2 : 1) * kLayerWarps * 32 * 4;
+    const int fixed = 1024 + kLayerWarps * p.warp_bytes + 2 * p.sums_bytes, slot = slot_weights(q.bits) + slot_consts(q.bits);
     if (fixed > kLayersSmem) return false;
     int slots = (kLayersSmem - fixed) / slot;
     if (slots > kMaxSlots) slots = kMaxSlots;
