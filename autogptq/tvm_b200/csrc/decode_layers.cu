@@ -1088,7 +1088,8 @@ B200GPTQ_API int b200gptq_step_plan_create(const b200gptq_step_shape* shape, con
     p.cos_t = static_cast<const __half*>(shape->cos_t);
     p.sin_t = static_cast<const __half*>(shape->sin_t);
     p.pos = static_cast<const long long*>(shape->pos);
-    B200GPTQ_CUDA_TRY(cudaFuncSetAttribute(plan.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, plan.smem));
+    // (the limit is the kernel's, not this plan's: the same for all, or a plan of less would refuse the launches of one of more)
+    B200GPTQ_CUDA_TRY(cudaFuncSetAttribute(plan.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kLayersSmem));
     int resident = 0;
     B200GPTQ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, plan.kernel, kLayerThreads, plan.smem));
     if (resident < 1) return B200GPTQ_ERR_TOO_LARGE;

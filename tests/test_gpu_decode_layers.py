@@ -157,3 +157,13 @@ def test_a_position_outside_the_caches_writes_none():
             assert torch.equal(L.k_cache, k) and torch.equal(L.v_cache, v)
         assert bool(torch.isfinite(x).all())
     ops.check_status(DEV)
+
+
+def test_a_smaller_model_leaves_the_larger_one_running():
+    """The limit of dynamic shared memory belongs to the kernel, not to a plan: a plan that needs less, made later, must not lower it."""
+    large, text = _model("llama", 4, False, 1, 1024, 8, 2816, 12)
+    want, _ = _steps(large, text, 12, True)
+    small, other = _model("llama", 4, False, 1, 256, 2, 512, 12)
+    _steps(small, other, 12, True)
+    assert small._plan[1] is not None and large._plan[1] is not None
+    assert torch.equal(_steps(large, text, 12, True)[0], want)
