@@ -394,6 +394,8 @@ class GPTQDecoder:
                         or not (m.bias is None or plain(m.bias, N))):
                     return None                    # (the layer's own call says what is wrong with them)
                 linears.append((m._qweight_run, m.qzeros, m.scales, m.bias, m._x_perm))
+            if L.down._x_perm is not None:
+                return None                        # (the kernel reads the activation as it lies)
             cache = (1, cfg.heads, cfg.max_seq, cfg.head_dim)
             norms = (L.norm1_w, L.norm2_w) + (() if rms else (L.norm1_b, L.norm2_b))
             if not (all(plain(t, H) for t in norms) and plain(L.k_cache, *cache) and plain(L.v_cache, *cache)):

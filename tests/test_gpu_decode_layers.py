@@ -7,7 +7,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 if torch.cuda.is_available():
-    from autogptq.tvm_b200 import decoder, ops
+    from autogptq.tvm_b200 import decoder, ops, synth
     DEV = torch.device("cuda:0")
 
 
@@ -167,3 +167,14 @@ def test_a_smaller_model_leaves_the_larger_one_running():
     _steps(small, other, 12, True)
     assert small._plan[1] is not None and large._plan[1] is not None
     assert torch.equal(_steps(large, text, 12, True)[0], want)
+
+
+@pytest.mark.parametrize("arch,bits", [("llama", 4), ("opt", 3)])
+def test_a_second_ffn_linear_with_rows_of_its_own_order_goes_kernel_by_kernel(arch, bits):
+    m, text = _model(arch, bits, False, 2, 512, 4, 1024, 12)
+    L = m.layers[1]
+    L.down = decoder._to_module(synth.make_layer(bits, 1024, 512, 128, True, bias=arch == "opt", seed=5, device=DEV), DEV)
+    assert L.down._x_perm is not None
+    want, _ = _steps(m, text, 12, False)
+    got, _ = _steps(m, text, 12, True)
+    assert torch.equal(got, want) and m._step_plan() is None
