@@ -149,7 +149,8 @@ class GPTQDecoder:
         (bit-identical).  Measured for Llama-7B: slower on one GPU (367 against 383-390 tok/s: every CTA then computes
         the activation of its K slice between the dependency wait and its first product), faster from two GPUs on,
         where the slices are short and a launch is a larger share of the step (536 against 508 tok/s at TP 2).
-        ``None`` picks accordingly."""
+        ``None`` picks accordingly, and leaves the step of one sequence to the one launch for all layers where that takes
+        the model (:meth:`_step_plan`); with ``True`` or ``False`` the kernels are launched one by one."""
         self.cfg, self.batch = cfg, batch
         self._fold_request = fold_activation
         self.fused = fused and cfg.head_dim in (64, 128)   # decode steps use the fused helper kernels
@@ -371,8 +372,9 @@ class GPTQDecoder:
         """The layers of a decode step as one launch, for one sequence on one GPU and layers that the kernel takes; None where the
         kernels of a layer are launched one by one.  Everything that the plan points to is looked at in every step that is not replayed."""
         cfg = self.cfg
-        if self.world > 1 or self.batch != 1 or not self.one_launch or _module._global_forward_hooks or _module._global_forward_pre_hooks:
-            return None
+        if (self.world > 1 or self.batch != 1 or not self.one_launch or self._fold_request is not None or self.fold_activation
+                or _module._global_forward_hooks or _module._global_forward_pre_hooks):
+            return None                            # (who says how the activation is launched gets it launched that way)
         key, layers = [], []
 
         def plain(t, *shape, dtype=torch.float16):

@@ -178,3 +178,13 @@ def test_a_second_ffn_linear_with_rows_of_its_own_order_goes_kernel_by_kernel(ar
     want, _ = _steps(m, text, 12, False)
     got, _ = _steps(m, text, 12, True)
     assert torch.equal(got, want) and m._step_plan() is None
+
+
+def test_the_folded_activation_that_was_asked_for_is_used():
+    m, text = _model("llama", 4, False, 2, 256, 2, 512, 12)
+    want, _ = _steps(m, text, 12, False)
+    m.fold_activation = True
+    down, calls = m.layers[1].down, []
+    down.forward_act = lambda *a: (calls.append(1), type(down).forward_act(down, *a))[1]
+    assert torch.equal(_steps(m, text, 12, True)[0], want), "bit-identical to the separate kernel"
+    assert len(calls) == 4
