@@ -375,12 +375,15 @@ class GPTQDecoder:
         if (self.world > 1 or self.batch != 1 or not self.one_launch or self._fold_request is not None or self.fold_activation
                 or _module._global_forward_hooks or _module._global_forward_pre_hooks):
             return None                            # (who says how the activation is launched gets it launched that way)
+        H, rms = cfg.hidden, cfg.arch == "llama"
+        # (before the tensors are looked at: 8 layers of 8 bits took 670 us a step for 508)
+        if not ops.StepPlan.takes(len(self.layers), H, cfg.heads, cfg.inter, cfg.max_seq, cfg.bits, cfg.group_size, rms):
+            return None
         key, layers = [], []
 
         def plain(t, *shape, dtype=torch.float16):
             return t is not None and t.dtype is dtype and t.shape == shape and t.is_contiguous() and t.device == self.pos.device
 
-        H, rms = cfg.hidden, cfg.arch == "llama"
         sizes = ((H, 3 * H), (H, H), (H, (2 if rms else 1) * cfg.inter), (cfg.inter, H))
         for L in self.layers:
             linears = []

@@ -476,14 +476,24 @@ class StepPlan:
     def __init__(self, handle, memory, keep):
         self._handle, self._memory, self._keep = handle, memory, keep
 
+    @staticmethod
+    def _shape(layers: int, hidden: int, heads: int, inter: int, max_seq: int, bits: int, group_size: int, llama: bool):
+        return _lib.StepShape(layers, 1, hidden, heads, inter, max_seq, bits, group_size, int(llama), int(llama), int(llama))
+
+    @classmethod
+    def takes(cls, *sizes) -> bool:
+        """Whether there is a plan for ``layers, hidden, heads, inter, max_seq, bits, group_size, llama``, whatever the tensors.  Host-only."""
+        import ctypes
+        return _lib.lib.b200gptq_step_plan_bytes(ctypes.byref(cls._shape(*sizes))) > 0
+
     @classmethod
     def make(cls, layers, hidden: int, heads: int, inter: int, bits: int, group_size: int, llama: bool, eps: float, cos, sin, pos):
         """``layers``: per layer ``(linears, norm_w, norm_b, k_cache, v_cache)``, four linears ``(qweight, qzeros, scales, bias, x_perm)`` in their
         run-time layout.  None for shapes that the kernel does not take."""
         import ctypes
-        device, max_seq, hd = pos.device, layers[0][3].shape[2], hidden // heads
-        shape = _lib.StepShape(len(layers), 1, hidden, heads, inter, max_seq, bits, group_size, int(llama), int(llama), int(llama), eps,
-                               1.0 / (hd ** 0.5), _ptr(cos), _ptr(sin), _ptr(pos))
+        device, hd = pos.device, hidden // heads
+        shape = cls._shape(len(layers), hidden, heads, inter, layers[0][3].shape[2], bits, group_size, llama)
+        shape.eps, shape.scale, shape.cos_t, shape.sin_t, shape.pos = eps, 1.0 / (hd ** 0.5), _ptr(cos), _ptr(sin), _ptr(pos)
         need = _lib.lib.b200gptq_step_plan_bytes(ctypes.byref(shape))
         if need == 0:
             return None

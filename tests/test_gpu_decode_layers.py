@@ -188,3 +188,14 @@ def test_the_folded_activation_that_was_asked_for_is_used():
     down.forward_act = lambda *a: (calls.append(1), type(down).forward_act(down, *a))[1]
     assert torch.equal(_steps(m, text, 12, True)[0], want), "bit-identical to the separate kernel"
     assert len(calls) == 4
+
+
+@pytest.mark.parametrize("bits,group", [(8, 128), (4, 64)])
+def test_tensors_of_a_shape_that_the_kernel_does_not_take_are_not_looked_at(bits, group):
+    """(that costs the host of a step without a graph as much as three launches per layer)"""
+    m, text = _model("llama", bits, False, 2, 256, 2, 512, 12, group)
+    m.prefill(text[:, :12].contiguous())
+    calls = []
+    for L in m.layers:
+        L.qkv._ready = lambda: (calls.append(1), True)[1]
+    assert m._step_plan() is None and not calls
