@@ -6,7 +6,8 @@
 //
 //  * A producer warp streams this CTA's weights of ALL linears of ALL layers, in the order they will be needed, through one
 //    ring of tensor boxes.  It depends on nothing but free slots, so the ring (170 KB per SM, 25 MB: the projection q|k|v of Llama-7B)
-//    fills while the CTAs exchange x, normalise, attend and add up.  Tensor maps of the next linear are prefetched.  A slot is one strip of
+//    fills while the CTAs exchange x, normalise, attend and add up.  Tensor maps of the next linear are prefetched; a warp
+//    of its own acquires them, layers ahead.  A slot is one strip of
 //    32 columns times 16 units of 128 rows with the units' scales and zero-points: one box each, one barrier for the CTA (a ring per warp,
 //    as in gemv_strip.cuh, needs 16 times the boxes).
 //  * Eight warps multiply, two units of every slot each, as gemv_strip.cuh's byte planes do (x in fixed point per unit, exact integer
@@ -123,6 +124,11 @@ __device__ __forceinline__ void consumers_meet() { asm volatile("bar.sync 1, %0;
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+// The maps lie in the plan's memory, where other maps may have lain before: what wrote them has to be made visible to the copies, once per map, launch
+// and CTA.
+__device__ __forceinline__ void acquire_map(const CUtensorMap* m) {
+    asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(m) : "memory");
+}
 __device__ __forceinline__ void prefetch_map(const CUtensorMap* m) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(m) : "memory");
 }
@@ -146,7 +152,7 @@ decode_layers_kernel(const StepParams p) {
     __shared__ __align__(8) uint64_t bars[2 * kMaxSlots];
     __shared__ __align__(16) float2 sm_sums[kLayerWarps];  // of x and x^2, per warp
     __shared__ __align__(16) StepPointers sm_layers[4];    // of the layers around the current one
-    __shared__ int sm_items[4][2];
+    __shared__ int sm_items[4][2], sm_maps;
     __shared__ __align__(16) __half q_sm[HD], knew_sm[HD], vnew_sm[HD];
     __shared__ float sm_m[kLayerWarps], sm_l[kLayerWarps];
 
@@ -156,6 +162,7 @@ decode_layers_kernel(const StepParams p) {
     const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8u * kMaxSlots;
     bool ok = true;
     if (tid == 0) {
+        sm_maps = 0;
         for (int s = 0; s < p.slots; ++s) {
             mbar_init(full0 + 8u * s, 1);
             mbar_init(empty0 + 8u * s, kLayerWarps);
@@ -172,14 +179,34 @@ decode_layers_kernel(const StepParams p) {
     if (warp >= kLayerWarps) {
         // ---- the producer ----
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kFewRegs));
-        if (warp == kLayerWarps && elect_one()) {
-            int slot = 0, parity = 1, issued = 0;          // (parity 1: the first round of slots is free)
-            for (int i = 0; i < 3; ++i) prefetch_map(&p.layers[0].w[0] + 4 * i);
+        if (warp == kLayerWarps + 1) {
+            // The maps of a layer, a lane each; how many layers of them, for the producer, which is a layer behind at least after the first.  (Acquired by
+            // the producer itself, whose copies in flight each fence waits for, a layer took 4 us longer.)
 #pragma unroll 1
             for (int l = 0; l < p.n_layers; ++l) {
+                if (lane < 12) acquire_map(&p.layers[l].w[0] + lane);
+                __syncwarp();
+                if (lane == 0) asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(smem_u32(&sm_maps)), "r"(l + 1) : "memory");
+            }
+        }
+        if (warp == kLayerWarps && elect_one()) {
+            int have = 0;
+            auto wait_for_maps = [&](int layers) {
+                const long long t0 = clock64();
+                while (have < layers && ok) {
+                    asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(have) : "r"(smem_u32(&sm_maps)) : "memory");
+                    if (clock64() - t0 > kWaitClocks) ok = false;
+                }
+            };
+            int slot = 0, parity = 1, issued = 0;          // (parity 1: the first round of slots is free)
+            wait_for_maps(1);
+            for (int i = 0; i < 3; ++i) prefetch_map(&p.layers[0].w[0] + 4 * i);
+#pragma unroll 1
+            for (int l = 0; l < p.n_layers && ok; ++l) {        // (none through a map that has not been acquired)
                 const StepLayer& layer = p.layers[l];
 #pragma unroll 1
                 for (int ph = 0; ph < 4; ++ph) {
+                    if (ph == 3) wait_for_maps(min(l + 2, p.n_layers));
                     const StepLayer& next = ph < 3 ? layer : p.layers[min(l + 1, p.n_layers - 1)];
                     for (int i = 0; i < 3; ++i) prefetch_map(&next.w[(ph + 1) & 3] + 4 * i);
                     const LinearShape& s = p.lin[ph];

@@ -199,3 +199,20 @@ def test_tensors_of_a_shape_that_the_kernel_does_not_take_are_not_looked_at(bits
     for L in m.layers:
         L.qkv._ready = lambda: (calls.append(1), True)[1]
     assert m._step_plan() is None and not calls
+
+
+def test_maps_of_a_plan_whose_memory_is_used_again():
+    """Every replaced tensor makes a plan, in memory that a plan of other tensor maps has left: the copies must not see those."""
+    m, text = _model("llama", 4, False, 2, 512, 4, 1024, 20)
+    _steps(m, text, 20, True)
+    at, pieces = [], []
+    for i in range(6):
+        L = m.layers[i % 2]
+        pieces.append(torch.empty(4096 * (i + 1), dtype=torch.uint8, device=DEV))     # (other addresses for what is replaced)
+        L.up.qweight = L.up.qweight.roll(32 * (i + 1), dims=1)
+        L.down.scales, L.o.qzeros = L.down.scales.flip(1).contiguous(), L.o.qzeros.roll(4, dims=1)
+        want, _ = _steps(m, text, 20, False)
+        got, _ = _steps(m, text, 20, True)
+        _close(got, want, 2)
+        at.append(m._plan[1]._memory.data_ptr())
+    assert len(set(at)) < len(at), "no plan's memory was used again"
