@@ -467,6 +467,8 @@ class GPTQDecoder:
         """Warm up (allocates scratch, builds run-time views) and capture one decode step in a CUDA graph."""
         check_positions(self._pos_host, 3, self.cfg.max_seq)   # two warm-up steps and the captured one
         saved_pos, saved_tok = self.pos.clone(), self.tokens.clone()
+        if self.fused:
+            self._step_plan()                      # its memory is the caller's stream's, where the graph is replayed, not the warm-up's
         s = torch.cuda.Stream(self.device)
         s.wait_stream(torch.cuda.current_stream(self.device))
         with torch.cuda.stream(s):

@@ -216,3 +216,13 @@ def test_maps_of_a_plan_whose_memory_is_used_again():
         _close(got, want, 2)
         at.append(m._plan[1]._memory.data_ptr())
     assert len(set(at)) < len(at), "no plan's memory was used again"
+
+
+def test_the_captured_plan_has_memory_of_the_stream_that_replays_it():
+    """Not of the warm-up's: freed with the model, that could be handed out on another stream while a replay still writes it."""
+    m, text = _model("llama", 4, False, 2, 512, 4, 1024, 20)
+    m.prefill(text[:, :20].contiguous())
+    m.capture()
+    at = m._graph_plan[1]._memory.data_ptr()
+    streams = [s["stream"] for s in torch.cuda.memory_snapshot() if s["address"] <= at < s["address"] + s["total_size"]]
+    assert streams == [torch.cuda.current_stream().cuda_stream]
