@@ -13,7 +13,7 @@
 //  * Eight warps multiply, two units of every slot each, as gemv_strip.cuh's byte planes do (x in fixed point per unit, exact integer
 //    products, scaled in fp32), and are added up through shared memory.  Two slots at a time: one alone is a chain of latencies.
 //  * What lies between the linears is done where the values are: residual sums and the activation by the warp that adds up a
-//    strip; the norm, the act-order gather and the planes by every CTA as it reads x; attention by up to four CTAs per head.
+//    strip; the norm, the act-order gather and the planes by every CTA as it reads x; attention by up to sixteen CTAs per head.
 //  * Values travel between CTAs as words that carry the number of their phase (put_word), so there is no barrier of the grid and
 //    no fence: a layer is five such exchanges.  All CTAs are resident (cooperative launch); every wait is bounded, and one
 //    that expires raises the sticky status word and ends the launch with undefined results.
@@ -41,7 +41,7 @@ static_assert(kLayerWarps * 32 * kMoreRegs + 128 * kFewRegs <= kLayerThreads * k
 constexpr int kSlotUnits = 2 * kLayerWarps;         // units of 128 rows in a slot: two per warp
 constexpr int kPasses = 3;                          // slots whose x is fetched at once; of a normalised x, all
 constexpr int kMaxSlots = 8;
-constexpr int kMaxSplit = 4;                        // CTAs that share a head
+constexpr int kMaxSplit = 16, kPartsAtOnce = 3;     // CTAs that share a head; parts of it that are fetched at once
 enum { kQkv = 0, kOut = 1, kUp = 2, kDown = 3 };
 
 // Bytes of a slot's weights and constants.  Zero-points: rows of 4 bits are one 16-byte piece per strip; 3 (2) bits are three (two)
@@ -257,8 +257,10 @@ decode_layers_kernel(const StepParams p) {
     const long long p64 = p.pos[0];
     const bool in_range = p64 >= 0 && p64 < p.max_seq;      // (a position outside the caches: no attention, as in b200gptq_attn_step)
     const int P = in_range ? (int)p64 : 0;
-    // CTAs that share a head: a part of fewer than 192 positions is not worth the meeting afterwards
-    const int n_split = max(1, min(min(ctas / p.heads, kMaxSplit), (P + 191) / 192));
+    // CTAs that share a head: as many as have a block of positions for each of their warps (a part per 192 positions, of four at most, made
+    // steps at 300 positions 4 to 6 % and at 16 000 positions of 8 heads 70 % longer)
+    constexpr int kRoundRows = kLayerWarps * 8 * (32 / (HD / 8));
+    const int n_split = max(1, min(min(ctas / p.heads, kMaxSplit), (P + kRoundRows - 1) / kRoundRows));
 
     // A wait for words: until every lane of the warp has seen its tag, or time is up.
     long long t0 = 0;
@@ -710,7 +712,9 @@ decode_layers_kernel(const StepParams p) {
     };
 
     // Single-query attention over positions 0 .. P: b200gptq_attn_step's arithmetic.  `split` CTAs share a head, their
-    // warps take blocks of kRows positions in turn; the first of them adds the parts up.
+    // warps take blocks of kRows positions in turn; the first of them adds the parts up.  us per layer, kernel by kernel / here: 32 heads of 128 (Llama-7B)
+    // 1000 positions 46.8 / 45.0, 4000 53.7 / 54.5, 16 000 81 / 92 (the cache that the shared memory leaves is too small for more loads in flight);
+    // 8 heads (hidden 1024) 1000 positions 23.9 / 20.0, 16 000 49.2 / 32.1.
     auto attention = [&](const StepPointers& layer, uint32_t tag) {
         constexpr int LP = HD / 8, GROUPS = 32 / LP, U = 8, kRows = U * GROUPS;    // lanes per position; positions per block
         constexpr int kWriters = HD / 32;                                          // warps that write, a lane per dim
@@ -726,16 +730,16 @@ decode_layers_kernel(const StepParams p) {
             const int head = item / split, sp = item - head * split;
             const size_t cache = (size_t)head * p.max_seq * HD;
             uint4 kv[U], vv[U];
-            auto request = [&](int t0) {
+            auto request = [&](const __half* from, int t0, uint4 (&to)[U]) {
 #pragma unroll
                 for (int i = 0; i < U; ++i) {
                     const int t = min(t0 + i * GROUPS + grp, p.max_seq - 1);
-                    kv[i] = *reinterpret_cast<const uint4*>(layer.k_cache + cache + (size_t)t * HD + dim);
-                    vv[i] = *reinterpret_cast<const uint4*>(layer.v_cache + cache + (size_t)t * HD + dim);
+                    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(to[i].x), "=r"(to[i].y), "=r"(to[i].z), "=r"(to[i].w)
+                                 : "l"(from + cache + (size_t)t * HD + dim));
                 }
             };
             int t_at = (warp * split + sp) * kRows;
-            if (t_at < P) request(t_at);
+            if (t_at < P) { request(layer.k_cache, t_at, kv); request(layer.v_cache, t_at, vv); }
             __half cs = __ushort_as_half(0), sn = cs;
             if (p.rope && d < HD / 2) { cs = p.cos_t[(size_t)P * (HD / 2) + d]; sn = p.sin_t[(size_t)P * (HD / 2) + d]; }
             if (warp < kWriters) {
@@ -815,6 +819,9 @@ decode_layers_kernel(const StepParams p) {
                     sc[i] = dot8(kv[i]);
                     if (t + i * GROUPS < P) m_new = fmaxf(m_new, sc[i]);
                 }
+                // (the next block's keys are on their way while the values are worked on, its values while the keys are)
+                t_at += stride;
+                if (t_at < P) request(layer.k_cache, t_at, kv);
                 const float corr = __expf(mx - m_new);
                 l *= corr;
 #pragma unroll
@@ -827,8 +834,7 @@ decode_layers_kernel(const StepParams p) {
                         add8(vv[i], w);
                     }
                 mx = m_new;
-                t_at += stride;
-                if (t_at < P) request(t_at);
+                if (t_at < P) request(layer.v_cache, t_at, vv);
             }
             if (sp == 0 && warp == kLayerWarps - 1) {
                 // the new position: one more step of the online softmax for the first group
@@ -880,37 +886,41 @@ decode_layers_kernel(const StepParams p) {
                     if (lane < 2) put_float(ml + 2 * sp + lane, lane ? cl : cm, tag);
                 } else {
                     if (split > 1) {
-                        unsigned long long a[kMaxSplit - 1], mlw = 0;
+                        // maxima and sums of weights of all parts, a lane each; the first parts with them, more of them in turn
+                        unsigned long long mlw = 0, a[kPartsAtOnce];
                         const bool has = lane >= 2 && lane < 2 * split;
-                        bool missing;
-                        t0 = 0;
-                        do {
-                            missing = false;
-                            if (has) {
-                                mlw = get_float(ml + lane);
-                                missing = (uint32_t)(mlw >> 32) != tag;
+                        float mine = 0.f, tm = cm;
+#pragma unroll 1
+                        for (int r0 = 1; r0 < split; r0 += kPartsAtOnce) {
+                            bool missing;
+                            t0 = 0;
+                            do {
+                                missing = false;
+                                if (has && r0 == 1) mlw = get_float(ml + lane);
+#pragma unroll
+                                for (int r = 0; r < kPartsAtOnce; ++r)
+                                    if (r0 + r < split) a[r] = get_float(part + (r0 + r) * HD + d);
+                                missing = has && (uint32_t)(mlw >> 32) != tag;
+#pragma unroll
+                                for (int r = 0; r < kPartsAtOnce; ++r)
+                                    if (r0 + r < split) missing = missing || (uint32_t)(a[r] >> 32) != tag;
+                            } while (again(missing));
+                            if (r0 == 1) {
+                                mine = __uint_as_float((uint32_t)mlw);
+                                if (has && !(lane & 1)) tm = fmaxf(cm, mine);
+#pragma unroll
+                                for (int o = 16; o > 0; o >>= 1) tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, o));
+                                const float e0 = __expf(cm - tm);
+                                cl *= e0; ca *= e0;
                             }
 #pragma unroll
-                            for (int r = 1; r < kMaxSplit; ++r)
-                                if (r < split) a[r - 1] = get_float(part + r * HD + d);
-#pragma unroll
-                            for (int r = 1; r < kMaxSplit; ++r)
-                                if (r < split) missing = missing || (uint32_t)(a[r - 1] >> 32) != tag;
-                        } while (again(missing));
-                        const float mine = __uint_as_float((uint32_t)mlw);
-                        float tm = cm;
-#pragma unroll
-                        for (int r = 1; r < kMaxSplit; ++r)
-                            if (r < split) tm = fmaxf(tm, __shfl_sync(0xffffffffu, mine, 2 * r));
-                        const float e0 = __expf(cm - tm);
-                        cl *= e0; ca *= e0;
-#pragma unroll
-                        for (int r = 1; r < kMaxSplit; ++r)
-                            if (r < split) {
-                                const float e = __expf(__shfl_sync(0xffffffffu, mine, 2 * r) - tm);
-                                cl += __shfl_sync(0xffffffffu, mine, 2 * r + 1) * e;
-                                ca += __uint_as_float((uint32_t)a[r - 1]) * e;
-                            }
+                            for (int r = 0; r < kPartsAtOnce; ++r)
+                                if (r0 + r < split) {
+                                    const float e = __expf(__shfl_sync(0xffffffffu, mine, 2 * (r0 + r)) - tm);
+                                    cl += __shfl_sync(0xffffffffu, mine, 2 * (r0 + r) + 1) * e;
+                                    ca += __uint_as_float((uint32_t)a[r]) * e;
+                                }
+                        }
                     }
                     put_word(p.att + head * HD + d, in_range ? __float2half_rn(ca / cl) : __low2half(zero2), tag);
                 }

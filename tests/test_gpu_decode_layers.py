@@ -50,6 +50,10 @@ def _close(got, want, layers):
     ("opt", 2, False, 1, 512, 4, 640, 5),
     ("llama", 4, False, 6, 2048, 16, 1024, 12),          # half the warps have no units of the second FFN linear and are ahead of the others
     ("opt", 3, True, 6, 1024, 8, 256, 40),
+    ("llama", 4, False, 1, 256, 2, 512, 2100),           # sixteen CTAs per head; a second block for some warps
+    ("llama", 4, False, 1, 1024, 8, 1152, 641),          # six, two batches of parts
+    ("opt", 3, False, 1, 512, 8, 1024, 1030),            # five of 64 dims, the last with a few positions; several blocks
+    ("llama", 2, False, 1, 4096, 32, 1024, 1500),        # four that go through several blocks
 ])
 def test_one_launch_computes_what_the_kernels_compute(shape):
     prompt, layers = shape[7], shape[3]
