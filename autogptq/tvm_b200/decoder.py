@@ -138,6 +138,18 @@ def _rmsnorm(x, w, eps=1e-6):
     return (xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + eps)).to(x.dtype) * w
 
 
+def one_launch_pays(bits: int, hidden: int, max_seq: int, sms: int) -> bool:
+    """Whether the decode step of one sequence is faster with its layers in one launch than kernel by kernel (a graph of the step, 180 models
+    of hidden 256 to 6144 with 2 to 4 bits, times as fast).  3 bits: 0.98 to 1.37.  2 and 4 bits, as long as the
+    linears that write ``hidden`` columns have a strip of 32 per SM at most: 0.98 to 1.4 up to 2000 positions; where they have more, 4864 and
+    up, a few SMs have two strips where the others have one, 0.91 to 1.07, mostly 0.93 to 0.99.  Hidden 3712 to 4224: the attention is the slower one
+    from 2500 positions on (4096, 4 bits: 200 positions 1.05, 2000 1.00, 4000 0.97, 16 000 0.88), so that a text of 4096 gains and longer ones lose.
+    Of other widths it is the faster one (4352, 16 000 positions 1.17; 3584 1.12)."""
+    if bits == 3:
+        return True
+    return hidden <= 32 * sms and (max_seq <= 4096 or not 3584 < hidden <= 4224)
+
+
 class GPTQDecoder:
     """Batch of sequences, one token per step after the prompt; greedy sampling."""
 
@@ -204,7 +216,7 @@ class GPTQDecoder:
         self.tokens = torch.zeros(batch, dtype=torch.long, device=dev)
         self.positions = torch.arange(cfg.max_seq, device=dev)
         self.graph: Optional[torch.cuda.CUDAGraph] = None
-        self.one_launch = True       # False: the kernels of a decode step's layers are launched one by one
+        self.one_launch: Optional[bool] = None   # a decode step's layers in one launch: where that pays, wherever it can be, never
         self._plan = None            # (what it was made from, ops.StepPlan or None)
         self._graph_plan = None      # the one whose memory the captured step uses
         self._pos_host = 0   # host copy of the position, for range checks
@@ -372,10 +384,12 @@ class GPTQDecoder:
         """The layers of a decode step as one launch, for one sequence on one GPU and layers that the kernel takes; None where the
         kernels of a layer are launched one by one.  Everything that the plan points to is looked at in every step that is not replayed."""
         cfg = self.cfg
-        if (self.world > 1 or self.batch != 1 or not self.one_launch or self._fold_request is not None or self.fold_activation
+        if (self.world > 1 or self.batch != 1 or self.one_launch is False or self._fold_request is not None or self.fold_activation
                 or _module._global_forward_hooks or _module._global_forward_pre_hooks):
             return None                            # (who says how the activation is launched gets it launched that way)
         H, rms = cfg.hidden, cfg.arch == "llama"
+        if self.one_launch is None and not one_launch_pays(cfg.bits, H, cfg.max_seq, torch.cuda.get_device_properties(self.device).multi_processor_count):
+            return None
         # (before the tensors are looked at: 8 layers of 8 bits took 670 us a step for 508)
         if not ops.StepPlan.takes(len(self.layers), H, cfg.heads, cfg.inter, cfg.max_seq, cfg.bits, cfg.group_size, rms):
             return None

@@ -22,3 +22,11 @@ def test_missing_tensors_are_refused():
     layers, table, plan = (_lib.StepLayer * 1)(), ctypes.create_string_buffer(_lib.lib.b200gptq_step_table_bytes(1)), ctypes.c_void_p()
     assert _lib.lib.b200gptq_step_plan_create(ctypes.byref(shape), layers, table, None) == -1
     assert _lib.lib.b200gptq_step_plan_run(None, None, None, None, None) == -1
+
+
+@pytest.mark.parametrize("bits,hidden,max_seq,pays", [
+    (4, 4096, 768, True), (4, 4096, 4096, True), (4, 4096, 4097, False), (2, 3712, 8192, False), (4, 3584, 8192, True), (4, 4352, 8192, True),
+    (4, 4736, 768, True), (4, 4864, 768, False), (2, 6144, 768, False), (3, 6144, 32768, True), (4, 256, 32768, True)])
+def test_where_one_launch_pays(bits, hidden, max_seq, pays):
+    from autogptq.tvm_b200.decoder import one_launch_pays
+    assert one_launch_pays(bits, hidden, max_seq, 148) == pays

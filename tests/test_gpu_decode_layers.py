@@ -230,3 +230,12 @@ def test_the_captured_plan_has_memory_of_the_stream_that_replays_it():
     at = m._graph_plan[1]._memory.data_ptr()
     streams = [s["stream"] for s in torch.cuda.memory_snapshot() if s["address"] <= at < s["address"] + s["total_size"]]
     assert streams == [torch.cuda.current_stream().cuda_stream]
+
+
+def test_a_model_that_is_faster_kernel_by_kernel_goes_that_way_unless_told():
+    m, text = _model("llama", 4, False, 1, 4864, 38, 512, 12)
+    assert m._step_plan() is None
+    m.one_launch = True
+    assert m._step_plan() is not None
+    m, text = _model("llama", 4, False, 1, 256, 2, 512, 12)
+    assert m._step_plan() is not None
