@@ -1,4 +1,5 @@
 // Host side of the decode GEMV (gemv_strip.cuh): plan, tensor map, launch.
+#include <mutex>
 #include <new>
 
 #include "gemv_strip.cuh"
@@ -47,6 +48,38 @@ const void* strip_kernel(int bits, int sub, int mode, int nt, int T, int warps, 
     return nullptr;
 }
 
+// Clusters of four (two) CTAs, one to an SM, that run at the same time: a cluster's SMs are neighbours, and what is left over of the
+// groups of them that a device has is lost (33 clusters of four on 148 SMs).  Looked up once per device.
+int clusters_at_once(int ctas) {
+    static std::once_flag once[64];
+    static int cached[64][2];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return sm_count() / ctas;
+    std::call_once(once[dev], [dev] {
+        for (int i = 0; i < 2; ++i) {
+            const void* kernel = strip_kernel(4, 1, kOne, 1, 1, 8, false, true);
+            cudaLaunchConfig_t cfg = {};
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = 2 << i;
+            attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+            cfg.gridDim = dim3(sm_count() / (2 << i) * (2 << i));
+            cfg.blockDim = dim3(32 * 8);
+            cfg.dynamicSmemBytes = kSmemMax;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            int n = 0;
+            if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax) != cudaSuccess ||
+                cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+                (void)cudaGetLastError();
+                n = sm_count() / (2 << i);
+            }
+            cached[dev][i] = n;
+        }
+    });
+    return cached[dev][ctas == 4];
+}
+
 }  // namespace
 
 // Groups of whole 32-row blocks, up to 16 rows of x.
@@ -75,16 +108,18 @@ int gemv_strip_prepare(GemvStripPlan* p, const int32_t* qweight, const int32_t* 
     s.per_cta = (s.strips + sm_count() - 1) / sm_count();
     // Fewer strips than half the SMs: clusters of two or four CTAs share one, where the units of K that a CTA is spared take longer than
     // the cluster's sum.  Hundredths of a us, from layers of 1024 to 2304 columns one behind the other, 1 to 16 rows of 1024 to 11008 values
-    // (600 of them): a unit takes 6 (one row) to 18, the cluster 150 and more with the number of strips, with a gather (every CTA copies x)
+    // (600 of them): a unit takes 6 (one row), 7 or 14 (more than eight), the cluster 150 and more with the number of strips, with a gather (every CTA copies x)
     // and 8 bits.  us, unsplit -> split: 4 bits, 11008 x 1024, one row 6.6 -> 4.4, 8 rows 9.4 -> 4.9, 16 rows 17.2 -> 6.4; 11008 x 2304, one row
     // 6.9 -> 6.4, 8 rows 9.9 -> 7.5, 16 rows 17.1 -> 10.4; 8192 x 1536, 3 bits act-order, 4 rows 8.0 -> 6.3.  Below the line 4096 x 1536, one
-    // row would be 3.1 -> 3.6 and 1024 x 1024 2.2 -> 2.8; rows in act-order gain less than they vary by from 57 strips on.
+    // row would be 3.1 -> 3.6 and 1024 x 1024 2.2 -> 2.8; rows in act-order gain less than they vary by from 57 strips on.  All clusters run at
+    // once: 34 to 37 strips by four CTAs each were two waves (8192 x 1120, one row 4.8 unsplit, 6.7 by four, 4.1 by two).
     s.split = 1;
     if (ctas_per_sm == 0 && !(permuted && M <= 8 && s.strips > 56))
         for (int split = 4; split > 1 && s.split == 1; split /= 2) {
             const int unit = M == 1 ? 6 : (M <= 8 ? 7 : 14), many = s.strips > 48 ? s.strips - 48 : 0;
             const int cluster = 150 + many + (gather ? 60 + 2 * many : 0) + (bits == 8 ? 60 : 0);
-            if (s.strips * split <= sm_count() && 10 * unit * (s.units - s.units / split) > 11 * cluster) s.split = split;
+            if (s.strips * split <= sm_count() && 10 * unit * (s.units - s.units / split) > 11 * cluster && s.strips <= clusters_at_once(split))
+                s.split = split;
         }
     s.cta_units = (s.units + s.split - 1) / s.split;
     // One and two rows: planes of x where they pay and fit; one row: x kept whole.  Planes take a CTA longer to prepare than x in operand

@@ -179,7 +179,7 @@ def test_folded_activation_equals_the_kernel_in_front(bits, K, gated, M):
 
 
 @pytest.mark.parametrize("bits,K,N,gs,gather,M", [
-    # four CTAs per strip (up to 37 strips): the shortest K of one row and of sixteen; units that do not divide; a cut last unit
+    # four CTAs per strip (up to 33 strips on 148 SMs): the shortest K of one row and of sixteen; units that do not divide; a cut last unit
     (4, 4864, 32, 128, False, 1), (4, 8032, 1184, 32, False, 2), (3, 8064, 1024, 128, True, 8), (2, 11008, 1024, 128, False, 16),
     (8, 10496, 1152, 128, False, 5), (4, 2176, 1024, 128, False, 16), (4, 2208, 992, 96, True, 9), (3, 10272, 64, -1, False, 3),
     # two CTAs (up to 74 strips); the largest and smallest number of them
@@ -205,6 +205,30 @@ def test_layers_of_few_strips_vs_oracle(bits, K, N, gs, gather, M):
     err = np.abs(y.cpu().numpy().astype(np.float64) - ref)
     bound = 2.0 ** -11 * np.abs(ref) + 2.0 ** -11 * np.linalg.norm(xg.numpy().astype(np.float64), axis=1)[:, None] * np.abs(W.astype(np.float64)).max()
     assert np.all(err <= bound), (err / bound).max()
+
+
+@pytest.mark.parametrize("K,M", [(4096, 8), (8192, 1), (11008, 16)])
+def test_clusters_that_share_a_strip_run_in_one_wave(K, M):
+    """34 to 37 strips by four CTAs each are no more CTAs than the GPU has SMs, but not all of their clusters run at once: two waves took 1.3 to
+    1.6 times what the next larger layers took, which two CTAs each share."""
+    def us(strips):
+        N = 32 * strips
+        d = [synth.make_layer(4, K, N, 128, False, seed=i, device=DEV) for i in range(4)]
+        plans = [ops.GemvPlan(l.qweight, l.qzeros, l.scales, None, None, None, M, 4, 128, None, 0) for l in d]
+        x = synth.make_x(M, K, device=DEV)
+        [p.run(x) for p in plans]
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            for i in range(40):
+                plans[i % 4].run(x)
+        times = []
+        for _ in range(20):
+            ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            ev[0].record(); graph.replay(); ev[1].record()
+            torch.cuda.synchronize()
+            times.append(ev[0].elapsed_time(ev[1]))
+        return min(times)
+    assert max(us(n) for n in (34, 35, 36, 37)) < 1.15 * us(38)
 
 
 @pytest.mark.parametrize("K,N,gs,gather", [
