@@ -73,7 +73,7 @@ int launch_pack(const int32_t* vals, int R, int C, int32_t* out, cudaStream_t st
 // writes its words, 128 bytes per warp and word-row.  (zero * scale, 1 / scale) of the 32 columns x all groups sit in
 // shared memory, column fastest, so that a look-up by any g_idx is one conflict-free 8-byte read; the rows are one entry
 // longer than the columns, so that the table is written without conflicts from coalesced reads of [N, G] too.  scales and
-// qzeros (and the copy of g_idx) are left to CTAs of their own.  4096 x 11008, 4 bits, groups of 128 in act-order: 35 us from fp16; in
+// qzeros are left to CTAs of their own.  4096 x 11008, 4 bits, groups of 128 in act-order: 35 us from fp16; in
 // order, where a row block is one group and needs no look-ups, 30 us.  fp16 weights of 2 to 4 bits have pack_pairs_kernel (26 and 25 us)
 // unless its table is too large; this kernel packs 8 bits, bf16 and fp32.
 //
@@ -138,13 +138,19 @@ __device__ __noinline__ void pack_divided(const T* row, const int* gr, const flo
     for (int i = 0; i < BITS; ++i) out[(size_t)i * N] = (int32_t)w[i];
 }
 
+// The group of row k (an index outside the groups is refused by the host when the layer is used).  The CTAs of the first strip, which read
+// every row's, leave the copy of g_idx.  (By the few CTAs that write the constants of a narrow layer it was a serial loop: 10720 x 320 7.9 us
+// instead of 5.8.)
+__device__ __forceinline__ int pack_group(const int32_t* __restrict__ g_idx, int k, int G, int32_t* __restrict__ g_idx_out) {
+    const int g = __ldg(g_idx + k);
+    if (g_idx_out && blockIdx.x == 0) g_idx_out[k] = g;
+    return min(max(g, 0), G - 1);
+}
+
 // scales_out and qzeros of one strip of 32 columns.  smem: 2 * 128 * kPackPitch floats
 template <int BITS, int THREADS>
 __device__ __forceinline__ void pack_constants(const float* __restrict__ scales, const float* __restrict__ zeros, int G, int N, int strip,
-                                               int32_t* __restrict__ qzeros, __half* __restrict__ scales_out, unsigned char* smem,
-                                               const int32_t* __restrict__ g_idx, int K, int32_t* __restrict__ g_idx_out) {
-    if (g_idx_out)                                                 // a copy, 32 of every 32 * strips by each strip
-        for (int k = strip * 32 + (threadIdx.x & 31); k < K && threadIdx.x < 32; k += 32 * gridDim.x) g_idx_out[k] = g_idx[k];
+                                               int32_t* __restrict__ qzeros, __half* __restrict__ scales_out, unsigned char* smem) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n0 = strip * kPackCols, n = n0 + lane;
     // scales and zero-points of the strip, 128 groups at a time: read along the groups, written along the columns
     constexpr int GT = 128;
@@ -205,13 +211,12 @@ pack_linear_kernel(const T* __restrict__ weight, const float* __restrict__ scale
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    // (an index outside the groups is refused by the host when the layer is used)
     auto group_of = [&](int c) {
         const int k = c * kPackChunk + threadIdx.x;
-        return k < K ? min(max(__ldg(g_idx + k), 0), G - 1) : 0;
+        return k < K ? pack_group(g_idx, k, G, g_idx_out) : 0;
     };
     if (blockIdx.y == gridDim.y - 1) {
-        pack_constants<BITS, kPackThreads>(scales, zeros, G, N, blockIdx.x, qzeros, scales_out, pack_smem, g_idx, K, g_idx_out);
+        pack_constants<BITS, kPackThreads>(scales, zeros, G, N, blockIdx.x, qzeros, scales_out, pack_smem);
         return;
     }
     fetch(c_begin, 0);
@@ -327,7 +332,7 @@ pack_pairs_kernel(const __half* __restrict__ weight, const float* __restrict__ s
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n0 = blockIdx.x * kPackCols;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (blockIdx.y == gridDim.y - 1) {
-        pack_constants<BITS, kPairThreads>(scales, zeros, G, N, blockIdx.x, qzeros, scales_out, pack_smem, g_idx, K, g_idx_out);
+        pack_constants<BITS, kPairThreads>(scales, zeros, G, N, blockIdx.x, qzeros, scales_out, pack_smem);
         return;
     }
     const int c_begin = blockIdx.y * chunks_per_cta, c_end = min((K + kPairChunk - 1) / kPairChunk, c_begin + chunks_per_cta);
@@ -347,9 +352,9 @@ pack_pairs_kernel(const __half* __restrict__ weight, const float* __restrict__ s
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    auto group_of = [&](int c, int i) {                            // (an index outside the groups is refused by the host when the layer is used)
+    auto group_of = [&](int c, int i) {
         const int k = c * kPairChunk + threadIdx.x + i * kPairThreads;
-        return k < K ? min(max(__ldg(g_idx + k), 0), G - 1) : 0;
+        return k < K ? pack_group(g_idx, k, G, g_idx_out) : 0;
     };
     fetch(c_begin, 0);
     if (c_begin + 1 < c_end) fetch(c_begin + 1, 1);

@@ -234,3 +234,28 @@ def test_pack_in_one_native_call_keeps_what_the_python_route_has():
     assert set(m.state_dict()) == {"qweight", "qzeros", "scales", "g_idx", "bias"}
     with pytest.raises(ValueError):
         m.pack(lin, scales[:, :2].contiguous(), zeros, g_idx)
+
+
+@pytest.mark.parametrize("K,N,gs,dtype", [(10720, 320, -1, torch.float16), (9984, 256, -1, torch.float32)])
+def test_the_copy_of_g_idx_costs_narrow_layers_little(K, N, gs, dtype):
+    """A narrow layer has few CTAs for its constants; the copy took them up to half as long as the whole launch."""
+    scales, zeros = torch.rand(N, 1, device=DEV) * 0.02 + 1e-3, torch.full((N, 1), 8.0, device=DEV)
+    lin = nn.Linear(K, N, bias=False, device=DEV, dtype=dtype)
+    lin.weight.data = (torch.randint(-8, 8, (N, K), device=DEV) * scales).to(dtype)
+    g_idx, m = torch.zeros(K, dtype=torch.int32, device=DEV), QuantLinear(4, gs, K, N, False).to(DEV)
+
+    def us(*given):
+        m.pack(lin, scales, zeros, *given)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            for _ in range(20):
+                m.pack(lin, scales, zeros, *given)
+        times = []
+        for _ in range(20):
+            ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            ev[0].record(), graph.replay(), ev[1].record()
+            torch.cuda.synchronize()
+            times.append(ev[0].elapsed_time(ev[1]))
+        return min(times)
+    assert us(g_idx) < 1.15 * us()
+    assert torch.equal(m.g_idx, g_idx)
