@@ -23,6 +23,18 @@ int sm_count() {
     return cached[dev];
 }
 
+EncodeTiledFn encode_tiled_fn() {
+    static const EncodeTiledFn fn = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            p = nullptr;
+        return reinterpret_cast<EncodeTiledFn>(p);
+    }();
+    return fn;
+}
+
 // implemented in the kernel translation units
 int dequant_dispatch(const int32_t*, const int32_t*, const __half*, const int32_t*, int, int, int, int, int8_t*,
                      __half*, cudaStream_t);

@@ -1,6 +1,7 @@
 // Shared device helpers: GPTQ field extraction and launch-side utilities.
 #pragma once
 
+#include <cuda.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -33,6 +34,12 @@ void set_last_cuda_error(int err);
     } while (0)
 
 int sm_count();  // multiprocessors of the current device (cached per device)
+
+// cuTensorMapEncodeTiled by way of the runtime (the library links against nothing else); null where there is no driver.
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiledFn encode_tiled_fn();
 
 // ---- field extraction ------------------------------------------------------------------
 // Field j (0..31) of one row block whose `BITS` words are w[0..BITS-1].  For 2/4/8 bits

@@ -51,12 +51,11 @@ constexpr int slot_zero_words(int bits) { return bits == 3 ? 8 : 4; }
 constexpr int slot_scales() { return kSlotUnits * 64; }
 constexpr int slot_consts(int bits) { return slot_scales() + kSlotUnits * slot_zero_words(bits) * 4; }
 
-struct StepPointers {
+struct alignas(128) StepPointers {
     const __half* bias[4];
     const int32_t* perm[3];         // rows of x that q|k|v, o and up read in order (null: as they lie)
     const __half *norm_w[2], *norm_b[2];
     __half *k_cache, *v_cache;
-    const void* unused[3];
 };
 static_assert(sizeof(StepPointers) == 128, "copied in 16-byte pieces");
 struct alignas(128) StepLayer {
@@ -366,7 +365,7 @@ decode_layers_kernel(const StepParams p) {
         // x of this warp's units, two units at a time (half a warp each, eight values per lane), ready to be multiplied.
         auto fetch_x = [&](const StepPointers& layer, int ph, uint32_t tag) {
             const LinearShape& s = p.lin[ph];
-            const int units = s.units, passes = s.slots, K = s.K;
+            const int units = s.units, passes = s.slots;
             const uint32_t* src = ph == kOut ? p.att : (ph == kDown ? p.act : p.xw);
             const bool normed = ph == kQkv || ph == kUp;
             const int which = ph == kQkv ? 0 : 1;
@@ -724,7 +723,6 @@ decode_layers_kernel(const StepParams p) {
         if (cta >= items) return;
         const int lane = d & 31, warp = d >> 5, grp = lane / LP, dim = (lane % LP) * 8, stride = kLayerWarps * split * kRows;
         float* own_acc = reinterpret_cast<float*>(base + p.off_x + warp * p.warp_bytes);                            // [HD] (x is not needed here)
-        const __half2 zero2 = __float2half2_rn(0.f);
 #pragma unroll 1
         for (int item = cta; item < items; item += ctas) {
             const int head = item / split, sp = item - head * split;
@@ -922,7 +920,7 @@ decode_layers_kernel(const StepParams p) {
                                 }
                         }
                     }
-                    put_word(p.att + head * HD + d, in_range ? __float2half_rn(ca / cl) : __low2half(zero2), tag);
+                    put_word(p.att + head * HD + d, in_range ? __float2half_rn(ca / cl) : __ushort_as_half(0), tag);
                 }
             }
             consumers_meet();                            // (the warps' sums have been read)
@@ -960,21 +958,6 @@ decode_layers_kernel(const StepParams p) {
     // all of them.)
     if (cta == ctas - 1 && tid == 0) *p.tag = tag0 + 2 * p.n_layers;
     if (!ok) atomicExch(p.status + kStatusWord, 1u);
-}
-
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn encode_tiled_fn() {
-    static const EncodeTiledFn fn = [] {
-        void* q = nullptr;
-        cudaDriverEntryPointQueryResult r;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &q, cudaEnableDefault, &r) != cudaSuccess ||
-            r != cudaDriverEntryPointSuccess)
-            q = nullptr;
-        return reinterpret_cast<EncodeTiledFn>(q);
-    }();
-    return fn;
 }
 
 const void* layers_kernel(int bits, int hd) {

@@ -23,21 +23,6 @@ namespace {
 constexpr int kSmemMax = 224 * 1024;      // dynamic shared memory of a CTA
 constexpr int kRawMax = 48 * 1024;        // largest x (all rows) that a CTA copies whole to gather from
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn encode_tiled_fn() {
-    static const EncodeTiledFn fn = [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            p = nullptr;
-        return reinterpret_cast<EncodeTiledFn>(p);
-    }();
-    return fn;
-}
-
 const void* strip_kernel(int bits, int sub, int mode, int nt, int T, int warps, bool apart, bool split) {
     switch (bits) {
         case 2: return gemv_strip_kernel_b2(sub, mode, nt, T, warps, apart, split);
@@ -112,7 +97,7 @@ int gemv_strip_prepare(GemvStripPlan* p, const int32_t* qweight, const int32_t* 
     // and 8 bits.  us, unsplit -> split: 4 bits, 11008 x 1024, one row 6.6 -> 4.4, 8 rows 9.4 -> 4.9, 16 rows 17.2 -> 6.4; 11008 x 2304, one row
     // 6.9 -> 6.4, 8 rows 9.9 -> 7.5, 16 rows 17.1 -> 10.4; 8192 x 1536, 3 bits act-order, 4 rows 8.0 -> 6.3.  Below the line 4096 x 1536, one
     // row would be 3.1 -> 3.6 and 1024 x 1024 2.2 -> 2.8; rows in act-order gain less than they vary by from 57 strips on.  All clusters run at
-    // once: 34 to 37 strips by four CTAs each were two waves (8192 x 1120, one row 4.8 unsplit, 6.7 by four, 4.1 by two).
+    // once: 34 to 37 strips by four CTAs each were two waves (8192 x 1120, one row 4.8 unsplit, 6.7 by four, 3.7 by two).
     s.split = 1;
     if (ctas_per_sm == 0 && !(permuted && M <= 8 && s.strips > 56))
         for (int split = 4; split > 1 && s.split == 1; split /= 2) {

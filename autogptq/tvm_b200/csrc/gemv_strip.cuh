@@ -283,7 +283,7 @@ template <int BITS, bool WHOLE> struct IntLayout;
 // 4 bits: a word-row is a step, nibbles 0 2 4 6 (q) and 1 3 5 7 (q << 4).  Whole units: its bytes are used as they are (low + 16 * high nibble) and
 // with the high nibble masked off; what the first product has too much of the low nibble is taken off the x of the second: (low + 16 high) X'
 // + low (16 X - X') = 16 (low X + high X').  One AND per word instead of two: one and two rows, groups of 128, 1.00 to 1.04 times as fast
-// (4096 x 4096 3.65 -> 3.57 us, 5120 x 10240 7.63 -> 7.38); with groups scaled apart in a unit 0.99 to 1.00, so these keep both.
+// (4096 x 4096 3.61 -> 3.57 us in each of eight processes, 5120 x 10240 7.63 -> 7.38); with groups scaled apart in a unit 0.99 to 1.00, so these keep both.
 template <bool WHOLE> struct IntLayout<4, WHOLE> {
     static constexpr int kSteps = 4, kPre = 4, kLoads = 4;
     __device__ static int load_row(int i, int j) { return WHOLE ? 2 * j + (i & 1) + 8 * (i >> 1) : 4 * i + j; }

@@ -239,3 +239,63 @@ def test_a_model_that_is_faster_kernel_by_kernel_goes_that_way_unless_told():
     assert m._step_plan() is not None
     m, text = _model("llama", 4, False, 1, 256, 2, 512, 12)
     assert m._step_plan() is not None
+
+
+def test_two_models_on_two_streams():
+    """Each launch holds the whole GPU, and is there as a whole or not at all: steps of two models that nothing orders wait for one another
+    and give what they give alone."""
+    models = [_model("llama", 4, False, 2, 512, 4, 1024, 20), _model("opt", 3, False, 3, 512, 8, 1024, 20)]
+    streams, want, got = [torch.cuda.Stream(DEV) for _ in models], [], []
+    for m, text in models:
+        want.append(_steps(m, text, 20, True, 1)[0][0])
+        m.prefill(text[:, :20].contiguous())
+        m.capture()
+        m.tokens.copy_(text[:, 20])
+    torch.cuda.synchronize()
+    for _ in range(20):
+        for (m, text), s in zip(models, streams):
+            with torch.cuda.stream(s):
+                m.tokens.copy_(text[:, 20])
+                m.pos.fill_(20)
+                m.graph.replay()
+                got.append(m.last_logits.double())
+    torch.cuda.synchronize()
+    ops.check_status(DEV)
+    for i, logits in enumerate(got):
+        assert torch.equal(logits, want[i % 2])
+
+
+@pytest.mark.parametrize("bits", [2, 3, 4])
+@pytest.mark.parametrize("big", [0, 512, 16384])
+def test_no_further_from_64_bits_than_the_kernels(bits, big):
+    """The second FFN linear of a step alone: the input is zero, the output projection's scales are zero, so that x becomes down(relu(bias of the
+    first)).  `big`: the largest value of every unit of 128 rows, which meets weights of zero, so that what x in fixed point takes from the
+    small ones' precision is seen: no more than the kernel by itself, which has fp16 products here, loses in fp32 sums (2 and 3 bits: far less)."""
+    H, inter = 1024, 4096
+    m, text = _model("opt", bits, False, 1, H, 8, inter, 4)
+    m.one_launch = True
+    L = m.layers[0]
+    gen = torch.Generator().manual_seed(bits + big)
+    act = torch.rand(inter, generator=gen) + 0.5
+    q = torch.randint(0, 2 ** bits, (inter, H), generator=gen)
+    zeros = torch.randint(1, 2 ** bits, (inter // 128, H), generator=gen)
+    if big:
+        at = torch.arange(inter // 128) * 128 + torch.randint(0, 128, (inter // 128,), generator=gen)
+        act[at] = float(big)
+        q[at] = zeros
+    act = act.half()
+    L.up.bias = act.to(DEV)
+    L.o.scales.zero_(), L.o.bias.zero_(), L.down.bias.zero_()
+    L.down.qweight = ops.pack_fields(q.to(torch.int32).to(DEV), bits)
+    L.down.qzeros = ops.pack_fields((zeros - 1).to(torch.int32).t().contiguous().to(DEV), bits).t().contiguous()
+    L.down.post_init()
+    W = (q - zeros.repeat_interleave(128, 0)).double() * L.down.scales.cpu().double().repeat_interleave(128, 0)
+    exact = act.double() @ W
+    m.pos.fill_(0)
+    x = torch.zeros(1, H, dtype=torch.float16, device=DEV)
+    assert m._step_plan().run(x)
+    one = (x.cpu().double()[0] - exact).norm() / exact.norm()
+    kernel = (L.down(act.to(DEV)[None]).cpu().double()[0] - exact).norm() / exact.norm()
+    ops.check_status(DEV)
+    # (both hold the result's rounding to fp16, 2.0e-4 of it, over 1024 columns: the same within a few per cent where that is all)
+    assert float(one) <= 1.1 * float(kernel), (float(one), float(kernel))
