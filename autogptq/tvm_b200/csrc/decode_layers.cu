@@ -1,6 +1,6 @@
 // The decoder layers of one decode step of one sequence in ONE launch.
 //
-// Launched one by one, a layer of such a step is eight kernels of 2.6 to 10 us (Llama-7B: 41 us a layer) whose weights need
+// Launched one by one, a layer of such a step is eight kernels of 2.6 to 10 us (Llama-7B: 40 us a layer) whose weights need
 // 16 us of HBM time: every launch waits for x, starts its weight rings, works through them and sums up, and while it does one of
 // these the others rest.  Here one CTA per SM stays for the whole step:
 //
@@ -18,12 +18,13 @@
 //    no fence: a layer is five such exchanges.  All CTAs are resident (cooperative launch); every wait is bounded, and one
 //    that expires raises the sticky status word and ends the launch with undefined results.
 //
-// us per layer with the kernels one by one -> here, 4 bits unless said (a graph of the whole step, the vocabulary projection in it): Llama-7B,
-// 512 positions 44.0 -> 40.0; hidden 1024, inter 2816, 100 positions 21.4 -> 16.4; hidden 2048, inter 5504, 200 positions 28.4 -> 26.2;
-// hidden 4096, 200 positions, 3 bits 52.9 -> 48.4, act-order 48.3 -> 44.4; OPT, hidden 2048, 3 bits act-order 34.1 -> 32.4.  The weights
-// alone stream in 18.4 of the 36.7 that a Llama-7B layer takes without its share of the projection; the exchanges without the products
-// take 30: what bounds it is their latency, five times read, norm, planes, sum and write.  Several sequences are left to the kernels one by
-// one: in the fp16 form of the products a step of two took 58 us a layer for 52.
+// us per layer with the kernels one by one -> here (a graph of the step; what 12 more layers take, / 12, so without the projection
+// to the vocabulary), 4 bits unless said: Llama-7B, 512 positions 39.9 -> 35.2, 200 positions 38.6 -> 33.6, 3 bits 44.2 -> 40.1, act-order 41.7 -> 36.0;
+// hidden 1024, inter 2816, 100 positions 20.9 -> 15.0; hidden 2048, inter 5504, 200 positions 23.6 -> 20.6; OPT, hidden 2048, inter 8192, 300 positions
+// 23.9 -> 21.3, 3 bits act-order 27.8 -> 26.1 (16 layers of hidden 2048 and less lie in L2).  When a Llama-7B layer took 36.7, the weights
+// alone streamed in 18.4 and the exchanges without the products took 30: what bounds it is their latency, five times read, norm,
+// planes, sum and write.  Where the kernels one by one are faster: one_launch_pays (decoder.py).  Several sequences are left to these:
+// in the fp16 form of the products a step of two took 58 us a layer for 52.
 #include <cstring>
 #include <new>
 
@@ -712,8 +713,8 @@ decode_layers_kernel(const StepParams p) {
 
     // Single-query attention over positions 0 .. P: b200gptq_attn_step's arithmetic.  `split` CTAs share a head, their
     // warps take blocks of kRows positions in turn; the first of them adds the parts up.  us per layer, kernel by kernel / here: 32 heads of 128 (Llama-7B)
-    // 1000 positions 46.8 / 45.0, 4000 53.7 / 54.5, 16 000 81 / 92 (the cache that the shared memory leaves is too small for more loads in flight);
-    // 8 heads (hidden 1024) 1000 positions 23.9 / 20.0, 16 000 49.2 / 32.1.
+    // 1000 positions 40.4 / 36.9, 4000 47.1 / 46.4, 16 000 75 / 83 (the cache that the shared memory leaves is too small for more loads in flight);
+    // 8 heads (hidden 1024) 1000 positions 22.3 / 17.3, 16 000 46.5 / 29.0; 4 heads (hidden 512) 32 000 positions 56.6 / 39.9.
     auto attention = [&](const StepPointers& layer, uint32_t tag) {
         constexpr int LP = HD / 8, GROUPS = 32 / LP, U = 8, kRows = U * GROUPS;    // lanes per position; positions per block
         constexpr int kWriters = HD / 32;                                          // warps that write, a lane per dim

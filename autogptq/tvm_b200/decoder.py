@@ -431,7 +431,7 @@ class GPTQDecoder:
 
     def _decode_step_fused(self):
         """One token per sequence: all layers in one launch where :meth:`_step_plan` has one, else the fused helper kernels, per
-        layer 5 small launches + 4 linears."""
+        layer 4 small launches + 4 linears."""
         cfg, B = self.cfg, self.batch
         hd, rms = cfg.head_dim, cfg.arch == "llama"
         eps = 1e-6 if rms else 1e-5
