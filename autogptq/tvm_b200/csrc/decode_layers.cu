@@ -19,9 +19,9 @@
 //    that expires raises the sticky status word and ends the launch with undefined results.
 //
 // us per layer with the kernels one by one -> here (a graph of the step; what 12 more layers take, / 12, so without the projection
-// to the vocabulary), 4 bits unless said: Llama-7B, 512 positions 39.9 -> 35.2, 200 positions 38.6 -> 33.6, 3 bits 44.2 -> 40.1, act-order 41.7 -> 36.0;
-// hidden 1024, inter 2816, 100 positions 20.9 -> 15.0; hidden 2048, inter 5504, 200 positions 23.6 -> 20.6; OPT, hidden 2048, inter 8192, 300 positions
-// 23.9 -> 21.3, 3 bits act-order 27.8 -> 26.1 (16 layers of hidden 2048 and less lie in L2).  When a Llama-7B layer took 36.7, the weights
+// to the vocabulary), 4 bits unless said: Llama-7B, 512 positions 39.5 -> 35.4, 200 positions 38.5 -> 33.8, 3 bits 44.5 -> 39.9, act-order 41.3 -> 36.2;
+// hidden 1024, inter 2816, 100 positions 21.0 -> 15.3; hidden 2048, inter 5504, 200 positions 24.0 -> 20.5; OPT, hidden 2048, inter 8192, 300 positions
+// 23.8 -> 21.2, 3 bits act-order 27.8 -> 26.1 (16 layers of hidden 2048 and less lie in L2).  When a Llama-7B layer took 36.7, the weights
 // alone streamed in 18.4 and the exchanges without the products took 30: what bounds it is their latency, five times read, norm,
 // planes, sum and write.  Where the kernels one by one are faster: one_launch_pays (decoder.py).  Several sequences are left to these:
 // in the fp16 form of the products a step of two took 58 us a layer for 52.
@@ -213,12 +213,15 @@ decode_layers_kernel(const StepParams p) {
                     const int end = sm_items[ph][1], pair = s.pair, n = s.slots, per_group = s.per_group;
                     const unsigned int inv = s.per_group_inv;
 #pragma unroll 1
-                    for (int it = sm_items[ph][0]; it < end; ++it)
+                    for (int it = sm_items[ph][0]; it < end && ok; ++it)
 #pragma unroll 1
-                        for (int i = 0; i < n; ++i)
+                        for (int i = 0; i < n && ok; ++i)
 #pragma unroll 1
                             for (int strip = it; strip <= it + pair; strip += pair ? pair : 1) {
+                                // (nothing more after a wait that has expired, and a slot is freed by warps that have seen its copy land only: two copies
+                                // on one barrier, and the wait at the end would not be for all of them)
                                 wait_for(empty0 + 8u * slot, parity, ok);
+                                if (!ok) break;
                                 const uint32_t bar = full0 + 8u * slot, cst = smem_u32(base) + p.off_const + slot * kConsts;
                                 const int group = (int)(per_group == 1 ? i * kSlotUnits : __umulhi(i * kSlotUnits, inv));
                                 mbar_expect(bar, kWeights + kConsts);
@@ -536,14 +539,14 @@ decode_layers_kernel(const StepParams p) {
                 to.zeros[v] = load_zeros<BITS>(cst + kScales + r * kZeroPitch + 4 * ((strip * BITS) & 3), 4 * g);
             }
             __syncwarp();                          // every lane has its part
-            if (lane == 0) mbar_arrive(empty0 + 8u * slot);
+            if (lane == 0 && ok) mbar_arrive(empty0 + 8u * slot);
             if (++slot == p.slots) { slot = 0; parity ^= 1; }
         };
         // (a slot of units past the last)
         auto pass_slot = [&]() {
             wait_for(full0 + 8u * slot, parity, ok);
             __syncwarp();
-            if (lane == 0) mbar_arrive(empty0 + 8u * slot);
+            if (lane == 0 && ok) mbar_arrive(empty0 + 8u * slot);
             if (++slot == p.slots) { slot = 0; parity ^= 1; }
         };
         auto column = [&](const uint4& v, int c) { return c == 0 ? v.x : (c == 1 ? v.y : (c == 2 ? v.z : v.w)); };
